@@ -116,6 +116,23 @@ int tk3d_knn(const void *query, const void *key, int64_t B, int64_t N1, int64_t 
              int64_t *index, int dtype, void *stream);
 
 /*
+ * The same two searches with a scratch buffer for spatially ordered copies of the clouds, which large
+ * float32 searches walk instead of sweeping every pair (same results, bit for bit).
+ *   xyz_channel_first, index_dtype   as for the *_layout entry points
+ *   scratch          device buffer of at least tk3d_*_scratch_bytes() bytes, contents ignored on entry;
+ *                    NULL or a smaller buffer sweeps.  The size functions return 0 where ordering the
+ *                    clouds does not pay or is not supported.
+ */
+size_t tk3d_chamfer_fwd_scratch_bytes(int64_t B, int64_t N1, int64_t N2, int dtype);
+int tk3d_chamfer_fwd_ws(const void *xyz1, const void *xyz2, int64_t B, int64_t N1, int64_t N2, int xyz_channel_first,
+                        void *dist1, int64_t *idx1, void *dist2, int64_t *idx2, double *sums, void *scratch,
+                        size_t scratch_bytes, int dtype, void *stream);
+size_t tk3d_knn_scratch_bytes(int64_t B, int64_t N1, int64_t N2, int64_t k, int dtype);
+int tk3d_knn_ws(const void *query, const void *key, int64_t B, int64_t N1, int64_t N2, int64_t k,
+                int xyz_channel_first, void *distance, void *index, int index_dtype, void *scratch,
+                size_t scratch_bytes, int dtype, void *stream);
+
+/*
  * Farthest point sampling, first sample = point 0, lowest index among exact maxima.
  * Replaces sample_farthest_points_cuda (torkit3d/csrc/include/sample_farthest_points.h:6-8,
  * torkit3d/csrc/cuda/sample_farthest_points_kernel.cu:106-165).

@@ -375,7 +375,14 @@ def knn_distance_cuda(query, key, k, version=0, *, channel_first=False, index_dt
     with _on(query.device):
         distance = torch.empty((B, N1, k), dtype=query.dtype, device=query.device)
         index = torch.empty((B, N1, k), dtype=index_dtype, device=query.device)
-        if channel_first or index_dtype != torch.int64:
+        # large searches order the clouds first; 0 where sweeping all pairs is faster
+        need = _lib.scratch_bytes("tk3d_knn", B, N1, N2, k, _dtype(query))
+        if need:
+            scratch = torch.empty((need,), dtype=torch.uint8, device=query.device)
+            check(lib.tk3d_knn_ws(_ptr(query), _ptr(key), B, N1, N2, k, 1 if channel_first else 0, _ptr(distance),
+                                  _ptr(index), _index_code(index_dtype), _ptr(scratch), need, _dtype(query),
+                                  _stream(query)))
+        elif channel_first or index_dtype != torch.int64:
             check(lib.tk3d_knn_layout(_ptr(query), _ptr(key), B, N1, N2, k, 1 if channel_first else 0,
                                       _ptr(distance), _ptr(index), _index_code(index_dtype), _dtype(query),
                                       _stream(query)))
@@ -444,7 +451,14 @@ def chamfer_distance_forward_cuda(xyz1, xyz2, sums=None, *, channel_first=False)
         if sums is not None:
             if not (sums.is_cuda and sums.dtype == torch.float64 and sums.numel() == 2 and sums.is_contiguous()):
                 raise RuntimeError("sums must be a contiguous float64 CUDA tensor with 2 elements")
-        if channel_first:
+        need = _lib.scratch_bytes("tk3d_chamfer_fwd", B, N1, N2, _dtype(xyz1))
+        if need:  # large problems order the clouds first
+            scratch = torch.empty((need,), dtype=torch.uint8, device=dev)
+            check(lib.tk3d_chamfer_fwd_ws(_ptr(xyz1), _ptr(xyz2), B, N1, N2, 1 if channel_first else 0, _ptr(dist1),
+                                          _ptr(idx1), _ptr(dist2), _ptr(idx2),
+                                          _ptr(sums) if sums is not None else None, _ptr(scratch), need,
+                                          _dtype(xyz1), _stream(xyz1)))
+        elif channel_first:
             check(lib.tk3d_chamfer_fwd_layout(_ptr(xyz1), _ptr(xyz2), B, N1, N2, 1, _ptr(dist1), _ptr(idx1),
                                               _ptr(dist2), _ptr(idx2), _ptr(sums) if sums is not None else None,
                                               _dtype(xyz1), _stream(xyz1)))

@@ -27,6 +27,11 @@ SIGNATURES = {
     "tk3d_chamfer_bwd_mean": (_int, [_vp, ctypes.c_double, ctypes.c_double, _vp, _vp, _vp, _vp, _i64, _i64, _i64,
                                      _vp, _vp, _int, _vp]),
     "tk3d_knn": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp, _int, _vp]),
+    "tk3d_chamfer_fwd_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _int]),
+    "tk3d_chamfer_fwd_ws": (_int, [_vp, _vp, _i64, _i64, _i64, _int, _vp, _vp, _vp, _vp, _vp, _vp, ctypes.c_size_t,
+                                   _int, _vp]),
+    "tk3d_knn_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64, _int]),
+    "tk3d_knn_ws": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _int, _vp, _vp, _int, _vp, ctypes.c_size_t, _int, _vp]),
     "tk3d_fps_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _int]),
     "tk3d_fps": (_int, [_vp, _i64, _i64, _i64, _vp, _vp, ctypes.c_size_t, _int, _vp]),
     "tk3d_fps_static_scratch_capacity": (ctypes.c_size_t, []),

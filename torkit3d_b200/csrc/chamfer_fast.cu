@@ -15,6 +15,7 @@
 // wins ties.
 //
 // Both directions run in one launch; each block adds its partial sum of distances to `sums`.
+#include "spatial.cuh"
 #include "sweep.cuh"
 
 namespace tk3d {
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(CF_THREADS, MINB)
 chamfer_fwd_fast_kernel(const float *__restrict__ xyz1, const float *__restrict__ xyz2, int64_t B, int N1, int N2,
                         float *__restrict__ dist1, int64_t *__restrict__ idx1, float *__restrict__ dist2,
                         int64_t *__restrict__ idx2, double *__restrict__ sums, int64_t blocks1,
-                        int64_t blocks_total, XyzLayout l1, XyzLayout l2) {
+                        int64_t blocks_total, XyzLayout l1, XyzLayout l2, SpOnly only) {
   constexpr int PER = CF_TILE / CF_THREADS;
   constexpr int GK = 8 / Q;  // keys per filter group: eight (key, query) pairs share one branch
   __shared__ float4 tile[2][CF_TILE];
@@ -80,6 +81,7 @@ chamfer_fwd_fast_kernel(const float *__restrict__ xyz1, const float *__restrict_
   static_assert(CF_TILE % CF_THREADS == 0, "tile is staged in whole rounds of the block");
   const int tid = threadIdx.x;
   const float pinf = __int_as_float(0x7f800000);
+  if (only.idle(B)) return;
 
   for (int64_t blk = blockIdx.x; blk < blocks_total; blk += gridDim.x) {
     const int dir = blk >= blocks1;
@@ -93,6 +95,7 @@ chamfer_fwd_fast_kernel(const float *__restrict__ xyz1, const float *__restrict_
     constexpr int QPB = CF_THREADS * Q / LANES;    // queries per block
     const int chunks = (nq + QPB - 1) / QPB;
     const int64_t b = id / chunks;
+    if (only.skip(b)) continue;
     const int i0 = (int)(id % chunks) * QPB;
     const int part = (tid & 31) / QL;              // which of a query's LANES lanes this is
     auto qindex = [&](int s) {
@@ -247,17 +250,19 @@ chamfer_fwd_fast_kernel(const float *__restrict__ xyz1, const float *__restrict_
 
 template <int Q, int MINB = 1, int UNR = 2, int CF_THREADS = 128, int LANES = 1>
 int launch(const float *xyz1, const float *xyz2, int64_t B, int N1, int N2, float *dist1, int64_t *idx1,
-           float *dist2, int64_t *idx2, double *sums, cudaStream_t st, XyzLayout l1, XyzLayout l2, int only_dir = -1) {
+           float *dist2, int64_t *idx2, double *sums, cudaStream_t st, XyzLayout l1, XyzLayout l2, int only_dir = -1,
+           SpOnly only = {}) {
   // only_dir: -1 = both directions in this launch, 0 = cloud 1 -> cloud 2 only, 1 = the other one
   const int64_t per = CF_THREADS * Q / LANES;
   const int64_t blocks1 = only_dir == 1 ? 0 : B * ((N1 + per - 1) / per);
   const int64_t blocks2 = only_dir == 0 ? 0 : B * ((N2 + per - 1) / per);
   const int64_t total = blocks1 + blocks2;
   if (total == 0) return TK3D_OK;
-  const int64_t cap = (int64_t)sm_count() * 256;
+  // behind a search over ordered clouds there is usually nothing left to do: one round of blocks looks
+  const int64_t cap = (int64_t)sm_count() * (only.q ? 6 : 256);
   const unsigned grid = (unsigned)(total < cap ? total : cap);
   chamfer_fwd_fast_kernel<Q, MINB, UNR, CF_THREADS, LANES><<<grid, CF_THREADS, 0, st>>>(
-      xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, blocks1, total, l1, l2);
+      xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, blocks1, total, l1, l2, only);
   return check_launch("chamfer_fwd_fast_kernel");
 }
 
@@ -489,6 +494,29 @@ int chamfer_fwd_f32_fast(const float *xyz1, const float *xyz2, int64_t B, int64_
     case 1: return launch_smwide(xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2);
     default: return launch<2, 6, 4>(xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2);
   }
+}
+
+// Both directions over spatially ordered clouds; what the order cannot serve is swept.
+int chamfer_fwd_f32_ordered(const float *xyz1, const float *xyz2, int64_t B, int64_t N1, int64_t N2, int channel_first,
+                            float *dist1, int64_t *idx1, float *dist2, int64_t *idx2, double *sums, void *scratch,
+                            cudaStream_t st) {
+  const int64_t step = sp_batch(B, N1, N2);
+  char *at = sp_align_ptr(scratch);
+  for (int64_t b0 = 0; b0 < B; b0 += step) {
+    const int64_t n = b0 + step < B ? step : B - b0;
+    const float *p1 = xyz1 + b0 * 3 * N1, *p2 = xyz2 + b0 * 3 * N2;
+    const SpCloud c1 = sp_cloud(p1, channel_first, n, N1, at);
+    const SpCloud c2 = sp_cloud(p2, channel_first, n, N2, at + sp_cloud_bytes(n, N1));
+    float *d1 = dist1 + b0 * N1, *d2 = dist2 + b0 * N2;
+    int64_t *i1 = idx1 + b0 * N1, *i2 = idx2 + b0 * N2;
+    int rc = sp_build(c1, &c2, n, st);
+    if (!rc) rc = sp_chamfer(c1, c2, n, d1, i1, d2, i2, sums, st);
+    if (!rc)
+      rc = launch<2, 6, 4>(p1, p2, n, (int)N1, (int)N2, d1, i1, d2, i2, sums, st, c1.l, c2.l, -1,
+                           SpOnly{c1.grid, c2.grid});
+    if (rc) return rc;
+  }
+  return TK3D_OK;
 }
 
 }  // namespace tk3d

@@ -6,6 +6,7 @@
 // and weights once (the reference re-reads them for every channel) and walks the channels; lanes
 // of a warp hold consecutive m, so stores coalesce along N2.
 #include "rows.cuh"
+#include "spatial.cuh"
 
 namespace tk3d {
 
@@ -257,7 +258,9 @@ extern "C" int tk3d_three_nn_weight(const void *distance, int64_t rows, int64_t 
 namespace tk3d {
 
 int three_nn_fused_f32(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, int channel_first,
-                       float eps, float *weight, int32_t *index32, cudaStream_t st);
+                       float eps, float *weight, int32_t *index32, void *scratch, size_t scratch_bytes,
+                       cudaStream_t st);
+bool knn_order_pays(int64_t B, int64_t N1, int64_t N2, int64_t k);
 
 namespace {
 
@@ -294,7 +297,10 @@ bool fused_interp_shape_ok(int64_t B, int64_t C, int64_t Nq, int64_t Nk) {
 
 extern "C" size_t tk3d_three_nn_interp_scratch_bytes(int64_t B, int64_t C, int64_t Nq, int64_t Nk, int dtype) {
   if (dtype != TK3D_F32 || !fused_interp_shape_ok(B, C, Nq, Nk) || B * C == 0) return 0;
-  return rows_scratch_bytes(B, C, Nk);
+  // the search's index and the transposed features are not needed at the same time
+  const size_t rows = rows_scratch_bytes(B, C, Nk);
+  const size_t order = knn_order_pays(B, Nq, Nk, 3) ? sp_search_bytes(B, Nq, Nk) : 0;
+  return rows > order ? rows : order;
 }
 
 extern "C" int tk3d_three_nn_interp_fwd(const void *query_xyz, const void *key_xyz, const void *key_feature,
@@ -313,7 +319,7 @@ extern "C" int tk3d_three_nn_interp_fwd(const void *query_xyz, const void *key_x
                "three_nn_interp_fwd: a pointer is NULL");
   cudaStream_t st = (cudaStream_t)stream;
   int rc = three_nn_fused_f32((const float *)query_xyz, (const float *)key_xyz, B, Nq, Nk, xyz_channel_first, eps,
-                              (float *)weight, index32, st);
+                              (float *)weight, index32, scratch, scratch_bytes, st);
   if (rc || C == 0) return rc;
   const size_t want = rows_scratch_bytes(B, C, Nk);
   TK3D_REQUIRE(scratch != nullptr && scratch_bytes >= want, TK3D_ERR_SCRATCH,

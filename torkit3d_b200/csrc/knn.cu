@@ -21,6 +21,7 @@
 // strict comparisons, so the retained set and its order are reproducible bit for bit.
 #include <stdlib.h>
 
+#include "spatial.cuh"
 #include "sweep.cuh"
 
 namespace tk3d {
@@ -56,7 +57,8 @@ __device__ __forceinline__ float4 make_key(const float *__restrict__ rb, int j, 
 template <int K, int Q, int LANES = 1, bool FIRSTX = false>
 __global__ void __launch_bounds__(KN_THREADS)
 knn_small_kernel(const float *__restrict__ query, const float *__restrict__ key, int64_t B, int N1, int N2,
-                 float *__restrict__ dist, IndexOut index, int64_t blocks_total, XyzLayout ql, XyzLayout kl) {
+                 float *__restrict__ dist, IndexOut index, int64_t blocks_total, XyzLayout ql, XyzLayout kl,
+                 SpOnly only) {
   constexpr int TILE = 512, PER = TILE / KN_THREADS;
   constexpr int GK = 8 / Q;  // keys per filter group: eight (key, query) pairs share one branch
   __shared__ float4 tile[2][TILE];  // pair layout of sweep.cuh
@@ -66,9 +68,11 @@ knn_small_kernel(const float *__restrict__ query, const float *__restrict__ key,
   constexpr int QPB = KN_THREADS * Q / LANES;         // queries per block
   const int chunks = (N1 + QPB - 1) / QPB;
   const int half = (tid & 31) / QL;                   // which of a query's LANES lanes this is
+  if (only.idle(B)) return;
 
   for (int64_t blk = blockIdx.x; blk < blocks_total; blk += gridDim.x) {
     const int64_t b = blk / chunks;
+    if (only.skip(b)) continue;
     const int i0 = (int)(blk % chunks) * QPB;
     // query s of this thread
     auto qindex = [&](int s) {
@@ -1053,6 +1057,7 @@ knn_generic_kernel(const T *__restrict__ query, const T *__restrict__ key, int64
 struct KnnIo {
   IndexOut index;
   XyzLayout ql, kl;
+  SpOnly only = {};  // behind a search over ordered clouds: the clouds it could not serve
 };
 
 template <typename T>
@@ -1071,14 +1076,14 @@ int knn_small(const float *query, const float *key, int64_t B, int N1, int N2, f
               cudaStream_t st) {
   const int64_t per = KN_THREADS * Q / LANES;
   const int64_t total = B * ((N1 + per - 1) / per);
-  const int64_t cap = (int64_t)sm_count() * 256;
+  const int64_t cap = (int64_t)sm_count() * (io.only.q ? 6 : 256);  // usually nothing is left: one round of blocks looks
   const unsigned grid = (unsigned)(total < cap ? total : cap);
   if (LANES > 1 && N2 <= 16384)  // few key tiles: the first one is worth extra exchanges
     knn_small_kernel<K, Q, LANES, (LANES > 1)><<<grid, KN_THREADS, 0, st>>>(query, key, B, N1, N2, dist, io.index, total,
-                                                                            io.ql, io.kl);
+                                                                            io.ql, io.kl, io.only);
   else
     knn_small_kernel<K, Q, LANES><<<grid, KN_THREADS, 0, st>>>(query, key, B, N1, N2, dist, io.index, total, io.ql,
-                                                               io.kl);
+                                                               io.kl, io.only);
   return check_launch("knn_small_kernel");
 }
 
@@ -1156,6 +1161,51 @@ int knn_twopass(const float *query, const float *key, int64_t B, int N1, int N2,
 
 }  // namespace
 
+// Whether ordering the clouds first pays: it costs 25 to 90 us, as much as sweeping some 6e7 pairs
+// (k = 3, sweep / ordered, us: 4 x 2048^2 46 / 56, 16 x 4096 x 1024 101 / 91, 8 x 4096^2 121 / 80).
+bool knn_order_pays(int64_t B, int64_t N1, int64_t N2, int64_t k) {
+  return k <= 4 && sp_supported(B, N1, N2) && (double)B * N1 * N2 >= 6e7;
+}
+
+__global__ void three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t N1, int64_t rows, float eps,
+                                               SpOnly only);
+
+// k <= 4 over spatially ordered clouds; what the order cannot serve is swept.
+int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, int k, int channel_first,
+                bool weights, float eps, float *dist, void *index, int index32, void *scratch, cudaStream_t st) {
+  const int64_t step = sp_batch(B, N1, N2);
+  char *at = sp_align_ptr(scratch);
+  for (int64_t b0 = 0; b0 < B; b0 += step) {
+    const int64_t n = b0 + step < B ? step : B - b0;
+    const float *q = query + b0 * 3 * N1, *r = key + b0 * 3 * N2;
+    const bool same = q == r && N1 == N2;
+    const SpCloud cq = sp_cloud(q, channel_first, n, N1, at);
+    const SpCloud ck = same ? cq : sp_cloud(r, channel_first, n, N2, at + sp_cloud_bytes(n, N1));
+    float *d = dist + b0 * N1 * k;
+    KnnIo io;
+    io.index = index_out((char *)index + b0 * N1 * k * (index32 ? 4 : 8), index32, n * N1 * k);
+    io.ql = cq.l;
+    io.kl = ck.l;
+    io.only = SpOnly{cq.grid, ck.grid};
+    int rc = sp_build(cq, same ? nullptr : &ck, n, st);
+    if (!rc) rc = sp_knn_small(cq, ck, n, k, weights, eps, d, io.index, st);
+    if (rc) return rc;
+    switch (k) {
+      case 1: rc = knn_small<1, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      case 2: rc = knn_small<2, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      case 3: rc = knn_small<3, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      default: rc = knn_small<4, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+    }
+    if (rc) return rc;
+    if (weights) {
+      three_nn_weight_inplace_kernel<<<sm_count(), 256, 0, st>>>(d, N1, n * N1, eps, io.only);
+      rc = check_launch("three_nn_weight_inplace_kernel");
+      if (rc) return rc;
+    }
+  }
+  return TK3D_OK;
+}
+
 // Three nearest keys of every query with inverse-distance weights, the front end of feature
 // interpolation: w_i = (1/max(d_i, eps)) / sum_j (1/max(d_j, eps)) and 32-bit indices; N2 >= 3.
 // The sweep writes the squared distances into `weight` and a second, tiny kernel turns every row
@@ -1164,8 +1214,10 @@ int knn_twopass(const float *query, const float *key, int64_t B, int N1, int N2,
 // per SM, i.e. out of reach for the half-filled launches that need it (8 x 16384 x 32768 with the
 // gather that follows: 1.24 -> 1.11 ms; 8 x 65536 x 32768: 6.80 -> 6.77).
 __global__ void __launch_bounds__(256)
-three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t rows, float eps) {
+three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t N1, int64_t rows, float eps, SpOnly only) {
+  if (only.idle(rows / N1)) return;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
+    if (only.q && only.skip(r / N1)) continue;
     float *w = weight + r * 3;
     float inv[3], sum = 0.f;
 #pragma unroll
@@ -1179,8 +1231,11 @@ three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t rows, float e
 }
 
 int three_nn_fused_f32(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, int channel_first,
-                       float eps, float *weight, int32_t *index32, cudaStream_t st) {
+                       float eps, float *weight, int32_t *index32, void *scratch, size_t scratch_bytes,
+                       cudaStream_t st) {
   if (B * N1 == 0) return TK3D_OK;
+  if (scratch && knn_order_pays(B, N1, N2, 3) && scratch_bytes >= sp_search_bytes(B, N1, N2))
+    return knn_ordered(query, key, B, N1, N2, 3, channel_first, true, eps, weight, index32, 1, scratch, st);
   KnnIo io;
   io.index = index_out(index32, 1, B * N1 * 3);
   io.ql = xyz_layout(channel_first, N1);
@@ -1188,7 +1243,7 @@ int three_nn_fused_f32(const float *query, const float *key, int64_t B, int64_t 
   int rc = knn_small_q<3>(query, key, B, (int)N1, (int)N2, weight, io, st);
   if (rc) return rc;
   const int64_t rows = B * N1, blocks = (rows + 255) / 256, cap = (int64_t)sm_count() * 8;
-  three_nn_weight_inplace_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(weight, rows, eps);
+  three_nn_weight_inplace_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(weight, N1, rows, eps, SpOnly{});
   return check_launch("three_nn_weight_inplace_kernel");
 }
 
@@ -1206,7 +1261,8 @@ bool knn_split_f64(const double *query, const double *key, int64_t B, int64_t N1
 using namespace tk3d;
 
 static int knn_impl(const void *query, const void *key, int64_t B, int64_t N1, int64_t N2, int64_t k,
-                    int channel_first, void *distance, void *index, int index32, int dtype, void *stream) {
+                    int channel_first, void *distance, void *index, int index32, int dtype, void *stream,
+                    void *scratch = nullptr, size_t scratch_bytes = 0) {
   TK3D_REQUIRE(dtype == TK3D_F32 || dtype == TK3D_F64, TK3D_ERR_DTYPE, "knn: dtype %d", dtype);
   TK3D_REQUIRE(B >= 0 && N1 >= 0 && N2 >= 0, TK3D_ERR_SHAPE, "knn: negative size");
   TK3D_REQUIRE(k >= 1, TK3D_ERR_K, "knn: k must be >= 1 (got %lld)", (long long)k);
@@ -1228,6 +1284,8 @@ static int knn_impl(const void *query, const void *key, int64_t B, int64_t N1, i
   }
   const float *q = (const float *)query, *r = (const float *)key;
   float *d = (float *)distance;
+  if (scratch && k <= 4 && sp_supported(B, N1, N2) && scratch_bytes >= sp_search_bytes(B, N1, N2))
+    return knn_ordered(q, r, B, N1, N2, (int)k, channel_first, false, 0.f, d, index, index32, scratch, st);
   switch (k) {
     case 1: return knn_small_q<1>(q, r, B, (int)N1, (int)N2, d, io, st);
     case 2: return knn_small_q<2>(q, r, B, (int)N1, (int)N2, d, io, st);
@@ -1277,6 +1335,20 @@ extern "C" int tk3d_knn_layout(const void *query, const void *key, int64_t B, in
   TK3D_REQUIRE(index_dtype == TK3D_I64 || index_dtype == TK3D_I32, TK3D_ERR_DTYPE, "knn: index_dtype %d", index_dtype);
   return knn_impl(query, key, B, N1, N2, k, xyz_channel_first != 0, distance, index, index_dtype == TK3D_I32, dtype,
                   stream);
+}
+
+extern "C" size_t tk3d_knn_scratch_bytes(int64_t B, int64_t N1, int64_t N2, int64_t k, int dtype) {
+  if (dtype != TK3D_F32 || k < 1 || k > N2 || !knn_order_pays(B, N1, N2, k)) return 0;
+  return sp_search_bytes(B, N1, N2);
+}
+
+extern "C" int tk3d_knn_ws(const void *query, const void *key, int64_t B, int64_t N1, int64_t N2, int64_t k,
+                           int xyz_channel_first, void *distance, void *index, int index_dtype, void *scratch,
+                           size_t scratch_bytes, int dtype, void *stream) {
+  TK3D_RANGE("tk3d_knn_ws");
+  TK3D_REQUIRE(index_dtype == TK3D_I64 || index_dtype == TK3D_I32, TK3D_ERR_DTYPE, "knn: index_dtype %d", index_dtype);
+  return knn_impl(query, key, B, N1, N2, k, xyz_channel_first != 0, distance, index, index_dtype == TK3D_I32, dtype,
+                  stream, scratch, scratch_bytes);
 }
 
 TK3D_BOUNDS_TU(knn)
