@@ -312,9 +312,10 @@ extern "C" int tk3d_chamfer_fwd_layout(const void *xyz1, const void *xyz2, int64
 
 extern "C" size_t tk3d_chamfer_fwd_scratch_bytes(int64_t B, int64_t N1, int64_t N2, int dtype) {
   if (dtype != TK3D_F32 || !sp_supported(B, N1, N2) || !sp_supported(B, N2, N1)) return 0;
-  // Ordering both clouds costs 25 to 100 us, as much as sweeping about 1e8 pairs (sweep / ordered, us:
-  // 64 x 1024^2 71 / 91, 8 x 4096^2 105 / 93, 24 x 2500 x 4099 161 / 114, 1 x 16384^2 193 / 113).
-  if (N1 < 1024 || N2 < 1024 || (double)B * N1 * N2 < 1.2e8) return 0;
+  // Ordering both clouds and walking them takes 45 us at least, as much as sweeping some 5e7 pairs
+  // (sweep / ordered, us: 32 x 1024^2 45 / 52, 2 x 4096^2 56 / 60, 64 x 1024^2 71 / 66, 16 x 2048^2 67 / 58,
+  // 8 x 4096^2 105 / 70, 24 x 2500 x 4099 162 / 107, 64 x 16384^2 5815 / 345 to 805).
+  if (N1 < 1024 || N2 < 1024 || (double)B * N1 * N2 < 6e7) return 0;
   return sp_search_bytes(B, N1, N2);
 }
 

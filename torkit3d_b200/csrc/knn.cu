@@ -1161,10 +1161,10 @@ int knn_twopass(const float *query, const float *key, int64_t B, int N1, int N2,
 
 }  // namespace
 
-// Whether ordering the clouds first pays: it costs 25 to 90 us, as much as sweeping some 6e7 pairs
-// (k = 3, sweep / ordered, us: 4 x 2048^2 46 / 56, 16 x 4096 x 1024 101 / 91, 8 x 4096^2 121 / 80).
+// Whether ordering the clouds first pays (k = 3, sweep / ordered, us: 4 x 2048^2 46 / 54, 64 x 1024 x 512
+// 54 / 56, 16 x 4096 x 1024 101 / 56, 8 x 4096^2 121 / 62, 8 x 131072 x 32768 6714 / 351 to 893).
 bool knn_order_pays(int64_t B, int64_t N1, int64_t N2, int64_t k) {
-  return k <= 4 && sp_supported(B, N1, N2) && (double)B * N1 * N2 >= 6e7;
+  return k <= 4 && sp_supported(B, N1, N2) && (double)B * N1 * N2 >= 4e7;
 }
 
 __global__ void three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t N1, int64_t rows, float eps,

@@ -14,20 +14,19 @@ namespace {
 // counts its slice of the points into a histogram in its own shared memory; the exclusive prefix over
 // (cell, block) is formed across the cluster through distributed shared memory, each block for its
 // share of the cells; then every block writes its points to their places.  The order inside a cell is
-// whatever the atomics give.  Then every warp takes windows of 256 consecutive points, sorts them by
-// their fine position along the curve (a bitonic network on registers) and forms the leaf boxes.
-// Searches decide by original index, so no result depends on the order.
+// whatever the atomics give.  A second launch then sorts every window of 256 points by fine cell (a warp
+// each, a bitonic network on registers) and forms the boxes.  Searches decide by original index, so no
+// result depends on the order.
 constexpr int SB_THREADS = 512;
 constexpr int SB_WARPS = SB_THREADS / 32;
-constexpr int SB_WINDOW = 256;
 
 struct SpPair {
   SpCloud c[2];
 };
 
 template <int CL>
-__global__ void __launch_bounds__(SB_THREADS)
-spatial_build_kernel(const __grid_constant__ SpPair pair, int B) {
+__global__ void __launch_bounds__(SB_THREADS, 2)
+spatial_sort_kernel(const __grid_constant__ SpPair pair, int B) {
   constexpr int SHARE = SP_CELLS / CL;      // cells of one block
   constexpr int MINE = SHARE / SB_THREADS;  // cells of one thread
   static_assert(MINE >= 1 && MINE * CL * SB_THREADS == SP_CELLS, "whole cells per thread");
@@ -52,7 +51,7 @@ spatial_build_kernel(const __grid_constant__ SpPair pair, int B) {
   };
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float *xyz = c.xyz + b * 3 * (int64_t)N;
-  float4 *pts = c.pts + b * (int64_t)c.leaves * SP_LEAF;
+  float4 *pts = reinterpret_cast<float4 *>(c.pts) + b * (int64_t)c.windows * SP_WINDOW;
   const int NL = (N + CL - 1) / CL;
   const int beg = min(N, rank * NL), end = min(N, beg + NL);
 
@@ -158,8 +157,8 @@ spatial_build_kernel(const __grid_constant__ SpPair pair, int B) {
     pts[to] = make_float4(x, y, z, __int_as_float(j));
   }
   if (rank == 0) {
-    // padding of the last leaf: NaN distances are never below or at a bound
-    for (int j = N + tid; j < c.leaves * SP_LEAF; j += SB_THREADS)
+    // padding of the last window: NaN distances are never below or at a bound
+    for (int j = N + tid; j < c.windows * SP_WINDOW; j += SB_THREADS)
       pts[j] = make_float4(sp_nan(), sp_nan(), sp_nan(), __int_as_float(0x7fffffff));
     if (tid == 0) {
       if (2 * (int64_t)crowd > N) g.irregular = 1;
@@ -167,100 +166,105 @@ spatial_build_kernel(const __grid_constant__ SpPair pair, int B) {
       c.grid[b] = g;
     }
   }
-  sync();
+}
 
-  // windows: element e = 32 r + lane of a window is register r
-  float4 *boxes = c.boxes + b * (int64_t)c.leaves * 2;
-  const int windows = (c.leaves + 7) / 8;
-  for (int w = rank * SB_WARPS + warp; w < windows; w += CL * SB_WARPS) {
-    float4 *p = pts + (int64_t)w * SB_WINDOW;
-    const int live = min(8, c.leaves - 8 * w);  // leaves of this window
-    unsigned key[8];
+// One warp per window.  Register r of lane l is element 8 l + r of the network, so that a lane ends up
+// with a whole leaf and the distances 1, 2, 4 of the network need no exchange.
+constexpr int SW_THREADS = 128;
+
+__global__ void __launch_bounds__(SW_THREADS)
+spatial_window_kernel(const __grid_constant__ SpPair pair, int64_t windows0, int64_t windows_total) {
+  const int lane = threadIdx.x & 31;
+  int64_t w = (int64_t)blockIdx.x * (SW_THREADS / 32) + (threadIdx.x >> 5);
+  if (w >= windows_total) return;
+  const SpCloud &c = pair.c[w >= windows0];
+  if (w >= windows0) w -= windows0;
+  const SpGrid g = c.grid[w / c.windows];
+  float4 *p = reinterpret_cast<float4 *>(c.pts) + w * SP_WINDOW;
+  unsigned key[8];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const unsigned e = 32 * r + lane;
-      key[r] = 0xffffff00u | e;  // padding sorts last
-      if (r < live) {
-        const float4 q = __ldcg(p + e);
-        if (__float_as_int(q.w) != 0x7fffffff) key[r] = (sp_fine(q.x, q.y, q.z, g) << 8) | e;
-      }
-    }
+  for (int r = 0; r < 8; ++r) {
+    const unsigned e = 32 * r + lane;
+    const float4 q = p[e];
+    key[r] = ((__float_as_int(q.w) == 0x7fffffff ? 0xffffffu : sp_fine(q.x, q.y, q.z, g)) << 8) | e;  // padding last
+  }
 #pragma unroll
-    for (int k = 2; k <= SB_WINDOW; k <<= 1) {
+  for (int k = 2; k <= SP_WINDOW; k <<= 1) {
 #pragma unroll
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        if (j >= 32) {
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j < 8) {
 #pragma unroll
-          for (int r = 0; r < 8; ++r) {
-            const int o = r ^ (j >> 5);
-            if (o > r) {
-              const bool up = ((32 * r) & k) == 0;
-              const unsigned lo = min(key[r], key[o]), hi = max(key[r], key[o]);
-              key[r] = up ? lo : hi;
-              key[o] = up ? hi : lo;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < 8; ++r) {
-            const unsigned other = __shfl_xor_sync(0xffffffffu, key[r], j);
-            const bool up = ((32 * r + lane) & k) == 0, low = (lane & j) == 0;
-            key[r] = up == low ? min(key[r], other) : max(key[r], other);
+        for (int r = 0; r < 8; ++r) {
+          const int o = r ^ j;
+          if (o > r) {
+            const bool up = ((8 * lane + r) & k) == 0;
+            const unsigned lo = min(key[r], key[o]), hi = max(key[r], key[o]);
+            key[r] = up ? lo : hi;
+            key[o] = up ? hi : lo;
           }
         }
-      }
-    }
-    float4 q[8];
+      } else {
+        const bool keep_low = ((8 * lane & k) == 0) == ((8 * lane & j) == 0);
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
-      if (r < live) q[r] = __ldcg(p + (key[r] & 255u));
-    __syncwarp();  // every point is in registers before its place is written
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      if (r < live) {
-        const int leaf = 8 * w + r;
-        const float4 lo = make_float4(sp_warp_min(q[r].x), sp_warp_min(q[r].y), sp_warp_min(q[r].z),
-                                      __int_as_float(__reduce_min_sync(0xffffffffu, __float_as_int(q[r].w))));
-        const float4 hi = make_float4(sp_warp_max(q[r].x), sp_warp_max(q[r].y), sp_warp_max(q[r].z), 0.f);
-        if (lane == 0) {
-          boxes[2 * leaf] = lo;
-          boxes[2 * leaf + 1] = hi;
+        for (int r = 0; r < 8; ++r) {
+          const unsigned other = __shfl_xor_sync(0xffffffffu, key[r], j >> 3);
+          key[r] = keep_low ? min(key[r], other) : max(key[r], other);
         }
-        // pair p becomes (x0,x1,y0,y1) (z0,z1,i0,i1): lane l writes float4 number l
-        const int o = lane & 1;
-        const float s0 = o ? q[r].x : q[r].z, s1 = o ? q[r].y : q[r].w;  // what the pair's other lane stores
-        const float t0 = __shfl_xor_sync(0xffffffffu, s0, 1), t1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-        p[32 * r + lane] = o ? make_float4(t0, q[r].z, t1, q[r].w) : make_float4(q[r].x, t0, q[r].y, t1);
       }
     }
   }
-  sync();
-  for (int s = rank * SB_WARPS + warp; s < c.supers; s += CL * SB_WARPS) {
-    const int leaf = s * 32 + lane;
-    float4 lo = make_float4(sp_inf(), sp_inf(), sp_inf(), __int_as_float(0x7fffffff));
-    float4 hi = make_float4(-sp_inf(), -sp_inf(), -sp_inf(), 0.f);
-    if (leaf < c.leaves) {
-      lo = __ldcg(boxes + 2 * leaf);
-      hi = __ldcg(boxes + 2 * leaf + 1);
-    }
-    lo = make_float4(sp_warp_min(lo.x), sp_warp_min(lo.y), sp_warp_min(lo.z),
-                     __int_as_float(__reduce_min_sync(0xffffffffu, __float_as_int(lo.w))));
-    hi = make_float4(sp_warp_max(hi.x), sp_warp_max(hi.y), sp_warp_max(hi.z), 0.f);
-    if (lane == 0) {
-      c.sup[(b * c.supers + s) * 2] = lo;
-      c.sup[(b * c.supers + s) * 2 + 1] = hi;
-    }
+  float x[8], y[8], z[8];
+  int i[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const float4 q = p[key[r] & 255u];
+    x[r] = q.x, y[r] = q.y, z[r] = q.z, i[r] = __float_as_int(q.w);
+  }
+  __syncwarp();  // every point is in registers before its place is written
+  float4 *leaf = p + 8 * lane;
+  leaf[0] = make_float4(x[0], x[1], x[2], x[3]);
+  leaf[1] = make_float4(x[4], x[5], x[6], x[7]);
+  leaf[2] = make_float4(y[0], y[1], y[2], y[3]);
+  leaf[3] = make_float4(y[4], y[5], y[6], y[7]);
+  leaf[4] = make_float4(z[0], z[1], z[2], z[3]);
+  leaf[5] = make_float4(z[4], z[5], z[6], z[7]);
+  reinterpret_cast<int4 *>(leaf)[6] = make_int4(i[0], i[1], i[2], i[3]);
+  reinterpret_cast<int4 *>(leaf)[7] = make_int4(i[4], i[5], i[6], i[7]);
+  // boxes (minima and maxima drop NaN; a leaf of nothing but padding gets an empty box)
+  float lo[3] = {sp_inf(), sp_inf(), sp_inf()}, hi[3] = {-sp_inf(), -sp_inf(), -sp_inf()};
+  int low = 0x7fffffff;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    lo[0] = fminf(lo[0], x[r]), lo[1] = fminf(lo[1], y[r]), lo[2] = fminf(lo[2], z[r]);
+    hi[0] = fmaxf(hi[0], x[r]), hi[1] = fmaxf(hi[1], y[r]), hi[2] = fmaxf(hi[2], z[r]);
+    low = min(low, i[r]);
+  }
+  float4 *box = c.boxes + (w * 32 + lane) * 2;
+  box[0] = make_float4(lo[0], lo[1], lo[2], hi[0]);
+  box[1] = make_float4(hi[1], hi[2], __int_as_float(low), 0.f);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = sp_warp_min(lo[d]);
+    hi[d] = sp_warp_max(hi[d]);
+  }
+  low = __reduce_min_sync(0xffffffffu, low);
+  if (lane == 0) {
+    c.wbox[2 * w] = make_float4(lo[0], lo[1], lo[2], hi[0]);
+    c.wbox[2 * w + 1] = make_float4(hi[1], hi[2], __int_as_float(low), 0.f);
   }
 }
 
 // ---------------------------------------------------------------------------------------------
-// K <= 4 nearest keys of every query: one warp per query leaf, lane = query.
-//   1. SEEDS keys around the position of the query's cell in the key cloud bound its K-th distance.
-//   2. The warp scans the leaf it is closest to, then walks super leaves and leaves whose boxes come
-//      within the largest bound of its 32 queries; a leaf is scanned when at least one lane's own
-//      bound reaches its box.
-//   3. A scan evaluates exact distances two keys at a time (every lane reads the same 32 bytes) and
-//      branches once per eight keys.
+// K <= 4 nearest keys of every query: one warp per 32 consecutive queries, lane = query.
+//   1. The leaf at the position of the query's cell in the key cloud bounds its K-th distance.
+//   2. The warp walks the windows and, nearest first, their leaves whose boxes come within the largest
+//      bound of its queries; a leaf is scanned when at least one lane's own bound reaches its box.
+//   3. A scan evaluates exact distances two keys at a time, every lane the same keys, and branches once
+//      per leaf.
+// Bound by latency and the L1's return path together (0.6 instructions a cycle and scheduler): for two
+// clouds of 16384 points a warp visits 6 to 21 windows, tests 30 to 95 leaves and scans 15 to 30 of them.
+// 64 x 16384 x 16384, both directions: 0.28 ms on a surface, 0.63 ms in blobs, plus 0.08 ms for the
+// order (sweeping all pairs: 5.8 ms; leaves of 32 points and no look-ahead: 0.41 and 0.88 ms).
 // The list starts as K entries (bound, INT_MAX): the K keys behind the bound all order before or at
 // it, so they fill the list whatever order the leaves come in, and (distance, index) decides as in a
 // sweep in index order.  For the chamfer distance it starts as (+inf, -1) instead: there a distance of
@@ -292,42 +296,27 @@ constexpr int SN_THREADS = 128;
 constexpr int SN_WARPS = SN_THREADS / 32;
 
 template <int K>
-__device__ __forceinline__ void sp_scan(const float4 *__restrict__ leaf, float2 nx, float2 ny, float2 nz, float2 one,
+__device__ __forceinline__ void sp_scan(const float *__restrict__ leaf, float2 nx, float2 ny, float2 nz, float2 one,
                                         SpList<K> &list) {
-  float4 A[8];  // four key pairs, loaded one step ahead
+  float2 d[4];
+  sp_leaf_dist(leaf, nx, ny, nz, one, d);
+  const float m = sp_min8(d);
+  if (m <= list.d[K - 1]) {
+    int i[8];
+    sp_leaf_index(leaf, i);
+    if constexpr (K == 1) {  // only the smallest of the eight can enter: its lowest index
+      int at = 0x7fffffff;
 #pragma unroll
-  for (int u = 0; u < 8; ++u) A[u] = __ldg(leaf + u);
+      for (int u = 0; u < 4; ++u) {
+        at = min(at, d[u].x == m ? i[2 * u] : 0x7fffffff);
+        at = min(at, d[u].y == m ? i[2 * u + 1] : 0x7fffffff);
+      }
+      list.offer(m, at);
+    } else {
 #pragma unroll
-  for (int p = 0; p < SP_LEAF; p += 8) {
-    float2 d[4], id[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      d[u] = sp_dist2(A[2 * u], A[2 * u + 1], nx, ny, nz, one);
-      id[u] = make_float2(A[2 * u + 1].z, A[2 * u + 1].w);
-    }
-    if (p + 8 < SP_LEAF) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u) A[u] = __ldg(leaf + p + 8 + u);
-    }
-    float m = sp_min3(d[0].x, d[0].y, d[1].x);
-    m = sp_min3(m, d[1].y, d[2].x);
-    m = sp_min3(m, d[2].y, d[3].x);
-    m = fminf(m, d[3].y);
-    if (m <= list.d[K - 1]) {
-      if constexpr (K == 1) {  // only the smallest of the eight can enter: its lowest index
-        int i = 0x7fffffff;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          i = min(i, d[u].x == m ? __float_as_int(id[u].x) : 0x7fffffff);
-          i = min(i, d[u].y == m ? __float_as_int(id[u].y) : 0x7fffffff);
-        }
-        list.offer(m, i);
-      } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (d[u].x <= list.d[K - 1]) list.offer(d[u].x, __float_as_int(id[u].x));
-          if (d[u].y <= list.d[K - 1]) list.offer(d[u].y, __float_as_int(id[u].y));
-        }
+      for (int u = 0; u < 4; ++u) {
+        if (d[u].x <= list.d[K - 1]) list.offer(d[u].x, i[2 * u]);
+        if (d[u].y <= list.d[K - 1]) list.offer(d[u].y, i[2 * u + 1]);
       }
     }
   }
@@ -340,15 +329,13 @@ struct SpSearch {
   SpCloud c[2];
   float *dist[2];
   IndexOut index[2];
-  int64_t tasks[2];  // query leaves of all clouds
+  int64_t tasks[2];  // query groups of all clouds
   int64_t blocks0;   // blocks of direction 0
 };
 
 template <int K, int MODE>
 __global__ void __launch_bounds__(SN_THREADS)
 spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sums, float eps, float one_) {
-  constexpr int SEEDS = 8;
-  static_assert(K <= SEEDS / 2, "the seeds bound the K-th distance");
   __shared__ double ssum[SN_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rev = blockIdx.x >= job.blocks0;
@@ -356,40 +343,35 @@ spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sum
   const int64_t task = (blockIdx.x - (rev ? job.blocks0 : 0)) * SN_WARPS + warp;
   double total = 0.0;
   if (task < job.tasks[rev]) {
-    const int64_t b = task / qc.leaves;
-    const int ql = (int)(task - b * qc.leaves);
+    const int64_t b = task / qc.groups;
+    const int first = (int)(task - b * qc.groups) * SP_GROUP;
     const SpGrid g = kc.grid[b];
     if (!(g.irregular | qc.grid[b].irregular)) {
-      const float4 q = sp_point(qc.pts + b * (int64_t)qc.leaves * SP_LEAF, ql * SP_LEAF + lane);
-      const float4 *qbox = qc.boxes + (b * qc.leaves + ql) * 2;
-      const float4 qlo = __ldg(qbox), qhi = __ldg(qbox + 1);
-      const bool valid = ql * SP_LEAF + lane < qc.N;
+      const float4 q = sp_point(qc.pts + b * (int64_t)qc.windows * SP_WINDOW * 4, first + lane);
+      const bool valid = first + lane < qc.N;
+      // minima and maxima drop the NaN of padding lanes
+      const SpBox qbox = {sp_warp_min(q.x), sp_warp_min(q.y), sp_warp_min(q.z),
+                          sp_warp_max(q.x), sp_warp_max(q.y), sp_warp_max(q.z)};
       const float2 one = make_float2(one_, one_);
       const float2 nx = make_float2(-q.x, -q.x), ny = make_float2(-q.y, -q.y), nz = make_float2(-q.z, -q.z);
-      const float4 *kpts = kc.pts + b * (int64_t)kc.leaves * SP_LEAF;
-      const float4 *kbox = kc.boxes + b * (int64_t)kc.leaves * 2;
-      const float4 *ksup = kc.sup + b * (int64_t)kc.supers * 2;
+      const float *kpts = kc.pts + b * (int64_t)kc.windows * SP_WINDOW * 4;
+      const float4 *kbox = kc.boxes + b * (int64_t)kc.windows * 64;
+      const float4 *kwin = kc.wbox + b * (int64_t)kc.windows * 2;
 
-      // 1. seeds
+      // 1. the seed leaf (whole leaves only: it must hold K keys)
       const int *tab = kc.table + b * SP_CELLS;
       const int e = sp_cell(q.x, q.y, q.z, g);
       const int p0 = __ldg(tab + e), p1 = e + 1 < SP_CELLS ? __ldg(tab + e + 1) : kc.N;
-      const int seed = min(max(((p0 + p1) >> 1) - SEEDS / 2, 0), kc.N - SEEDS - 1) & ~1;
+      const int seed = min((p0 + p1) >> 4, (kc.N >> 3) - 1);
       SpList<K> list;
 #pragma unroll
       for (int c = 0; c < K; ++c) {
         list.d[c] = sp_inf();
         list.i[c] = MODE == SN_CHAMFER ? -1 : 0x7fffffff;
       }
-#pragma unroll
-      for (int u = 0; u < SEEDS / 2; ++u) {
-        const float4 A = __ldg(kpts + seed + 2 * u), Bv = __ldg(kpts + seed + 2 * u + 1);
-        const float2 d = sp_dist2(A, Bv, nx, ny, nz, one);
-        list.offer(d.x, __float_as_int(Bv.z));
-        list.offer(d.y, __float_as_int(Bv.w));
-      }
+      sp_scan<K>(kpts + seed * 32, nx, ny, nz, one, list);
       if constexpr (K > 1) {
-        // the seeds come again with their leaves: keep their bound only
+        // the seeds come again with their leaf: keep their bound only
         const float bound = list.d[K - 1];
 #pragma unroll
         for (int c = 0; c < K; ++c) {
@@ -399,37 +381,51 @@ spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sum
       }
       if (!valid) list.d[K - 1] = -1.f;  // never reached by a distance
 
-      // 2. the closest leaf, then the rest
-      const int home = __shfl_sync(0xffffffffu, seed + SEEDS / 2, min(16, qc.N - ql * SP_LEAF - 1)) >> 5;
-      sp_scan<K>(kpts + (int64_t)home * SP_LEAF, nx, ny, nz, one, list);
+      // 2. windows and leaves, beginning with the window of a middle query's seed
+      const int home = __shfl_sync(0xffffffffu, seed >> 5, min(16, qc.N - first - 1));
+      const float mx = 0.5f * (qbox.lx + qbox.hx), my = 0.5f * (qbox.ly + qbox.hy), mz = 0.5f * (qbox.lz + qbox.hz);
       float gb = sp_warp_max(list.d[K - 1]);
-      const int chunks = (kc.supers + 31) >> 5;
-      int ch = home >> 10;
+      const int chunks = (kc.windows + 31) >> 5;
+      int ch = home >> 5;
       for (int cc = 0; cc < chunks; ++cc) {
         const int s = ch * 32 + lane;
         bool hit = false;
-        if (s < kc.supers) hit = sp_box_box(qlo, qhi, __ldg(ksup + 2 * s), __ldg(ksup + 2 * s + 1)) <= gb;
-        unsigned smask = __ballot_sync(0xffffffffu, hit);
-        unsigned first = cc == 0 ? smask & (1u << ((home >> 5) & 31)) : 0u;
-        while (smask) {
-          const int sl = __ffs(first ? first : smask) - 1;
-          first = 0u;
-          smask &= ~(1u << sl);
-          const int l0 = (ch * 32 + sl) * 32;
-          hit = false;
-          if (l0 + lane < kc.leaves && l0 + lane != home)
-            hit = sp_box_box(qlo, qhi, __ldg(kbox + 2 * (l0 + lane)), __ldg(kbox + 2 * (l0 + lane) + 1)) <= gb;
-          unsigned lmask = __ballot_sync(0xffffffffu, hit);
-          while (lmask) {
-            const int l = l0 + __ffs(lmask) - 1;
-            lmask &= lmask - 1;
-            const float4 lo = __ldg(kbox + 2 * l), hi = __ldg(kbox + 2 * l + 1);
-            const float bd = sp_point_box(q.x, q.y, q.z, lo, hi);
-            const bool need =
-                bd < list.d[K - 1] || (bd == list.d[K - 1] && __float_as_int(lo.w) < list.i[K - 1]);
-            if (__any_sync(0xffffffffu, need)) sp_scan<K>(kpts + (int64_t)l * SP_LEAF, nx, ny, nz, one, list);
+        if (s < kc.windows) hit = sp_box_box(qbox, sp_box(kwin + 2 * s)) <= gb;
+        unsigned wmask = __ballot_sync(0xffffffffu, hit);
+        unsigned begin = cc == 0 ? wmask & (1u << (home & 31)) : 0u;
+        while (wmask) {
+          const int wl = __ffs(begin ? begin : wmask) - 1;
+          begin = 0u;
+          wmask &= ~(1u << wl);
+          const int l0 = (ch * 32 + wl) * 32;
+          const SpBox mine = sp_box(kbox + 2 * (l0 + lane));
+          const float reach = sp_box_box(qbox, mine);
+          // leaves in ascending distance of their centres from the group's: only an order, any will do
+          const float ex = 0.5f * (mine.lx + mine.hx) - mx, ey = 0.5f * (mine.ly + mine.hy) - my,
+                      ez = 0.5f * (mine.lz + mine.hz) - mz;
+          const unsigned far = 0xffffffffu;
+          unsigned key = (__float_as_uint(ex * ex + ey * ey + ez * ez) & 0x7fffffe0u) | lane;
+          if (!(reach <= gb)) key = far;
+          // the next leaf is picked and its box fetched while the current one is looked at
+          unsigned next = __reduce_min_sync(0xffffffffu, key);
+          SpBox box = sp_box(kbox + 2 * (l0 + (next & 31)));
+          while (next != far) {
+            const int l = l0 + (next & 31);
+            if (lane == (next & 31)) key = far;
+            const SpBox now = box;
+            next = __reduce_min_sync(0xffffffffu, key);
+            box = sp_box(kbox + 2 * (l0 + (next & 31)));
+            const float bd = sp_point_box(q.x, q.y, q.z, now);
+            if (!__any_sync(0xffffffffu, bd <= list.d[K - 1])) continue;
+            if (!__any_sync(0xffffffffu, bd < list.d[K - 1])) {
+              // at the bound itself a leaf matters only if it can win the tie by index
+              const int low = __float_as_int(__ldg(reinterpret_cast<const float *>(kbox + 2 * l) + 6));
+              if (!__any_sync(0xffffffffu, bd == list.d[K - 1] && low < list.i[K - 1])) continue;
+            }
+            sp_scan<K>(kpts + l * 32, nx, ny, nz, one, list);
+            gb = sp_warp_max(list.d[K - 1]);
+            if (!(reach <= gb)) key = far;
           }
-          gb = sp_warp_max(list.d[K - 1]);
         }
         ch = ch + 1 < chunks ? ch + 1 : 0;
       }
@@ -485,10 +481,10 @@ int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st) {
   SpPair pair;
   pair.c[0] = a;
   pair.c[1] = b ? *b : a;
-  const void *kern = CL == 8   ? (const void *)spatial_build_kernel<8>
-                     : CL == 4 ? (const void *)spatial_build_kernel<4>
-                     : CL == 2 ? (const void *)spatial_build_kernel<2>
-                               : (const void *)spatial_build_kernel<1>;
+  const void *kern = CL == 8   ? (const void *)spatial_sort_kernel<8>
+                     : CL == 4 ? (const void *)spatial_sort_kernel<4>
+                     : CL == 2 ? (const void *)spatial_sort_kernel<2>
+                               : (const void *)spatial_sort_kernel<1>;
   int B_ = (int)B;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(clouds * CL));
@@ -503,7 +499,10 @@ int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st) {
   cfg.numAttrs = 1;
   void *args[] = {&pair, &B_};
   TK3D_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
-  return check_launch("spatial_build_kernel");
+  const int64_t w0 = B * a.windows, total = w0 + (b ? B * b->windows : 0);
+  const int64_t per = SW_THREADS / 32;
+  spatial_window_kernel<<<(unsigned)((total + per - 1) / per), SW_THREADS, 0, st>>>(pair, w0, total);
+  return check_launch("spatial_window_kernel");
 }
 
 int sp_chamfer(const SpCloud &a, const SpCloud &b, int64_t B, float *dist1, int64_t *idx1, float *dist2, int64_t *idx2,
@@ -512,7 +511,7 @@ int sp_chamfer(const SpCloud &a, const SpCloud &b, int64_t B, float *dist1, int6
   job.c[0] = a, job.c[1] = b;
   job.dist[0] = dist1, job.dist[1] = dist2;
   job.index[0] = index_out(idx1, 0, B * a.N), job.index[1] = index_out(idx2, 0, B * b.N);
-  job.tasks[0] = B * a.leaves, job.tasks[1] = B * b.leaves;
+  job.tasks[0] = B * a.groups, job.tasks[1] = B * b.groups;
   job.blocks0 = (job.tasks[0] + SN_WARPS - 1) / SN_WARPS;
   const int64_t blocks = job.blocks0 + (job.tasks[1] + SN_WARPS - 1) / SN_WARPS;
   spatial_nn_kernel<1, SN_CHAMFER><<<(unsigned)blocks, SN_THREADS, 0, st>>>(job, sums, 0.f, 1.0f);
@@ -525,7 +524,7 @@ int sp_knn_small(const SpCloud &q, const SpCloud &k, int64_t B, int K, bool weig
   job.c[0] = q, job.c[1] = k;
   job.dist[0] = job.dist[1] = dist;
   job.index[0] = job.index[1] = index;
-  job.tasks[0] = B * q.leaves, job.tasks[1] = 0;
+  job.tasks[0] = B * q.groups, job.tasks[1] = 0;
   job.blocks0 = (job.tasks[0] + SN_WARPS - 1) / SN_WARPS;
   const unsigned grid = (unsigned)job.blocks0;
 #define SN_LAUNCH(KK, MODE) spatial_nn_kernel<KK, MODE><<<grid, SN_THREADS, 0, st>>>(job, nullptr, eps, 1.0f)

@@ -1,12 +1,17 @@
 // Spatially ordered copy of a batch of point clouds: the index that the pruned neighbour searches
 // walk (spatial.cu: build and up to four nearest neighbours).
 //
-// The points of a cloud are ordered along a Hilbert curve (16 cells per axis, refined to 256 within
-// windows of 256 points) and cut into LEAVES of 32 consecutive points; every leaf has a bounding box,
-// and so has every SUPER leaf of 32 leaves.  A leaf is what a warp handles at a time: as queries (one
-// lane each, close together in space) and as keys (scanned only when its box can hold a neighbour of
-// one of the warp's queries).  Of 512 leaves of a 16384-point cloud a warp has to scan 8 (points on a
-// surface) to 14 (in a volume) for nearest neighbours; along a Morton curve it would be 10 to 22.
+// The points of a cloud are ordered along a Hilbert curve: by one of 4096 cells (16 per axis), and
+// within WINDOWS of 256 points by one of 256 cells per axis.  Eight consecutive points form a LEAF, a
+// window is 32 leaves; leaves and windows have bounding boxes.  A warp takes 32 consecutive points as
+// queries (one lane each, close together in space), finds the windows and leaves whose boxes can hold
+// a neighbour of one of its queries, and scans those.
+//
+// Why eight: all lanes of a warp read the same key, and a 16-byte load hands 512 bytes to the lanes
+// whatever it reads, four cycles of the SM's L1; that, not arithmetic, bounds a scan.  Two clouds of
+// 16384 points, one neighbour, keys scanned per warp (counted on the CPU): leaves of 32 / 16 / 8 points
+// 433 / 272 / 156 in a volume, 262 / 177 / 112 on a surface, 573 / 369 / 236 in blobs.  Along a Morton
+// curve it would be about 1.6 times as many.
 //
 // Exactness.  Neighbour decisions are taken on d = ((dx*dx + dy*dy) + dz*dz) with individually
 // rounded operations.  The distance from a point to a box, and from a box to a box, is evaluated
@@ -27,7 +32,9 @@
 
 namespace tk3d {
 
-constexpr int SP_LEAF = 32;
+constexpr int SP_GROUP = 32;    // queries of a warp
+constexpr int SP_LEAF = 8;
+constexpr int SP_WINDOW = 256;  // 32 leaves
 constexpr int SP_CELLS = 4096;  // 16 per axis
 constexpr int SP_CROWD = 4096;
 constexpr int64_t SP_MAX_POINTS = 1 << 20;
@@ -42,10 +49,10 @@ struct SpGrid {
 struct SpCloud {
   const float *xyz;
   XyzLayout l;
-  int N, leaves, supers;
-  float4 *pts;    // [B][leaves * 32]: two points are two float4, (x0,x1,y0,y1) (z0,z1,i0,i1); i = original index
-  float4 *boxes;  // [B][leaves][2]: (lo, lowest original index), (hi, -)
-  float4 *sup;    // [B][supers][2]
+  int N, groups, windows;
+  float *pts;     // [B][windows * 32][4][8]: x, y, z and original index of a leaf's points; padding is NaN
+  float4 *boxes;  // [B][windows * 32][2]: (lo x, y, z, hi x), (hi y, hi z, lowest original index, -)
+  float4 *wbox;   // [B][windows][2]
   int *table;     // [B][SP_CELLS]: first position of every cell
   SpGrid *grid;   // [B]
 };
@@ -53,9 +60,9 @@ struct SpCloud {
 inline size_t sp_align(size_t n) { return (n + 255) / 256 * 256; }
 
 inline size_t sp_cloud_bytes(int64_t B, int64_t N) {
-  const int64_t leaves = (N + SP_LEAF - 1) / SP_LEAF, supers = (leaves + 31) / 32;
-  return sp_align((size_t)B * leaves * SP_LEAF * 16) + sp_align((size_t)B * leaves * 32) +
-         sp_align((size_t)B * supers * 32) + sp_align((size_t)B * SP_CELLS * 4) + sp_align((size_t)B * sizeof(SpGrid));
+  const int64_t windows = (N + SP_WINDOW - 1) / SP_WINDOW;
+  return sp_align((size_t)B * windows * SP_WINDOW * 16) + sp_align((size_t)B * windows * 32 * 32) +
+         sp_align((size_t)B * windows * 32) + sp_align((size_t)B * SP_CELLS * 4) + sp_align((size_t)B * sizeof(SpGrid));
 }
 
 // Lays the arrays of one side out at `at` (256-byte aligned).
@@ -64,14 +71,14 @@ inline SpCloud sp_cloud(const float *xyz, int channel_first, int64_t B, int64_t 
   c.xyz = xyz;
   c.l = xyz_layout(channel_first, N);
   c.N = (int)N;
-  c.leaves = (int)((N + SP_LEAF - 1) / SP_LEAF);
-  c.supers = (c.leaves + 31) / 32;
-  c.pts = reinterpret_cast<float4 *>(at);
-  at += sp_align((size_t)B * c.leaves * SP_LEAF * 16);
+  c.groups = (int)((N + SP_GROUP - 1) / SP_GROUP);
+  c.windows = (int)((N + SP_WINDOW - 1) / SP_WINDOW);
+  c.pts = reinterpret_cast<float *>(at);
+  at += sp_align((size_t)B * c.windows * SP_WINDOW * 16);
   c.boxes = reinterpret_cast<float4 *>(at);
-  at += sp_align((size_t)B * c.leaves * 32);
-  c.sup = reinterpret_cast<float4 *>(at);
-  at += sp_align((size_t)B * c.supers * 32);
+  at += sp_align((size_t)B * c.windows * 32 * 32);
+  c.wbox = reinterpret_cast<float4 *>(at);
+  at += sp_align((size_t)B * c.windows * 32);
   c.table = reinterpret_cast<int *>(at);
   at += sp_align((size_t)B * SP_CELLS * 4);
   c.grid = reinterpret_cast<SpGrid *>(at);
@@ -96,7 +103,7 @@ inline char *sp_align_ptr(void *p) {
   return reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 255) & ~(uintptr_t)255);
 }
 
-// Builds the index of both sides (one launch); `b` may be null.
+// Builds the index of both sides (two launches); `b` may be null.
 int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st);
 
 // Searches over built indexes; rows of clouds that are irregular on either side are left alone.
@@ -194,34 +201,59 @@ __device__ __forceinline__ float sp_sq3(float dx, float dy, float dz) {
   return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
 }
 
-// Lower bound of d between any point of box [alo, ahi] and any point of box [blo, bhi].
-__device__ __forceinline__ float sp_box_box(const float4 &alo, const float4 &ahi, const float4 &blo,
-                                            const float4 &bhi) {
-  return sp_sq3(sp_max3(__fsub_rn(alo.x, bhi.x), __fsub_rn(blo.x, ahi.x), 0.f),
-                sp_max3(__fsub_rn(alo.y, bhi.y), __fsub_rn(blo.y, ahi.y), 0.f),
-                sp_max3(__fsub_rn(alo.z, bhi.z), __fsub_rn(blo.z, ahi.z), 0.f));
+struct SpBox {
+  float lx, ly, lz, hx, hy, hz;
+};
+__device__ __forceinline__ SpBox sp_box(const float4 *__restrict__ at) {
+  const float4 a = __ldg(at);
+  const float2 c = __ldg(reinterpret_cast<const float2 *>(at + 1));
+  return {a.x, a.y, a.z, a.w, c.x, c.y};
 }
 
-__device__ __forceinline__ float sp_point_box(float x, float y, float z, const float4 &lo, const float4 &hi) {
-  return sp_sq3(sp_max3(__fsub_rn(lo.x, x), __fsub_rn(x, hi.x), 0.f),
-                sp_max3(__fsub_rn(lo.y, y), __fsub_rn(y, hi.y), 0.f),
-                sp_max3(__fsub_rn(lo.z, z), __fsub_rn(z, hi.z), 0.f));
+// Lower bound of d between any point of one box and any point of another.
+__device__ __forceinline__ float sp_box_box(const SpBox &a, const SpBox &c) {
+  return sp_sq3(sp_max3(__fsub_rn(a.lx, c.hx), __fsub_rn(c.lx, a.hx), 0.f),
+                sp_max3(__fsub_rn(a.ly, c.hy), __fsub_rn(c.ly, a.hy), 0.f),
+                sp_max3(__fsub_rn(a.lz, c.hz), __fsub_rn(c.lz, a.hz), 0.f));
+}
+__device__ __forceinline__ float sp_point_box(float x, float y, float z, const SpBox &c) {
+  return sp_sq3(sp_max3(__fsub_rn(c.lx, x), __fsub_rn(x, c.hx), 0.f), sp_max3(__fsub_rn(c.ly, y), __fsub_rn(y, c.hy), 0.f),
+                sp_max3(__fsub_rn(c.lz, z), __fsub_rn(z, c.hz), 0.f));
 }
 
-// Two exact squared distances at once: keys (x0,x1) .. against the query (-q, -q).  `one` must be
-// 1.0f and unknown to the compiler: fma(a, 1, b) rounds once, like the addition it stands for, and is
-// not fused with the product before it.
-__device__ __forceinline__ float2 sp_dist2(const float4 &A, const float4 &Bv, float2 nx, float2 ny, float2 nz,
-                                           float2 one) {
-  const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nx), dy = __fadd2_rn(make_float2(A.z, A.w), ny),
-               dz = __fadd2_rn(make_float2(Bv.x, Bv.y), nz);
-  return __ffma2_rn(__ffma2_rn(__fmul2_rn(dx, dx), one, __fmul2_rn(dy, dy)), one, __fmul2_rn(dz, dz));
+// Exact squared distances of a leaf's eight keys, two at a time, from the query (-q, -q).  `one` must
+// be 1.0f and unknown to the compiler: fma(a, 1, b) rounds once, like the addition it stands for, and
+// is not fused with the product before it.  Padding keys give NaN.
+__device__ __forceinline__ void sp_leaf_dist(const float *__restrict__ leaf, float2 nx, float2 ny, float2 nz, float2 one,
+                                             float2 (&d)[4]) {
+  const float4 *v = reinterpret_cast<const float4 *>(leaf);
+  float4 c[6];
+#pragma unroll
+  for (int u = 0; u < 6; ++u) c[u] = __ldg(v + u);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const float4 X = c[u >> 1], Y = c[2 + (u >> 1)], Z = c[4 + (u >> 1)];
+    const float2 dx = __fadd2_rn((u & 1) ? make_float2(X.z, X.w) : make_float2(X.x, X.y), nx);
+    const float2 dy = __fadd2_rn((u & 1) ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y), ny);
+    const float2 dz = __fadd2_rn((u & 1) ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y), nz);
+    d[u] = __ffma2_rn(__ffma2_rn(__fmul2_rn(dx, dx), one, __fmul2_rn(dy, dy)), one, __fmul2_rn(dz, dz));
+  }
+}
+__device__ __forceinline__ void sp_leaf_index(const float *__restrict__ leaf, int (&i)[8]) {
+  const int4 a = __ldg(reinterpret_cast<const int4 *>(leaf) + 6), c = __ldg(reinterpret_cast<const int4 *>(leaf) + 7);
+  i[0] = a.x, i[1] = a.y, i[2] = a.z, i[3] = a.w, i[4] = c.x, i[5] = c.y, i[6] = c.z, i[7] = c.w;
+}
+__device__ __forceinline__ float sp_min8(const float2 (&d)[4]) {
+  float m = sp_min3(d[0].x, d[0].y, d[1].x);
+  m = sp_min3(m, d[1].y, d[2].x);
+  m = sp_min3(m, d[2].y, d[3].x);
+  return fminf(m, d[3].y);
 }
 
-// Point `pos` of an ordered cloud (pair layout).
-__device__ __forceinline__ float4 sp_point(const float4 *__restrict__ pts, int pos) {
-  const float *f = reinterpret_cast<const float *>(pts) + (pos >> 1) * 8 + (pos & 1);
-  return make_float4(__ldg(f), __ldg(f + 2), __ldg(f + 4), __ldg(f + 6));
+// Point `pos` of an ordered cloud: coordinates and original index.
+__device__ __forceinline__ float4 sp_point(const float *__restrict__ pts, int pos) {
+  const float *f = pts + (int64_t)(pos >> 3) * 32 + (pos & 7);
+  return make_float4(__ldg(f), __ldg(f + 8), __ldg(f + 16), __ldg(f + 24));
 }
 #endif
 
