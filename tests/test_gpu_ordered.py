@@ -81,7 +81,7 @@ def test_chamfer(kind, B, N, M, cf):
 
 
 @pytest.mark.parametrize("kind", KINDS)
-@pytest.mark.parametrize("k", [1, 2, 3, 4])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 16, 17, 32, 33, 64])  # every list size, both ends of each class count
 @pytest.mark.parametrize("B,N,M,cf", [(3, 33, 1100, 0), (2, 4097, 1056, 1), (1, 700, 40001, 0)])
 def test_knn(kind, k, B, N, M, cf):
     from torkit3d_b200 import _lib

@@ -2,7 +2,8 @@
 //
 // Four kernels here, two more in files of their own (knn_select.cu: float32 with 64 < k <= 256, or
 // 40 < k with fewer than 16 keys per wanted neighbour, by radix selection; knn_split.cu: float64
-// with few queries):
+// with few queries).  Large float32 problems whose caller provides scratch do not sweep: they walk
+// spatially ordered clouds (spatial.cu, spatial_knn.cu).
 //   knn_small_kernel<K,Q>  fp32, k <= 4: per-thread top-K in registers, filter-then-verify sweep
 //                          (sweep.cuh), insertion straight from the verify branch.  With k << N2
 //                          the branch is rare (about k ln(N2/k) times per query).
@@ -21,6 +22,7 @@
 // strict comparisons, so the retained set and its order are reproducible bit for bit.
 #include <stdlib.h>
 
+#include "knn_list.cuh"
 #include "spatial.cuh"
 #include "sweep.cuh"
 
@@ -34,7 +36,6 @@ constexpr int KN_CAP = 16;   // candidate buffer entries per query
 constexpr int KN_STEP = 8;   // keys processed between two buffer-occupancy checks
 
 __device__ __forceinline__ float qnan() { return __int_as_float(0x7fc00000); }
-__device__ __forceinline__ float pinf() { return __int_as_float(0x7f800000); }
 
 // Stage one key tile (padded with points that can only reach the verify path, where they are
 // rejected by index) from registers or global memory.
@@ -492,25 +493,6 @@ constexpr size_t kt_smem_bytes() {
   return (size_t)2 * KT_TILE * 16 + (size_t)KT_NCH * 32 * Q * 4 + (size_t)KT_QCAP * 32 * Q * 4;
 }
 
-// Predicated append: if a < thr, claim a slot of the query's list and store v there (when the
-// slot exists).  Written in PTX so that it stays five straight-line instructions.
-template <int STRIDE_BYTES, int KT_QCAP>
-__device__ __forceinline__ void kt_append(float a, float thr, unsigned cnt_addr, unsigned cand_addr, int v) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      ".reg .pred q;\n\t"
-      ".reg .s32 sl;\n\t"
-      ".reg .u32 ad;\n\t"
-      "setp.ltu.f32 p, %0, %1;\n\t"
-      "@p atom.shared.add.s32 sl, [%2], 1;\n\t"
-      "setp.lt.and.s32 q, sl, %5, p;\n\t"
-      "mad.lo.u32 ad, sl, %6, %3;\n\t"
-      "@q st.shared.s32 [ad], %4;\n\t"
-      "}" ::"f"(a),
-      "f"(thr), "r"(cnt_addr), "r"(cand_addr), "r"(v), "n"(KT_QCAP), "n"(STRIDE_BYTES));
-}
-
 // Compare-exchange of a sorting network.
 __device__ __forceinline__ void kt_cx(float &a, float &b) {
   const float lo = fminf(a, b), hi = fmaxf(a, b);
@@ -523,7 +505,8 @@ __device__ __forceinline__ void kt_cx(float &a, float &b) {
 template <int Q, int KT_NCH, int KT_QCAP, int MINB, int KT_TILE>
 __global__ void __launch_bounds__(KT_THREADS, MINB)
 knn_twopass_kernel(const float *__restrict__ query, const float *__restrict__ key, int64_t B, int N1, int N2, int k,
-                   float *__restrict__ dist, IndexOut index, int64_t blocks_total, XyzLayout ql, XyzLayout kl) {
+                   float *__restrict__ dist, IndexOut index, int64_t blocks_total, XyzLayout ql, XyzLayout kl,
+                   SpOnly only) {
   constexpr int PER = KT_TILE / KT_THREADS;
   constexpr int CPW = KT_NCH / KT_SPLIT;          // classes per warp: 8, 16, 32 or 64
   constexpr int NPAIR = KT_TILE / 2 / KT_SPLIT;   // key pairs per warp and tile: 32 or 64
@@ -553,8 +536,10 @@ knn_twopass_kernel(const float *__restrict__ query, const float *__restrict__ ke
   const unsigned cnt_base = (unsigned)__cvta_generic_to_shared(ccnt);
   const unsigned cand_base = (unsigned)__cvta_generic_to_shared(cand);
 
+  if (only.idle(B)) return;
   for (int64_t blk = blockIdx.x; blk < blocks_total; blk += gridDim.x) {
     const int64_t b = blk / chunks;
+    if (only.skip(b)) continue;
     const int ibase = (int)(blk % chunks) * QS;
     float qx[Q], qy[Q], qz[Q], qq[Q];
     float2 mx[Q], my[Q], mz[Q];
@@ -843,80 +828,11 @@ knn_twopass_kernel(const float *__restrict__ query, const float *__restrict__ ke
     if (sub == 0) ccnt[col] = (qvalid && !listed) ? 1 : 0;
     __syncthreads();
 
-    // ---- exact scan of the queries flagged above, one warp per query: lanes take 32 consecutive
-    // keys at a time; a key that beats the current k-th entry is inserted into the sorted list kept
-    // in the first k slots of the query's own column of cd / cand (position by counting, entries
-    // behind it moved up by the lanes together).  Keys arrive in ascending index order, so a key
-    // equal to the k-th distance never enters a full list and equal distances stay in index order.
-    // A NaN distance counts as +inf for the ordering.
+    // ---- exact scan of the queries flagged above, one warp per query (knn_list.cuh)
     for (int fc = part; fc < QS; fc += KT_SPLIT) {
       if (ccnt[fc] == 0) continue;  // uniform over the warp
-      const int fq = ibase + fc;
-      float fx, fy, fz;
-      load_xyz(query + b * 3 * (int64_t)N1, fq, ql, fx, fy, fz);
-      int nk = 0;
-      float kth = pinf();
-      for (int base = 0; base < N2; base += 32) {
-        const int j = base + lane;
-        float d = pinf();
-        if (j < N2) {
-          float rx, ry, rz;
-          load_xyz(rb, j, kl, rx, ry, rz);
-          d = sqdist<float>(rx, ry, rz, fx, fy, fz);
-        }
-        const float dv = d == d ? d : pinf();  // ordering value
-        unsigned mask = __ballot_sync(0xffffffffu, j < N2 && (nk < k || dv < kth));
-        while (mask) {
-          const int l = __ffs(mask) - 1;
-          mask &= mask - 1;
-          const float dn = __shfl_sync(0xffffffffu, d, l), dnv = __shfl_sync(0xffffffffu, dv, l);
-          if (nk == k && !(dnv < kth)) continue;  // the k-th entry tightened since the ballot
-          // position: entries ordering at or before the new key (equal distances hold lower indices)
-          int before = 0;
-          for (int r = lane; r < nk; r += 32) {
-            const float w = cd[r * QS + fc];
-            before += ((w == w ? w : pinf()) <= dnv) ? 1 : 0;
-          }
-          const int pos = __reduce_add_sync(0xffffffffu, before);
-          const int last = nk < k ? nk : k - 1;  // slot that receives the old entry last - 1
-          // move entries [pos, last) up by one: read them all, then write them all
-          float mv[4];
-          int mj[4];
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            const int r = lane + 32 * q4;
-            if (r >= pos && r < last) {
-              mv[q4] = cd[r * QS + fc];
-              mj[q4] = cand[r * QS + fc];
-            }
-          }
-          __syncwarp();
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            const int r = lane + 32 * q4;
-            if (r >= pos && r < last) {
-              cd[(r + 1) * QS + fc] = mv[q4];
-              cand[(r + 1) * QS + fc] = mj[q4];
-            }
-          }
-          if (lane == 0) {
-            cd[pos * QS + fc] = dn;
-            cand[pos * QS + fc] = base + l;
-          }
-          __syncwarp();
-          if (nk < k) ++nk;
-          if (nk == k) {
-            const float w = cd[(k - 1) * QS + fc];
-            kth = w == w ? w : pinf();
-          }
-        }
-      }
-      float *od = dist + (b * N1 + fq) * (int64_t)k;
-      const int64_t orow = (b * N1 + fq) * (int64_t)k;
-      for (int c = lane; c < k; c += 32) {
-        od[c] = cd[c * QS + fc];
-        index.put(orow + c, cand[c * QS + fc]);
-      }
+      kt_exact_scan<QS>(query + b * 3 * (int64_t)N1, rb, ibase + fc, N2, k, ql, kl, cd + fc, cand + fc, dist, index,
+                        (b * N1 + ibase + fc) * (int64_t)k);
     }
   }
 }
@@ -1150,27 +1066,36 @@ template <int Q, int NCH, int QCAP, int MINB, int TILE = 256>
 int knn_twopass(const float *query, const float *key, int64_t B, int N1, int N2, int k, float *dist, const KnnIo &io,
                 cudaStream_t st) {
   const int64_t total = B * ((N1 + 32 * Q - 1) / (32 * Q));
-  const int64_t gcap = (int64_t)sm_count() * 256;
+  const int64_t gcap = (int64_t)sm_count() * (io.only.q ? MINB : 256);
   const size_t smem = kt_smem_bytes<Q, NCH, QCAP, TILE>();
   if (smem + 4096 > 48 * 1024)  // static shared memory of the kernel counts towards the 48 KB default limit
     TK3D_CUDA(raise_smem_limit((const void *)knn_twopass_kernel<Q, NCH, QCAP, MINB, TILE>, (int)smem));
   knn_twopass_kernel<Q, NCH, QCAP, MINB, TILE><<<(unsigned)(total < gcap ? total : gcap), KT_THREADS, smem, st>>>(
-      query, key, B, N1, N2, k, dist, io.index, total, io.ql, io.kl);
+      query, key, B, N1, N2, k, dist, io.index, total, io.ql, io.kl, io.only);
   return check_launch("knn_twopass_kernel");
 }
 
 }  // namespace
 
-// Whether ordering the clouds first pays (k = 3, sweep / ordered, us: 4 x 2048^2 46 / 54, 64 x 1024 x 512
-// 54 / 56, 16 x 4096 x 1024 101 / 56, 8 x 4096^2 121 / 62, 8 x 131072 x 32768 6714 / 351 to 893).
+// Whether the ordered search takes this k, and whether ordering the clouds first pays.
+bool knn_order_takes(int64_t B, int64_t N1, int64_t N2, int64_t k) {
+  return sp_supported(B, N1, N2) && (k <= 4 || (k <= 64 && N2 >= 16 * k && N2 <= SP_SELECT_POINTS));
+}
+// Measured on B200, sweep / ordered, us (two numbers: points in a volume, on a surface):
+//   k = 3    4 x 2048^2 46 / 54, 64 x 1024 x 512 54 / 56, 16 x 4096 x 1024 101 / 56, 8 x 4096^2 121 / 62
+//   k = 16   32 x 1024^2 55 / 74, 64; 8 x 2048^2 52 / 62, 52; 16 x 4096^2 175 / 136, 98; 4 x 512 x 10000 116 / 80, 60
+//   k = 32   4 x 1024^2 48 / 64; 32 x 1024^2 124 / 126, 107; 8 x 2048^2 89 / 91, 74; 32 x 2048 x 8192 545 / 273, 195
+//   k = 64   4 x 1024^2 101 / 107, 102; 8 x 2048^2 195 / 162, 152; 32 x 2048 x 8192 936 / 551, 425
 bool knn_order_pays(int64_t B, int64_t N1, int64_t N2, int64_t k) {
-  return k <= 4 && sp_supported(B, N1, N2) && (double)B * N1 * N2 >= 4e7;
+  const double pairs = (double)B * N1 * N2;
+  const double least = k <= 4 ? 4e7 : k > 32 || N2 >= 8192 ? 2e7 : k > 16 ? 4e7 : 1e8;
+  return knn_order_takes(B, N1, N2, k) && pairs >= least;
 }
 
 __global__ void three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t N1, int64_t rows, float eps,
                                                SpOnly only);
 
-// k <= 4 over spatially ordered clouds; what the order cannot serve is swept.
+// k <= 64 over spatially ordered clouds; what the order cannot serve is swept.
 int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, int k, int channel_first,
                 bool weights, float eps, float *dist, void *index, int index32, void *scratch, cudaStream_t st) {
   const int64_t step = sp_batch(B, N1, N2);
@@ -1188,13 +1113,19 @@ int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int
     io.kl = ck.l;
     io.only = SpOnly{cq.grid, ck.grid};
     int rc = sp_build(cq, same ? nullptr : &ck, n, st);
-    if (!rc) rc = sp_knn_small(cq, ck, n, k, weights, eps, d, io.index, st);
+    if (!rc)
+      rc = k <= 4 ? sp_knn_small(cq, ck, n, k, weights, eps, d, io.index, st)
+                  : sp_knn_select(cq, ck, n, k, d, io.index, st);
     if (rc) return rc;
     switch (k) {
       case 1: rc = knn_small<1, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
       case 2: rc = knn_small<2, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
       case 3: rc = knn_small<3, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
-      default: rc = knn_small<4, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      case 4: rc = knn_small<4, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      default:
+        rc = k <= 16   ? knn_twopass<1, 32, 56, 7>(q, r, n, (int)N1, (int)N2, k, d, io, st)
+             : k <= 32 ? knn_twopass<1, 64, 104, 5>(q, r, n, (int)N1, (int)N2, k, d, io, st)
+                       : knn_twopass<1, 128, 192, 4>(q, r, n, (int)N1, (int)N2, k, d, io, st);
     }
     if (rc) return rc;
     if (weights) {
@@ -1284,7 +1215,7 @@ static int knn_impl(const void *query, const void *key, int64_t B, int64_t N1, i
   }
   const float *q = (const float *)query, *r = (const float *)key;
   float *d = (float *)distance;
-  if (scratch && k <= 4 && sp_supported(B, N1, N2) && scratch_bytes >= sp_search_bytes(B, N1, N2))
+  if (scratch && knn_order_takes(B, N1, N2, k) && scratch_bytes >= sp_search_bytes(B, N1, N2))
     return knn_ordered(q, r, B, N1, N2, (int)k, channel_first, false, 0.f, d, index, index32, scratch, st);
   switch (k) {
     case 1: return knn_small_q<1>(q, r, B, (int)N1, (int)N2, d, io, st);

@@ -1,5 +1,5 @@
 // Spatially ordered copy of a batch of point clouds: the index that the pruned neighbour searches
-// walk (spatial.cu: build and up to four nearest neighbours).
+// walk (spatial.cu: build and up to four nearest neighbours, spatial_knn.cu: up to 64).
 //
 // The points of a cloud are ordered along a Hilbert curve: by one of 4096 cells (16 per axis), and
 // within WINDOWS of 256 points by one of 256 cells per axis.  Eight consecutive points form a LEAF, a
@@ -111,6 +111,8 @@ int sp_chamfer(const SpCloud &a, const SpCloud &b, int64_t B, float *dist1, int6
                double *sums, cudaStream_t st);
 int sp_knn_small(const SpCloud &q, const SpCloud &k, int64_t B, int K, bool weights, float eps, float *dist,
                  IndexOut index, cudaStream_t st);
+int sp_knn_select(const SpCloud &q, const SpCloud &k, int64_t B, int K, float *dist, IndexOut index, cudaStream_t st);
+constexpr int64_t SP_SELECT_POINTS = 1 << 19;  // keys at most: leaf numbers are kept in 16 bits
 
 // For the sweeping kernels launched behind a search: the grids of the two sides, null for a launch on its own.
 struct SpOnly {
