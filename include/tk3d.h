@@ -116,7 +116,7 @@ int tk3d_knn(const void *query, const void *key, int64_t B, int64_t N1, int64_t 
              int64_t *index, int dtype, void *stream);
 
 /*
- * The same two searches with a scratch buffer for spatially ordered copies of the clouds, which large
+ * These two searches and the ball query with a scratch buffer for spatially ordered copies of the clouds, which large
  * float32 searches walk instead of sweeping every pair (same results, bit for bit).
  *   xyz_channel_first, index_dtype   as for the *_layout entry points
  *   scratch          device buffer of at least tk3d_*_scratch_bytes() bytes, contents ignored on entry;
@@ -131,6 +131,10 @@ size_t tk3d_knn_scratch_bytes(int64_t B, int64_t N1, int64_t N2, int64_t k, int 
 int tk3d_knn_ws(const void *query, const void *key, int64_t B, int64_t N1, int64_t N2, int64_t k,
                 int xyz_channel_first, void *distance, void *index, int index_dtype, void *scratch,
                 size_t scratch_bytes, int dtype, void *stream);
+size_t tk3d_ball_query_scratch_bytes(int64_t B, int64_t N1, int64_t N2, int64_t k, int dtype);
+int tk3d_ball_query_ws(const void *query, const void *key, int64_t B, int64_t N1, int64_t N2, float radius, int64_t k,
+                       int xyz_channel_first, void *index, int index_dtype, void *scratch, size_t scratch_bytes,
+                       int dtype, void *stream);
 
 /*
  * Farthest point sampling, first sample = point 0, lowest index among exact maxima.

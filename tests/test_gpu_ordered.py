@@ -99,6 +99,51 @@ def test_knn(kind, k, B, N, M, cf):
         assert _same(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
 
 
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("radius", [0.0, 0.03, 0.15, 0.4, 30.0, float("inf"), float("nan")])  # none, sparse, dense, all
+@pytest.mark.parametrize("B,N,M,k,cf", [(2, 333, 1100, 8, 0), (2, 1001, 4099, 40, 1), (1, 2000, 33000, 200, 0)])
+def test_ball_query(kind, radius, B, N, M, k, cf):
+    from torkit3d_b200 import _lib
+
+    lib = _lib.load()
+    a, b = _pair(kind, B, N, M, cf)
+    for itype, code in ((torch.int64, _lib.I64), (torch.int32, _lib.I32)):
+        res = []
+        for buf in (None, _scratch()):
+            i = torch.full((B, N, k), -7, dtype=itype, device=DEV)
+            assert lib.tk3d_ball_query_ws(a.data_ptr(), b.data_ptr(), B, N, M, radius, k, cf, i.data_ptr(), code,
+                                          buf.data_ptr() if buf is not None else None,
+                                          buf.numel() if buf is not None else 0, _lib.F32, _stream()) == 0
+            res.append(i)
+        assert torch.equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("K", [7, 32])
+@pytest.mark.parametrize("radius", [0.05, 0.5])
+def test_set_abstraction_from_ordered_neighbours(radius, K):
+    from torkit3d_b200 import _lib
+
+    lib = _lib.load()
+    B, C, N, M = 4, 12, 16400, 2100
+    a, b = _pair("uniform", B, M, N, 1)  # centroids, points
+    f = torch.randn(B, C, N, device=DEV)
+    need, rows = lib.tk3d_sa_group_scratch_bytes(B, C, N, M, K, _lib.F32), B * C * N * 4
+    assert need > rows
+    for want_index in (True, False):
+        res = []
+        for n in (rows, need):  # the smaller buffer holds the transposed features only: the kernel sweeps
+            buf = torch.zeros(n, dtype=torch.uint8, device=DEV)
+            out = torch.empty(B, C + 3, M, K, device=DEV)
+            i = torch.full((B, M, K), -7, dtype=torch.int32, device=DEV)
+            st = torch.zeros(1, dtype=torch.int32, device=DEV)
+            assert lib.tk3d_sa_group_fwd(b.data_ptr(), a.data_ptr(), f.data_ptr(), B, C, N, M, radius, K, 1, 1,
+                                         out.data_ptr(), i.data_ptr() if want_index else None, st.data_ptr(),
+                                         buf.data_ptr(), n, _lib.F32, _stream()) == 0
+            torch.cuda.synchronize()
+            res.append((out, i, st))
+        assert _same(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1]) and torch.equal(res[0][2], res[1][2])
+
+
 @pytest.mark.parametrize("kind", ["uniform", "nonfinite", "zeros"])
 def test_three_nn_weights_of_the_fused_interpolation(kind):
     from torkit3d_b200 import _fused, ops

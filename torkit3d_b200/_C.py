@@ -167,7 +167,14 @@ def ball_query_cuda(query, key, radius, max_neighbors, *, channel_first=False, i
     k = int(max_neighbors)
     with _on(query.device):
         index = torch.empty((B, N1, k), dtype=index_dtype, device=query.device)
-        if channel_first or index_dtype != torch.int64:
+        # large searches order the clouds first; 0 where sweeping all pairs is faster
+        need = _lib.scratch_bytes("tk3d_ball_query", B, N1, N2, k, _dtype(query))
+        if need:
+            scratch = torch.empty((need,), dtype=torch.uint8, device=query.device)
+            check(lib.tk3d_ball_query_ws(_ptr(query), _ptr(key), B, N1, N2, float(radius), k,
+                                         1 if channel_first else 0, _ptr(index), _index_code(index_dtype),
+                                         _ptr(scratch), need, _dtype(query), _stream(query)))
+        elif channel_first or index_dtype != torch.int64:
             check(lib.tk3d_ball_query_layout(_ptr(query), _ptr(key), B, N1, N2, float(radius), k,
                                              1 if channel_first else 0, _ptr(index), _index_code(index_dtype),
                                              _dtype(query), _stream(query)))

@@ -32,6 +32,9 @@ SIGNATURES = {
                                    _int, _vp]),
     "tk3d_knn_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64, _int]),
     "tk3d_knn_ws": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _int, _vp, _vp, _int, _vp, ctypes.c_size_t, _int, _vp]),
+    "tk3d_ball_query_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64, _int]),
+    "tk3d_ball_query_ws": (_int, [_vp, _vp, _i64, _i64, _i64, ctypes.c_float, _i64, _int, _vp, _int, _vp,
+                                  ctypes.c_size_t, _int, _vp]),
     "tk3d_fps_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _int]),
     "tk3d_fps": (_int, [_vp, _i64, _i64, _i64, _vp, _vp, ctypes.c_size_t, _int, _vp]),
     "tk3d_fps_static_scratch_capacity": (ctypes.c_size_t, []),

@@ -7,6 +7,8 @@
 // -inf) and a block leaves the key loop as soon as all its queries are full -- the reference keeps
 // scanning to the end of the cloud.  Short rows are padded with the first hit, rows without a hit
 // are filled with -1, so every output element is written here.
+#include "ball_sweep.cuh"
+#include "spatial.cuh"
 #include "sweep.cuh"
 
 namespace tk3d {
@@ -106,118 +108,22 @@ ball_query_fast_kernel(const float *__restrict__ query, const float *__restrict_
   }
 }
 
-// Few queries (B*N1 below a few hundred thousand): one query per thread cannot fill 148 SMs.  Here a
-// block of SPLIT warps serves 32 queries (lane = query) and warp s sweeps the s-th slice of every
-// 256-key tile, so SPLIT times as many warps are in flight.  A thread records the hits of its slice
-// as a bit mask (at most 64 keys), the slices' hit counts of the tile are exchanged through shared
-// memory at the tile's barrier, and every thread then knows where its hits belong in the query's
-// row (hits of earlier tiles + hits of lower slices of this tile) and writes them there: rows come
-// out in ascending key order without a merge, for any K.  A query with K hits stops testing, and
-// the block leaves the key loop at the first barrier after all its queries are full.
-constexpr int BS_TILE = 256;
-
+// Few queries (B*N1 below a few hundred thousand): one query per thread cannot fill 148 SMs, several
+// warps share 32 queries (ball_sweep.cuh).
 template <int SPLIT>
 __global__ void __launch_bounds__(32 * SPLIT)
 ball_query_split_kernel(const float *__restrict__ query, const float *__restrict__ key, int64_t B, int N1, int N2,
                         float r2, int k, IndexOut index, int64_t blocks_total, XyzLayout ql, XyzLayout kl) {
-  constexpr int THREADS = 32 * SPLIT;
-  constexpr int PER = BS_TILE / THREADS;
-  constexpr int QK = BS_TILE / SPLIT;  // keys per warp per tile (64 or 32)
-  static_assert(PER >= 1 && QK <= 64 && QK % 8 == 0, "slice must fit a 64-bit hit mask");
-  __shared__ float4 tile[2][BS_TILE];
-  __shared__ int tcount[2][SPLIT][32];
-  const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
+  __shared__ BallSweepSmem<SPLIT> sm;
   const int chunks = (N1 + 31) / 32;
-  const float never = __int_as_float(0xff800000);
-
   for (int64_t blk = blockIdx.x; blk < blocks_total; blk += gridDim.x) {
     const int64_t b = blk / chunks;
-    const int i = (int)(blk % chunks) * 32 + lane;
+    const int i = (int)(blk % chunks) * 32 + (threadIdx.x & 31);
     const bool valid = i < N1;
     float qx = 0.f, qy = 0.f, qz = 0.f;
     if (valid) load_xyz(query + b * 3 * (int64_t)N1, i, ql, qx, qy, qz);
-    const float2 mx[1] = {make_float2(-2.f * qx, -2.f * qx)}, my[1] = {make_float2(-2.f * qy, -2.f * qy)},
-                 mz[1] = {make_float2(-2.f * qz, -2.f * qz)};
-    const float open_thr = sweep_threshold(r2, sweep_qq(qx, qy, qz));
-    float thr[1] = {valid ? open_thr : never};
-    const int64_t row = (b * N1 + (valid ? i : 0)) * (int64_t)k;
-    int done = 0;  // hits of this query in the tiles swept so far (the same number in every warp)
-    const float *rb = key + b * (int64_t)N2 * 3;
-    const int ntiles = (N2 + BS_TILE - 1) / BS_TILE;
-
-    float4 nxt[PER];
-    auto fetch = [&](int t0) {
-#pragma unroll
-      for (int p = 0; p < PER; ++p) {
-        const int j = t0 + tid + p * THREADS;
-        float4 v = make_float4(0.f, 0.f, 0.f, __int_as_float(0x7f800000));
-        if (j < N2) {
-          float x, y, z;
-          load_xyz(rb, j, kl, x, y, z);
-          v = make_float4(x, y, z, sweep_key_w(x, y, z));
-        }
-        nxt[p] = v;
-      }
-    };
-    auto commit = [&](float4 *dst) {
-#pragma unroll
-      for (int p = 0; p < PER; ++p) sweep_store_key(dst, tid + p * THREADS, nxt[p].x, nxt[p].y, nxt[p].z, nxt[p].w);
-    };
-    fetch(0);
-    commit(tile[0]);
-    __syncthreads();
-    for (int t = 0; t < ntiles; ++t) {
-      const int t0 = t * BS_TILE + part * QK;
-      const float4 *tl = tile[t & 1] + part * QK;
-      if (t + 1 < ntiles) fetch((t + 1) * BS_TILE);
-      unsigned long long mask = 0;
-      int cnt = 0;
-      const bool was_full = !valid || done >= k;
-#pragma unroll 2
-      for (int u0 = 0; u0 < QK; u0 += 8) {
-        float2 a[4];
-        if (__builtin_expect(sweep_group2<1, true>(tl + u0, mx, my, mz, thr, a), 0)) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const float av = (u & 1) ? a[u >> 1].y : a[u >> 1].x;
-            if (!(av >= thr[0])) {  // padding keys carry +inf; a full row has thr = -inf
-              const float4 r = sweep_load_key(tl, u0 + u);
-              const float d = sqdist<float>(r.x, r.y, r.z, qx, qy, qz);
-              if (d < r2) {
-                mask |= 1ull << (u0 + u);
-                if (done + ++cnt >= k) thr[0] = never;  // whatever the lower slices found, this row is full
-              }
-            }
-          }
-        }
-      }
-      tcount[t & 1][part][lane] = cnt;
-      if (t + 1 < ntiles) commit(tile[(t + 1) & 1]);
-      // One barrier per tile; it also votes on "every query of this block was full before this tile"
-      // (such a tile recorded no hit anywhere, so nothing is left to write).
-      if (__syncthreads_and(was_full)) break;
-      int before = 0, total = 0;
-#pragma unroll
-      for (int s = 0; s < SPLIT; ++s) {
-        const int c = tcount[t & 1][s][lane];
-        if (s < part) before += c;
-        total += c;
-      }
-      int pos = done + before;
-      while (mask != 0 && pos < k) {
-        const int bit = __ffsll((long long)mask) - 1;
-        mask &= mask - 1;
-        index.put(row + pos, t0 + bit);
-        ++pos;
-      }
-      done += total;
-      if (done >= k) thr[0] = never;
-    }
-    __syncthreads();  // the row's first entry, written by whichever warp found it, is visible now
-    if (valid && done < k) {
-      const int64_t first = done > 0 ? index.get(row) : -1;
-      for (int c = done + part; c < k; c += SPLIT) index.put(row + c, first);
-    }
+    ball_sweep<SPLIT>(key + b * (int64_t)N2 * 3, N2, kl, qx, qy, qz, valid, r2, k,
+                      (b * N1 + (valid ? i : 0)) * (int64_t)k, index, sm);
     __syncthreads();
   }
 }
@@ -359,7 +265,8 @@ ball_query_generic_kernel(const T *__restrict__ query, const T *__restrict__ key
 using namespace tk3d;
 
 static int ball_query_impl(const void *query, const void *key, int64_t B, int64_t N1, int64_t N2, float radius,
-                           int64_t k, int channel_first, void *index, int index32, int dtype, void *stream) {
+                           int64_t k, int channel_first, void *index, int index32, int dtype, void *stream,
+                           void *scratch = nullptr, size_t scratch_bytes = 0) {
   TK3D_REQUIRE(dtype == TK3D_F32 || dtype == TK3D_F64, TK3D_ERR_DTYPE, "ball_query: dtype %d", dtype);
   TK3D_REQUIRE(B >= 0 && N1 >= 0 && N2 >= 0, TK3D_ERR_SHAPE, "ball_query: negative size");
   TK3D_REQUIRE(k >= 1 && k < (1LL << 31), TK3D_ERR_K, "ball_query: max_neighbors must be >= 1 (got %lld)",
@@ -370,6 +277,10 @@ static int ball_query_impl(const void *query, const void *key, int64_t B, int64_
   cudaStream_t st = (cudaStream_t)stream;
   const XyzLayout ql = xyz_layout(channel_first, N1), kl = xyz_layout(channel_first, N2);
   const IndexOut io = index_out(index, index32, B * N1 * k);
+  if (dtype == TK3D_F32 && scratch && sp_supported(B, N1, N2) && N2 <= SP_SELECT_POINTS &&
+      scratch_bytes >= sp_search_bytes(B, N1, N2))
+    return sp_ball_query((const float *)query, (const float *)key, B, N1, N2, channel_first, radius * radius, (int)k,
+                         index, index32, scratch, st);
   if (dtype == TK3D_F32) {
     const float r2 = radius * radius;  // squared in fp32, as the reference does for float tensors
     const int64_t cap = (int64_t)sm_count() * 256;
@@ -418,6 +329,31 @@ extern "C" int tk3d_ball_query_layout(const void *query, const void *key, int64_
                index_dtype);
   return ball_query_impl(query, key, B, N1, N2, radius, k, xyz_channel_first != 0, index, index_dtype == TK3D_I32,
                          dtype, stream);
+}
+
+namespace tk3d {
+// Whether ordering the clouds first pays.  Measured on B200, sweep / ordered, us, balls of 0.6 to 1.5 times
+// the wanted hits: 32 x 512 queries of 2048 keys 43 / 54, 8 x 2048 of 4096 56 / 42 to 48, 32 x 1024 of 8192
+// 133 / 70 to 79, 32 x 4096 of 16384 845 / 260 to 312.  Dense balls are found out by a sample and swept:
+// the looking costs 12 us (32 x 1024 of 8192, 1000 hits: 29 / 41), hence not below 1.2e8 pairs.
+bool ball_order_pays(int64_t B, int64_t N1, int64_t N2) {
+  return sp_supported(B, N1, N2) && N2 <= SP_SELECT_POINTS && (double)B * N1 * N2 >= 1.2e8;
+}
+}  // namespace tk3d
+
+extern "C" size_t tk3d_ball_query_scratch_bytes(int64_t B, int64_t N1, int64_t N2, int64_t k, int dtype) {
+  if (dtype != TK3D_F32 || k < 1 || k >= (1LL << 31) || !ball_order_pays(B, N1, N2)) return 0;
+  return sp_search_bytes(B, N1, N2);
+}
+
+extern "C" int tk3d_ball_query_ws(const void *query, const void *key, int64_t B, int64_t N1, int64_t N2, float radius,
+                                  int64_t k, int xyz_channel_first, void *index, int index_dtype, void *scratch,
+                                  size_t scratch_bytes, int dtype, void *stream) {
+  TK3D_RANGE("tk3d_ball_query_ws");
+  TK3D_REQUIRE(index_dtype == TK3D_I64 || index_dtype == TK3D_I32, TK3D_ERR_DTYPE, "ball_query: index_dtype %d",
+               index_dtype);
+  return ball_query_impl(query, key, B, N1, N2, radius, k, xyz_channel_first != 0, index, index_dtype == TK3D_I32,
+                         dtype, stream, scratch, scratch_bytes);
 }
 
 TK3D_BOUNDS_TU(ball_query)

@@ -21,7 +21,11 @@
 // all 1024 blocks are resident at once and pass through the two phases together, so the time is
 // close to the sum of a ball query (0.13 ms) and a gather (0.11 ms); larger batches, whose blocks
 // come in several waves, let the sweep of one block overlap the traffic of another.
+//
+// Large problems whose scratch allows it find the neighbours over spatially ordered clouds first
+// (spatial_ball.cu); the kernel then starts from those lists.
 #include "rows.cuh"
+#include "spatial.cuh"
 #include "sweep.cuh"
 
 namespace tk3d {
@@ -55,7 +59,8 @@ __global__ void __launch_bounds__(32 * SPLIT)
 sa_group_fwd_kernel(const float *__restrict__ points, const float *__restrict__ centroids,
                     const float *__restrict__ featT, int64_t B, int C, int N, int M, int pps, int pcs, int cps,
                     int cpc, float r2, int K, int use_xyz, int vec, float *__restrict__ out,
-                    int32_t *__restrict__ index32, int32_t *__restrict__ status, int64_t blocks_total) {
+                    const int32_t *__restrict__ given, int32_t *__restrict__ index32, int32_t *__restrict__ status,
+                    int64_t blocks_total) {
   constexpr int THREADS = 32 * SPLIT;  // SPLIT warps share every tile of points
   constexpr int PER = SA_TILE / THREADS;
   constexpr int QK = SA_TILE / SPLIT;
@@ -100,7 +105,7 @@ sa_group_fwd_kernel(const float *__restrict__ points, const float *__restrict__ 
     int done = 0;                   // hits of this centroid in the tiles swept so far (same in every warp)
     int *row = sidx + lane * S1;    // its hit list, ascending point index
     const float *rb = points + b * 3 * (int64_t)N;
-    const int ntiles = (N + SA_TILE - 1) / SA_TILE;
+    const int ntiles = given ? 0 : (N + SA_TILE - 1) / SA_TILE;
 
     // ---- phase A: ball query ----------------------------------------------------------------
     float4 nxt[PER];
@@ -176,7 +181,11 @@ sa_group_fwd_kernel(const float *__restrict__ points, const float *__restrict__ 
       if (done >= K) thr[0] = never;
     }
     __syncthreads();  // the lists' first entries are visible to every warp
-    if (done < K) {   // short lists repeat their first hit; empty ones (and padding lanes) hold -1
+    if (given) {      // complete lists, found beforehand
+      const int32_t *gp = given + b * E + (int64_t)m0 * K;
+      for (int e = tid; e < nv * K; e += THREADS) sidx[(e / K) * S1 + (e % K)] = gp[e];
+      if (part == 0 && valid && status && gp[(int64_t)lane * K] < 0) atomicOr(status, 1);
+    } else if (done < K) {   // short lists repeat their first hit; empty ones (and padding lanes) hold -1
       const int first = valid && done > 0 ? row[0] : -1;
       for (int c = (valid ? done : 0) + part; c < K; c += SPLIT) row[c] = first;
       if (part == 0 && valid && done == 0 && status) atomicOr(status, 1);
@@ -343,9 +352,16 @@ extern "C" int tk3d_sa_group_supported(int64_t B, int64_t C, int64_t N, int64_t 
   return dtype == TK3D_F32 && sa_shape_ok(B, C, N, M, K) ? 1 : 0;
 }
 
+namespace tk3d {
+bool ball_order_pays(int64_t B, int64_t N1, int64_t N2);
+}
+static size_t sa_align(size_t n) { return (n + 255) & ~(size_t)255; }
+
 extern "C" size_t tk3d_sa_group_scratch_bytes(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K, int dtype) {
   if (!tk3d_sa_group_supported(B, C, N, M, K, dtype) || C == 0) return 0;
-  return rows_scratch_bytes(B, C, N);
+  const size_t rows = rows_scratch_bytes(B, C, N);
+  return ball_order_pays(B, M, N) ? sa_align(rows) + sp_search_bytes(B, M, N) + sizeof(int32_t) * (size_t)(B * M * K)
+                                  : rows;
 }
 
 extern "C" int tk3d_sa_group_fwd(const void *points, const void *centroids, const void *feature, int64_t B, int64_t C,
@@ -371,6 +387,16 @@ extern "C" int tk3d_sa_group_fwd(const void *points, const void *centroids, cons
     if (rc) return rc;
     featT = (const float *)scratch;
   }
+  const int32_t *given = nullptr;
+  if (C > 0 && ball_order_pays(B, M, N) &&
+      scratch_bytes >= tk3d_sa_group_scratch_bytes(B, C, N, M, K, dtype)) {
+    char *order = (char *)scratch + sa_align(rows_scratch_bytes(B, C, N));
+    int32_t *lists = index32 ? index32 : reinterpret_cast<int32_t *>(order + sp_search_bytes(B, M, N));
+    int rc = sp_ball_query((const float *)centroids, (const float *)points, B, M, N, xyz_channel_first, radius * radius,
+                           (int)K, lists, 1, order, st);
+    if (rc) return rc;
+    given = lists;
+  }
   const int vec = C > 0 && C % 4 == 0 && K % 4 == 0 &&
                   ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
   const SaSmem sm = sa_smem((int)C, (int)K, vec);
@@ -387,11 +413,11 @@ extern "C" int tk3d_sa_group_fwd(const void *points, const void *centroids, cons
   if (wide)
     sa_group_fwd_kernel<8><<<grid, 256, sm.total, st>>>(
         (const float *)points, (const float *)centroids, featT, B, (int)C, (int)N, (int)M, pps, pcs, cps, cpc, r2,
-        (int)K, use_xyz ? 1 : 0, vec, (float *)out, index32, status, total);
+        (int)K, use_xyz ? 1 : 0, vec, (float *)out, given, given ? nullptr : index32, status, total);
   else
     sa_group_fwd_kernel<4><<<grid, 128, sm.total, st>>>(
         (const float *)points, (const float *)centroids, featT, B, (int)C, (int)N, (int)M, pps, pcs, cps, cpc, r2,
-        (int)K, use_xyz ? 1 : 0, vec, (float *)out, index32, status, total);
+        (int)K, use_xyz ? 1 : 0, vec, (float *)out, given, given ? nullptr : index32, status, total);
   return check_launch("sa_group_fwd_kernel");
 }
 

@@ -24,9 +24,19 @@ struct SpPair {
   SpCloud c[2];
 };
 
+// A ball query's radius and row length (k = 0: another search).  Where balls hold more than about twice
+// the wanted hits, sweeping the keys in index order stops early and ordering them is wasted: the sort
+// looks at 16 queries and 512 keys of its cloud pair first (every block at the same ones) and flags
+// such a pair as irregular.  32 x 1024 queries of 8192 keys, k = 32, 20 / 100 / 1000 hits, us: sweep 137,
+// 95, 29; ordered 72, 171, 145.
+struct SpPeek {
+  float r2;
+  int k;
+};
+
 template <int CL>
 __global__ void __launch_bounds__(SB_THREADS, 2)
-spatial_sort_kernel(const __grid_constant__ SpPair pair, int B) {
+spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
   constexpr int SHARE = SP_CELLS / CL;      // cells of one block
   constexpr int MINE = SHARE / SB_THREADS;  // cells of one thread
   static_assert(MINE >= 1 && MINE * CL * SB_THREADS == SP_CELLS, "whole cells per thread");
@@ -54,6 +64,31 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B) {
   float4 *pts = reinterpret_cast<float4 *>(c.pts) + b * (int64_t)c.windows * SP_WINDOW;
   const int NL = (N + CL - 1) / CL;
   const int beg = min(N, rank * NL), end = min(N, beg + NL);
+
+  if (peek.k > 0) {
+    const SpCloud &qc = pair.c[0], &kc = pair.c[1];
+    float kx, ky, kz;
+    load_xyz(kc.xyz + b * 3 * (int64_t)kc.N, (int64_t)tid * kc.N / SB_THREADS, kc.l, kx, ky, kz);
+    int hits = 0;
+#pragma unroll 4
+    for (int i = 0; i < 16; ++i) {
+      float x, y, z;
+      load_xyz(qc.xyz + b * 3 * (int64_t)qc.N, (int64_t)i * qc.N / 16, qc.l, x, y, z);
+      hits += sqdist<float>(kx, ky, kz, x, y, z) < peek.r2 ? 1 : 0;
+    }
+    hits = __reduce_add_sync(0xffffffffu, hits);
+    if (lane == 0) warp_total[warp] = hits;
+    __syncthreads();
+    hits = 0;
+#pragma unroll
+    for (int w = 0; w < SB_WARPS; ++w) hits += warp_total[w];
+    // hits per query = hits * N2 / (16 * 512)
+    if ((double)hits * kc.N > 2.0 * 16 * SB_THREADS * peek.k) {  // the same in all blocks of the cluster
+      if (rank == 0 && tid == 0) c.grid[b].irregular = 1;
+      return;
+    }
+    __syncthreads();
+  }
 
 #pragma unroll
   for (int e = 0; e < SP_CELLS / SB_THREADS; ++e) hist[tid + e * SB_THREADS] = 0;
@@ -180,6 +215,7 @@ spatial_window_kernel(const __grid_constant__ SpPair pair, int64_t windows0, int
   const SpCloud &c = pair.c[w >= windows0];
   if (w >= windows0) w -= windows0;
   const SpGrid g = c.grid[w / c.windows];
+  if (g.irregular) return;  // no search looks at it
   float4 *p = reinterpret_cast<float4 *>(c.pts) + w * SP_WINDOW;
   unsigned key[8];
 #pragma unroll
@@ -472,7 +508,7 @@ spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sum
 
 }  // namespace
 
-int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st) {
+int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st, float r2, int k) {
   const int64_t clouds = b ? 2 * B : B;
   const int big = b && b->N > a.N ? b->N : a.N;
   // Blocks per cloud: as many as the SMs hold at once (two each), at least 512 points per block.
@@ -497,7 +533,8 @@ int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void *args[] = {&pair, &B_};
+  SpPeek peek{r2, k};
+  void *args[] = {&pair, &B_, &peek};
   TK3D_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
   const int64_t w0 = B * a.windows, total = w0 + (b ? B * b->windows : 0);
   const int64_t per = SW_THREADS / 32;

@@ -1,5 +1,6 @@
 // Spatially ordered copy of a batch of point clouds: the index that the pruned neighbour searches
-// walk (spatial.cu: build and up to four nearest neighbours, spatial_knn.cu: up to 64).
+// walk (spatial.cu: build and up to four nearest neighbours, spatial_knn.cu: up to 64,
+// spatial_ball.cu: ball query).
 //
 // The points of a cloud are ordered along a Hilbert curve: by one of 4096 cells (16 per axis), and
 // within WINDOWS of 256 points by one of 256 cells per axis.  Eight consecutive points form a LEAF, a
@@ -24,7 +25,7 @@
 // What the index cannot serve is flagged per cloud (SpGrid::irregular): non-finite coordinates
 // (their ordering rules belong to the sweeping kernels), and clouds of which more than half sit in
 // cells of more than SP_CROWD points (duplicates, or an outlier that stretches the grid), where boxes
-// prune little.  The searches skip flagged clouds and the sweeping kernels, launched behind them,
+// prune little; a ball query also flags pairs of clouds whose balls are dense.  The searches skip flagged clouds and the sweeping kernels, launched behind them,
 // skip all others.
 #pragma once
 
@@ -103,8 +104,9 @@ inline char *sp_align_ptr(void *p) {
   return reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 255) & ~(uintptr_t)255);
 }
 
-// Builds the index of both sides (two launches); `b` may be null.
-int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st);
+// Builds the index of both sides (two launches); `b` may be null.  r2, k: of a ball query of a's points in
+// b's (k = 0: another search); pairs of clouds with dense balls are flagged irregular.
+int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st, float r2 = 0.f, int k = 0);
 
 // Searches over built indexes; rows of clouds that are irregular on either side are left alone.
 int sp_chamfer(const SpCloud &a, const SpCloud &b, int64_t B, float *dist1, int64_t *idx1, float *dist2, int64_t *idx2,
@@ -112,6 +114,8 @@ int sp_chamfer(const SpCloud &a, const SpCloud &b, int64_t B, float *dist1, int6
 int sp_knn_small(const SpCloud &q, const SpCloud &k, int64_t B, int K, bool weights, float eps, float *dist,
                  IndexOut index, cudaStream_t st);
 int sp_knn_select(const SpCloud &q, const SpCloud &k, int64_t B, int K, float *dist, IndexOut index, cudaStream_t st);
+int sp_ball_query(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, int channel_first, float r2,
+                  int k, void *index, int index32, void *scratch, cudaStream_t st);
 constexpr int64_t SP_SELECT_POINTS = 1 << 19;  // keys at most: leaf numbers are kept in 16 bits
 
 // For the sweeping kernels launched behind a search: the grids of the two sides, null for a launch on its own.
