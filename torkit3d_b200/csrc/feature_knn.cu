@@ -9,14 +9,18 @@
 // FP32 instructions per pair and channel -- and needs no tensor cores at DGCNN's sizes: 32 clouds
 // of 1024 points with 64 channels are 4.3 GFLOP.)
 //
-// A block of 8 warps owns 32 queries; warp w owns queries 4w .. 4w+3 and, for every tile of 128
-// keys, lane l holds the 4 x 4 distances of those queries to keys l, l+32, l+64, l+96 in registers
-// (channel slices of 16 are staged in shared memory: one broadcast LDS.128 for the queries and
-// four conflict-free LDS.32 for the keys feed 16 subtractions and 16 FMAs).  The same warp then
-// selects: each query's k best so far form a list sorted by (distance, index) that is spread over
-// the warp's registers (entry m lives in lane m % 32, slot m / 32); candidates that order before
-// the k-th entry are found with a ballot and inserted one at a time with a rank count (ballot +
-// popc) and a one-lane shift (shfl_up).  Ties go to the lower index; rows come out sorted.
+// Every warp owns four queries; the eight warps of a block share tiles of 256 keys, staged 16 channels at
+// a time with asynchronous copies into two buffers.  Lane l holds the 4 x 8 distances of its queries to
+// keys 2l, 2l + 1 of each 64 in registers and advances two keys per packed operation (eight queries per
+// warp halve the loads per operation, but leave 16 warps on an SM, and were 10 % slower).
+// Selection: distances that can enter a query's list are appended to a 64-entry buffer in shared
+// memory; 32 of them at a time are sorted across the warp's lanes (bitonic, on the 64-bit word of
+// distance bits and index) and merged with the list.  A list of 32 * KS entries is kept sorted; a block
+// of 32 new entries first meets the topmost 32, of which the lower half stays, and the exchange then
+// goes down the list.  Ties go to the lower index; rows come out sorted.
+//
+// 32 x 1024 x 1024, 64 channels, k = 20: 0.232 ms; one key per lane and one candidate at a time into the
+// list took 0.400 ms.  Half of the issue slots are the packed operations, the rest mostly selection.
 #include <limits.h>
 
 #include "tk3d_common.cuh"
@@ -25,161 +29,222 @@ namespace tk3d {
 namespace {
 
 constexpr int FK_THREADS = 256;
-constexpr int FK_QT = 32;   // queries per block
-constexpr int FK_KT = 128;  // keys per tile
+constexpr int FK_WARPS = FK_THREADS / 32;
+constexpr int FK_QW = 4;    // queries per warp
+constexpr int FK_KT = 256;  // keys per tile
 constexpr int FK_CS = 16;   // channels per slice
+constexpr int FK_BUF = 64;  // buffered candidates per query: fewer than 32, and up to 32 more
 constexpr unsigned FULL = 0xffffffffu;
 
-__device__ __forceinline__ bool before(float d, int i, float e, int j) { return d < e || (d == e && i < j); }
+using u64 = unsigned long long;
 
-// KS: list slots per lane (capacity 32 * KS >= k).  CF: channel-first tensors [B, C, N], otherwise
-// point-major [B, N, C].
-template <int KS, bool CF>
+template <int KS>
+struct FkSmem {
+  float k[2][FK_CS][FK_KT];
+  float q[2][FK_CS][FK_QW * FK_WARPS];
+  u64 buf[FK_QW * FK_WARPS][FK_BUF];
+  u64 list[FK_QW * FK_WARPS][32 * KS];
+};
+
+// BYTES (4 or 16) bytes, or zeros where the source does not exist.
+template <int BYTES>
+__device__ __forceinline__ void fk_copy(float *dst, const float *src, bool there) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "n"(BYTES), "r"(there ? BYTES : 0)
+               : "memory");
+}
+
+__device__ __forceinline__ u64 fk_exchange(u64 v, int o, bool low) {
+  const u64 w = __shfl_xor_sync(FULL, v, o);
+  return (w < v) == low ? w : v;
+}
+// Sorts a bitonic sequence over the lanes.
+__device__ __forceinline__ u64 fk_merge(u64 v, int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fk_exchange(v, o, (lane & o) == 0);
+  return v;
+}
+__device__ __forceinline__ u64 fk_sort(u64 v, int lane) {
+#pragma unroll
+  for (int n = 2; n <= 32; n <<= 1)
+#pragma unroll
+    for (int o = n >> 1; o > 0; o >>= 1) v = fk_exchange(v, o, ((lane & o) == 0) == ((lane & n) == 0));
+  return v;
+}
+
+// Takes the first 32 buffered candidates (of `n`) into the list; returns the list's k-th entry.
+template <int KS>
+__device__ __noinline__ u64 fk_flush(u64 *buf, u64 *list, int n, int k, int lane) {
+  const u64 none = 0x7f8000007fffffffull;  // (+inf, INT_MAX): orders after every real entry
+  __syncwarp();
+  u64 v = fk_sort(lane < n ? buf[lane] : none, lane);
+  if (lane + 32 < n) buf[lane] = buf[lane + 32];
+  v = __shfl_xor_sync(FULL, v, 31);  // descending, against the ascending list
+  const u64 top = list[32 * (KS - 1) + lane];
+  v = fk_merge(v < top ? v : top, lane);
+#pragma unroll
+  for (int s = KS - 2; s >= 0; --s) {
+    const u64 up = __shfl_xor_sync(FULL, v, 31), mine = list[32 * s + lane];
+    list[32 * (s + 1) + lane] = fk_merge(up < mine ? mine : up, lane);
+    v = fk_merge(up < mine ? up : mine, lane);
+  }
+  list[lane] = v;
+  __syncwarp();
+  return list[k - 1];
+}
+
+// KS: list capacity 32 * KS >= k.  LAYOUT: point-major tensors [B, N, C], or channel-first [B, C, N]
+// copied by four bytes, or by sixteen (N1 and N2 multiples of four, 16-byte aligned tensors).
+enum { FK_POINTS = 0, FK_CHANNELS = 1, FK_CHANNELS16 = 2 };
+
+template <int KS, int LAYOUT>
 __global__ void __launch_bounds__(FK_THREADS, KS <= 2 ? 3 : 2)
 feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ key, int C, int N1, int N2, int k,
                    float *__restrict__ dist, int64_t *__restrict__ index, int64_t blocks_total) {
-  __shared__ __align__(16) float qs[FK_CS][FK_QT];
-  __shared__ float ks[FK_CS][FK_KT + 1];  // + 1: the point-major staging stores spread over the banks
+  extern __shared__ __align__(16) unsigned char fk_smem[];
+  constexpr int QW = FK_QW, V = LAYOUT == FK_CHANNELS16 ? 4 : 1;
+  constexpr bool CF = LAYOUT != FK_POINTS;
+  FkSmem<KS> &sm = *reinterpret_cast<FkSmem<KS> *>(fk_smem);
+  constexpr int QT = QW * FK_WARPS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int chunks = (N1 + FK_QT - 1) / FK_QT;
+  const int chunks = (N1 + QT - 1) / QT;
+  const int slices = (C + FK_CS - 1) / FK_CS;
   const float pinf = __int_as_float(0x7f800000);
-  const int kslot = (k - 1) >> 5, klane = (k - 1) & 31;
 
   for (int64_t blk = blockIdx.x; blk < blocks_total; blk += gridDim.x) {
     const int64_t b = blk / chunks;
-    const int q0 = (int)(blk % chunks) * FK_QT;
+    const int q0 = (int)(blk % chunks) * QT;
     const float *qb = query + b * (int64_t)C * N1;
     const float *kb = key + b * (int64_t)C * N2;
-
-    float ld[4][KS], thd[4];
-    int li[4][KS], thi[4];
+    // slice `s` of the tile at key j0 goes to buffer `to`
+    auto stage = [&](int j0, int s, int to) {
+      const int c0 = s * FK_CS;
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
+      for (int r = 0; r < (FK_CS * QT / V + FK_THREADS - 1) / FK_THREADS; ++r) {
+        const int e = (tid + r * FK_THREADS) * V;
+        if (FK_CS * QT / V < FK_THREADS && e >= FK_CS * QT) break;
+        const int c = CF ? e / QT : e % FK_CS, i = CF ? e % QT : e / FK_CS;
+        const bool there = c0 + c < C && q0 + i < N1;
+        const int64_t off = CF ? (int64_t)(c0 + c) * N1 + q0 + i : (int64_t)(q0 + i) * C + c0 + c;
+        fk_copy<4 * V>(&sm.q[to][c][i], qb + (there ? off : 0), there);
+      }
+#pragma unroll
+      for (int r = 0; r < FK_CS * FK_KT / V / FK_THREADS; ++r) {
+        const int e = (tid + r * FK_THREADS) * V;
+        const int c = CF ? e / FK_KT : e % FK_CS, j = CF ? e % FK_KT : e / FK_CS;
+        const bool there = c0 + c < C && j0 + j < N2;
+        const int64_t off = CF ? (int64_t)(c0 + c) * N2 + j0 + j : (int64_t)(j0 + j) * C + c0 + c;
+        fk_copy<4 * V>(&sm.k[to][c][j], kb + (there ? off : 0), there);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    float thd[QW];
+    int thi[QW], cnt[QW];
+#pragma unroll
+    for (int a = 0; a < QW; ++a) {
       thd[a] = pinf;
       thi[a] = INT_MAX;
+      cnt[a] = 0;
 #pragma unroll
-      for (int s = 0; s < KS; ++s) {
-        ld[a][s] = pinf;
-        li[a][s] = INT_MAX;  // sentinel: orders after every real (distance, index)
-      }
+      for (int s = 0; s < KS; ++s) sm.list[warp * QW + a][32 * s + lane] = 0x7f8000007fffffffull;
     }
 
+    stage(0, 0, 0);
+    int at = 0;
     for (int j0 = 0; j0 < N2; j0 += FK_KT) {
-      float acc[4][4];
+      float2 acc[QW][4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < QW; ++a)
 #pragma unroll
-        for (int bb = 0; bb < 4; ++bb) acc[a][bb] = 0.f;
+        for (int p = 0; p < 4; ++p) acc[a][p] = make_float2(0.f, 0.f);
 
-      for (int c0 = 0; c0 < C; c0 += FK_CS) {
-        __syncthreads();  // the previous slice has been consumed
-#pragma unroll
-        for (int r = 0; r < FK_CS * FK_QT / FK_THREADS; ++r) {
-          const int e = tid + r * FK_THREADS;
-          const int c = CF ? e / FK_QT : e % FK_CS, i = CF ? e % FK_QT : e / FK_CS;
-          float v = 0.f;  // channels past C and queries past N1 read as zero on both sides
-          if (c0 + c < C && q0 + i < N1)
-            v = CF ? qb[(int64_t)(c0 + c) * N1 + q0 + i] : qb[(int64_t)(q0 + i) * C + c0 + c];
-          qs[c][i] = v;
-        }
-#pragma unroll
-        for (int r = 0; r < FK_CS * FK_KT / FK_THREADS; ++r) {
-          const int e = tid + r * FK_THREADS;
-          const int c = CF ? e / FK_KT : e % FK_CS, j = CF ? e % FK_KT : e / FK_CS;
-          float v = 0.f;
-          if (c0 + c < C && j0 + j < N2)
-            v = CF ? kb[(int64_t)(c0 + c) * N2 + j0 + j] : kb[(int64_t)(j0 + j) * C + c0 + c];
-          ks[c][j] = v;
-        }
-        __syncthreads();
-#pragma unroll
+      for (int s = 0; s < slices; ++s, at ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // this slice has landed, and the other buffer has been consumed
+        if (s + 1 < slices) stage(j0, s + 1, at ^ 1);
+        else if (j0 + FK_KT < N2) stage(j0 + FK_KT, 0, at ^ 1);
+#pragma unroll 2
         for (int c = 0; c < FK_CS; ++c) {
-          const float4 qv = *reinterpret_cast<const float4 *>(&qs[c][4 * warp]);
-          const float q[4] = {qv.x, qv.y, qv.z, qv.w};
+          float2 kv[4];
 #pragma unroll
-          for (int bb = 0; bb < 4; ++bb) {
-            const float kv = ks[c][lane + 32 * bb];
+          for (int p = 0; p < 4; ++p) kv[p] = *reinterpret_cast<const float2 *>(&sm.k[at][c][64 * p + 2 * lane]);
+#pragma unroll
+          for (int a0 = 0; a0 < QW; a0 += 4) {
+            const float4 qv = *reinterpret_cast<const float4 *>(&sm.q[at][c][warp * QW + a0]);
+            const float q[4] = {-qv.x, -qv.y, -qv.z, -qv.w};
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-              const float df = __fsub_rn(kv, q[a]);
-              acc[a][bb] = __fmaf_rn(df, df, acc[a][bb]);
+              const float2 q2 = make_float2(q[a], q[a]);
+#pragma unroll
+              for (int p = 0; p < 4; ++p) {
+                const float2 df = __fadd2_rn(kv[p], q2);
+                acc[a0 + a][p] = __ffma2_rn(df, df, acc[a0 + a][p]);
+              }
             }
           }
         }
       }
 
-      // Selection: this warp's four queries against the 128 keys of the tile.
+      // Selection: this warp's queries against the 256 keys of the tile.
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
+      for (int a = 0; a < QW; ++a) {
+        u64 *buf = sm.buf[warp * QW + a], *list = sm.list[warp * QW + a];
 #pragma unroll
-        for (int bb = 0; bb < 4; ++bb) {
-          const int j = j0 + lane + 32 * bb;
-          const float d = j < N2 ? acc[a][bb] : pinf;
-          const int id = j < N2 ? j : INT_MAX;
-          unsigned mask = __ballot_sync(FULL, before(d, id, thd[a], thi[a]));
-          while (mask) {
-            const int src = __ffs(mask) - 1;
-            mask &= mask - 1;
-            const float cd = __shfl_sync(FULL, d, src);
-            const int ci = __shfl_sync(FULL, id, src);
-            if (!before(cd, ci, thd[a], thi[a])) continue;  // the k-th entry moved since the ballot
-            int pos = 0;                                     // entries that order before the candidate
-#pragma unroll
-            for (int s = 0; s < KS; ++s) pos += __popc(__ballot_sync(FULL, before(ld[a][s], li[a][s], cd, ci)));
-#pragma unroll
-            for (int s = KS - 1; s >= 0; --s) {  // top slot first: lower slots still hold the old entries
-              float ud = __shfl_up_sync(FULL, ld[a][s], 1);
-              int ui = __shfl_up_sync(FULL, li[a][s], 1);
-              if (s > 0) {
-                const float wd = __shfl_sync(FULL, ld[a][s - 1], 31);
-                const int wi = __shfl_sync(FULL, li[a][s - 1], 31);
-                if (lane == 0) ud = wd, ui = wi;
-              }
-              const int m = lane + 32 * s;
-              if (m == pos) ld[a][s] = cd, li[a][s] = ci;
-              else if (m > pos) ld[a][s] = ud, li[a][s] = ui;
-            }
-            float td = ld[a][0];
-            int ti = li[a][0];
-#pragma unroll
-            for (int s = 1; s < KS; ++s)
-              if (s == kslot) td = ld[a][s], ti = li[a][s];
-            thd[a] = __shfl_sync(FULL, td, klane);
-            thi[a] = __shfl_sync(FULL, ti, klane);
+        for (int e = 0; e < 8; ++e) {
+          const int j = j0 + 64 * (e >> 1) + 2 * lane + (e & 1);
+          const float d = (e & 1) ? acc[a][e >> 1].y : acc[a][e >> 1].x;
+          const bool in = j < N2 && (d < thd[a] || (d == thd[a] && j < thi[a]));
+          const unsigned mask = __ballot_sync(FULL, in);
+          if (mask == 0) continue;
+          if (in)
+            buf[cnt[a] + __popc(mask & ((1u << lane) - 1u))] =
+                ((u64)__float_as_uint(d) << 32) | (unsigned)j;  // d >= +0: the bits order like the value
+          cnt[a] += __popc(mask);
+          if (cnt[a] >= 32) {
+            const u64 last = fk_flush<KS>(buf, list, cnt[a], k, lane);
+            cnt[a] -= 32;
+            thd[a] = __uint_as_float((unsigned)(last >> 32));
+            thi[a] = (int)(unsigned)last;
           }
         }
       }
     }
 
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int qi = q0 + 4 * warp + a;
+    for (int a = 0; a < QW; ++a) {
+      const int qi = q0 + warp * QW + a;
       if (qi < N1) {
+        u64 *list = sm.list[warp * QW + a];
+        if (cnt[a] > 0) fk_flush<KS>(sm.buf[warp * QW + a], list, cnt[a], k, lane);
         float *od = dist + (b * N1 + qi) * (int64_t)k;
         int64_t *oi = index + (b * N1 + qi) * (int64_t)k;
-#pragma unroll
-        for (int s = 0; s < KS; ++s) {
-          const int m = lane + 32 * s;
-          if (m < k) {
-            od[m] = ld[a][s];
-            oi[m] = li[a][s] == INT_MAX ? (int64_t)-1 : (int64_t)li[a][s];  // only with NaN inputs
-          }
+        for (int m = lane; m < k; m += 32) {
+          const u64 v = list[m];
+          od[m] = __uint_as_float((unsigned)(v >> 32));
+          oi[m] = (unsigned)v == 0x7fffffffu ? (int64_t)-1 : (int64_t)(unsigned)v;  // only with NaN inputs
         }
       }
     }
+    __syncthreads();  // the next task's first slice may land in a buffer that a slower warp still reads
   }
 }
 
 template <int KS>
 int launch(const float *query, const float *key, int64_t B, int C, int N1, int N2, int k, bool cf, float *dist,
            int64_t *index, cudaStream_t st) {
-  const int64_t total = B * ((N1 + FK_QT - 1) / FK_QT);
+  constexpr int QT = FK_QW * FK_WARPS;
+  const int64_t total = B * ((N1 + QT - 1) / QT);
   const int64_t cap = (int64_t)sm_count() * 32;
   const unsigned grid = (unsigned)(total < cap ? total : cap);
-  if (cf)
-    feature_knn_kernel<KS, true><<<grid, FK_THREADS, 0, st>>>(query, key, C, N1, N2, k, dist, index, total);
-  else
-    feature_knn_kernel<KS, false><<<grid, FK_THREADS, 0, st>>>(query, key, C, N1, N2, k, dist, index, total);
+  const size_t smem = sizeof(FkSmem<KS>);
+  const bool wide = N1 % 4 == 0 && N2 % 4 == 0 &&
+                    ((reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(key)) & 15) == 0;
+  auto kern = !cf    ? feature_knn_kernel<KS, FK_POINTS>
+              : wide ? feature_knn_kernel<KS, FK_CHANNELS16>
+                     : feature_knn_kernel<KS, FK_CHANNELS>;
+  TK3D_CUDA(raise_smem_limit((const void *)kern, (int)smem));
+  kern<<<grid, FK_THREADS, smem, st>>>(query, key, C, N1, N2, k, dist, index, total);
   return check_launch("feature_knn_kernel");
 }
 
