@@ -29,26 +29,37 @@ constexpr int FC_MAX_CL = 16;  // 8 is the portable cluster size; 16 needs an op
 
 // ---------------------------------------------------------------------------------------------
 // No block or cluster barrier in the step.  Every WARP finds its own farthest point (two REDUX)
-// and sends it -- 20 bytes: distance bits, index, coordinates -- straight into the shared memory of
-// every block of the cluster with st.async, which also counts the bytes on an mbarrier of the
-// receiving block.  A warp then waits on its own block's mbarrier until the candidates of all
-// warps of the cluster have landed, and lane l looks at candidates l, l + 32, ...: two more REDUX
-// pick the winner (highest distance, lowest index), the same in every warp.  The candidate slots
-// and mbarriers are double buffered by the step's parity: a warp can send for step i+2 only after
-// it has seen every warp's candidate of step i+1, which those warps send after they have read
-// step i.  The fewer warps a cluster has the shorter the step (its floor is the exchange over
-// distributed shared memory, about 0.45 us), hence up to 32 points per thread.  Every wait is
-// limited (limit_ns: one second in regular calls); a warp that runs into the limit stops, the
-// rest of its cloud's index row is set to -1, fw_expired_waits counts it, and every block still
-// leaves through the final cluster barrier.
+// and sends it -- 24 bytes: distance bits, index, coordinates, and a bound on what its other points
+// could be worth -- straight into the shared memory of every block of the cluster with st.async, which
+// also counts the bytes on an mbarrier of the receiving block.  A warp then waits on its own block's
+// mbarrier until the candidates of all warps of the cluster have landed.
+//
+// One exchange yields several samples.  The bound is the largest running minimum among the warp's
+// points after its own candidate would have been sampled.  With the candidates in hand every warp
+// goes through the samples that follow, all warps the same: the farthest remaining candidate (lowest
+// index among equals) is the next sample as long as (a) it lies strictly above the bounds of the
+// warps whose candidates have been taken, and (b) none of the samples taken since the exchange came
+// closer to it than its running minimum.  Nothing else can be farther: a warp whose candidate has not
+// been taken has no point above it.  The first candidate always passes, so the sequence is the one
+// of single steps, bit for bit.  Counted on the CPU, an exchange yields 3.5 to 4.3 samples; it costs
+// 0.45 us and more, a sample taken from it about 0.15 us.
+//
+// The candidate slots and mbarriers are double buffered by the parity of the exchange: a warp can send
+// for exchange i+2 only after it has seen every warp's candidate of exchange i+1, which those warps
+// send after they are done with exchange i.  The fewer warps a cluster has the shorter the exchange,
+// hence up to 32 points per thread.  Every wait is limited (limit_ns: one second in regular calls); a
+// warp that runs into the limit stops, the rest of its cloud's index row is set to -1,
+// fw_expired_waits counts it, and every block still leaves through the final cluster barrier.
 struct __align__(16) FwCandidate {
   unsigned bits;
   int idx;
   float x, y;
   float z;
-  int pad[3];
+  unsigned rest;  // bits of the bound on the warp's other points
+  int pad[2];
 };
-constexpr unsigned FW_CAND_BYTES = 20;
+constexpr unsigned FW_CAND_BYTES = 24;
+constexpr int FW_BATCH = 16;  // samples of one exchange, at most 32
 
 __device__ __forceinline__ unsigned fw_smem(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned fw_mapa(unsigned addr, unsigned rank) {
@@ -158,31 +169,45 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
   const unsigned rbar0 = fw_mapa(bar0, tgt), rbar1 = fw_mapa(bar1, tgt);
 
   const float2 one2 = make_float2(one, one);
-  bool failed = false;
-  int it = 1;
-  for (; it < S; ++it) {
-    const int par = it & 1;
-    const float2 ncx = make_float2(-cx, -cx), ncy = make_float2(-cy, -cy), ncz = make_float2(-cz, -cz);
-    float bm = 0.f;
+  // Point pairs of this thread: coordinates from registers or the block's copy.
+  auto pair = [&](int i, float2 &qx_, float2 &qy_, float2 &qz_) {
+    if constexpr (FW_REGS) {
+      qx_ = px[i];
+      qy_ = py[i];
+      qz_ = pz[i];
+    } else {
+      const float *a0 = sxyz + 3 * ((2 * i) * T + tid), *a1 = sxyz + 3 * ((2 * i + 1) * T + tid);
+      qx_ = make_float2(a0[0], a1[0]);
+      qy_ = make_float2(a0[1], a1[1]);
+      qz_ = make_float2(a0[2], a1[2]);
+    }
+  };
+  // Exact squared distances of a pair to (x, y, z), given as (-x, -x) ...
+  auto dist2 = [&](int i, float2 nx, float2 ny, float2 nz) {
+    float2 qx_, qy_, qz_;
+    pair(i, qx_, qy_, qz_);
+    const float2 dx = __fadd2_rn(qx_, nx), dy = __fadd2_rn(qy_, ny), dz = __fadd2_rn(qz_, nz);
+    return __ffma2_rn(__ffma2_rn(__fmul2_rn(dx, dx), one2, __fmul2_rn(dy, dy)), one2, __fmul2_rn(dz, dz));
+  };
+  auto apply = [&](float x, float y, float z) {
+    const float2 nx = make_float2(-x, -x), ny = make_float2(-y, -y), nz = make_float2(-z, -z);
 #pragma unroll
     for (int i = 0; i < FW_P2; ++i) {
-      float2 qx_, qy_, qz_;
-      if constexpr (FW_REGS) {
-        qx_ = px[i];
-        qy_ = py[i];
-        qz_ = pz[i];
-      } else {
-        const float *a0 = sxyz + 3 * ((2 * i) * T + tid), *a1 = sxyz + 3 * ((2 * i + 1) * T + tid);
-        qx_ = make_float2(a0[0], a1[0]);
-        qy_ = make_float2(a0[1], a1[1]);
-        qz_ = make_float2(a0[2], a1[2]);
-      }
-      const float2 dx = __fadd2_rn(qx_, ncx), dy = __fadd2_rn(qy_, ncy), dz = __fadd2_rn(qz_, ncz);
-      const float2 d = __ffma2_rn(__ffma2_rn(__fmul2_rn(dx, dx), one2, __fmul2_rn(dy, dy)), one2, __fmul2_rn(dz, dz));
+      const float2 d = dist2(i, nx, ny, nz);
       md[i].x = fminf(md[i].x, d.x);
       md[i].y = fminf(md[i].y, d.y);
-      asm("max.f32 %0, %0, %1, %2;" : "+f"(bm) : "f"(md[i].x), "f"(md[i].y));
     }
+  };
+  apply(cx, cy, cz);  // sample 0
+
+  constexpr int CPL = FW_SLOTS / 32;  // candidates of a lane
+  bool failed = false;
+  int n = 1;  // samples so far
+  for (int ex = 1; n < S; ++ex) {
+    const int par = ex & 1;
+    float bm = 0.f;
+#pragma unroll
+    for (int i = 0; i < FW_P2; ++i) asm("max.f32 %0, %0, %1, %2;" : "+f"(bm) : "f"(md[i].x), "f"(md[i].y));
     const unsigned bits = __float_as_uint(bm);
     const unsigned gb = __reduce_max_sync(0xffffffffu, bits);
     int mine = 0x7fffffff;
@@ -194,21 +219,34 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       }
     }
     const int loc = __reduce_min_sync(0xffffffffu, mine);  // lowest local index holding the warp's maximum
-    if (lane < CL && !(it == drop_step && gw == 0)) {  // drop_step: diagnostic only, -1 otherwise
-      const bool real = loc < nloc;
-      const float x = real ? sxyz[3 * loc + 0] : 0.f, y = real ? sxyz[3 * loc + 1] : 0.f,
-                  z = real ? sxyz[3 * loc + 2] : 0.f;
+    const bool real = loc < nloc;
+    const float x = real ? sxyz[3 * loc + 0] : 0.f, y = real ? sxyz[3 * loc + 1] : 0.f,
+                z = real ? sxyz[3 * loc + 2] : 0.f;
+    float rm = 0.f;  // running minima if this candidate were sampled
+    {
+      const float2 nx = make_float2(-x, -x), ny = make_float2(-y, -y), nz = make_float2(-z, -z);
+#pragma unroll
+      for (int i = 0; i < FW_P2; ++i) {
+        const float2 d = dist2(i, nx, ny, nz);
+        asm("max.f32 %0, %0, %1, %2;" : "+f"(rm) : "f"(fminf(md[i].x, d.x)), "f"(fminf(md[i].y, d.y)));
+      }
+    }
+    const unsigned rest = __reduce_max_sync(0xffffffffu, __float_as_uint(rm));
+    // drop_step: diagnostic only (-1 otherwise): warp 0 is silent in the exchange for that sample
+    const int stop = n < drop_step && drop_step < S ? drop_step : S;
+    if (lane < CL && !(n == drop_step && gw == 0)) {
       const unsigned rc = par ? rcand1 : rcand0, rb = par ? rbar1 : rbar0;
       asm volatile(
           "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(rc),
           "r"(gb), "r"(base + loc), "r"(__float_as_uint(x)), "r"(__float_as_uint(y)), "r"(rb)
           : "memory");
-      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(rc + 16),
-                   "r"(__float_as_uint(z)), "r"(rb)
+      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(
+                       rc + 16),
+                   "r"(__float_as_uint(z)), "r"(rest), "r"(rb)
                    : "memory");
     }
     // wait until the candidates of all warps of the cluster have landed in this block
-    const unsigned lb = par ? bar1 : bar0, phase = (unsigned)((it - 1) >> 1) & 1u;
+    const unsigned lb = par ? bar1 : bar0, phase = (unsigned)((ex - 1) >> 1) & 1u;
     unsigned ok = fw_try_wait(lb, phase);
     if (!ok) {  // bounded by time (limit_ns: one second) and by count
       const unsigned long long t0 = fw_now();
@@ -221,46 +259,82 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       failed = true;
       break;
     }
-    // the barrier just completed is used again two steps on
-    if (tid == 0 && it + 2 < S)
+    // the barrier just completed is used again two exchanges on
+    if (tid == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(lb), "r"(expect) : "memory");
-    // lane l looks at candidates l, l + 32, ...: highest distance, then lowest index
-    const bool has = lane < nw;
-    unsigned cb = 0u;
-    int ci = 0x7fffffff, slot = lane;
-    if constexpr (FW_SLOTS <= 32) {
-      cb = has ? cand[par][lane].bits : 0u;
-      ci = has ? cand[par][lane].idx : 0x7fffffff;
-    } else {
-      for (int sl = lane; sl < nw; sl += 32) {
-        const unsigned b_ = cand[par][sl].bits;
-        const int i_ = cand[par][sl].idx;
-        if (b_ > cb || (b_ == cb && i_ < ci)) {
-          cb = b_;
-          ci = i_;
-          slot = sl;
+
+    // lane l holds candidates l, l + 32, ...
+    unsigned cb[CPL];
+    int ci[CPL];
+    float kx[CPL], ky[CPL], kz[CPL];
+    bool reduced[CPL];  // a sample of this exchange lies closer than the candidate's running minimum
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      const int sl = lane + 32 * c;
+      const bool has = sl < nw;
+      cb[c] = has ? cand[par][sl].bits : 0u;
+      ci[c] = has ? cand[par][sl].idx : 0x7fffffff;
+      kx[c] = has ? cand[par][sl].x : 0.f;
+      ky[c] = has ? cand[par][sl].y : 0.f;
+      kz[c] = has ? cand[par][sl].z : 0.f;
+      reduced[c] = false;
+    }
+    unsigned bound = 0u;
+    int taken = 0, where = 0;  // lane j keeps the slot of the j-th sample
+    while (true) {
+      unsigned b_ = cb[0];
+      int i_ = ci[0], slot = lane;
+      bool red = reduced[0];
+#pragma unroll
+      for (int c = 1; c < CPL; ++c) {
+        if (cb[c] > b_ || (cb[c] == b_ && ci[c] < i_)) {
+          b_ = cb[c];
+          i_ = ci[c];
+          slot = lane + 32 * c;
+          red = reduced[c];
         }
       }
+      const unsigned wb = __reduce_max_sync(0xffffffffu, b_);
+      if (taken > 0 && wb <= bound) break;
+      const int wi = __reduce_min_sync(0xffffffffu, b_ == wb ? i_ : 0x7fffffff);
+      const bool owner = b_ == wb && i_ == wi;
+      if (__any_sync(0xffffffffu, owner && red)) break;
+      // (several lanes own it only where all candidates are gone or zero; they agree on index INT_MAX or 0)
+      const int src = __shfl_sync(0xffffffffu, slot, __ffs(__ballot_sync(0xffffffffu, owner)) - 1);
+      cx = cand[par][src].x;
+      cy = cand[par][src].y;
+      cz = cand[par][src].z;
+      bound = max(bound, cand[par][src].rest);
+      if (lane == taken) where = src;
+      if (writer) {
+        out[n] = wi;
+        if (sm) {
+          sm[(int64_t)n * sps] = cx;
+          sm[(int64_t)n * sps + scs] = cy;
+          sm[(int64_t)n * sps + 2 * (int64_t)scs] = cz;
+        }
+      }
+      ++n;
+      if (++taken == FW_BATCH || n >= stop) break;
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        if (lane + 32 * c == src) {
+          cb[c] = 0u;
+          ci[c] = 0x7fffffff;
+        }
+        reduced[c] |= sqdist<float>(kx[c], ky[c], kz[c], cx, cy, cz) < __uint_as_float(cb[c]);
+      }
     }
-    const unsigned wb = __reduce_max_sync(0xffffffffu, cb);
-    const int wi = __reduce_min_sync(0xffffffffu, (has && cb == wb) ? ci : 0x7fffffff);
-    int src = __ffs(__ballot_sync(0xffffffffu, has && cb == wb && ci == wi)) - 1;
-    if constexpr (FW_SLOTS > 32) src = __shfl_sync(0xffffffffu, slot, src);
-    cx = cand[par][src].x;
-    cy = cand[par][src].y;
-    cz = cand[par][src].z;
-    if (writer) {
-      out[it] = wi;
-      if (sm) {
-        sm[(int64_t)it * sps] = cx;
-        sm[(int64_t)it * sps + scs] = cy;
-        sm[(int64_t)it * sps + 2 * (int64_t)scs] = cz;
+    if (n < S) {
+      for (int j = 0; j < taken; ++j) {
+        const FwCandidate &w = cand[par][__shfl_sync(0xffffffffu, where, j)];
+        apply(w.x, w.y, w.z);
       }
     }
   }
   if (failed && lane == 0) atomicAdd(&fw_expired_waits, 1u);
   if (failed && rank == 0 && warp == 0 && lane == 0)
-    for (int r = it; r < S; ++r) out[r] = -1;  // a wait ran into its limit: the rest of the row is marked
+    for (int r = n; r < S; ++r) out[r] = -1;  // a wait ran into its limit: the rest of the row is marked
   cluster.sync();  // no block leaves while a candidate may still be on its way into its shared memory
 }
 
@@ -494,12 +568,12 @@ static bool fps_warpcast64_launch(const double *points, int64_t B, int64_t N, in
 template <int THREADS, int P2>
 static bool fps_warpcast_launch(const float *points, int64_t B, int64_t N, int64_t S, int ps, int64_t cs, int64_t *index,
                                 float *sampled, cudaStream_t st, int *rc, int CL, FwWait wt) {
-  if (CL * (THREADS / 32) > 512 || (int64_t)CL * THREADS * 2 * P2 < N) return false;  // a slot per warp, a register per point
-  if (CL * (THREADS / 32) <= 32)
-    return fps_cluster_launch_kernel(fps_warpcast_kernel<THREADS, P2, 32>, THREADS, points, B, N, S, ps, cs, index,
-                                     sampled, st, rc, CL, wt);
-  return fps_cluster_launch_kernel(fps_warpcast_kernel<THREADS, P2, 512>, THREADS, points, B, N, S, ps, cs, index,
-                                   sampled, st, rc, CL, wt);
+  const int warps = CL * (THREADS / 32);
+  if (warps > 128 || (int64_t)CL * THREADS * 2 * P2 < N) return false;  // a slot per warp, a register per point
+  return fps_cluster_launch_kernel(warps <= 32   ? fps_warpcast_kernel<THREADS, P2, 32>
+                                   : warps <= 64 ? fps_warpcast_kernel<THREADS, P2, 64>
+                                                 : fps_warpcast_kernel<THREADS, P2, 128>,
+                                   THREADS, points, B, N, S, ps, cs, index, sampled, st, rc, CL, wt);
 }
 
 // Launches a cluster kernel when the clouds suit one (float32, 4096 < N <= 262144); returns false
