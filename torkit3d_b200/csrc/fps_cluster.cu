@@ -198,16 +198,29 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       md[i].y = fminf(md[i].y, d.y);
     }
   };
-  apply(cx, cy, cz);  // sample 0
+  // The same, returning the thread's largest running minimum.
+  auto apply_max = [&](float x, float y, float z) {
+    const float2 nx = make_float2(-x, -x), ny = make_float2(-y, -y), nz = make_float2(-z, -z);
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < FW_P2; ++i) {
+      const float2 d = dist2(i, nx, ny, nz);
+      md[i].x = fminf(md[i].x, d.x);
+      md[i].y = fminf(md[i].y, d.y);
+      asm("max.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(md[i].x), "f"(md[i].y));
+    }
+    return m;
+  };
+  float bm = apply_max(cx, cy, cz);  // sample 0
 
   constexpr int CPL = FW_SLOTS / 32;  // candidates of a lane
   bool failed = false;
   int n = 1;  // samples so far
+  // Where exchanges keep yielding a single sample (points on a lattice: ties), the bounds are left out
+  // for 48 exchanges at a time; the same in all warps.
+  int again = 0, single = 0;
   for (int ex = 1; n < S; ++ex) {
     const int par = ex & 1;
-    float bm = 0.f;
-#pragma unroll
-    for (int i = 0; i < FW_P2; ++i) asm("max.f32 %0, %0, %1, %2;" : "+f"(bm) : "f"(md[i].x), "f"(md[i].y));
     const unsigned bits = __float_as_uint(bm);
     const unsigned gb = __reduce_max_sync(0xffffffffu, bits);
     int mine = 0x7fffffff;
@@ -222,16 +235,17 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
     const bool real = loc < nloc;
     const float x = real ? sxyz[3 * loc + 0] : 0.f, y = real ? sxyz[3 * loc + 1] : 0.f,
                 z = real ? sxyz[3 * loc + 2] : 0.f;
-    float rm = 0.f;  // running minima if this candidate were sampled
-    {
+    unsigned rest = gb;
+    if (ex >= again) {  // running minima if this candidate were sampled
+      float rm = 0.f;
       const float2 nx = make_float2(-x, -x), ny = make_float2(-y, -y), nz = make_float2(-z, -z);
 #pragma unroll
       for (int i = 0; i < FW_P2; ++i) {
         const float2 d = dist2(i, nx, ny, nz);
         asm("max.f32 %0, %0, %1, %2;" : "+f"(rm) : "f"(fminf(md[i].x, d.x)), "f"(fminf(md[i].y, d.y)));
       }
+      rest = __reduce_max_sync(0xffffffffu, __float_as_uint(rm));
     }
-    const unsigned rest = __reduce_max_sync(0xffffffffu, __float_as_uint(rm));
     // drop_step: diagnostic only (-1 otherwise): warp 0 is silent in the exchange for that sample
     const int stop = n < drop_step && drop_step < S ? drop_step : S;
     if (lane < CL && !(n == drop_step && gw == 0)) {
@@ -272,14 +286,17 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
     for (int c = 0; c < CPL; ++c) {
       const int sl = lane + 32 * c;
       const bool has = sl < nw;
-      cb[c] = has ? cand[par][sl].bits : 0u;
-      ci[c] = has ? cand[par][sl].idx : 0x7fffffff;
-      kx[c] = has ? cand[par][sl].x : 0.f;
-      ky[c] = has ? cand[par][sl].y : 0.f;
-      kz[c] = has ? cand[par][sl].z : 0.f;
+      // whole words: the slots are 32 bytes apart, and single words would meet in four banks
+      const uint4 v = *reinterpret_cast<const uint4 *>(&cand[par][has ? sl : 0]);
+      cb[c] = has ? v.x : 0u;
+      ci[c] = has ? (int)v.y : 0x7fffffff;
+      kx[c] = __uint_as_float(v.z);
+      ky[c] = __uint_as_float(v.w);
+      kz[c] = cand[par][has ? sl : 0].z;
       reduced[c] = false;
     }
     unsigned bound = 0u;
+    unsigned stale = 0u;       // reduced[0] of all lanes
     int taken = 0, where = 0;  // lane j keeps the slot of the j-th sample
     while (true) {
       unsigned b_ = cb[0];
@@ -297,10 +314,15 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       const unsigned wb = __reduce_max_sync(0xffffffffu, b_);
       if (taken > 0 && wb <= bound) break;
       const int wi = __reduce_min_sync(0xffffffffu, b_ == wb ? i_ : 0x7fffffff);
-      const bool owner = b_ == wb && i_ == wi;
-      if (__any_sync(0xffffffffu, owner && red)) break;
-      // (several lanes own it only where all candidates are gone or zero; they agree on index INT_MAX or 0)
-      const int src = __shfl_sync(0xffffffffu, slot, __ffs(__ballot_sync(0xffffffffu, owner)) - 1);
+      // (several lanes own it only where all candidates are gone or zero)
+      const unsigned owners = __ballot_sync(0xffffffffu, b_ == wb && i_ == wi);
+      int src = __ffs(owners) - 1;
+      if constexpr (CPL == 1) {
+        if ((stale >> src) & 1u) break;
+      } else {
+        src = __shfl_sync(0xffffffffu, slot | (red ? 0x10000 : 0), src);
+        if (src & 0x10000) break;
+      }
       cx = cand[par][src].x;
       cy = cand[par][src].y;
       cz = cand[par][src].z;
@@ -315,7 +337,7 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
         }
       }
       ++n;
-      if (++taken == FW_BATCH || n >= stop) break;
+      if (++taken == FW_BATCH || n >= stop || ex < again) break;
 #pragma unroll
       for (int c = 0; c < CPL; ++c) {
         if (lane + 32 * c == src) {
@@ -324,12 +346,21 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
         }
         reduced[c] |= sqdist<float>(kx[c], ky[c], kz[c], cx, cy, cz) < __uint_as_float(cb[c]);
       }
+      if constexpr (CPL == 1) stale = __ballot_sync(0xffffffffu, reduced[0]);
+    }
+    if (ex >= again) {
+      single = taken == 1 ? single + 1 : 0;
+      if (single >= 12) {
+        again = ex + 49;
+        single = 10;
+      }
     }
     if (n < S) {
-      for (int j = 0; j < taken; ++j) {
+      for (int j = 0; j + 1 < taken; ++j) {
         const FwCandidate &w = cand[par][__shfl_sync(0xffffffffu, where, j)];
         apply(w.x, w.y, w.z);
       }
+      bm = apply_max(cx, cy, cz);
     }
   }
   if (failed && lane == 0) atomicAdd(&fw_expired_waits, 1u);
