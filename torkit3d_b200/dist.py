@@ -138,6 +138,11 @@ def _one(device, dtype):
 
 
 # ---- training step without autograd ---------------------------------------------------------------
+def _chamfer_scratch(_lib, B, n1, n2, dt, dev):
+    """Scratch of a chamfer forward; empty where the library sweeps all pairs."""
+    return torch.empty((_lib.scratch_bytes("tk3d_chamfer_fwd", B, n1, n2, dt),), dtype=torch.uint8, device=dev)
+
+
 def chamfer_step(xyz1, xyz2, global_batch=None, group=None, workspace=None):
     """Mean chamfer loss over a batch sharded across ranks AND its gradients, in one call.
 
@@ -177,13 +182,14 @@ def chamfer_step(xyz1, xyz2, global_batch=None, group=None, workspace=None):
             bufs = (torch.empty((B, n1), dtype=a.dtype, device=dev), torch.empty((B, n2), dtype=a.dtype, device=dev),
                     torch.empty((B, n1), dtype=torch.int64, device=dev),
                     torch.empty((B, n2), dtype=torch.int64, device=dev), torch.empty_like(a), torch.empty_like(b),
-                    torch.empty(2, dtype=torch.float64, device=dev), torch.empty((), dtype=a.dtype, device=dev))
+                    torch.empty(2, dtype=torch.float64, device=dev), torch.empty((), dtype=a.dtype, device=dev),
+                    _chamfer_scratch(_lib, B, n1, n2, dt, dev))
             if workspace is not None:
                 workspace[key] = bufs
-        d1, d2, i1, i2, ga, gb, sums, loss = bufs
+        d1, d2, i1, i2, ga, gb, sums, loss, scratch = bufs
         one = _one(dev, a.dtype)
-        _lib.check(lib.tk3d_chamfer_fwd(_ptr(a), _ptr(b), B, n1, n2, _ptr(d1), _ptr(i1), _ptr(d2), _ptr(i2),
-                                        _ptr(sums), dt, st))
+        _lib.check(lib.tk3d_chamfer_fwd_ws(_ptr(a), _ptr(b), B, n1, n2, 0, _ptr(d1), _ptr(i1), _ptr(d2), _ptr(i2),
+                                           _ptr(sums), _ptr(scratch), scratch.numel(), dt, st))
         work = dist.all_reduce(sums, op=dist.ReduceOp.SUM, group=group, async_op=True) if world > 1 else None
         _lib.check(lib.tk3d_chamfer_bwd_mean(_ptr(one), count1, count2, _ptr(a), _ptr(b), _ptr(i1), _ptr(i2), B, n1,
                                              n2, _ptr(ga), _ptr(gb), dt, st))
@@ -255,6 +261,7 @@ def chamfer_step_from_host(xyz1_host, xyz2_host, device, global_batch=None, grou
         ga, gbt = torch.empty_like(a), torch.empty_like(b)
         sums = torch.zeros((nch, 2), dtype=torch.float64, device=dev)  # the kernel overwrites its row
         per = (B + nch - 1) // nch if B > 0 else 0
+        scratch = _chamfer_scratch(_lib, per, n1, n2, _lib.F32, dev)  # the chunks follow one another on one stream
         one = _one(dev, torch.float32)  # upstream gradient of the loss
         copy.wait_stream(compute)  # the buffers above exist before the side stream writes them
         for t in (a, b):
@@ -270,9 +277,10 @@ def chamfer_step_from_host(xyz1_host, xyz2_host, device, global_batch=None, grou
                 ready.record(copy)
             compute.wait_event(ready)
             st = compute.cuda_stream
-            check(lib.tk3d_chamfer_fwd(a[b0:b1].data_ptr(), b[b0:b1].data_ptr(), b1 - b0, n1, n2,
-                                       d1[b0:b1].data_ptr(), i1[b0:b1].data_ptr(), d2[b0:b1].data_ptr(),
-                                       i2[b0:b1].data_ptr(), sums[c].data_ptr(), _lib.F32, st))
+            check(lib.tk3d_chamfer_fwd_ws(a[b0:b1].data_ptr(), b[b0:b1].data_ptr(), b1 - b0, n1, n2, 0,
+                                          d1[b0:b1].data_ptr(), i1[b0:b1].data_ptr(), d2[b0:b1].data_ptr(),
+                                          i2[b0:b1].data_ptr(), sums[c].data_ptr(), scratch.data_ptr(),
+                                          scratch.numel(), _lib.F32, st))
             check(lib.tk3d_chamfer_bwd_mean(one.data_ptr(), count1, count2, a[b0:b1].data_ptr(),
                                             b[b0:b1].data_ptr(), i1[b0:b1].data_ptr(), i2[b0:b1].data_ptr(),
                                             b1 - b0, n1, n2, ga[b0:b1].data_ptr(), gbt[b0:b1].data_ptr(), _lib.F32,
