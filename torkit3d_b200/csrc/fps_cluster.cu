@@ -198,20 +198,14 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       md[i].y = fminf(md[i].y, d.y);
     }
   };
-  // The same, returning the thread's largest running minimum.
-  auto apply_max = [&](float x, float y, float z) {
-    const float2 nx = make_float2(-x, -x), ny = make_float2(-y, -y), nz = make_float2(-z, -z);
+  auto thread_max = [&]() {
     float m = 0.f;
 #pragma unroll
-    for (int i = 0; i < FW_P2; ++i) {
-      const float2 d = dist2(i, nx, ny, nz);
-      md[i].x = fminf(md[i].x, d.x);
-      md[i].y = fminf(md[i].y, d.y);
-      asm("max.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(md[i].x), "f"(md[i].y));
-    }
+    for (int i = 0; i < FW_P2; ++i) asm("max.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(md[i].x), "f"(md[i].y));
     return m;
   };
-  float bm = apply_max(cx, cy, cz);  // sample 0
+  apply(cx, cy, cz);  // sample 0
+  float bm = thread_max();
 
   constexpr int CPL = FW_SLOTS / 32;  // candidates of a lane
   bool failed = false;
@@ -297,7 +291,7 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
     }
     unsigned bound = 0u;
     unsigned stale = 0u;       // reduced[0] of all lanes
-    int taken = 0, where = 0;  // lane j keeps the slot of the j-th sample
+    int taken = 0;
     while (true) {
       unsigned b_ = cb[0];
       int i_ = ci[0], slot = lane;
@@ -327,7 +321,6 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       cy = cand[par][src].y;
       cz = cand[par][src].z;
       bound = max(bound, cand[par][src].rest);
-      if (lane == taken) where = src;
       if (writer) {
         out[n] = wi;
         if (sm) {
@@ -337,7 +330,7 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
         }
       }
       ++n;
-      if (++taken == FW_BATCH || n >= stop || ex < again) break;
+      ++taken;
 #pragma unroll
       for (int c = 0; c < CPL; ++c) {
         if (lane + 32 * c == src) {
@@ -347,6 +340,9 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
         reduced[c] |= sqdist<float>(kx[c], ky[c], kz[c], cx, cy, cz) < __uint_as_float(cb[c]);
       }
       if constexpr (CPL == 1) stale = __ballot_sync(0xffffffffu, reduced[0]);
+      // in the shadow of the next pick's reductions
+      apply(cx, cy, cz);
+      if (taken == FW_BATCH || n >= stop || ex < again) break;
     }
     if (ex >= again) {
       single = taken == 1 ? single + 1 : 0;
@@ -355,13 +351,7 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
         single = 10;
       }
     }
-    if (n < S) {
-      for (int j = 0; j + 1 < taken; ++j) {
-        const FwCandidate &w = cand[par][__shfl_sync(0xffffffffu, where, j)];
-        apply(w.x, w.y, w.z);
-      }
-      bm = apply_max(cx, cy, cz);
-    }
+    bm = thread_max();
   }
   if (failed && lane == 0) atomicAdd(&fw_expired_waits, 1u);
   if (failed && rank == 0 && warp == 0 && lane == 0)
