@@ -1,0 +1,39 @@
+"""Cluster FPS, where one exchange yields several samples: the sequence is the oracle's, index by index.
+
+Sizes cover every cluster shape (one, two and four candidates per lane; coordinates in registers and in
+shared memory); the inputs what ends a batch early: exact ties within and between warps, duplicates whose
+distances run out, a sample next to the following candidate, more samples than one batch holds.
+"""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _cloud(kind, B, N):
+    g = np.random.default_rng(N)
+    if kind == "random":
+        return g.random((B, N, 3), dtype=np.float32)
+    if kind == "lattice":
+        return g.integers(0, 7, (B, N, 3)).astype(np.float32) * np.float32(0.25)
+    if kind == "few":  # 40 distinct points, then only zero distances
+        return g.random((B, 40, 3), dtype=np.float32)[:, g.integers(0, 40, N)]
+    if kind == "far":  # a handful of far points among near ones: long batches, then none
+        p = g.random((B, N, 3), dtype=np.float32) * np.float32(0.01)
+        p[:, ::997] += g.standard_normal((B, len(range(0, N, 997)), 3)).astype(np.float32) * 10
+        return p
+    p = g.random((B, N, 3), dtype=np.float32)  # sorted along x: neighbours share a warp
+    return np.take_along_axis(p, np.argsort(p[..., :1], axis=1, kind="stable"), axis=1)
+
+
+@pytest.mark.parametrize("kind", ["random", "lattice", "few", "far", "sorted"])
+@pytest.mark.parametrize("B,N,S", [(2, 4097, 200), (1, 8192, 300), (2, 8193, 100), (1, 16385, 150), (1, 40000, 90),
+                                   (1, 65537, 90), (1, 131073, 60)])
+def test_sequence(oracle, kind, B, N, S):
+    from torkit3d_b200.ops import sample_farthest_points
+
+    p = np.ascontiguousarray(_cloud(kind, B, N))
+    got = sample_farthest_points(torch.from_numpy(p).to(DEV), S).cpu().numpy()
+    np.testing.assert_array_equal(got, oracle.fps(p, S))

@@ -175,3 +175,29 @@ def test_a_scratch_buffer_that_is_too_small_sweeps():
         assert bool(buf.any()) == (n == need)
         res.append((d, i))
     assert _same(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+
+
+def test_ordered_searches_are_captured_and_replayed_on_new_inputs():
+    from torkit3d_b200 import ops
+
+    a, b = _pair("uniform", 2, 9000, 9000, 0)
+
+    def run():
+        return ops.nn_distance(a, b) + list(ops.knn_points(a, b, 3)) + list(ops.knn_points(a, b, 20)) + [
+            ops.ball_query(a, b, 0.05, 16)]
+
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        run()
+    torch.cuda.current_stream().wait_stream(s)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = run()
+    for kind in ("plane", "outlier"):
+        a2, b2 = _pair(kind, 2, 9000, 9000, 0)
+        a.copy_(a2), b.copy_(b2)
+        graph.replay()
+        torch.cuda.synchronize()
+        for x, y in zip(out, run()):
+            assert _same(x, y)

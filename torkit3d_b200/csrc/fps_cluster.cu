@@ -7,8 +7,8 @@
 // L2 in every step (4 clouds of 65536 points: 19 us per step).  Here a cluster of 4, 8 or 16 small
 // blocks shares a cloud: every block keeps a contiguous slice of the points and their running
 // minima in registers (8 to 32 points per thread), and the step has no block or cluster barrier at
-// all -- see fps_warpcast_kernel.  32 clouds of 8192 points, 1024 samples: 0.56 ms against 0.70 ms;
-// 4 clouds of 65536 points, 2048 samples: 2.0 ms against 39.9 ms for the streaming kernel.
+// all -- see fps_warpcast_kernel.  32 clouds of 8192 points, 1024 samples: 0.34 ms against 0.70 ms;
+// 4 clouds of 65536 points, 2048 samples: 1.12 ms against 39.9 ms for the streaming kernel.
 //
 // Measured and dropped: the same clusters with 1024-thread blocks that reduce inside the block
 // first (two block barriers) and exchange one candidate per block behind a cluster barrier per
@@ -41,8 +41,11 @@ constexpr int FC_MAX_CL = 16;  // 8 is the portable cluster size; 16 needs an op
 // warps whose candidates have been taken, and (b) none of the samples taken since the exchange came
 // closer to it than its running minimum.  Nothing else can be farther: a warp whose candidate has not
 // been taken has no point above it.  The first candidate always passes, so the sequence is the one
-// of single steps, bit for bit.  Counted on the CPU, an exchange yields 3.5 to 4.3 samples; it costs
-// 0.45 us and more, a sample taken from it about 0.15 us.
+// of single steps, bit for bit.  Counted on the CPU, an exchange yields 3.5 to 4.3 samples; taking one
+// costs about 0.15 us, an exchange 0.45 us and more.  32 clouds of 8192 points, 1024 samples: 0.34 ms,
+// one sample per exchange 0.56; 4 clouds of 65536 points, 2048 samples: 1.12 ms, 1.95.  Where most
+// distances tie (a lattice of 1000 positions) exchanges yield little more than one sample, at 1.05 to
+// 1.2 times the cost.
 //
 // The candidate slots and mbarriers are double buffered by the parity of the exchange: a warp can send
 // for exchange i+2 only after it has seen every warp's candidate of exchange i+1, which those warps
@@ -212,7 +215,7 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
   int n = 1;  // samples so far
   // Where exchanges keep yielding a single sample (points on a lattice: ties), the bounds are left out
   // for 48 exchanges at a time; the same in all warps.
-  int again = 0, single = 0;
+  int again = FW_REGS ? 0 : 0x7fffffff, single = 0;
   for (int ex = 1; n < S; ++ex) {
     const int par = ex & 1;
     const unsigned bits = __float_as_uint(bm);
@@ -271,6 +274,48 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
     if (tid == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(lb), "r"(expect) : "memory");
 
+    if constexpr (!FW_REGS) {
+      // coordinates in shared memory: a bound costs more than it saves (2 x 200000 -> 200 593 us, without
+      // bounds 419), so every exchange gives one sample
+      unsigned b_ = 0u;
+      int i_ = 0x7fffffff, slot = lane;
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        const int sl = lane + 32 * c;
+        const uint2 v = *reinterpret_cast<const uint2 *>(&cand[par][sl < nw ? sl : 0]);
+        if (sl < nw && (c == 0 || v.x > b_ || (v.x == b_ && (int)v.y < i_))) {
+          b_ = v.x;
+          i_ = (int)v.y;
+          slot = sl;
+        }
+      }
+      const unsigned wb = __reduce_max_sync(0xffffffffu, b_);
+      const int wi = __reduce_min_sync(0xffffffffu, b_ == wb ? i_ : 0x7fffffff);
+      int src = __ffs(__ballot_sync(0xffffffffu, b_ == wb && i_ == wi)) - 1;
+      if constexpr (CPL > 1) src = __shfl_sync(0xffffffffu, slot, src);
+      cx = cand[par][src].x;
+      cy = cand[par][src].y;
+      cz = cand[par][src].z;
+      if (writer) {
+        out[n] = wi;
+        if (sm) {
+          sm[(int64_t)n * sps] = cx;
+          sm[(int64_t)n * sps + scs] = cy;
+          sm[(int64_t)n * sps + 2 * (int64_t)scs] = cz;
+        }
+      }
+      ++n;
+      const float2 nx = make_float2(-cx, -cx), ny = make_float2(-cy, -cy), nz = make_float2(-cz, -cz);
+      bm = 0.f;
+#pragma unroll
+      for (int i = 0; i < FW_P2; ++i) {
+        const float2 d = dist2(i, nx, ny, nz);
+        md[i].x = fminf(md[i].x, d.x);
+        md[i].y = fminf(md[i].y, d.y);
+        asm("max.f32 %0, %0, %1, %2;" : "+f"(bm) : "f"(md[i].x), "f"(md[i].y));
+      }
+      continue;
+    }
     // lane l holds candidates l, l + 32, ...
     unsigned cb[CPL];
     int ci[CPL];
