@@ -184,7 +184,7 @@ def test_ordered_searches_are_captured_and_replayed_on_new_inputs():
 
     def run():
         return ops.nn_distance(a, b) + list(ops.knn_points(a, b, 3)) + list(ops.knn_points(a, b, 20)) + [
-            ops.ball_query(a, b, 0.05, 16)]
+            ops.ball_query(a, b, 0.05, 16, transpose=False)]
 
     s = torch.cuda.Stream()
     s.wait_stream(torch.cuda.current_stream())
