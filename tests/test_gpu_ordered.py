@@ -201,3 +201,60 @@ def test_ordered_searches_are_captured_and_replayed_on_new_inputs():
         torch.cuda.synchronize()
         for x, y in zip(out, run()):
             assert _same(x, y)
+
+
+def test_batches_beyond_the_scratch_limit_are_cut():
+    from torkit3d_b200 import _lib
+
+    lib = _lib.load()
+    B, N = 9001, 1024  # about 670 MB of index: built in two parts
+    g = torch.Generator(device=DEV).manual_seed(1)
+    a, b = (torch.randn(B, N, 3, generator=g, device=DEV) for _ in range(2))
+    a[4000, 3, 1] = float("nan")
+    need = lib.tk3d_chamfer_fwd_scratch_bytes(B, N, N, _lib.F32)
+    assert 0 < need < (600 << 20) and need == lib.tk3d_chamfer_fwd_scratch_bytes(2 * B, N, N, _lib.F32)
+    buf, res = torch.empty(need, dtype=torch.uint8, device=DEV), []
+    for n in (0, need):
+        d = [torch.empty(B, N, device=DEV) for _ in range(2)]
+        i = [torch.empty(B, N, dtype=torch.int64, device=DEV) for _ in range(2)]
+        sums = torch.empty(2, dtype=torch.float64, device=DEV)
+        assert lib.tk3d_chamfer_fwd_ws(a.data_ptr(), b.data_ptr(), B, N, N, 0, d[0].data_ptr(), i[0].data_ptr(),
+                                       d[1].data_ptr(), i[1].data_ptr(), sums.data_ptr(), buf.data_ptr(), n, _lib.F32,
+                                       _stream()) == 0
+        res.append(d + i + [sums])
+    for x, y in zip(res[0][:4], res[1][:4]):
+        assert _same(x, y)
+
+
+@pytest.mark.parametrize("N,M,cf", [(1025, 4097, 0), (4096, 2048, 1), (1024, 20001, 1)])
+@pytest.mark.parametrize("kind", ["uniform", "zeros", "nonfinite"])
+def test_nothing_outside_the_scratch_and_the_outputs_is_written(kind, N, M, cf):
+    from torkit3d_b200 import _lib
+
+    lib = _lib.load()
+    B, pad = 41, 4096
+    a, b = _pair(kind, B, N, M, cf)
+
+    def guarded(nbytes):
+        t = torch.full((nbytes + 2 * pad,), 0x5A, dtype=torch.uint8, device=DEV)
+        guards.append((t, nbytes))
+        return t.data_ptr() + pad
+
+    for k, ball in ((0, 0), (3, 0), (16, 0), (40, 0), (16, 1)):
+        guards = []
+        if k == 0:
+            need = lib.tk3d_chamfer_fwd_scratch_bytes(B, N, M, _lib.F32)
+            rc = lib.tk3d_chamfer_fwd_ws(a.data_ptr(), b.data_ptr(), B, N, M, cf, guarded(B * N * 4),
+                                         guarded(B * N * 8), guarded(B * M * 4), guarded(B * M * 8), None,
+                                         guarded(need), need, _lib.F32, _stream())
+        elif ball:
+            need = lib.tk3d_ball_query_scratch_bytes(B, N, M, k, _lib.F32)
+            rc = lib.tk3d_ball_query_ws(a.data_ptr(), b.data_ptr(), B, N, M, 0.1, k, cf, guarded(B * N * k * 8),
+                                        _lib.I64, guarded(need), need, _lib.F32, _stream())
+        else:
+            need = lib.tk3d_knn_scratch_bytes(B, N, M, k, _lib.F32)
+            rc = lib.tk3d_knn_ws(a.data_ptr(), b.data_ptr(), B, N, M, k, cf, guarded(B * N * k * 4),
+                                 guarded(B * N * k * 8), _lib.I64, guarded(need), need, _lib.F32, _stream())
+        assert rc == 0 and need > 0
+        for t, n in guards:
+            assert bool((t[:pad] == 0x5A).all()) and bool((t[pad + n:] == 0x5A).all())
