@@ -1083,12 +1083,13 @@ bool knn_order_takes(int64_t B, int64_t N1, int64_t N2, int64_t k) {
 }
 // Measured on B200, sweep / ordered, us (two numbers: points in a volume, on a surface):
 //   k = 3    4 x 2048^2 46 / 54, 64 x 1024 x 512 54 / 56, 16 x 4096 x 1024 101 / 56, 8 x 4096^2 121 / 62
+//   k = 5    8 x 2048^2 39 / 47, 42; 29 x 4478 x 961 97 / 107, 89; 32 x 4096 x 2048 142 / 121, 95
 //   k = 16   32 x 1024^2 55 / 74, 64; 8 x 2048^2 52 / 62, 52; 16 x 4096^2 175 / 136, 98; 4 x 512 x 10000 116 / 80, 60
 //   k = 32   4 x 1024^2 48 / 64; 32 x 1024^2 124 / 126, 107; 8 x 2048^2 89 / 91, 74; 32 x 2048 x 8192 545 / 273, 195
 //   k = 64   4 x 1024^2 101 / 107, 102; 8 x 2048^2 195 / 162, 152; 32 x 2048 x 8192 936 / 551, 425
 bool knn_order_pays(int64_t B, int64_t N1, int64_t N2, int64_t k) {
   const double pairs = (double)B * N1 * N2;
-  const double least = k <= 4 ? 4e7 : k > 32 || N2 >= 8192 ? 2e7 : k > 16 ? 4e7 : 1e8;
+  const double least = k <= 4 ? 4e7 : k > 32 || N2 >= 8192 ? 2e7 : k > 16 ? 4e7 : k > 8 ? 1e8 : 1.6e8;
   return knn_order_takes(B, N1, N2, k) && pairs >= least;
 }
 
