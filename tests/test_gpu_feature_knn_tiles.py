@@ -54,3 +54,25 @@ def test_infinite_distances_rank_last_and_nan_never():
     order = [j for j in range(40) if j not in (10, 11)]
     assert i[0, 0].tolist() == order + [10, -1]
     assert d[0, 0, :38].tolist() == [float(j * j) for j in order] and np.isinf(d[0, 0, 38:]).all()
+
+
+def test_point_major_rows_are_staged_without_bank_conflicts():
+    """Staging point-major tensors costs strided reads, not bank conflicts (with them 1.85 times the channel-first call)."""
+    from torkit3d_b200 import _C
+
+    g = torch.Generator(device=DEV).manual_seed(0)
+    a = torch.randn(4, 128, 4096, generator=g, device=DEV)
+    p = a.transpose(1, 2).contiguous()
+
+    def us(fn):
+        best = float("inf")
+        for _ in range(6):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            fn()
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1) * 1e3)
+        return best
+
+    assert us(lambda: _C.feature_knn_cuda(p, p, 40, channel_first=False)) < 1.6 * us(lambda: _C.feature_knn_cuda(a, a, 40))

@@ -19,8 +19,9 @@
 // of 32 new entries first meets the topmost 32, of which the lower half stays, and the exchange then
 // goes down the list.  Ties go to the lower index; rows come out sorted.
 //
-// 32 x 1024 x 1024, 64 channels, k = 20: 0.232 ms; one key per lane and one candidate at a time into the
-// list took 0.400 ms.  Half of the issue slots are the packed operations, the rest mostly selection.
+// 32 x 1024 x 1024, 64 channels, k = 20: 0.229 ms, point-major tensors 0.298 (0.391 with unpadded rows); one key per
+// lane and one candidate at a time into the list took 0.400 and 0.422 ms.  Half of the issue slots are the packed
+// operations, the rest mostly selection.
 #include <limits.h>
 
 #include "tk3d_common.cuh"
@@ -38,10 +39,12 @@ constexpr unsigned FULL = 0xffffffffu;
 
 using u64 = unsigned long long;
 
-template <int KS>
+// Row lengths: point-major tensors are staged along the channels, sixteen rows at a time, and rows of 256 words would
+// meet in one bank; 258 spread sixteen channels of two keys over all banks, 36 those of two queries over half of them.
+template <int KS, bool POINTS>
 struct FkSmem {
-  float k[2][FK_CS][FK_KT];
-  float q[2][FK_CS][FK_QW * FK_WARPS];
+  float k[2][FK_CS][POINTS ? FK_KT + 2 : FK_KT];
+  float q[2][FK_CS][POINTS ? FK_QW * FK_WARPS + 4 : FK_QW * FK_WARPS];
   u64 buf[FK_QW * FK_WARPS][FK_BUF];
   u64 list[FK_QW * FK_WARPS][32 * KS];
 };
@@ -104,7 +107,8 @@ feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ ke
   extern __shared__ __align__(16) unsigned char fk_smem[];
   constexpr int QW = FK_QW, V = LAYOUT == FK_CHANNELS16 ? 4 : 1;
   constexpr bool CF = LAYOUT != FK_POINTS;
-  FkSmem<KS> &sm = *reinterpret_cast<FkSmem<KS> *>(fk_smem);
+  using Smem = FkSmem<KS, LAYOUT == FK_POINTS>;
+  Smem &sm = *reinterpret_cast<Smem *>(fk_smem);
   constexpr int QT = QW * FK_WARPS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chunks = (N1 + QT - 1) / QT;
@@ -237,7 +241,7 @@ int launch(const float *query, const float *key, int64_t B, int C, int N1, int N
   const int64_t total = B * ((N1 + QT - 1) / QT);
   const int64_t cap = (int64_t)sm_count() * 32;
   const unsigned grid = (unsigned)(total < cap ? total : cap);
-  const size_t smem = sizeof(FkSmem<KS>);
+  const size_t smem = cf ? sizeof(FkSmem<KS, false>) : sizeof(FkSmem<KS, true>);
   const bool wide = N1 % 4 == 0 && N2 % 4 == 0 &&
                     ((reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(key)) & 15) == 0;
   auto kern = !cf    ? feature_knn_kernel<KS, FK_POINTS>
