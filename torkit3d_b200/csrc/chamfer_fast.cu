@@ -68,12 +68,12 @@ __device__ __forceinline__ void chamfer_verify(const float4 *tl, int u0, int t0,
 // distance; taken one ulp higher, because a key AT that distance with a lower index must still pass
 // this lane's filter -- and at the end the best (distance, index) of all lanes is kept.  Same pairs
 // per shared-memory load, LANES times the warps.
-template <int Q, int MINB = 1, int UNR = 2, int CF_THREADS = 128, int LANES = 1>
+template <int Q, int MINB, int UNR, int CF_THREADS, int LANES, typename Only>
 __global__ void __launch_bounds__(CF_THREADS, MINB)
 chamfer_fwd_fast_kernel(const float *__restrict__ xyz1, const float *__restrict__ xyz2, int64_t B, int N1, int N2,
                         float *__restrict__ dist1, int64_t *__restrict__ idx1, float *__restrict__ dist2,
                         int64_t *__restrict__ idx2, double *__restrict__ sums, int64_t blocks1,
-                        int64_t blocks_total, XyzLayout l1, XyzLayout l2, SpOnly only) {
+                        int64_t blocks_total, XyzLayout l1, XyzLayout l2, Only only) {
   constexpr int PER = CF_TILE / CF_THREADS;
   constexpr int GK = 8 / Q;  // keys per filter group: eight (key, query) pairs share one branch
   __shared__ float4 tile[2][CF_TILE];
@@ -261,8 +261,12 @@ int launch(const float *xyz1, const float *xyz2, int64_t B, int N1, int N2, floa
   // behind a search over ordered clouds there is usually nothing left to do: one round of blocks looks
   const int64_t cap = (int64_t)sm_count() * (only.q ? 6 : 256);
   const unsigned grid = (unsigned)(total < cap ? total : cap);
-  chamfer_fwd_fast_kernel<Q, MINB, UNR, CF_THREADS, LANES><<<grid, CF_THREADS, 0, st>>>(
-      xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, blocks1, total, l1, l2, only);
+  if (only.q)
+    chamfer_fwd_fast_kernel<Q, MINB, UNR, CF_THREADS, LANES, SpOnly><<<grid, CF_THREADS, 0, st>>>(
+        xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, blocks1, total, l1, l2, only);
+  else
+    chamfer_fwd_fast_kernel<Q, MINB, UNR, CF_THREADS, LANES, SpAll><<<grid, CF_THREADS, 0, st>>>(
+        xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, blocks1, total, l1, l2, SpAll{});
   return check_launch("chamfer_fwd_fast_kernel");
 }
 

@@ -55,11 +55,11 @@ __device__ __forceinline__ float4 make_key(const float *__restrict__ rb, int j, 
 // end the lists are merged by (distance, index) in log2(LANES) butterfly steps.  Same pairs per shared-memory load, same staging, but
 // LANES times the warps for a given number of queries: for launches that cannot fill the GPU with
 // one lane per query, whose time is the critical path of a single warp.
-template <int K, int Q, int LANES = 1, bool FIRSTX = false>
+template <int K, int Q, int LANES, bool FIRSTX, typename Only>
 __global__ void __launch_bounds__(KN_THREADS)
 knn_small_kernel(const float *__restrict__ query, const float *__restrict__ key, int64_t B, int N1, int N2,
                  float *__restrict__ dist, IndexOut index, int64_t blocks_total, XyzLayout ql, XyzLayout kl,
-                 SpOnly only) {
+                 Only only) {
   constexpr int TILE = 512, PER = TILE / KN_THREADS;
   constexpr int GK = 8 / Q;  // keys per filter group: eight (key, query) pairs share one branch
   __shared__ float4 tile[2][TILE];  // pair layout of sweep.cuh
@@ -502,11 +502,11 @@ __device__ __forceinline__ void kt_cx(float &a, float &b) {
 
 // Q = queries per lane (1 or 2): a block serves 32*Q queries.  Two queries per lane halve the
 // shared-memory reads per pair, one keeps more blocks in flight when queries are few.
-template <int Q, int KT_NCH, int KT_QCAP, int MINB, int KT_TILE>
+template <int Q, int KT_NCH, int KT_QCAP, int MINB, int KT_TILE, typename Only>
 __global__ void __launch_bounds__(KT_THREADS, MINB)
 knn_twopass_kernel(const float *__restrict__ query, const float *__restrict__ key, int64_t B, int N1, int N2, int k,
                    float *__restrict__ dist, IndexOut index, int64_t blocks_total, XyzLayout ql, XyzLayout kl,
-                   SpOnly only) {
+                   Only only) {
   constexpr int PER = KT_TILE / KT_THREADS;
   constexpr int CPW = KT_NCH / KT_SPLIT;          // classes per warp: 8, 16, 32 or 64
   constexpr int NPAIR = KT_TILE / 2 / KT_SPLIT;   // key pairs per warp and tile: 32 or 64
@@ -973,7 +973,7 @@ knn_generic_kernel(const T *__restrict__ query, const T *__restrict__ key, int64
 struct KnnIo {
   IndexOut index;
   XyzLayout ql, kl;
-  SpOnly only = {};  // behind a search over ordered clouds: the clouds it could not serve
+  SpOnly only = {};  // behind a search over ordered clouds (grids not null): the clouds it could not serve
 };
 
 template <typename T>
@@ -992,14 +992,21 @@ int knn_small(const float *query, const float *key, int64_t B, int N1, int N2, f
               cudaStream_t st) {
   const int64_t per = KN_THREADS * Q / LANES;
   const int64_t total = B * ((N1 + per - 1) / per);
-  const int64_t cap = (int64_t)sm_count() * (io.only.q ? 6 : 256);  // usually nothing is left: one round of blocks looks
+  // behind a search usually nothing is left: about a round of blocks looks
+  const int64_t cap = (int64_t)sm_count() * (io.only.q ? 6 : 256);
   const unsigned grid = (unsigned)(total < cap ? total : cap);
-  if (LANES > 1 && N2 <= 16384)  // few key tiles: the first one is worth extra exchanges
-    knn_small_kernel<K, Q, LANES, (LANES > 1)><<<grid, KN_THREADS, 0, st>>>(query, key, B, N1, N2, dist, io.index, total,
-                                                                            io.ql, io.kl, io.only);
-  else
-    knn_small_kernel<K, Q, LANES><<<grid, KN_THREADS, 0, st>>>(query, key, B, N1, N2, dist, io.index, total, io.ql,
-                                                               io.kl, io.only);
+  const bool firstx = LANES > 1 && N2 <= 16384;  // few key tiles: the first one is worth extra exchanges
+  auto go = [&](auto only) {
+    using Only = decltype(only);
+    if (firstx)
+      knn_small_kernel<K, Q, LANES, (LANES > 1), Only><<<grid, KN_THREADS, 0, st>>>(query, key, B, N1, N2, dist, io.index,
+                                                                                    total, io.ql, io.kl, only);
+    else
+      knn_small_kernel<K, Q, LANES, false, Only><<<grid, KN_THREADS, 0, st>>>(query, key, B, N1, N2, dist, io.index,
+                                                                              total, io.ql, io.kl, only);
+  };
+  if (io.only.q) go(io.only);
+  else go(SpAll{});
   return check_launch("knn_small_kernel");
 }
 
@@ -1068,11 +1075,15 @@ int knn_twopass(const float *query, const float *key, int64_t B, int N1, int N2,
   const int64_t total = B * ((N1 + 32 * Q - 1) / (32 * Q));
   const int64_t gcap = (int64_t)sm_count() * (io.only.q ? MINB : 256);
   const size_t smem = kt_smem_bytes<Q, NCH, QCAP, TILE>();
-  if (smem + 4096 > 48 * 1024)  // static shared memory of the kernel counts towards the 48 KB default limit
-    TK3D_CUDA(raise_smem_limit((const void *)knn_twopass_kernel<Q, NCH, QCAP, MINB, TILE>, (int)smem));
-  knn_twopass_kernel<Q, NCH, QCAP, MINB, TILE><<<(unsigned)(total < gcap ? total : gcap), KT_THREADS, smem, st>>>(
-      query, key, B, N1, N2, k, dist, io.index, total, io.ql, io.kl, io.only);
-  return check_launch("knn_twopass_kernel");
+  const unsigned grid = (unsigned)(total < gcap ? total : gcap);
+  auto go = [&](auto only) {
+    auto kern = knn_twopass_kernel<Q, NCH, QCAP, MINB, TILE, decltype(only)>;
+    if (smem + 4096 > 48 * 1024)  // static shared memory of the kernel counts towards the 48 KB default limit
+      TK3D_CUDA(raise_smem_limit((const void *)kern, (int)smem));
+    kern<<<grid, KT_THREADS, smem, st>>>(query, key, B, N1, N2, k, dist, io.index, total, io.ql, io.kl, only);
+    return check_launch("knn_twopass_kernel");
+  };
+  return io.only.q ? go(io.only) : go(SpAll{});
 }
 
 }  // namespace
@@ -1093,8 +1104,9 @@ bool knn_order_pays(int64_t B, int64_t N1, int64_t N2, int64_t k) {
   return knn_order_takes(B, N1, N2, k) && pairs >= least;
 }
 
+template <typename Only>
 __global__ void three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t N1, int64_t rows, float eps,
-                                               SpOnly only);
+                                               Only only);
 
 // k <= 64 over spatially ordered clouds; what the order cannot serve is swept.
 int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, int k, int channel_first,
@@ -1145,11 +1157,12 @@ int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int
 // epilogue saved that launch but left the sweep's two-lane variant with 79 registers, six blocks
 // per SM, i.e. out of reach for the half-filled launches that need it (8 x 16384 x 32768 with the
 // gather that follows: 1.24 -> 1.11 ms; 8 x 65536 x 32768: 6.80 -> 6.77).
+template <typename Only>
 __global__ void __launch_bounds__(256)
-three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t N1, int64_t rows, float eps, SpOnly only) {
+three_nn_weight_inplace_kernel(float *__restrict__ weight, int64_t N1, int64_t rows, float eps, Only only) {
   if (only.idle(rows / N1)) return;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
-    if (only.q && only.skip(r / N1)) continue;
+    if (only.skip(r / N1)) continue;
     float *w = weight + r * 3;
     float inv[3], sum = 0.f;
 #pragma unroll
@@ -1175,7 +1188,7 @@ int three_nn_fused_f32(const float *query, const float *key, int64_t B, int64_t 
   int rc = knn_small_q<3>(query, key, B, (int)N1, (int)N2, weight, io, st);
   if (rc) return rc;
   const int64_t rows = B * N1, blocks = (rows + 255) / 256, cap = (int64_t)sm_count() * 8;
-  three_nn_weight_inplace_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(weight, N1, rows, eps, SpOnly{});
+  three_nn_weight_inplace_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(weight, N1, rows, eps, SpAll{});
   return check_launch("three_nn_weight_inplace_kernel");
 }
 

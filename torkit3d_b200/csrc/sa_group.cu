@@ -54,7 +54,8 @@ inline SaSmem sa_smem(int C, int K, bool vec) {
 
 // Point j, coordinate d of cloud b lives at base[b*3*N + j*ps + d*cs]: (ps, cs) = (3, 1) for
 // [B,N,3] and (1, N) for [B,3,N].
-template <int SPLIT>
+// GIVEN: the neighbours have been found beforehand.
+template <int SPLIT, bool GIVEN>
 __global__ void __launch_bounds__(32 * SPLIT)
 sa_group_fwd_kernel(const float *__restrict__ points, const float *__restrict__ centroids,
                     const float *__restrict__ featT, int64_t B, int C, int N, int M, int pps, int pcs, int cps,
@@ -105,7 +106,7 @@ sa_group_fwd_kernel(const float *__restrict__ points, const float *__restrict__ 
     int done = 0;                   // hits of this centroid in the tiles swept so far (same in every warp)
     int *row = sidx + lane * S1;    // its hit list, ascending point index
     const float *rb = points + b * 3 * (int64_t)N;
-    const int ntiles = given ? 0 : (N + SA_TILE - 1) / SA_TILE;
+    const int ntiles = GIVEN ? 0 : (N + SA_TILE - 1) / SA_TILE;
 
     // ---- phase A: ball query ----------------------------------------------------------------
     float4 nxt[PER];
@@ -181,7 +182,7 @@ sa_group_fwd_kernel(const float *__restrict__ points, const float *__restrict__ 
       if (done >= K) thr[0] = never;
     }
     __syncthreads();  // the lists' first entries are visible to every warp
-    if (given) {      // complete lists, found beforehand
+    if constexpr (GIVEN) {  // complete lists
       const int32_t *gp = given + b * E + (int64_t)m0 * K;
       for (int e = tid; e < nv * K; e += THREADS) sidx[(e / K) * S1 + (e % K)] = gp[e];
       if (part == 0 && valid && status && gp[(int64_t)lane * K] < 0) atomicOr(status, 1);
@@ -402,22 +403,16 @@ extern "C" int tk3d_sa_group_fwd(const void *points, const void *centroids, cons
   const SaSmem sm = sa_smem((int)C, (int)K, vec);
   const int64_t total = B * ((M + SA_Q - 1) / SA_Q);
   const bool wide = total <= 2 * (int64_t)sm_count();  // few blocks: eight warps per 32 centroids
-  if (sm.total > 48 * 1024)
-    TK3D_CUDA(raise_smem_limit(wide ? (const void *)sa_group_fwd_kernel<8> : (const void *)sa_group_fwd_kernel<4>,
-                               (int)sm.total));
+  auto kern = given ? (wide ? sa_group_fwd_kernel<8, true> : sa_group_fwd_kernel<4, true>)
+                    : (wide ? sa_group_fwd_kernel<8, false> : sa_group_fwd_kernel<4, false>);
+  if (sm.total > 48 * 1024) TK3D_CUDA(raise_smem_limit((const void *)kern, (int)sm.total));
   const int64_t cap = (int64_t)sm_count() * 64;
   const float r2 = radius * radius;
   const int pps = xyz_channel_first ? 1 : 3, pcs = xyz_channel_first ? (int)N : 1;
   const int cps = xyz_channel_first ? 1 : 3, cpc = xyz_channel_first ? (int)M : 1;
-  const unsigned grid = (unsigned)(total < cap ? total : cap);
-  if (wide)
-    sa_group_fwd_kernel<8><<<grid, 256, sm.total, st>>>(
-        (const float *)points, (const float *)centroids, featT, B, (int)C, (int)N, (int)M, pps, pcs, cps, cpc, r2,
-        (int)K, use_xyz ? 1 : 0, vec, (float *)out, given, given ? nullptr : index32, status, total);
-  else
-    sa_group_fwd_kernel<4><<<grid, 128, sm.total, st>>>(
-        (const float *)points, (const float *)centroids, featT, B, (int)C, (int)N, (int)M, pps, pcs, cps, cpc, r2,
-        (int)K, use_xyz ? 1 : 0, vec, (float *)out, given, given ? nullptr : index32, status, total);
+  kern<<<(unsigned)(total < cap ? total : cap), wide ? 256 : 128, sm.total, st>>>(
+      (const float *)points, (const float *)centroids, featT, B, (int)C, (int)N, (int)M, pps, pcs, cps, cpc, r2, (int)K,
+      use_xyz ? 1 : 0, vec, (float *)out, given, given ? nullptr : index32, status, total);
   return check_launch("sa_group_fwd_kernel");
 }
 
