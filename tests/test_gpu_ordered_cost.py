@@ -1,0 +1,83 @@
+"""What the searches over ordered clouds cost on inputs that the order does not serve, against the same entry point
+without scratch (which sweeps all pairs), and that the results are the same.  The limits leave room for the order itself
+(20 to 35 us) and for noise; each input took two to ten times its limit before it was looked after."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _sphere(B, N, g):
+    p = torch.randn(B, N, 3, generator=g, device=DEV)
+    return p / p.norm(dim=2, keepdim=True) + 0.01 * torch.randn(B, N, 3, generator=g, device=DEV)
+
+
+def _cloud(kind, B, N, g):
+    p = _sphere(B, N, g)
+    if kind == "blobs":
+        centres = torch.rand(B, 8, 3, generator=torch.Generator(device=DEV).manual_seed(7), device=DEV) * 2 - 1
+        pick = torch.randint(0, 8, (B, N, 1), generator=g, device=DEV).expand(-1, -1, 3)
+        p = torch.gather(centres, 1, pick) + 0.1 * torch.randn(B, N, 3, generator=g, device=DEV)
+    elif kind == "collapsed":
+        p = 0.01 * torch.randn(B, N, 3, generator=g, device=DEV)
+    elif kind == "outlier":
+        p[:, N // 3] = torch.tensor([1000.0, 0, 0], device=DEV)
+    elif kind == "away":
+        p += 10
+    elif kind == "nan":
+        p[:, N // 3] = float("nan")
+    return p
+
+
+def _us(fn):
+    for _ in range(3):
+        fn()
+    best = float("inf")
+    for _ in range(7):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        for _ in range(3):
+            fn()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3 / 3)
+    return best
+
+
+def _both(k, B, N, M, kinds):
+    """Times without and with scratch; the results have to be equal."""
+    from torkit3d_b200 import _lib
+
+    lib = _lib.load()
+    g = torch.Generator(device=DEV).manual_seed(N + M)
+    a, b = _cloud(kinds[0], B, N, g), _cloud(kinds[1], B, M, g)
+    buf = torch.empty(64 << 20, dtype=torch.uint8, device=DEV)
+    st = torch.cuda.current_stream().cuda_stream
+    if k == 0:
+        out = [torch.empty(B, n, dtype=t, device=DEV) for n in (N, M) for t in (torch.float32, torch.int64)]
+
+        def run(n):
+            assert lib.tk3d_chamfer_fwd_ws(a.data_ptr(), b.data_ptr(), B, N, M, 0, *(o.data_ptr() for o in out), None,
+                                           buf.data_ptr(), n, _lib.F32, st) == 0
+    else:
+        out = [torch.empty(B, N, k, dtype=t, device=DEV) for t in (torch.float32, torch.int64)]
+
+        def run(n):
+            assert lib.tk3d_knn_ws(a.data_ptr(), b.data_ptr(), B, N, M, k, 0, out[0].data_ptr(), out[1].data_ptr(),
+                                   _lib.I64, buf.data_ptr(), n, _lib.F32, st) == 0
+
+    res, times = [], []
+    for n in (0, buf.numel()):
+        times.append(_us(lambda: run(n)))
+        res.append([o.clone() for o in out])
+    for x, y in zip(*res):
+        assert torch.equal(x.view(torch.int32) if x.dtype == torch.float32 else x,
+                           y.view(torch.int32) if y.dtype == torch.float32 else y)
+    return times
+
+
+@pytest.mark.parametrize("k,B,N,M", [(0, 1, 2048, 65536), (0, 2, 8192, 8192), (3, 1, 1000, 100000), (3, 16, 4096, 4096)])
+def test_flagged_clouds_are_swept_by_the_kernel_that_serves_a_call_without_scratch(k, B, N, M):
+    plain, ordered = _both(k, B, N, M, ("nan", "nan"))
+    assert ordered < 1.25 * plain + 40

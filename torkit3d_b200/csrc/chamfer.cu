@@ -166,7 +166,7 @@ chamfer_bwd_scatter_kernel(const T *__restrict__ g1, const T *__restrict__ g2, c
 
 int chamfer_fwd_f32_fast(const float *xyz1, const float *xyz2, int64_t B, int64_t N1, int64_t N2, float *dist1,
                          int64_t *idx1, float *dist2, int64_t *idx2, double *sums, cudaStream_t st, XyzLayout l1,
-                         XyzLayout l2);
+                         XyzLayout l2, SpOnly only);
 
 template <typename T>
 static int chamfer_fwd_generic(const T *xyz1, const T *xyz2, int64_t B, int64_t N1, int64_t N2, T *dist1,
@@ -291,7 +291,7 @@ static int chamfer_fwd_impl(const void *xyz1, const void *xyz2, int64_t B, int64
                                    idx1, (float *)dist2, idx2, sums, scratch, st);
   if (dtype == TK3D_F32)
     return chamfer_fwd_f32_fast((const float *)xyz1, (const float *)xyz2, B, N1, N2, (float *)dist1, idx1,
-                                (float *)dist2, idx2, sums, st, l1, l2);
+                                (float *)dist2, idx2, sums, st, l1, l2, SpOnly{});
   return chamfer_fwd_generic<double>((const double *)xyz1, (const double *)xyz2, B, N1, N2, (double *)dist1, idx1,
                                      (double *)dist2, idx2, sums, st, l1, l2);
 }

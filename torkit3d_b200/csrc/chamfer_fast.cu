@@ -15,6 +15,8 @@
 // wins ties.
 //
 // Both directions run in one launch; each block adds its partial sum of distances to `sums`.
+#include <type_traits>
+
 #include "spatial.cuh"
 #include "sweep.cuh"
 
@@ -258,8 +260,8 @@ int launch(const float *xyz1, const float *xyz2, int64_t B, int N1, int N2, floa
   const int64_t blocks2 = only_dir == 0 ? 0 : B * ((N2 + per - 1) / per);
   const int64_t total = blocks1 + blocks2;
   if (total == 0) return TK3D_OK;
-  // behind a search over ordered clouds there is usually nothing left to do: one round of blocks looks
-  const int64_t cap = (int64_t)sm_count() * (only.q ? 6 : 256);
+  // behind a search over ordered clouds there is usually nothing left to do: about one round of blocks looks
+  const int64_t cap = (int64_t)sm_count() * (only.q ? 12 : 256);
   const unsigned grid = (unsigned)(total < cap ? total : cap);
   if (only.q)
     chamfer_fwd_fast_kernel<Q, MINB, UNR, CF_THREADS, LANES, SpOnly><<<grid, CF_THREADS, 0, st>>>(
@@ -282,12 +284,12 @@ int launch(const float *xyz1, const float *xyz2, int64_t B, int N1, int N2, floa
 // (its groups are bound to their block, so an SM's last tasks of a round run with the SM partly
 // empty).  The launcher therefore picks this kernel only for one or two nearly full rounds of
 // tasks.  896 threads leave 72 registers per thread.
-template <int UNR>
+template <int UNR, typename Only>
 __global__ void __launch_bounds__(896, 1)
 chamfer_fwd_smwide_kernel(const float *__restrict__ xyz1, const float *__restrict__ xyz2, int N1, int N2,
                           float *__restrict__ dist1, int64_t *__restrict__ idx1, float *__restrict__ dist2,
                           int64_t *__restrict__ idx2, double *__restrict__ sums, int blocks1,
-                          int blocks_total, XyzLayout l1, XyzLayout l2) {
+                          int blocks_total, XyzLayout l1, XyzLayout l2, int B, Only only) {
   constexpr int Q = 2, TH = 128;
   constexpr int PER = CF_TILE / TH;
   extern __shared__ float4 group_tiles[];  // [groups][2][CF_TILE]
@@ -296,9 +298,13 @@ chamfer_fwd_smwide_kernel(const float *__restrict__ xyz1, const float *__restric
   const int groups = blockDim.x >> 7;
   float4(*tile)[CF_TILE] = reinterpret_cast<float4(*)[CF_TILE]>(group_tiles + (size_t)grp * 2 * CF_TILE);
   const float pinf = __int_as_float(0x7f800000);
+  if (only.idle(B)) return;
 
-  // Every group walks its own tasks; groups never wait for one another.
-  for (int blk = blockIdx.x * groups + grp; blk < blocks_total; blk += gridDim.x * groups) {
+  // Every group walks its own tasks; groups never wait for one another.  Behind a search the tasks of the few clouds
+  // that it left are next to one another: they go to one SM after the other.
+  constexpr bool SPREAD = !std::is_same<Only, SpAll>::value;
+  for (int blk = SPREAD ? blockIdx.x + grp * gridDim.x : blockIdx.x * groups + grp; blk < blocks_total;
+       blk += gridDim.x * groups) {
     const int dir = blk >= blocks1;
     const int id = dir ? blk - blocks1 : blk;
     const float *qpts = dir ? xyz2 : xyz1;
@@ -308,6 +314,7 @@ chamfer_fwd_smwide_kernel(const float *__restrict__ xyz1, const float *__restric
     const XyzLayout lq = dir ? l2 : l1, lr = dir ? l1 : l2;
     const int chunks = (nq + TH * Q - 1) / (TH * Q);
     const int64_t b = id / chunks;
+    if (only.skip(b)) continue;
     const int i0 = (id % chunks) * (TH * Q) + tid;
 
     float qx[Q], qy[Q], qz[Q], thr[Q], best[Q];
@@ -411,16 +418,21 @@ chamfer_fwd_smwide_kernel(const float *__restrict__ xyz1, const float *__restric
 constexpr int SMWIDE_GROUPS = 7;
 
 int launch_smwide(const float *xyz1, const float *xyz2, int64_t B, int N1, int N2, float *dist1, int64_t *idx1,
-                  float *dist2, int64_t *idx2, double *sums, cudaStream_t st, XyzLayout l1, XyzLayout l2) {
+                  float *dist2, int64_t *idx2, double *sums, cudaStream_t st, XyzLayout l1, XyzLayout l2,
+                  SpOnly only) {
   const int64_t blocks1 = B * ((N1 + 255) / 256), blocks2 = B * ((N2 + 255) / 256);
   const int64_t total = blocks1 + blocks2;
   const size_t smem = (size_t)SMWIDE_GROUPS * 2 * CF_TILE * sizeof(float4);  // 112 KB
-  TK3D_CUDA(raise_smem_limit((const void *)chamfer_fwd_smwide_kernel<4>, (int)smem));
   const int64_t blocks = (total + SMWIDE_GROUPS - 1) / SMWIDE_GROUPS;
   const int64_t cap = sm_count();
-  chamfer_fwd_smwide_kernel<4><<<(unsigned)(blocks < cap ? blocks : cap), 128 * SMWIDE_GROUPS, smem, st>>>(
-      xyz1, xyz2, N1, N2, dist1, idx1, dist2, idx2, sums, (int)blocks1, (int)total, l1, l2);
-  return check_launch("chamfer_fwd_smwide_kernel");
+  auto go = [&](auto what) {
+    auto kern = chamfer_fwd_smwide_kernel<4, decltype(what)>;
+    TK3D_CUDA(raise_smem_limit((const void *)kern, (int)smem));
+    kern<<<(unsigned)(blocks < cap ? blocks : cap), 128 * SMWIDE_GROUPS, smem, st>>>(
+        xyz1, xyz2, N1, N2, dist1, idx1, dist2, idx2, sums, (int)blocks1, (int)total, l1, l2, (int)B, what);
+    return check_launch("chamfer_fwd_smwide_kernel");
+  };
+  return only.q ? go(only) : go(SpAll{});
 }
 
 }  // namespace
@@ -464,18 +476,21 @@ static int chamfer_lanes(int64_t nq) {
 // One direction (or both) with one query per thread and the lane count that suits `nq` queries.
 static int launch_lanes(int64_t nq, const float *xyz1, const float *xyz2, int64_t B, int N1, int N2, float *dist1,
                         int64_t *idx1, float *dist2, int64_t *idx2, double *sums, cudaStream_t st, XyzLayout l1,
-                        XyzLayout l2, int only_dir) {
-  switch (chamfer_lanes(nq)) {
-    case 8: return launch<1, 1, 2, 128, 8>(xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, only_dir);
-    case 4: return launch<1, 1, 2, 128, 4>(xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, only_dir);
-    case 2: return launch<1, 1, 2, 128, 2>(xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, only_dir);
-    default: return launch<1, 1, 2>(xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, only_dir);
-  }
+                        XyzLayout l2, int only_dir, SpOnly only) {
+  const int lanes = chamfer_lanes(nq);
+  auto go = lanes == 8   ? launch<1, 1, 2, 128, 8>
+            : lanes == 4 ? launch<1, 1, 2, 128, 4>
+            : lanes == 2 ? launch<1, 1, 2, 128, 2>
+                         : launch<1, 1, 2, 128, 1>;
+  return go(xyz1, xyz2, B, N1, N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, only_dir, only);
 }
 
 int chamfer_fwd_f32_fast(const float *xyz1, const float *xyz2, int64_t B, int64_t N1, int64_t N2, float *dist1,
                          int64_t *idx1, float *dist2, int64_t *idx2, double *sums, cudaStream_t st, XyzLayout l1,
-                         XyzLayout l2) {
+                         XyzLayout l2, SpOnly only) {
+  // `only`: behind a search over ordered clouds, the pairs that it left.  They are swept in the shape for all pairs,
+  // which is right where all are left (chamfer 1 x 2048 x 65536 with a NaN 1.57 ms, 5.03 in the shape for large batches;
+  // k = 3, 1 x 1000 x 100000 1.45, 8.20).
   const int64_t sms = sm_count();
   const int64_t small = B * (N1 < N2 ? N1 : N2), large = B * (N1 < N2 ? N2 : N1);
   // Clouds of very different sizes: the direction with few queries sweeps the large cloud and is
@@ -483,20 +498,22 @@ int chamfer_fwd_f32_fast(const float *xyz1, const float *xyz2, int64_t B, int64_
   // and its own shape (1 x 300 x 50000: 0.54 -> 0.19 ms).
   if (small > 0 && large >= 4 * small && 2 * small < sms * 2 * 128 * 2) {
     const int few = N1 < N2 ? 0 : 1;  // the direction whose queries are the small cloud
-    int rc = launch_lanes(2 * small, xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, few);
+    int rc = launch_lanes(2 * small, xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, few,
+                          only);
     if (rc) return rc;
     if (2 * large < sms * 2 * 128 * 2)
       return launch_lanes(2 * large, xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2,
-                          1 - few);
-    return launch<2, 6, 4>(xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, 1 - few);
+                          1 - few, only);
+    return launch<2, 6, 4>(xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, 1 - few, only);
   }
   // Measured on B200 (B=64, N=M=16384): two queries per thread, six resident blocks per SM and a
   // four-fold unrolled key loop beat four queries per thread by about 10 %.
   switch (chamfer_fwd_f32_plan(B, N1, N2)) {
     case 0:
-      return launch_lanes(B * (N1 + N2), xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, -1);
-    case 1: return launch_smwide(xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2);
-    default: return launch<2, 6, 4>(xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2);
+      return launch_lanes(B * (N1 + N2), xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2,
+                          -1, only);
+    case 1: return launch_smwide(xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, only);
+    default: return launch<2, 6, 4>(xyz1, xyz2, B, (int)N1, (int)N2, dist1, idx1, dist2, idx2, sums, st, l1, l2, -1, only);
   }
 }
 
@@ -516,8 +533,7 @@ int chamfer_fwd_f32_ordered(const float *xyz1, const float *xyz2, int64_t B, int
     int rc = sp_build(c1, &c2, n, st);
     if (!rc) rc = sp_chamfer(c1, c2, n, d1, i1, d2, i2, sums, st);
     if (!rc)
-      rc = launch<2, 6, 4>(p1, p2, n, (int)N1, (int)N2, d1, i1, d2, i2, sums, st, c1.l, c2.l, -1,
-                           SpOnly{c1.grid, c2.grid});
+      rc = chamfer_fwd_f32_fast(p1, p2, n, N1, N2, d1, i1, d2, i2, sums, st, c1.l, c2.l, SpOnly{c1.grid, c2.grid});
     if (rc) return rc;
   }
   return TK3D_OK;

@@ -993,7 +993,7 @@ int knn_small(const float *query, const float *key, int64_t B, int N1, int N2, f
   const int64_t per = KN_THREADS * Q / LANES;
   const int64_t total = B * ((N1 + per - 1) / per);
   // behind a search usually nothing is left: about a round of blocks looks
-  const int64_t cap = (int64_t)sm_count() * (io.only.q ? 6 : 256);
+  const int64_t cap = (int64_t)sm_count() * (io.only.q ? 12 : 256);
   const unsigned grid = (unsigned)(total < cap ? total : cap);
   const bool firstx = LANES > 1 && N2 <= 16384;  // few key tiles: the first one is worth extra exchanges
   auto go = [&](auto only) {
@@ -1086,6 +1086,18 @@ int knn_twopass(const float *query, const float *key, int64_t B, int N1, int N2,
   return io.only.q ? go(io.only) : go(SpAll{});
 }
 
+// 4 < k <= 64
+int knn_twopass_k(const float *query, const float *key, int64_t B, int N1, int N2, int k, float *dist, const KnnIo &io,
+                  cudaStream_t st) {
+  if (k <= 16) {
+    if (B * N1 >= (int64_t)sm_count() * 4 * 64)
+      return knn_twopass<2, 32, 56, 7>(query, key, B, N1, N2, k, dist, io, st);
+    return knn_twopass<1, 32, 56, 7>(query, key, B, N1, N2, k, dist, io, st);
+  }
+  if (k <= 32) return knn_twopass<1, 64, 104, 5>(query, key, B, N1, N2, k, dist, io, st);
+  return knn_twopass<1, 128, 192, 4>(query, key, B, N1, N2, k, dist, io, st);
+}
+
 }  // namespace
 
 // Whether the ordered search takes this k, and whether ordering the clouds first pays.
@@ -1130,15 +1142,13 @@ int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int
       rc = k <= 4 ? sp_knn_small(cq, ck, n, k, weights, eps, d, io.index, st)
                   : sp_knn_select(cq, ck, n, k, d, io.index, st);
     if (rc) return rc;
+    // what the order left is swept by the kernel that serves a call without scratch
     switch (k) {
-      case 1: rc = knn_small<1, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
-      case 2: rc = knn_small<2, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
-      case 3: rc = knn_small<3, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
-      case 4: rc = knn_small<4, 2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
-      default:
-        rc = k <= 16   ? knn_twopass<1, 32, 56, 7>(q, r, n, (int)N1, (int)N2, k, d, io, st)
-             : k <= 32 ? knn_twopass<1, 64, 104, 5>(q, r, n, (int)N1, (int)N2, k, d, io, st)
-                       : knn_twopass<1, 128, 192, 4>(q, r, n, (int)N1, (int)N2, k, d, io, st);
+      case 1: rc = knn_small_q<1>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      case 2: rc = knn_small_q<2>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      case 3: rc = knn_small_q<3>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      case 4: rc = knn_small_q<4>(q, r, n, (int)N1, (int)N2, d, io, st); break;
+      default: rc = knn_twopass_k(q, r, n, (int)N1, (int)N2, k, d, io, st);
     }
     if (rc) return rc;
     if (weights) {
@@ -1245,15 +1255,8 @@ static int knn_impl(const void *query, const void *key, int64_t B, int64_t N1, i
   // With fewer than 16 keys per wanted neighbour the class minima stop bounding anything for
   // k > 40 (16 x 4096 x 300, k = 64: 0.47 ms two-pass, 0.26 ms by radix).
   const bool by_radix = (k > 64 || (k > 40 && N2 < 16 * k)) && k <= 256 && N2 < (1LL << 31);
-  if (!by_radix && k <= 64 && N2 >= 4 * k && N2 >= 256) {
-    if (k <= 16) {
-      if (B * N1 >= (int64_t)sm_count() * 4 * 64)
-        return knn_twopass<2, 32, 56, 7>(q, r, B, (int)N1, (int)N2, (int)k, d, io, st);
-      return knn_twopass<1, 32, 56, 7>(q, r, B, (int)N1, (int)N2, (int)k, d, io, st);
-    }
-    if (k <= 32) return knn_twopass<1, 64, 104, 5>(q, r, B, (int)N1, (int)N2, (int)k, d, io, st);
-    return knn_twopass<1, 128, 192, 4>(q, r, B, (int)N1, (int)N2, (int)k, d, io, st);
-  }
+  if (!by_radix && k <= 64 && N2 >= 4 * k && N2 >= 256)
+    return knn_twopass_k(q, r, B, (int)N1, (int)N2, (int)k, d, io, st);
   // key clouds too small for the two-pass kernel: buffered lists up to k = 40 (16 x 4096 x 300:
   // 0.069 ms at k = 16 against 0.195 by radix, 0.47 against 0.26 at k = 64)
   if (k <= 40) {
