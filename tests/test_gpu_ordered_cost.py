@@ -81,3 +81,9 @@ def _both(k, B, N, M, kinds):
 def test_flagged_clouds_are_swept_by_the_kernel_that_serves_a_call_without_scratch(k, B, N, M):
     plain, ordered = _both(k, B, N, M, ("nan", "nan"))
     assert ordered < 1.25 * plain + 40
+
+
+@pytest.mark.parametrize("k", [5, 16, 32])
+def test_keys_away_from_the_queries_are_told_apart(k):
+    plain, ordered = _both(k, 16, 4096, 4096, ("away", "sphere"))
+    assert ordered < 1.25 * plain + 40

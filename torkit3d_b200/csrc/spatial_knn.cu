@@ -50,6 +50,7 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
   int *cand = reinterpret_cast<int *>(sk_smem + QCAP * 32 * 4);  // [QCAP][32] leaves, then key indices
   unsigned short *list = reinterpret_cast<unsigned short *>(sk_smem + QCAP * 32 * 8);  // [2][SK_LIST]
   __shared__ int counts[2][SK_WARPS][32];
+  __shared__ float least[SK_WARPS][32];
   __shared__ int ccnt[32], fcnt[32], hcnt[32];
   __shared__ int nlist[3];
   __shared__ float4 sq[32];  // the queries and their bounds
@@ -77,10 +78,15 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
     if (lane < 3) nlist[lane] = 0;
   }
 
-  // a bound with at least k class minima at or below it, starting from `hi`, which is one
+  // a bound with at least k class minima at or below it, starting from `hi`, which is one, and the smallest
   float cmin[CPW];
   auto kth_bound = [&](float hi) {
-    float lo = 0.f;
+    float lo = cmin[0];
+#pragma unroll
+    for (int c = 1; c < CPW; ++c) lo = fminf(lo, cmin[c]);
+    least[part][lane] = lo;
+    __syncthreads();
+    lo = fminf(fminf(least[0][lane], least[1][lane]), fminf(least[2][lane], least[3][lane]));
 #pragma unroll 1
     for (int it = 0; it < SK_STEPS; ++it) {
       const float mid = 0.5f * (lo + hi);
