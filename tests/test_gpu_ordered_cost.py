@@ -87,3 +87,9 @@ def test_flagged_clouds_are_swept_by_the_kernel_that_serves_a_call_without_scrat
 def test_keys_away_from_the_queries_are_told_apart(k):
     plain, ordered = _both(k, 16, 4096, 4096, ("away", "sphere"))
     assert ordered < 1.25 * plain + 40
+
+
+@pytest.mark.parametrize("k,N", [(64, 1024), (16, 4096)])
+def test_groups_with_long_lists_do_not_go_through_all_leaves(k, N):
+    plain, ordered = _both(k, 4, N, 65536, ("blobs", "blobs"))
+    assert ordered < 1.25 * plain + 40

@@ -16,7 +16,9 @@
 //      ties) falls back to an exact scan of all keys by one warp.
 // All distances are the exactly rounded ones (two keys per packed operation), so the bounds need no
 // error analysis.  A bound is found by bisection over the class minima, which stay in registers: any
-// value with k minima at or below it will do, and eight steps come within 1/256 of the best.
+// value with k minima at or below it will do, and eight steps from the smallest minimum come within 1/256 of the
+// best (from 0 the keys of a cloud that lies away from the queries could not be told apart, lists overflowed, and
+// 16 x 4096 x 4096, k = 16, ten radii away, took 1.03 ms; now 0.087).
 //
 // 0.5 instructions a cycle and scheduler, bound by latency (barriers of the bisection, gathers of the
 // selection): 16 x 4096 x 4096, k = 16: 0.11 ms plus 0.03 ms for the order (two passes over all keys:
@@ -30,12 +32,12 @@ namespace {
 
 constexpr int SK_THREADS = 128;
 constexpr int SK_WARPS = SK_THREADS / 32;
-constexpr int SK_LIST = 1024;  // listed leaves; more than that and the block goes through all of them
+constexpr int SK_LIST = 2048;  // leaves of the second sweep; more than that and it goes over those of the first one
 constexpr int SK_STEPS = 8;
 
 template <int QCAP>
 constexpr size_t sk_smem_bytes() {
-  return (size_t)QCAP * 32 * 8 + 2 * SK_LIST * 2;
+  return (size_t)QCAP * 32 * 8 + SK_LIST * 2;
 }
 
 template <int NCH, int QCAP, int MINB>
@@ -48,7 +50,12 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
   extern __shared__ __align__(16) unsigned char sk_smem[];
   float *cd = reinterpret_cast<float *>(sk_smem);                // [QCAP][32] exact distances
   int *cand = reinterpret_cast<int *>(sk_smem + QCAP * 32 * 4);  // [QCAP][32] leaves, then key indices
-  unsigned short *list = reinterpret_cast<unsigned short *>(sk_smem + QCAP * 32 * 8);  // [2][SK_LIST]
+  // Leaves within reach of the group, in the place of the candidates; of one query, in the place of the distances; and
+  // those of the second sweep.  Tails of a cloud have long lists (65536 points in blobs, k = 16: up to 1500 leaves;
+  // a group that went through all 8192 instead took 1.2 ms by itself).
+  constexpr int FIRST = QCAP * 64;
+  unsigned short *list0 = reinterpret_cast<unsigned short *>(cand), *list1 = reinterpret_cast<unsigned short *>(cd),
+                 *list2 = reinterpret_cast<unsigned short *>(sk_smem + QCAP * 32 * 8);
   __shared__ int counts[2][SK_WARPS][32];
   __shared__ float least[SK_WARPS][32];
   __shared__ int ccnt[32], fcnt[32], hcnt[32];
@@ -148,14 +155,14 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
         int at = 0;
         if (lane == 0 && m) at = atomicAdd(&nlist[0], __popc(m));
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
-        if (hit && at < SK_LIST) list[at] = (unsigned short)l;
+        if (hit && at < FIRST) list0[at] = (unsigned short)l;
       }
     }
   }
   if (part == 0) sq[lane] = make_float4(q.x, q.y, q.z, valid ? tau0 : -1.f);
   __syncthreads();
   // leaves of `from` (or all of them) within reach of one of the queries go to `to`
-  auto cut = [&](const unsigned short *from, int count, unsigned short *to, int *total) {
+  auto cut = [&](const unsigned short *from, int count, unsigned short *to, int room, int *total) {
     for (int l0 = part * 32; l0 < count; l0 += SK_THREADS) {
       const int l = l0 + lane < count ? (from ? from[l0 + lane] : l0 + lane) : -1;
       bool hit = false;
@@ -171,13 +178,13 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
       int at = 0;
       if (lane == 0 && m) at = atomicAdd(total, __popc(m));
       at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
-      if (hit && at < SK_LIST) to[at] = (unsigned short)l;
+      if (hit && at < room) to[at] = (unsigned short)l;
     }
   };
-  const bool most = nlist[0] > SK_LIST;
-  cut(most ? nullptr : list, most ? kc.windows * 32 : nlist[0], list + SK_LIST, &nlist[1]);
+  const bool most = nlist[0] > FIRST;
+  cut(most ? nullptr : list0, most ? kc.windows * 32 : nlist[0], list1, FIRST, &nlist[1]);
   __syncthreads();
-  const bool all = nlist[1] > SK_LIST;
+  const bool all = nlist[1] > FIRST;
   const int n1 = all ? kc.windows * 32 : nlist[1];
 
   // ---- 3. class minima over the listed leaves
@@ -187,26 +194,25 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = li + u * SK_WARPS;
-      if (i < n1) take(kpts + (all ? i : list[SK_LIST + i]) * 32, 8 * u);
+      if (i < n1) take(kpts + (all ? i : list1[i]) * 32, 8 * u);
     }
   }
   const float tau1 = kth_bound(tau0);
 
   // ---- 4. leaves with a distance at or below tau1
-  if (!all) {
-    if (part == 0) sq[lane].w = valid ? tau1 : -1.f;
-    __syncthreads();
-    cut(list + SK_LIST, n1, list, &nlist[2]);
-    __syncthreads();
-  }
-  const int n2 = all ? n1 : nlist[2];
+  if (part == 0) sq[lane].w = valid ? tau1 : -1.f;
+  __syncthreads();
+  cut(all ? nullptr : list1, n1, list2, SK_LIST, &nlist[2]);
+  __syncthreads();
+  const unsigned short *last = nlist[2] <= SK_LIST ? list2 : all ? nullptr : list1;
+  const int n2 = nlist[2] <= SK_LIST ? nlist[2] : n1;
   // the next float above tau1 (tau1 >= 0): "below it" is "at or below tau1"
   const float thr = valid ? (tau1 < pinf() ? __int_as_float(__float_as_int(tau1) + 1) : tau1) : -pinf();
   const unsigned cnt_addr = (unsigned)__cvta_generic_to_shared(ccnt + lane);
   const unsigned cand_addr = (unsigned)__cvta_generic_to_shared(cand + lane);
 #pragma unroll 2
   for (int li = part; li < n2; li += SK_WARPS) {
-    const int leaf = all ? li : list[li];
+    const int leaf = last ? last[li] : li;
     float2 d[4];
     sp_leaf_dist(kpts + leaf * 32, nx, ny, nz, one, d);
     // padding keys have NaN distances, which the minima drop; a leaf of nothing else gives +inf
