@@ -93,3 +93,10 @@ def test_keys_away_from_the_queries_are_told_apart(k):
 def test_groups_with_long_lists_do_not_go_through_all_leaves(k, N):
     plain, ordered = _both(k, 4, N, 65536, ("blobs", "blobs"))
     assert ordered < 1.25 * plain + 40
+
+
+@pytest.mark.parametrize("kinds", [("collapsed", "sphere"), ("outlier", "outlier")])
+@pytest.mark.parametrize("k,B,N", [(0, 32, 4096), (0, 2, 8192), (1, 16, 4096), (3, 16, 4096), (16, 16, 4096)])
+def test_clouds_that_the_order_does_not_serve_are_found_out(k, B, N, kinds):
+    plain, ordered = _both(k, B, N, N, kinds)
+    assert ordered < 1.25 * plain + 40

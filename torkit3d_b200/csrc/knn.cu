@@ -1137,7 +1137,7 @@ int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int
     io.ql = cq.l;
     io.kl = ck.l;
     io.only = SpOnly{cq.grid, ck.grid};
-    int rc = sp_build(cq, same ? nullptr : &ck, n, st);
+    int rc = sp_build(cq, same ? nullptr : &ck, n, SpUse{false, k <= 32 || N2 > 8192, k <= 4, 0, 0.f}, st);
     if (!rc)
       rc = k <= 4 ? sp_knn_small(cq, ck, n, k, weights, eps, d, io.index, st)
                   : sp_knn_select(cq, ck, n, k, d, io.index, st);

@@ -24,19 +24,41 @@ struct SpPair {
   SpCloud c[2];
 };
 
-// A ball query's radius and row length (k = 0: another search).  Where balls hold more than about twice
-// the wanted hits, sweeping the keys in index order stops early and ordering them is wasted: the sort
-// looks at 16 queries and 512 keys of its cloud pair first (every block at the same ones) and flags
-// such a pair as irregular.  32 x 1024 queries of 8192 keys, k = 32, 20 / 100 / 1000 hits, us: sweep 137,
-// 95, 29; ordered 72, 171, 145.
-struct SpPeek {
-  float r2;
-  int k;
-};
+// Inputs that the order would not serve are found out from a sample before anything is sorted, and flagged as
+// irregular.
+//
+// Dense balls (16 queries and 512 keys).  Where balls hold more than about twice the wanted hits, sweeping the keys
+// in index order stops early and ordering them is wasted.  32 x 1024 queries of 8192 keys, k = 32, 20 / 100 /
+// 1000 hits, us: sweep 137, 95, 29; ordered 72, 171, 145.
+//
+// Nothing to prune.  Where most sampled keys are no farther from a query than its nearest sampled key and the
+// spacing of the sample together, most leaves come within reach of every group of queries: a cloud that has
+// collapsed, or lies in the middle of the other one.  The share of such keys was at most 0.1 for volumes, surfaces,
+// blobs, lattices and clouds away from one another, and 0.9 and more for a cloud of radius 0.01 in the middle
+// of a sphere (sweep / ordered, us: chamfer 32 x 4096^2 208 / 384, 2 x 8192^2 102 / 309, k = 3 16 x 4096^2
+// 133 / 246, k = 16 168 / 342, k = 32 340 / 450, k = 64 709 / 700: flagged above a half, up to 32 neighbours).
+// The look costs 2 to 3 us; a flagged pair pays 10 to 20 us over its sweep.
+//
+// A grid too coarse.  Where a fine cell around a point holds a good part of the cloud, the windows cannot be sorted:
+// an outlier that squeezes all other points into a few cells, heavy tails.  Share of the cloud in such a cell and
+// sweep / ordered, us, chamfer 32 x 4096^2: a sphere with an outlier at 10 radii 0.0001, 229 / 83; at 100 radii
+// 0.012, 229 / 255; at 1000 all of it, 229 / 616; points on a line 0.004, 245 / 93: flagged above 1 / PK_COARSE.
+// More than four neighbours are found twice to ten times as fast in order even then (16 x 4096^2, k = 16, 1000
+// radii: 1950 / 460), because the sweep's lists overflow.
+constexpr int PK_SAMPLE = 8;  // queries, and keys whose surroundings are looked at
+constexpr int PK_KEYS = 128;  // keys they are held against
+constexpr int PK_COARSE = 32;
+static_assert(PK_KEYS == 128 && SB_WARPS == 16, "two directions, four slices of the keys, two halves of the queries");
+
+// Sampled key i of N: one of each PK_KEYS-th of the cloud, at varying places (a cloud that repeats itself must not
+// give the same points over and over).
+__device__ __forceinline__ int64_t pk_key(int i, int N) {
+  return ((int64_t)(i * PK_KEYS + ((i * 73) & (PK_KEYS - 1))) * N) / (PK_KEYS * PK_KEYS);
+}
 
 template <int CL>
 __global__ void __launch_bounds__(SB_THREADS, 2)
-spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
+spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpUse use) {
   constexpr int SHARE = SP_CELLS / CL;      // cells of one block
   constexpr int MINE = SHARE / SB_THREADS;  // cells of one thread
   static_assert(MINE >= 1 && MINE * CL * SB_THREADS == SP_CELLS, "whole cells per thread");
@@ -50,7 +72,9 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
   __shared__ float red[SB_WARPS][8];
   __shared__ float part[8];  // this block's (lo, hi, non-finite)
   __shared__ int warp_total[SB_WARPS];
-  __shared__ int block_total, crowd;
+  __shared__ int block_total, crowd, close;
+  __shared__ __align__(16) float least[2][2][PK_SAMPLE / CL][PK_KEYS / 32];
+  __shared__ int near[2];  // sampled keys that would come within reach
   auto sync = [&]() {
     if constexpr (CL > 1) cluster.sync();
     else __syncthreads();
@@ -65,7 +89,7 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
   const int NL = (N + CL - 1) / CL;
   const int beg = min(N, rank * NL), end = min(N, beg + NL);
 
-  if (peek.k > 0) {
+  if (use.row > 0) {
     const SpCloud &qc = pair.c[0], &kc = pair.c[1];
     float kx, ky, kz;
     load_xyz(kc.xyz + b * 3 * (int64_t)kc.N, (int64_t)tid * kc.N / SB_THREADS, kc.l, kx, ky, kz);
@@ -74,7 +98,7 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
     for (int i = 0; i < 16; ++i) {
       float x, y, z;
       load_xyz(qc.xyz + b * 3 * (int64_t)qc.N, (int64_t)i * qc.N / 16, qc.l, x, y, z);
-      hits += sqdist<float>(kx, ky, kz, x, y, z) < peek.r2 ? 1 : 0;
+      hits += sqdist<float>(kx, ky, kz, x, y, z) < use.r2 ? 1 : 0;
     }
     hits = __reduce_add_sync(0xffffffffu, hits);
     if (lane == 0) warp_total[warp] = hits;
@@ -83,7 +107,7 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
 #pragma unroll
     for (int w = 0; w < SB_WARPS; ++w) hits += warp_total[w];
     // hits per query = hits * N2 / (16 * 512)
-    if ((double)hits * kc.N > 2.0 * 16 * SB_THREADS * peek.k) {  // the same in all blocks of the cluster
+    if ((double)hits * kc.N > 2.0 * 16 * SB_THREADS * use.row) {  // the same in all blocks of the cluster
       if (rank == 0 && tid == 0) c.grid[b].irregular = 1;
       return;
     }
@@ -92,7 +116,32 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
 
 #pragma unroll
   for (int e = 0; e < SP_CELLS / SB_THREADS; ++e) hist[tid + e * SB_THREADS] = 0;
-  if (tid == 0) crowd = 0;
+  if (tid == 0) crowd = close = 0;
+
+  // This block's share of the sample, PER queries in each direction: 0 searches a's points in b, 1 the other way round.
+  // A warp takes one direction, 32 of the keys and half of the queries.
+  constexpr int PER = PK_SAMPLE / CL, HALF = (PER + 1) / 2;
+  const int dir = warp & 1, slice = (warp >> 1) & (PK_KEYS / 32 - 1), i0 = (warp >> 3) * HALF;
+  const bool looks = use.prunes && (dir == 0 || use.both) && i0 < PER;
+  float reach[HALF];
+  if (looks) {
+    const SpCloud &qc = pair.c[dir], &kc = pair.c[1 - dir];
+    const float *kx = kc.xyz + b * 3 * (int64_t)kc.N, *qx = qc.xyz + b * 3 * (int64_t)qc.N;
+    float x, y, z;
+    load_xyz(kx, pk_key(slice * 32 + lane, kc.N), kc.l, x, y, z);
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {  // nearest sampled key of every query, nearest other one of every key
+      const int s = rank * PER + i0 + i;
+      float u, w, r;
+      load_xyz(qx, (int64_t)s * qc.N / PK_SAMPLE, qc.l, u, w, r);
+      reach[i] = sp_sq3(u - x, w - y, r - z);
+      load_xyz(kx, pk_key(s * (PK_KEYS / PK_SAMPLE), kc.N), kc.l, u, w, r);
+      const float e = sp_sq3(u - x, w - y, r - z);
+      const float dq = sp_warp_min(reach[i]), dk = sp_warp_min(e > 0.f ? e : sp_inf());
+      if (lane == 0) least[dir][0][i0 + i][slice] = dq, least[dir][1][i0 + i][slice] = dk;
+    }
+  }
+  if (tid < 2) near[tid] = 0;
   float v[7] = {sp_inf(), sp_inf(), sp_inf(), -sp_inf(), -sp_inf(), -sp_inf(), 0.f};
 #pragma unroll 4
   for (int j = beg + tid; j < end; j += SB_THREADS) {
@@ -117,6 +166,22 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
       if (lane == 0) part[i] = r;
     }
   }
+  if (looks) {
+    auto min4 = [](const float(&m)[PK_KEYS / 32]) { return fminf(fminf(m[0], m[1]), fminf(m[2], m[3])); };
+    // the geometric mean of the spacings: neither an outlier nor a pair of close keys weighs much
+    float lg = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) lg += 0.5f * __log2f(fminf(fmaxf(min4(least[dir][1][i]), 1e-30f), 1e30f));
+    const float spacing = exp2f(lg / PER);
+    int hits = 0;
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {
+      const float r = sqrtf(min4(least[dir][0][i0 + i])) + spacing;
+      hits += reach[i] <= r * r ? 1 : 0;
+    }
+    hits = __reduce_add_sync(0xffffffffu, hits);
+    if (lane == 0) atomicAdd(&near[dir], hits);
+  }
   sync();
 #pragma unroll
   for (int i = 0; i < 7; ++i) {
@@ -133,7 +198,36 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
   const float ext = fmaxf(fmaxf(v[3] - v[0], v[4] - v[1]), v[5] - v[2]);
   g.inv = (ext > 0.f && ext < sp_inf()) ? 256.f / ext : 0.f;
   g.irregular = v[6] != 0.f;
+  g.pad[0] = g.pad[1] = g.pad[2] = 0;
+  if (use.prunes) {
+    int within[2] = {0, 0};
+#pragma unroll
+    for (int o = 0; o < CL; ++o) {
+      within[0] += remote(near, o)[0];
+      within[1] += remote(near, o)[1];
+    }
+    constexpr int MOST = PK_SAMPLE * PK_KEYS / 2;
+    if (within[0] > MOST || (use.both && within[1] > MOST)) g.irregular = 1;
+  }
+  if (g.irregular) {  // no search looks at the cloud; the same in all blocks, and nobody leaves before all have read
+    if (rank == 0 && tid == 0) c.grid[b] = g;
+    sync();
+    return;
+  }
 
+  if (use.resolves) {
+    const float half = 0.5f * ext * (1.f / 256.f);
+    float x, y, z;
+    load_xyz(xyz, pk_key((warp & (PK_KEYS / 32 - 1)) * 32 + lane, N), c.l, x, y, z);
+    int same = 0;
+    for (int i = warp / (PK_KEYS / 32); i < PER; i += SB_WARPS / (PK_KEYS / 32)) {
+      float u, w, r;
+      load_xyz(xyz, pk_key((rank * PER + i) * (PK_KEYS / PK_SAMPLE), N), c.l, u, w, r);
+      const float e = fmaxf(fmaxf(fabsf(u - x), fabsf(w - y)), fabsf(r - z));
+      same += __popc(__ballot_sync(0xffffffffu, e > 0.f && e <= half));
+    }
+    if (lane == 0 && same) atomicAdd(remote(&close, 0), same);
+  }
 #pragma unroll 4
   for (int j = beg + tid; j < end; j += SB_THREADS) {
     float x, y, z;
@@ -173,6 +267,8 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
     sync();
     for (int o = 0; o < rank; ++o) at += *remote(&block_total, o);
   }
+  g.irregular = 2 * (int64_t)*remote(&crowd, 0) > N;  // complete since the last barrier
+  if (use.resolves && *remote(&close, 0) * PK_COARSE > PK_SAMPLE * PK_KEYS) g.irregular = 1;
 #pragma unroll
   for (int i = 0; i < MINE; ++i) {
     c.table[b * SP_CELLS + c0 + i] = at;
@@ -182,7 +278,9 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
       at += n[o][i];
     }
   }
-  sync();
+  sync();  // the last access to another block's shared memory lies behind every block
+  if (rank == 0 && tid == 0) c.grid[b] = g;
+  if (g.irregular) return;
 
 #pragma unroll 4
   for (int j = beg + tid; j < end; j += SB_THREADS) {
@@ -195,11 +293,6 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpPeek peek) {
     // padding of the last window: NaN distances are never below or at a bound
     for (int j = N + tid; j < c.windows * SP_WINDOW; j += SB_THREADS)
       pts[j] = make_float4(sp_nan(), sp_nan(), sp_nan(), __int_as_float(0x7fffffff));
-    if (tid == 0) {
-      if (2 * (int64_t)crowd > N) g.irregular = 1;
-      g.pad[0] = g.pad[1] = g.pad[2] = 0;
-      c.grid[b] = g;
-    }
   }
 }
 
@@ -508,7 +601,7 @@ spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sum
 
 }  // namespace
 
-int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st, float r2, int k) {
+int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, const SpUse &use, cudaStream_t st) {
   const int64_t clouds = b ? 2 * B : B;
   const int big = b && b->N > a.N ? b->N : a.N;
   // Blocks per cloud: as many as the SMs hold at once (two each), at least 512 points per block.
@@ -533,8 +626,8 @@ int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st, flo
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  SpPeek peek{r2, k};
-  void *args[] = {&pair, &B_, &peek};
+  SpUse use_ = use;
+  void *args[] = {&pair, &B_, &use_};
   TK3D_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
   const int64_t w0 = B * a.windows, total = w0 + (b ? B * b->windows : 0);
   const int64_t per = SW_THREADS / 32;

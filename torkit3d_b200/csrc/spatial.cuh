@@ -22,11 +22,12 @@
 // without any slack.  A leaf also carries the lowest original index among its points, so a leaf
 // whose box is exactly at the current distance is visited only if it can win the tie.
 //
-// What the index cannot serve is flagged per cloud (SpGrid::irregular): non-finite coordinates
-// (their ordering rules belong to the sweeping kernels), and clouds of which more than half sit in
-// cells of more than SP_CROWD points (duplicates, or an outlier that stretches the grid), where boxes
-// prune little; a ball query also flags pairs of clouds whose balls are dense.  The searches skip flagged clouds and the sweeping kernels, launched behind them,
-// skip all others.
+// What the index cannot serve is flagged per cloud (SpGrid::irregular): non-finite coordinates (their ordering
+// rules belong to the sweeping kernels), and clouds of which more than half sit in cells of more than SP_CROWD
+// points (duplicates, or an outlier that stretches the grid), where boxes prune little.  A sample finds more of
+// them out before anything is sorted (spatial.cu): a grid too coarse for the cloud, pairs of clouds so placed
+// that most leaves are within reach of every query, balls too dense.  The searches skip flagged clouds, and the
+// sweeping kernels, launched behind them, skip all others (a ball query sweeps where it is).
 #pragma once
 
 #include "tk3d_common.cuh"
@@ -104,9 +105,18 @@ inline char *sp_align_ptr(void *p) {
   return reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 255) & ~(uintptr_t)255);
 }
 
-// Builds the index of both sides (two launches); `b` may be null.  r2, k: of a ball query of a's points in
-// b's (k = 0: another search); pairs of clouds with dense balls are flagged irregular.
-int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, cudaStream_t st, float r2 = 0.f, int k = 0);
+// What the index is built for: a search of a's points in b, `both`: and the other way round.  Pairs of clouds that the
+// order would not serve are flagged irregular (spatial.cu):
+struct SpUse {
+  bool both;
+  bool prunes;    // where nothing would be pruned
+  bool resolves;  // where the grid is too coarse
+  int row;        // of a ball query: its row length and squared radius; where balls are dense
+  float r2;
+};
+
+// Builds the index of both sides (two launches); `b` may be null: both sides are a.
+int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, const SpUse &use, cudaStream_t st);
 
 // Searches over built indexes; rows of clouds that are irregular on either side are left alone.
 int sp_chamfer(const SpCloud &a, const SpCloud &b, int64_t B, float *dist1, int64_t *idx1, float *dist2, int64_t *idx2,

@@ -169,7 +169,7 @@ int sp_ball_query(const float *query, const float *key, int64_t B, int64_t N1, i
     const int64_t n = b0 + step < B ? step : B - b0;
     const SpCloud cq = sp_cloud(query + b0 * 3 * N1, channel_first, n, N1, at);
     const SpCloud ck = sp_cloud(key + b0 * 3 * N2, channel_first, n, N2, at + sp_cloud_bytes(n, N1));
-    int rc = sp_build(cq, &ck, n, st, r2, k);
+    int rc = sp_build(cq, &ck, n, SpUse{false, false, true, k, r2}, st);
     if (rc) return rc;
     spatial_ball_kernel<<<(unsigned)(n * cq.groups), SQ_THREADS, 0, st>>>(
         cq, ck, r2, k, index_out((char *)index + b0 * N1 * k * (index32 ? 4 : 8), index32, n * N1 * k), 1.0f);
