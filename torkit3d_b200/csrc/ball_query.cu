@@ -337,7 +337,10 @@ namespace tk3d {
 // 133 / 70 to 79, 32 x 4096 of 16384 845 / 260 to 312.  Dense balls are found out by a sample and swept:
 // the looking costs 12 us (32 x 1024 of 8192, 1000 hits: 29 / 41), hence not below 1.2e8 pairs.
 bool ball_order_pays(int64_t B, int64_t N1, int64_t N2) {
-  return sp_supported(B, N1, N2) && N2 <= SP_SELECT_POINTS && (double)B * N1 * N2 >= 1.2e8;
+  if (!sp_supported(B, N1, N2) || N2 > SP_SELECT_POINTS || (double)B * N1 * N2 < 1.2e8) return false;
+  // Few queries strewn over many keys (on a surface, in blobs, 25 hits): 16 x 512 x 16384 110 / 176, 217; 4 x 2048 x 65536
+  // 344 / 447, 490; but 16 x 1024 x 16384 168 / 72, 220; 4 x 2048 x 16384 111 / 47, 160; 1 x 4096 x 65536 304 / 68, 437.
+  return N2 <= 16 * N1 || B * N1 >= 200 * (int64_t)sm_count();
 }
 }  // namespace tk3d
 

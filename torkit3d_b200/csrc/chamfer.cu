@@ -316,6 +316,13 @@ extern "C" size_t tk3d_chamfer_fwd_scratch_bytes(int64_t B, int64_t N1, int64_t 
   // (sweep / ordered, us: 32 x 1024^2 45 / 52, 2 x 4096^2 56 / 60, 64 x 1024^2 71 / 66, 16 x 2048^2 67 / 58,
   // 8 x 4096^2 105 / 70, 24 x 2500 x 4099 162 / 107, 64 x 16384^2 5815 / 345 to 805).
   if (N1 < 1024 || N2 < 1024 || (double)B * N1 * N2 < 6e7) return 0;
+  // Few points strewn over a large cloud: groups of 32 of them reach for many leaves, and there are too few groups to
+  // hide it (sweep / ordered, points on a surface, in blobs: 4 x 1024 x 16384 136 / 80, 173; 4 x 1024 x 65536 357 /
+  // 250, 622; 1 x 2048 x 65536 350 / 146, 388; but 4 x 2048 x 16384 181 / 60, 168; 1 x 4096 x 65536 393 / 109, 251;
+  // 16 x 1024 x 16384 226 / 108, 190).
+  const int64_t small = N1 < N2 ? N1 : N2, large = N1 < N2 ? N2 : N1;
+  const bool many = B * small >= 200 * (int64_t)sm_count();
+  if (!many && (large > 16 * small || (large > 8 * small && small < 4096 && B * small < 16384))) return 0;
   return sp_search_bytes(B, N1, N2);
 }
 

@@ -1113,7 +1113,22 @@ bool knn_order_takes(int64_t B, int64_t N1, int64_t N2, int64_t k) {
 bool knn_order_pays(int64_t B, int64_t N1, int64_t N2, int64_t k) {
   const double pairs = (double)B * N1 * N2;
   const double least = k <= 4 ? 4e7 : k > 32 || N2 >= 8192 ? 2e7 : k > 16 ? 4e7 : k > 8 ? 1e8 : 1.6e8;
-  return knn_order_takes(B, N1, N2, k) && pairs >= least;
+  if (!knn_order_takes(B, N1, N2, k) || pairs < least) return false;
+  // Few queries strewn over many keys: a group of 32 reaches for many leaves, one after another, and there are too few
+  // groups to hide it, while the sweep takes several lanes per query.  k = 3, sweep / ordered (on a surface, in
+  // blobs): 16 x 1024 x 4096 69 / 83, 124; 4 x 4096 x 4096 69 / 45, 91; 4 x 2048 x 16384 142 / 92, 257; 4 x 4096 x
+  // 16384 192 / 73, 205; 1 x 8192 x 16384 140 / 60, 132; 1 x 16384 x 16384 191 / 58, 123; 16 x 2048 x 4096
+  // 113 / 79, 118; 4 x 8192 x 16384 265 / 84, 178; 1 x 1000 x 100000 421 / 337, 767.
+  if (k <= 4) {
+    const int64_t sms = sm_count(), nq = B * N1;
+    if (nq >= 200 * sms) return true;
+    if (N1 >= 8192) return nq >= 100 * sms ? pairs >= 1e8 : nq >= 50 * sms && pairs >= 1.3e8;
+    return N1 >= 4096 && nq >= 100 * sms && pairs >= 2e8;
+  }
+  // More neighbours: a block serves the 32 queries, which hides more (k = 32: 4 x 512 x 65536 706 / 190, 860; 16 x 256 x
+  // 65536 708 / 235, 870; k = 64: 16 x 512 x 65536 831 / 320, 985; k = 8: 1 x 256 x 100000 947 / 218, 1100; k = 16:
+  // 1 x 64 x 400000 4460 / 1600, 8190).
+  return k <= 16 ? N2 < 1024 * N1 : N2 < 128 * N1;
 }
 
 template <typename Only>
