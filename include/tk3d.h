@@ -121,7 +121,9 @@ int tk3d_knn(const void *query, const void *key, int64_t B, int64_t N1, int64_t 
  *   xyz_channel_first, index_dtype   as for the *_layout entry points
  *   scratch          device buffer of at least tk3d_*_scratch_bytes() bytes, contents ignored on entry;
  *                    NULL or a smaller buffer sweeps.  The size functions return 0 where ordering the
- *                    clouds does not pay or is not supported.
+ *                    clouds does not pay or is not supported; 512 MB at most (larger batches are cut).
+ * Pairs of clouds that the order would not serve are found out on the device and swept, and so is the whole
+ * call where the device refuses a thread-block cluster.
  */
 size_t tk3d_chamfer_fwd_scratch_bytes(int64_t B, int64_t N1, int64_t N2, int dtype);
 int tk3d_chamfer_fwd_ws(const void *xyz1, const void *xyz2, int64_t B, int64_t N1, int64_t N2, int xyz_channel_first,
@@ -468,8 +470,9 @@ int tk3d_diag_fps_wait_limit(const void *points, int64_t B, int64_t N, int64_t n
 int tk3d_diag_ffma(int64_t iters, float *sink, double *flop, void *stream);
 
 /*
- * Diagnostic with no counterpart in the reference: the name of the kernel that tk3d_chamfer_fwd
- * launches for these sizes on the current device (a static string; launches nothing).  The fp32
+ * Diagnostic with no counterpart in the reference: the name of the kernel that tk3d_chamfer_fwd, the sweep
+ * of all pairs, launches for these sizes on the current device (a static string; launches nothing).  With
+ * scratch (tk3d_chamfer_fwd_ws) the work is done by spatial_nn_kernel, and that kernel sweeps what is left.  The fp32
  * forward has three: "chamfer_fwd_fast_kernel<1>" (small inputs, one query per thread),
  * "chamfer_fwd_smwide_kernel" (one 896-thread block per SM, for one or two nearly full rounds of
  * 256-query tasks) and "chamfer_fwd_fast_kernel<2>" (everything larger); fp64 has

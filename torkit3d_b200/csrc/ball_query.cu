@@ -262,6 +262,29 @@ ball_query_generic_kernel(const T *__restrict__ query, const T *__restrict__ key
 }  // namespace
 }  // namespace tk3d
 
+namespace tk3d {
+
+// All pairs in float32.
+int ball_query_sweep_f32(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, float r2, int k,
+                         const IndexOut &index, XyzLayout ql, XyzLayout kl, cudaStream_t st) {
+  const int64_t cap = (int64_t)sm_count() * 256;
+  if (B * N1 < (int64_t)sm_count() * 16 * BQ_THREADS) {
+    const int64_t total = B * ((N1 + 31) / 32);
+    const unsigned grid = (unsigned)(total < cap ? total : cap);
+    if (total <= 2 * (int64_t)sm_count())  // very few queries: eight warps per 32 queries
+      ball_query_split_kernel<8><<<grid, 256, 0, st>>>(query, key, B, (int)N1, (int)N2, r2, k, index, total, ql, kl);
+    else
+      ball_query_split_kernel<4><<<grid, 128, 0, st>>>(query, key, B, (int)N1, (int)N2, r2, k, index, total, ql, kl);
+    return check_launch("ball_query_split_kernel");
+  }
+  const int64_t total = B * ((N1 + BQ_THREADS - 1) / BQ_THREADS);
+  ball_query_fast_kernel<<<(unsigned)(total < cap ? total : cap), BQ_THREADS, 0, st>>>(query, key, B, (int)N1, (int)N2, r2,
+                                                                                      k, index, total, ql, kl);
+  return check_launch("ball_query_fast_kernel");
+}
+
+}  // namespace tk3d
+
 using namespace tk3d;
 
 static int ball_query_impl(const void *query, const void *key, int64_t B, int64_t N1, int64_t N2, float radius,
@@ -281,25 +304,9 @@ static int ball_query_impl(const void *query, const void *key, int64_t B, int64_
       scratch_bytes >= sp_search_bytes(B, N1, N2))
     return sp_ball_query((const float *)query, (const float *)key, B, N1, N2, channel_first, radius * radius, (int)k,
                          index, index32, scratch, st);
-  if (dtype == TK3D_F32) {
-    const float r2 = radius * radius;  // squared in fp32, as the reference does for float tensors
-    const int64_t cap = (int64_t)sm_count() * 256;
-    if (B * N1 < (int64_t)sm_count() * 16 * BQ_THREADS) {
-      const int64_t total = B * ((N1 + 31) / 32);
-      const unsigned grid = (unsigned)(total < cap ? total : cap);
-      if (total <= 2 * (int64_t)sm_count())  // very few queries: eight warps per 32 queries
-        ball_query_split_kernel<8><<<grid, 256, 0, st>>>((const float *)query, (const float *)key, B, (int)N1, (int)N2,
-                                                         r2, (int)k, io, total, ql, kl);
-      else
-        ball_query_split_kernel<4><<<grid, 128, 0, st>>>((const float *)query, (const float *)key, B, (int)N1, (int)N2,
-                                                         r2, (int)k, io, total, ql, kl);
-      return check_launch("ball_query_split_kernel");
-    }
-    const int64_t total = B * ((N1 + BQ_THREADS - 1) / BQ_THREADS);
-    ball_query_fast_kernel<<<(unsigned)(total < cap ? total : cap), BQ_THREADS, 0, st>>>(
-        (const float *)query, (const float *)key, B, (int)N1, (int)N2, r2, (int)k, io, total, ql, kl);
-    return check_launch("ball_query_fast_kernel");
-  }
+  if (dtype == TK3D_F32)  // the radius is squared in fp32, as the reference does for float tensors
+    return ball_query_sweep_f32((const float *)query, (const float *)key, B, N1, N2, radius * radius, (int)k, io, ql, kl,
+                                st);
   const double r = (double)radius;
   if (B * N1 < (int64_t)sm_count() * 8 * 256) {  // too few queries for one thread each
     const int64_t tot = B * ((N1 + 31) / 32);

@@ -531,9 +531,9 @@ int chamfer_fwd_f32_ordered(const float *xyz1, const float *xyz2, int64_t B, int
     float *d1 = dist1 + b0 * N1, *d2 = dist2 + b0 * N2;
     int64_t *i1 = idx1 + b0 * N1, *i2 = idx2 + b0 * N2;
     int rc = sp_build(c1, &c2, n, SpUse{true, true, true, 0, 0.f}, st);
+    const SpOnly only = rc == SP_DECLINED ? SpOnly{} : SpOnly{c1.grid, c2.grid};
     if (!rc) rc = sp_chamfer(c1, c2, n, d1, i1, d2, i2, sums, st);
-    if (!rc)
-      rc = chamfer_fwd_f32_fast(p1, p2, n, N1, N2, d1, i1, d2, i2, sums, st, c1.l, c2.l, SpOnly{c1.grid, c2.grid});
+    if (!rc || !only.q) rc = chamfer_fwd_f32_fast(p1, p2, n, N1, N2, d1, i1, d2, i2, sums, st, c1.l, c2.l, only);
     if (rc) return rc;
   }
   return TK3D_OK;

@@ -1153,10 +1153,14 @@ int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int
     io.kl = ck.l;
     io.only = SpOnly{cq.grid, ck.grid};
     int rc = sp_build(cq, same ? nullptr : &ck, n, SpUse{false, k <= 32 || N2 > 8192, k <= 4, 0, 0.f}, st);
-    if (!rc)
-      rc = k <= 4 ? sp_knn_small(cq, ck, n, k, weights, eps, d, io.index, st)
-                  : sp_knn_select(cq, ck, n, k, d, io.index, st);
-    if (rc) return rc;
+    if (rc == SP_DECLINED) {
+      io.only = {};
+    } else {
+      if (!rc)
+        rc = k <= 4 ? sp_knn_small(cq, ck, n, k, weights, eps, d, io.index, st)
+                    : sp_knn_select(cq, ck, n, k, d, io.index, st);
+      if (rc) return rc;
+    }
     // what the order left is swept by the kernel that serves a call without scratch
     switch (k) {
       case 1: rc = knn_small_q<1>(q, r, n, (int)N1, (int)N2, d, io, st); break;
@@ -1167,7 +1171,8 @@ int knn_ordered(const float *query, const float *key, int64_t B, int64_t N1, int
     }
     if (rc) return rc;
     if (weights) {
-      three_nn_weight_inplace_kernel<<<sm_count(), 256, 0, st>>>(d, N1, n * N1, eps, io.only);
+      if (io.only.q) three_nn_weight_inplace_kernel<<<sm_count(), 256, 0, st>>>(d, N1, n * N1, eps, io.only);
+      else three_nn_weight_inplace_kernel<<<sm_count(), 256, 0, st>>>(d, N1, n * N1, eps, SpAll{});
       rc = check_launch("three_nn_weight_inplace_kernel");
       if (rc) return rc;
     }

@@ -628,7 +628,10 @@ int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, const SpUse &use, cu
   cfg.numAttrs = 1;
   SpUse use_ = use;
   void *args[] = {&pair, &B_, &use_};
-  TK3D_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
+  if (cudaLaunchKernelExC(&cfg, kern, args) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return SP_DECLINED;
+  }
   const int64_t w0 = B * a.windows, total = w0 + (b ? B * b->windows : 0);
   const int64_t per = SW_THREADS / 32;
   spatial_window_kernel<<<(unsigned)((total + per - 1) / per), SW_THREADS, 0, st>>>(pair, w0, total);

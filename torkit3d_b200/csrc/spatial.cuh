@@ -115,7 +115,9 @@ struct SpUse {
   float r2;
 };
 
-// Builds the index of both sides (two launches); `b` may be null: both sides are a.
+// Builds the index of both sides (two launches); `b` may be null: both sides are a.  SP_DECLINED where the device
+// refuses the cluster launch (a partition without room for it): nothing was built, the caller sweeps.
+constexpr int SP_DECLINED = -1;
 int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, const SpUse &use, cudaStream_t st);
 
 // Searches over built indexes; rows of clouds that are irregular on either side are left alone.

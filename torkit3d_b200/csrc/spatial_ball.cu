@@ -161,6 +161,9 @@ spatial_ball_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ 
 
 }  // namespace
 
+int ball_query_sweep_f32(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, float r2, int k,
+                         const IndexOut &index, XyzLayout ql, XyzLayout kl, cudaStream_t st);
+
 int sp_ball_query(const float *query, const float *key, int64_t B, int64_t N1, int64_t N2, int channel_first, float r2,
                   int k, void *index, int index32, void *scratch, cudaStream_t st) {
   const int64_t step = sp_batch(B, N1, N2);
@@ -170,10 +173,13 @@ int sp_ball_query(const float *query, const float *key, int64_t B, int64_t N1, i
     const SpCloud cq = sp_cloud(query + b0 * 3 * N1, channel_first, n, N1, at);
     const SpCloud ck = sp_cloud(key + b0 * 3 * N2, channel_first, n, N2, at + sp_cloud_bytes(n, N1));
     int rc = sp_build(cq, &ck, n, SpUse{false, false, true, k, r2}, st);
-    if (rc) return rc;
-    spatial_ball_kernel<<<(unsigned)(n * cq.groups), SQ_THREADS, 0, st>>>(
-        cq, ck, r2, k, index_out((char *)index + b0 * N1 * k * (index32 ? 4 : 8), index32, n * N1 * k), 1.0f);
-    rc = check_launch("spatial_ball_kernel");
+    const IndexOut io = index_out((char *)index + b0 * N1 * k * (index32 ? 4 : 8), index32, n * N1 * k);
+    if (rc == SP_DECLINED) {
+      rc = ball_query_sweep_f32(cq.xyz, ck.xyz, n, N1, N2, r2, k, io, cq.l, ck.l, st);
+    } else if (!rc) {
+      spatial_ball_kernel<<<(unsigned)(n * cq.groups), SQ_THREADS, 0, st>>>(cq, ck, r2, k, io, 1.0f);
+      rc = check_launch("spatial_ball_kernel");
+    }
     if (rc) return rc;
   }
   return TK3D_OK;
