@@ -1,4 +1,4 @@
-"""Searches over spatially ordered clouds, continued: a device that refuses the cluster launch."""
+"""Searches over spatially ordered clouds, continued: memory that is short, a device that refuses the cluster launch."""
 import os
 import subprocess
 import sys
@@ -15,6 +15,45 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 def _same(x, y):
     return torch.equal(x.view(torch.int32) if x.dtype == torch.float32 else x,
                        y.view(torch.int32) if y.dtype == torch.float32 else y)
+
+
+@pytest.mark.parametrize("op", ["chamfer", "knn", "ball", "interp", "sa", "step"])
+def test_calls_sweep_where_the_memory_for_the_order_is_missing(op):
+    """The order takes scratch that a sweep does not: a call that just fits without it still runs."""
+    from torkit3d_b200 import _fused, _lib, dist, ops
+
+    B, N = 64, 16384
+    g = torch.Generator(device=DEV).manual_seed(2)
+    a, b = (torch.rand(B, N, 3, generator=g, device=DEV) for _ in range(2))
+    acf, bcf = (t.transpose(1, 2).contiguous() for t in (a, b))
+    f = torch.randn(B, 2, N, generator=g, device=DEV)
+    run = {
+        "chamfer": lambda: ops.nn_distance(a, b),
+        "knn": lambda: ops.knn_points(a, b, 3),
+        "ball": lambda: [ops.ball_query(a, b, 0.02, 4, transpose=False)],
+        "interp": lambda: _fused.three_nn_interp_forward(acf, bcf, f),
+        "sa": lambda: _fused.sa_group_forward(bcf, acf, f, 0.02, 4),
+        "step": lambda: dist.chamfer_step(a, b),
+    }[op]
+    margin = 28 << 20
+    assert _lib.scratch_bytes("tk3d_chamfer_fwd", B, N, N, _lib.F32) > margin + (12 << 20)
+    want = list(run())
+    results = sum(t.numel() * t.element_size() for t in want)
+    if op == "step":  # distances and indices are temporaries
+        results += 2 * B * N * 12
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + results + margin) / total)
+    try:
+        got = list(run())
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for x, y in zip(want, got):
+        if op == "step":
+            torch.testing.assert_close(x, y, rtol=1e-5, atol=1e-9)  # float32 sums in any order
+        else:
+            assert _same(x, y)
 
 
 def test_a_device_that_refuses_the_cluster_launch_is_swept(tmp_path):

@@ -124,6 +124,16 @@ def _ptr(t):
     return t.data_ptr()  # 0 for an empty tensor, which ctypes passes as NULL
 
 
+def _order_scratch(need, device, least=0):
+    """Scratch of ``need`` bytes for a search over spatially ordered clouds (about 21 bytes a point and 16 KB a cloud,
+    512 MB at most: larger batches are cut).  Where that much is not free, ``least`` bytes (0: None), with which the
+    library sweeps all pairs."""
+    try:
+        return torch.empty((need,), dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return torch.empty((least,), dtype=torch.uint8, device=device) if least else None
+
+
 def sample_farthest_points_cuda(points, num_samples, *, channel_first=False):
     """points [B,N,3] ([B,3,N] with ``channel_first``) -> index [B,num_samples] int64 (first sample is point 0)."""
     _check_cuda_contig(points=points)
@@ -169,8 +179,8 @@ def ball_query_cuda(query, key, radius, max_neighbors, *, channel_first=False, i
         index = torch.empty((B, N1, k), dtype=index_dtype, device=query.device)
         # large searches order the clouds first; 0 where sweeping all pairs is faster
         need = _lib.scratch_bytes("tk3d_ball_query", B, N1, N2, k, _dtype(query))
-        if need:
-            scratch = torch.empty((need,), dtype=torch.uint8, device=query.device)
+        scratch = _order_scratch(need, query.device) if need else None
+        if scratch is not None:
             check(lib.tk3d_ball_query_ws(_ptr(query), _ptr(key), B, N1, N2, float(radius), k,
                                          1 if channel_first else 0, _ptr(index), _index_code(index_dtype),
                                          _ptr(scratch), need, _dtype(query), _stream(query)))
@@ -384,8 +394,8 @@ def knn_distance_cuda(query, key, k, version=0, *, channel_first=False, index_dt
         index = torch.empty((B, N1, k), dtype=index_dtype, device=query.device)
         # large searches order the clouds first; 0 where sweeping all pairs is faster
         need = _lib.scratch_bytes("tk3d_knn", B, N1, N2, k, _dtype(query))
-        if need:
-            scratch = torch.empty((need,), dtype=torch.uint8, device=query.device)
+        scratch = _order_scratch(need, query.device) if need else None
+        if scratch is not None:
             check(lib.tk3d_knn_ws(_ptr(query), _ptr(key), B, N1, N2, k, 1 if channel_first else 0, _ptr(distance),
                                   _ptr(index), _index_code(index_dtype), _ptr(scratch), need, _dtype(query),
                                   _stream(query)))
@@ -459,8 +469,8 @@ def chamfer_distance_forward_cuda(xyz1, xyz2, sums=None, *, channel_first=False)
             if not (sums.is_cuda and sums.dtype == torch.float64 and sums.numel() == 2 and sums.is_contiguous()):
                 raise RuntimeError("sums must be a contiguous float64 CUDA tensor with 2 elements")
         need = _lib.scratch_bytes("tk3d_chamfer_fwd", B, N1, N2, _dtype(xyz1))
-        if need:  # large problems order the clouds first
-            scratch = torch.empty((need,), dtype=torch.uint8, device=dev)
+        scratch = _order_scratch(need, dev) if need else None  # large problems order the clouds first
+        if scratch is not None:
             check(lib.tk3d_chamfer_fwd_ws(_ptr(xyz1), _ptr(xyz2), B, N1, N2, 1 if channel_first else 0, _ptr(dist1),
                                           _ptr(idx1), _ptr(dist2), _ptr(idx2),
                                           _ptr(sums) if sums is not None else None, _ptr(scratch), need,

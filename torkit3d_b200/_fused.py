@@ -7,7 +7,7 @@ and element-wise PyTorch expressions in ``torkit3d/layers/pointnet2.py`` and
 import torch
 
 from . import _lib
-from ._C import _check_cuda, _check_eq, _on, _ptr, _stream
+from ._C import _check_cuda, _check_eq, _on, _order_scratch, _ptr, _stream
 from ._lib import check, load
 
 
@@ -80,7 +80,8 @@ def sa_group_forward(points, centroids, feature, radius, max_neighbors, use_xyz=
         out = torch.empty((B, C + (3 if use_xyz else 0), M, K), dtype=torch.float32, device=dev)
         index32 = torch.empty((B, M, K), dtype=torch.int32, device=dev) if want_index else None
         need = _lib.scratch_bytes("tk3d_sa_group", B, C, N, M, K, _lib.F32)
-        scratch = _scratch(need, dev)
+        scratch = _order_scratch(need, dev, 4 * B * C * N) if need else None
+        need = scratch.numel() if need else 0
         check(lib.tk3d_sa_group_fwd(_ptr(points), _ptr(centroids), _ptr(feature) if C else None, B, C, N, M,
                                     float(radius), K, 1 if channel_first else 0, 1 if use_xyz else 0, _ptr(out),
                                     _ptr(index32) if want_index else None, None, _ptr(scratch) if need else None,
@@ -105,7 +106,8 @@ def sa_group_backward(grad_out, index32, C, N, use_xyz=True, channel_first=True,
             if (xyz and need_points) else None
         gcen = torch.empty((B, 3, M) if channel_first else (B, M, 3), dtype=torch.float32, device=dev) \
             if (xyz and need_centroids) else None
-        need = _lib.scratch_bytes("tk3d_sa_group", B, C, N, M, K, _lib.F32) if gfeat is not None else 0
+        # the transposed gradient alone; the rest of that size is the forward's search
+        need = 4 * B * C * N if gfeat is not None and _lib.scratch_bytes("tk3d_sa_group", B, C, N, M, K, _lib.F32) else 0
         scratch = _scratch(need, dev)
         check(lib.tk3d_sa_group_bwd(_ptr(grad_out), _ptr(index32), B, C, N, M, K, 1 if channel_first else 0,
                                     1 if use_xyz else 0, _ptr(gfeat) if gfeat is not None else None,
@@ -134,7 +136,8 @@ def three_nn_interp_forward(query_xyz, key_xyz, key_feature, eps=1e-10, channel_
         index32 = torch.empty((B, Nq, 3), dtype=torch.int32, device=dev)
         weight = torch.empty((B, Nq, 3), dtype=torch.float32, device=dev)
         need = _lib.scratch_bytes("tk3d_three_nn_interp", B, C, Nq, Nk, _lib.F32)
-        scratch = _scratch(need, dev)
+        scratch = _order_scratch(need, dev, 4 * B * C * Nk) if need else None
+        need = scratch.numel() if need else 0
         check(lib.tk3d_three_nn_interp_fwd(_ptr(query_xyz), _ptr(key_xyz), _ptr(key_feature), B, C, Nq, Nk,
                                            1 if channel_first else 0, float(eps), _ptr(out), _ptr(index32),
                                            _ptr(weight), None, _ptr(scratch) if need else None, need, _lib.F32,
@@ -152,7 +155,8 @@ def three_nn_interp_backward(grad_out, index32, weight, Nk):
     dev = grad_out.device
     with _on(dev):
         gfeat = torch.empty((B, C, Nk), dtype=torch.float32, device=dev)
-        need = _lib.scratch_bytes("tk3d_three_nn_interp", B, C, Nq, Nk, _lib.F32)
+        # the transposed gradient alone; the rest of that size is the forward's search
+        need = 4 * B * C * Nk if _lib.scratch_bytes("tk3d_three_nn_interp", B, C, Nq, Nk, _lib.F32) else 0
         scratch = _scratch(need, dev)
         check(lib.tk3d_three_nn_interp_bwd(_ptr(grad_out), _ptr(index32), _ptr(weight), B, C, Nq, Nk, _ptr(gfeat),
                                            None, _ptr(scratch) if need else None, need, _lib.F32,

@@ -139,8 +139,12 @@ def _one(device, dtype):
 
 # ---- training step without autograd ---------------------------------------------------------------
 def _chamfer_scratch(_lib, B, n1, n2, dt, dev):
-    """Scratch of a chamfer forward; empty where the library sweeps all pairs."""
-    return torch.empty((_lib.scratch_bytes("tk3d_chamfer_fwd", B, n1, n2, dt),), dtype=torch.uint8, device=dev)
+    """Scratch of a chamfer forward (up to about 512 MB); empty where the library sweeps all pairs, or memory is short."""
+    from ._C import _order_scratch
+
+    need = _lib.scratch_bytes("tk3d_chamfer_fwd", B, n1, n2, dt)
+    scratch = _order_scratch(need, dev) if need else None
+    return scratch if scratch is not None else torch.empty((0,), dtype=torch.uint8, device=dev)
 
 
 def chamfer_step(xyz1, xyz2, global_batch=None, group=None, workspace=None):
@@ -149,8 +153,9 @@ def chamfer_step(xyz1, xyz2, global_batch=None, group=None, workspace=None):
     The loss is linear in the per-point distances, so the gradient kernels need only the counts,
     not the reduced loss: they are launched right behind the forward kernel while the all-reduce of
     the two partial sums is in flight (``async_op``), and only the final loss kernel waits for it.
-    Five launches per step (forward, two gradient kernels, the collective, the loss), no
-    element-wise PyTorch kernel, no autograd graph.
+    Five launches per step (forward, two gradient kernels, the collective, the loss), eight where the
+    forward orders the clouds first (sort, windows, search, the sweep of what is left); no element-wise
+    PyTorch kernel, no autograd graph.
 
     Args:
         xyz1: [B_local, N1, 3] float32/float64 CUDA tensor, this rank's clouds;  xyz2: [B_local, N2, 3].
@@ -158,7 +163,9 @@ def chamfer_step(xyz1, xyz2, global_batch=None, group=None, workspace=None):
         workspace: optional dict owned by the caller.  The outputs and intermediate tensors of the
             step are then kept in it and reused by the next call with the same shapes (ten fewer
             allocations per step, which matters when a step takes less than a millisecond); the
-            tensors returned by one call are overwritten by the next call with that workspace.
+            tensors returned by one call are overwritten by the next call with that workspace.  Where the
+            forward orders the clouds its scratch is kept too (about 21 bytes a point and 16 KB a cloud,
+            512 MB at most).
 
     Returns:
         (loss, grad_xyz1, grad_xyz2): the global mean loss (0-dim, identical on every rank) and
