@@ -37,3 +37,17 @@ def test_sequence(oracle, kind, B, N, S):
     p = np.ascontiguousarray(_cloud(kind, B, N))
     got = sample_farthest_points(torch.from_numpy(p).to(DEV), S).cpu().numpy()
     np.testing.assert_array_equal(got, oracle.fps(p, S))
+
+
+@pytest.mark.parametrize("kind", ["random", "lattice", "few", "far", "sorted"])
+@pytest.mark.parametrize("B,N,S", [(2, 4097, 200), (2, 8193, 100), (1, 16385, 150), (1, 40000, 90), (1, 65537, 90)])
+def test_sequence_of_batches_whatever_the_number_of_samples(oracle, kind, B, N, S):
+    """The diagnostic entry takes several samples per exchange also where a regular call takes one (few samples)."""
+    from torkit3d_b200 import _lib
+
+    p = np.ascontiguousarray(_cloud(kind, B, N))
+    pts = torch.from_numpy(p).to(DEV)
+    idx = torch.empty(B, S, dtype=torch.int64, device=DEV)
+    assert _lib.load().tk3d_diag_fps_wait_limit(pts.data_ptr(), B, N, S, idx.data_ptr(), 1000, -1,
+                                                torch.cuda.current_stream().cuda_stream) == 0
+    np.testing.assert_array_equal(idx.cpu().numpy(), oracle.fps(p, S))

@@ -19,6 +19,8 @@
 // torkit3d/csrc/cuda/sample_farthest_points_kernel.cu:33-103 (one block per cloud, any size).
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "tk3d_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -94,7 +96,8 @@ __device__ unsigned int fw_expired_waits = 0;
 
 // FW_REGS false (clouds beyond 131072 points): the coordinates stay in shared memory, which then
 // holds FW_THREADS * 2 * FW_P2 points, and only the running minima live in registers.
-template <int FW_THREADS, int FW_P2, int FW_SLOTS, bool FW_REGS = true>
+// FW_BATCHED false: one sample per exchange.
+template <int FW_THREADS, int FW_P2, int FW_SLOTS, bool FW_REGS = true, bool FW_BATCHED = FW_REGS>
 __global__ void __launch_bounds__(FW_THREADS)
 fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int64_t *__restrict__ index, int ps, int cs,
                     float *__restrict__ sampled, float one, unsigned long long limit_ns, int drop_step) {
@@ -215,7 +218,7 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
   int n = 1;  // samples so far
   // Where exchanges keep yielding a single sample (points on a lattice: ties), the bounds are left out
   // for 48 exchanges at a time; the same in all warps.
-  int again = FW_REGS ? 0 : 0x7fffffff, single = 0;
+  int again = FW_BATCHED ? 0 : 0x7fffffff, single = 0;
   for (int ex = 1; n < S; ++ex) {
     const int par = ex & 1;
     const unsigned bits = __float_as_uint(bm);
@@ -274,9 +277,7 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
     if (tid == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(lb), "r"(expect) : "memory");
 
-    if constexpr (!FW_REGS) {
-      // coordinates in shared memory: a bound costs more than it saves (2 x 200000 -> 200 593 us, without
-      // bounds 419), so every exchange gives one sample
+    if constexpr (!FW_BATCHED) {
       unsigned b_ = 0u;
       int i_ = 0x7fffffff, slot = lane;
 #pragma unroll
@@ -633,13 +634,17 @@ static bool fps_warpcast64_launch(const double *points, int64_t B, int64_t N, in
 
 template <int THREADS, int P2>
 static bool fps_warpcast_launch(const float *points, int64_t B, int64_t N, int64_t S, int ps, int64_t cs, int64_t *index,
-                                float *sampled, cudaStream_t st, int *rc, int CL, FwWait wt) {
+                                float *sampled, cudaStream_t st, int *rc, int CL, FwWait wt, bool batched) {
   const int warps = CL * (THREADS / 32);
   if (warps > 128 || (int64_t)CL * THREADS * 2 * P2 < N) return false;  // a slot per warp, a register per point
-  return fps_cluster_launch_kernel(warps <= 32   ? fps_warpcast_kernel<THREADS, P2, 32>
-                                   : warps <= 64 ? fps_warpcast_kernel<THREADS, P2, 64>
-                                                 : fps_warpcast_kernel<THREADS, P2, 128>,
-                                   THREADS, points, B, N, S, ps, cs, index, sampled, st, rc, CL, wt);
+  auto pick = [&](auto several) -> FpsClusterKernel {
+    constexpr bool BATCHED = decltype(several)::value;
+    return warps <= 32   ? fps_warpcast_kernel<THREADS, P2, 32, true, BATCHED>
+           : warps <= 64 ? fps_warpcast_kernel<THREADS, P2, 64, true, BATCHED>
+                         : fps_warpcast_kernel<THREADS, P2, 128, true, BATCHED>;
+  };
+  return fps_cluster_launch_kernel(batched ? pick(std::true_type{}) : pick(std::false_type{}), THREADS, points, B, N, S,
+                                   ps, cs, index, sampled, st, rc, CL, wt);
 }
 
 // Launches a cluster kernel when the clouds suit one (float32, 4096 < N <= 262144); returns false
@@ -656,25 +661,37 @@ static bool fps_warpcast_launch(const float *points, int64_t B, int64_t N, int64
 // Beyond about half a cloud per SM the blocks of several clusters share SMs and the one-block
 // kernel is as fast; up to 4096 points its step (0.43 us) is shorter than the exchange over
 // distributed shared memory (0.45 to 0.5 us).
+//
+// Several samples per exchange, where enough of them are taken: the first ones are far from all others, and their
+// exchanges yield one each.  One / several, us, points on a surface, in a volume, all the same:
+//   samples       64                128              256              512              2048
+//   32 x  8192    38 / 46, 44, 45   73 / 72, 81, 86  144 / 118, 122, 167  284 / 195, 194, 329  1125 / 616, 622, 1301
+//    4 x 16384    42 / 46, 43, 46   78 / 77, 71, 84  152 / 130, 118, 163  302 / 218, 205, 320  1185 / 715, 699, 1259
+//   16 x 20000    56 / 72, 70, 68   106 / 120, 114, 127  205 / 206, 199, 243  407 / 364, 360, 478  1612 / 1237, 1227, 1884
+//    4 x 65536    68 / 80, 77, 74   128 / 138, 127, 137  249 / 226, 209, 264  492 / 384, 353, 518  1945 / 1156, 1119, 2038
+//    2 x 131072   97 / 126, 125, 123  186 / 230, 208, 233  365 / 400, 353, 454  718 / 647, 595, 890  2833 / 1899, 1820, 3505
+// `force`: the diagnostic entry, several always.
 static bool fps_cluster_dispatch(const float *points, int64_t B, int64_t N, int64_t S, int ps, int64_t cs,
                                  int64_t *index, float *sampled, cudaStream_t st, int *rc, FwWait wt, bool force) {
+  const bool batched = force || S >= (N <= 16384 ? 192 : 384);
   if (N > 4096 && N <= 16384) {
     if (N <= 8192) {
       if (!force && B * 15 > (int64_t)sm_count() * 7) return false;
-      return fps_warpcast_launch<256, 4>(points, B, N, S, ps, cs, index, sampled, st, rc, 4, wt);
+      return fps_warpcast_launch<256, 4>(points, B, N, S, ps, cs, index, sampled, st, rc, 4, wt, batched);
     }
     if (!force && B * 15 > (int64_t)sm_count() * 8) return false;
-    return fps_warpcast_launch<128, 8>(points, B, N, S, ps, cs, index, sampled, st, rc, 8, wt);
+    return fps_warpcast_launch<128, 8>(points, B, N, S, ps, cs, index, sampled, st, rc, 8, wt, batched);
   }
   if (N <= 16384 || N > 262144 || B * FC_MAX_CL >= (1LL << 31)) return false;
-  if (N > 131072)  // 64 points per thread: running minima in registers, coordinates in 192 KB of shared memory
+  if (N > 131072)  // 64 points per thread: running minima in registers, coordinates in 192 KB of shared memory, where
+                   // a bound costs more than it saves (2 x 200000 -> 200: 593 us, one sample per exchange 419)
     return fps_cluster_launch_kernel(fps_warpcast_kernel<256, 32, 128, false>, 256, points, B, N, S, ps, cs, index,
                                      sampled, st, rc, 16, wt, (size_t)256 * 64 * 12);
   // larger clouds: 32 points per thread, so that a cluster has at most 128 warps (4 clouds, 512 samples:
   // 32768 points 0.375 ms, 0.48 with 16 points per thread and twice the warps; 65536 points 0.51 / 0.60)
-  if (N <= 32768) return fps_warpcast_launch<128, 16>(points, B, N, S, ps, cs, index, sampled, st, rc, 8, wt);
-  if (N <= 65536) return fps_warpcast_launch<128, 16>(points, B, N, S, ps, cs, index, sampled, st, rc, 16, wt);
-  return fps_warpcast_launch<256, 16>(points, B, N, S, ps, cs, index, sampled, st, rc, 16, wt);
+  if (N <= 32768) return fps_warpcast_launch<128, 16>(points, B, N, S, ps, cs, index, sampled, st, rc, 8, wt, batched);
+  if (N <= 65536) return fps_warpcast_launch<128, 16>(points, B, N, S, ps, cs, index, sampled, st, rc, 16, wt, batched);
+  return fps_warpcast_launch<256, 16>(points, B, N, S, ps, cs, index, sampled, st, rc, 16, wt, batched);
 }
 
 // float64: few clouds of 2049 to 8192 points (the one-block kernel's step is 1.1 us at 4096 points),
