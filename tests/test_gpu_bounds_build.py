@@ -100,3 +100,60 @@ def test_bounds_build_counts_no_violation_and_matches_the_regular_build():
 
     both(wide_ball)
     assert chk.tk3d_bounds_violations() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["random", "collapsed", "nonfinite"])
+@pytest.mark.parametrize("B,n1,n2,cf", [(2, 33, 512, 0), (3, 700, 1111, 1), (1, 4099, 9001, 0)])
+def test_bounds_build_over_ordered_clouds(kind, B, n1, n2, cf):
+    """The searches with scratch: positions, leaves and the outputs."""
+    from torkit3d_b200 import _lib
+
+    reg, chk = _lib.load(), _lib.load_bounds_checked()
+    st = torch.cuda.current_stream().cuda_stream
+    g = torch.Generator().manual_seed(n2)
+    q, r = torch.randn(B, n1, 3, generator=g), torch.randn(B, n2, 3, generator=g)
+    if kind == "collapsed":
+        q *= 1e-3
+    elif kind == "nonfinite":
+        r[B - 1, 5, 1] = float("nan")
+    q, r = ((t.transpose(1, 2).contiguous() if cf else t).to(DEV) for t in (q, r))
+    buf = torch.empty(16 << 20, dtype=torch.uint8, device=DEV)
+    before = chk.tk3d_bounds_violations()
+
+    def both(fn):
+        a, b = fn(reg), fn(chk)
+        torch.cuda.synchronize()
+        for x, y in zip(a, b):
+            assert torch.equal(x, y)
+
+    for k in (1, 3, 4, 5, 16, 32, 64):
+        if n2 < 16 * k:
+            continue
+
+        def knn(lib):
+            d = torch.empty(B, n1, k, device=DEV)
+            i = torch.empty(B, n1, k, dtype=torch.int32, device=DEV)
+            assert lib.tk3d_knn_ws(q.data_ptr(), r.data_ptr(), B, n1, n2, k, cf, d.data_ptr(), i.data_ptr(), _lib.I32,
+                                   buf.data_ptr(), buf.numel(), _lib.F32, st) == 0
+            return d.nan_to_num(), i
+
+        both(knn)
+
+    def ball(lib):
+        i = torch.empty(B, n1, 24, dtype=torch.int64, device=DEV)
+        assert lib.tk3d_ball_query_ws(q.data_ptr(), r.data_ptr(), B, n1, n2, 0.3, 24, cf, i.data_ptr(), _lib.I64,
+                                      buf.data_ptr(), buf.numel(), _lib.F32, st) == 0
+        return (i,)
+
+    both(ball)
+    if n1 >= 512:
+
+        def chamfer(lib):
+            out = [torch.empty(B, n, dtype=t, device=DEV) for n in (n1, n2) for t in (torch.float32, torch.int64)]
+            assert lib.tk3d_chamfer_fwd_ws(q.data_ptr(), r.data_ptr(), B, n1, n2, cf, *(o.data_ptr() for o in out), None,
+                                           buf.data_ptr(), buf.numel(), _lib.F32, st) == 0
+            return [o.nan_to_num() for o in out]
+
+        both(chamfer)
+    assert chk.tk3d_bounds_violations() == before == 0

@@ -2,8 +2,8 @@
 
 Both run through the same C entry point: with a scratch buffer the clouds are ordered, without one
 every pair is swept (and the sweeping kernels are compared with the oracle elsewhere).  Sizes sit at
-the edges of the structure: leaves of 32 points, windows of 256, super leaves of 1024, clusters of one
-to eight blocks, several chunks of super leaves.  The inputs cover what orders badly: duplicates, a
+the edges of the structure: leaves of 8 points, windows of 256, clusters of one to eight blocks, several
+chunks of 32 windows.  The inputs cover what orders badly: duplicates, a
 lattice full of ties, a plane, an outlier that stretches the grid, NaN and infinite coordinates.
 All results are decided on exactly rounded distances, so the comparison is exact.
 """

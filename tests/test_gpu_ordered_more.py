@@ -1,4 +1,6 @@
-"""Searches over spatially ordered clouds, continued: memory that is short, a device that refuses the cluster launch."""
+"""Searches over spatially ordered clouds, continued: a cloud searched in itself, clouds that are away from one another,
+collapsed, or so far apart that distances overflow, batches of which only some clouds are ordered, sums of cut batches,
+memory that is short, a device that refuses the cluster launch."""
 import os
 import subprocess
 import sys
@@ -12,9 +14,113 @@ DEV = "cuda:0"
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
 def _same(x, y):
     return torch.equal(x.view(torch.int32) if x.dtype == torch.float32 else x,
                        y.view(torch.int32) if y.dtype == torch.float32 else y)
+
+
+def _knn(a, b, k, cf, scratch):
+    from torkit3d_b200 import _lib
+
+    B, N, M = a.shape[0], a.shape[2 if cf else 1], b.shape[2 if cf else 1]
+    d, i = torch.empty(B, N, k, device=DEV), torch.empty(B, N, k, dtype=torch.int64, device=DEV)
+    assert _lib.load().tk3d_knn_ws(a.data_ptr(), b.data_ptr(), B, N, M, k, cf, d.data_ptr(), i.data_ptr(), _lib.I64,
+                                   scratch.data_ptr() if scratch is not None else None,
+                                   scratch.numel() if scratch is not None else 0, _lib.F32, _stream()) == 0
+    return d, i
+
+
+def _chamfer(a, b, scratch):
+    from torkit3d_b200 import _lib
+
+    B, N, M = a.shape[0], a.shape[1], b.shape[1]
+    out = [torch.empty(B, n, dtype=t, device=DEV) for n in (N, M) for t in (torch.float32, torch.int64)]
+    sums = torch.empty(2, dtype=torch.float64, device=DEV)
+    assert _lib.load().tk3d_chamfer_fwd_ws(a.data_ptr(), b.data_ptr(), B, N, M, 0, *(o.data_ptr() for o in out),
+                                           sums.data_ptr(), scratch.data_ptr() if scratch is not None else None,
+                                           scratch.numel() if scratch is not None else 0, _lib.F32, _stream()) == 0
+    return out + [sums]
+
+
+@pytest.mark.parametrize("kind", ["random", "lattice", "zeros", "outlier", "nonfinite"])
+@pytest.mark.parametrize("k", [1, 3, 4, 5, 16, 32, 64])
+@pytest.mark.parametrize("B,N,cf", [(2, 1024, 0), (3, 1025, 1), (1, 8200, 0)])
+def test_a_cloud_searched_in_itself(kind, k, B, N, cf):
+    g = torch.Generator().manual_seed(N)
+    p = torch.randn(B, N, 3, generator=g)
+    if kind == "lattice":
+        p = torch.randint(0, 9, (B, N, 3), generator=g).float() * 0.1
+    elif kind == "zeros":
+        p[torch.rand(B, N, generator=g) < 0.3] = 0
+    elif kind == "outlier":
+        p[:, N // 2] = 1e6
+    elif kind == "nonfinite":
+        p[B - 1, 7, 1] = float("nan")
+    p = (p.transpose(1, 2).contiguous() if cf else p).to(DEV)
+    scratch = torch.full((32 << 20,), 0xA5, dtype=torch.uint8, device=DEV)
+    for x, y in zip(_knn(p, p, k, cf, None), _knn(p, p, k, cf, scratch)):
+        assert _same(x, y)
+
+
+@pytest.mark.parametrize("kind", ["away", "collapsed", "inside", "overflow", "halves"])
+@pytest.mark.parametrize("B,N,M", [(2, 1030, 4099), (1, 4096, 1024)])
+def test_clouds_that_lie_badly_to_each_other(kind, B, N, M):
+    g = torch.Generator().manual_seed(M)
+    a, b = torch.randn(B, N, 3, generator=g), torch.randn(B, M, 3, generator=g)
+    if kind == "away":
+        a += 100
+    elif kind == "collapsed":
+        a[:] = 0.25
+    elif kind == "inside":
+        a *= 1e-3
+        b /= b.norm(dim=2, keepdim=True)
+    elif kind == "overflow":  # finite coordinates, infinite distances: no nearest neighbour in the chamfer distance
+        a -= 3e19
+        b += 3e19
+    else:  # half of the queries like the keys, half away: some lists are short, some long
+        a[:, ::2] += 50
+    a, b = a.to(DEV), b.to(DEV)
+    scratch = torch.full((32 << 20,), 0xA5, dtype=torch.uint8, device=DEV)
+    for x, y in zip(_chamfer(a, b, None)[:4], _chamfer(a, b, scratch)[:4]):
+        assert _same(x, y)
+    for k in (1, 3, 5, 16, 40, 64):
+        for x, y in zip(_knn(a, b, k, 0, None), _knn(a, b, k, 0, scratch)):
+            assert _same(x, y)
+
+
+@pytest.mark.parametrize("bad", [(0,), (1,), (2,), (0, 2)])
+def test_weights_of_a_batch_of_which_some_clouds_are_swept(bad):
+    from torkit3d_b200 import _fused, ops
+
+    B, C, N, M = 3, 4, 11000, 4100
+    g = torch.Generator(device=DEV).manual_seed(5)
+    a, b = torch.randn(B, 3, N, generator=g, device=DEV), torch.randn(B, 3, M, generator=g, device=DEV)
+    for i in bad:
+        b[i, 1, 77] = float("inf")
+    f = torch.randn(B, C, M, generator=g, device=DEV)
+    _, index, weight = _fused.three_nn_interp_forward(a, b, f)
+    for q0 in range(0, N, 2000):  # too few pairs to be ordered
+        d, i = ops.knn_points(a[:, :, q0:q0 + 2000].contiguous(), b, 3, transpose=True)
+        assert torch.equal(index[:, q0:q0 + 2000].long(), i)
+        assert _same(weight[:, q0:q0 + 2000].contiguous(), ops.three_nn_weight(d))
+
+
+def test_sums_of_a_batch_that_is_cut():
+    from torkit3d_b200 import _lib
+
+    B, N = 9001, 1024  # built in two parts
+    g = torch.Generator(device=DEV).manual_seed(1)
+    a, b = (torch.randn(B, N, 3, generator=g, device=DEV) for _ in range(2))
+    a[4000, 3], a[B - 1, 5] = 1e4, 1e4  # one swept cloud in each part
+    need = _lib.load().tk3d_chamfer_fwd_scratch_bytes(B, N, N, _lib.F32)
+    x, y = _chamfer(a, b, None), _chamfer(a, b, torch.empty(need, dtype=torch.uint8, device=DEV))
+    for p, q in zip(x[:4], y[:4]):
+        assert _same(p, q)
+    torch.testing.assert_close(x[4], y[4], rtol=1e-12, atol=0)
 
 
 @pytest.mark.parametrize("op", ["chamfer", "knn", "ball", "interp", "sa", "step"])

@@ -287,7 +287,7 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpUse use) {
     float x, y, z;
     load_xyz(xyz, j, c.l, x, y, z);
     const int to = atomicAdd(&hist[sp_cell(x, y, z, g)], 1);
-    pts[to] = make_float4(x, y, z, __int_as_float(j));
+    pts[sp_checked(to, N)] = make_float4(x, y, z, __int_as_float(j));
   }
   if (rank == 0) {
     // padding of the last window: NaN distances are never below or at a bound
@@ -476,7 +476,7 @@ spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sum
     const int first = (int)(task - b * qc.groups) * SP_GROUP;
     const SpGrid g = kc.grid[b];
     if (!(g.irregular | qc.grid[b].irregular)) {
-      const float4 q = sp_point(qc.pts + b * (int64_t)qc.windows * SP_WINDOW * 4, first + lane);
+      const float4 q = sp_point(qc.pts + b * (int64_t)qc.windows * SP_WINDOW * 4, first + lane, qc.windows);
       const bool valid = first + lane < qc.N;
       // minima and maxima drop the NaN of padding lanes
       const SpBox qbox = {sp_warp_min(q.x), sp_warp_min(q.y), sp_warp_min(q.z),
@@ -498,7 +498,7 @@ spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sum
         list.d[c] = sp_inf();
         list.i[c] = MODE == SN_CHAMFER ? -1 : 0x7fffffff;
       }
-      sp_scan<K>(kpts + seed * 32, nx, ny, nz, one, list);
+      sp_scan<K>(sp_leaf(kpts, seed, kc.windows), nx, ny, nz, one, list);
       if constexpr (K > 1) {
         // the seeds come again with their leaf: keep their bound only
         const float bound = list.d[K - 1];
@@ -551,7 +551,7 @@ spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sum
               const int low = __float_as_int(__ldg(reinterpret_cast<const float *>(kbox + 2 * l) + 6));
               if (!__any_sync(0xffffffffu, bd == list.d[K - 1] && low < list.i[K - 1])) continue;
             }
-            sp_scan<K>(kpts + l * 32, nx, ny, nz, one, list);
+            sp_scan<K>(sp_leaf(kpts, l, kc.windows), nx, ny, nz, one, list);
             gb = sp_warp_max(list.d[K - 1]);
             if (!(reach <= gb)) key = far;
           }

@@ -274,8 +274,19 @@ __device__ __forceinline__ float sp_min8(const float2 (&d)[4]) {
   return fminf(m, d[3].y);
 }
 
+// Positions and leaves of an ordered cloud of `windows` windows; the range-checked build counts those outside.
+#ifdef TK3D_BOUNDS
+__device__ __forceinline__ int sp_checked(int i, int n) { return (int)tk3d_checked(i, n); }
+#else
+__device__ __forceinline__ int sp_checked(int i, int) { return i; }
+#endif
+__device__ __forceinline__ const float *sp_leaf(const float *__restrict__ pts, int leaf, int windows) {
+  return pts + sp_checked(leaf, windows * 32) * 32;
+}
+
 // Point `pos` of an ordered cloud: coordinates and original index.
-__device__ __forceinline__ float4 sp_point(const float *__restrict__ pts, int pos) {
+__device__ __forceinline__ float4 sp_point(const float *__restrict__ pts, int pos, int windows) {
+  pos = sp_checked(pos, windows * SP_WINDOW);
   const float *f = pts + (int64_t)(pos >> 3) * 32 + (pos & 7);
   return make_float4(__ldg(f), __ldg(f + 8), __ldg(f + 16), __ldg(f + 24));
 }

@@ -50,7 +50,7 @@ spatial_ball_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ 
     q.w = __int_as_float(valid ? first_q + lane : 0);
     if (valid) load_xyz(qc.xyz + b * 3 * (int64_t)qc.N, first_q + lane, qc.l, q.x, q.y, q.z);
   } else {
-    q = sp_point(qc.pts + b * (int64_t)qc.windows * SP_WINDOW * 4, first_q + lane);
+    q = sp_point(qc.pts + b * (int64_t)qc.windows * SP_WINDOW * 4, first_q + lane, qc.windows);
   }
   const int64_t row = (b * qc.N + (valid ? __float_as_int(q.w) : 0)) * (int64_t)k;
 
@@ -114,7 +114,7 @@ spatial_ball_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ 
       const float lim = valid ? r2 : 0.f;  // no distance is below 0
 #pragma unroll 2
       for (int li = part; li < n1; li += SQ_WARPS) {
-        const float *leaf = kpts + sm.b.list[1][li] * 32;
+        const float *leaf = sp_leaf(kpts, sm.b.list[1][li], kc.windows);
         float2 d[4];
         sp_leaf_dist(leaf, nx, ny, nz, one, d);
         if (sp_min8(d) < lim) {

@@ -67,7 +67,7 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
   const SpGrid g = kc.grid[b];
   if (g.irregular | qc.grid[b].irregular) return;  // the whole block
 
-  float4 q = sp_point(qc.pts + b * (int64_t)qc.windows * SP_WINDOW * 4, first_q + lane);
+  float4 q = sp_point(qc.pts + b * (int64_t)qc.windows * SP_WINDOW * 4, first_q + lane, qc.windows);
   const bool valid = first_q + lane < qc.N;
   const SpBox qbox = {sp_warp_min(q.x), sp_warp_min(q.y), sp_warp_min(q.z),
                       sp_warp_max(q.x), sp_warp_max(q.y), sp_warp_max(q.z)};
@@ -128,7 +128,8 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
     const int p0 = __ldg(tab + e), p1 = e + 1 < SP_CELLS ? __ldg(tab + e + 1) : kc.N;
     const int seed = min(max(((p0 + p1) >> 4) - SEED / 2, 0), (kc.N >> 3) - SEED);
 #pragma unroll
-    for (int i = 0; i < SEED / SK_WARPS; ++i) take(kpts + (seed + i * SK_WARPS + part) * 32, 8 * (i % U));
+    for (int i = 0; i < SEED / SK_WARPS; ++i)
+      take(sp_leaf(kpts, seed + i * SK_WARPS + part, kc.windows), 8 * (i % U));
   }
   float top = cmin[0];
 #pragma unroll
@@ -194,7 +195,7 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = li + u * SK_WARPS;
-      if (i < n1) take(kpts + (all ? i : list1[i]) * 32, 8 * u);
+      if (i < n1) take(sp_leaf(kpts, all ? i : list1[i], kc.windows), 8 * u);
     }
   }
   const float tau1 = kth_bound(tau0);
@@ -214,7 +215,7 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
   for (int li = part; li < n2; li += SK_WARPS) {
     const int leaf = last ? last[li] : li;
     float2 d[4];
-    sp_leaf_dist(kpts + leaf * 32, nx, ny, nz, one, d);
+    sp_leaf_dist(sp_leaf(kpts, leaf, kc.windows), nx, ny, nz, one, d);
     // padding keys have NaN distances, which the minima drop; a leaf of nothing else gives +inf
     kt_append<32 * 4, QCAP>(fminf(sp_min8(d), pinf()), thr, cnt_addr, cand_addr, leaf);
   }
@@ -225,7 +226,7 @@ spatial_knn_kernel(const __grid_constant__ SpCloud qc, const __grid_constant__ S
   if (valid && n <= QCAP) {
     int hits = 0;
     for (int c = part; c < n; c += SK_WARPS) {
-      const float *leaf = kpts + cand[c * 32 + lane] * 32;
+      const float *leaf = sp_leaf(kpts, cand[c * 32 + lane], kc.windows);
       float2 d2[4];
       int ji[8];
       sp_leaf_dist(leaf, nx, ny, nz, one, d2);
