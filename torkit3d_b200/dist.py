@@ -226,7 +226,7 @@ def chamfer_step_from_host(xyz1_host, xyz2_host, device, global_batch=None, grou
     possible because the mean loss is linear in the per-point distances: d loss / d dist is the
     constant 1/count, known before any distance is, so each slice's gradient kernels can run right
     after its forward kernel.  Slicing adds launches and host work per slice: on B200, 64 pairs of
-    16384-point clouds in 8 slices ran slower (7.3 ms) than unsliced (6.85 ms).  To hide the copy of
+    16384-point clouds took 1.30 ms unsliced, 1.19 in 2 slices, 1.36 in 4, 1.82 in 8.  To hide the copy of
     such batches use ``HostCloudPrefetcher`` across steps.
 
     Args:
