@@ -123,22 +123,16 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpUse use) {
   constexpr int PER = PK_SAMPLE / CL, HALF = (PER + 1) / 2;
   const int dir = warp & 1, slice = (warp >> 1) & (PK_KEYS / 32 - 1), i0 = (warp >> 3) * HALF;
   const bool looks = use.prunes && (dir == 0 || use.both) && i0 < PER;
-  float reach[HALF];
-  if (looks) {
+  float kx, ky, kz, qx[HALF], qy[HALF], qz[HALF], nx[HALF], ny[HALF], nz[HALF];
+  if (looks) {  // loaded ahead, looked at behind the first pass
     const SpCloud &qc = pair.c[dir], &kc = pair.c[1 - dir];
-    const float *kx = kc.xyz + b * 3 * (int64_t)kc.N, *qx = qc.xyz + b * 3 * (int64_t)qc.N;
-    float x, y, z;
-    load_xyz(kx, pk_key(slice * 32 + lane, kc.N), kc.l, x, y, z);
+    const float *kp = kc.xyz + b * 3 * (int64_t)kc.N, *qp = qc.xyz + b * 3 * (int64_t)qc.N;
+    load_xyz(kp, pk_key(slice * 32 + lane, kc.N), kc.l, kx, ky, kz);
 #pragma unroll
-    for (int i = 0; i < HALF; ++i) {  // nearest sampled key of every query, nearest other one of every key
+    for (int i = 0; i < HALF; ++i) {
       const int s = rank * PER + i0 + i;
-      float u, w, r;
-      load_xyz(qx, (int64_t)s * qc.N / PK_SAMPLE, qc.l, u, w, r);
-      reach[i] = sp_sq3(u - x, w - y, r - z);
-      load_xyz(kx, pk_key(s * (PK_KEYS / PK_SAMPLE), kc.N), kc.l, u, w, r);
-      const float e = sp_sq3(u - x, w - y, r - z);
-      const float dq = sp_warp_min(reach[i]), dk = sp_warp_min(e > 0.f ? e : sp_inf());
-      if (lane == 0) least[dir][0][i0 + i][slice] = dq, least[dir][1][i0 + i][slice] = dk;
+      load_xyz(qp, (int64_t)s * qc.N / PK_SAMPLE, qc.l, qx[i], qy[i], qz[i]);
+      load_xyz(kp, pk_key(s * (PK_KEYS / PK_SAMPLE), kc.N), kc.l, nx[i], ny[i], nz[i]);
     }
   }
   if (tid < 2) near[tid] = 0;
@@ -150,6 +144,16 @@ spatial_sort_kernel(const __grid_constant__ SpPair pair, int B, SpUse use) {
     v[0] = fminf(v[0], x), v[1] = fminf(v[1], y), v[2] = fminf(v[2], z);
     v[3] = fmaxf(v[3], x), v[4] = fmaxf(v[4], y), v[5] = fmaxf(v[5], z);
     if (!(fabsf(x) < sp_inf() && fabsf(y) < sp_inf() && fabsf(z) < sp_inf())) v[6] = 1.f;
+  }
+  float reach[HALF];
+  if (looks) {  // nearest sampled key of every query, nearest other one of every key
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {
+      reach[i] = sp_sq3(qx[i] - kx, qy[i] - ky, qz[i] - kz);
+      const float e = sp_sq3(nx[i] - kx, ny[i] - ky, nz[i] - kz);
+      const float dq = sp_warp_min(reach[i]), dk = sp_warp_min(e > 0.f ? e : sp_inf());
+      if (lane == 0) least[dir][0][i0 + i][slice] = dq, least[dir][1][i0 + i][slice] = dk;
+    }
   }
 #pragma unroll
   for (int i = 0; i < 7; ++i) v[i] = i < 3 ? sp_warp_min(v[i]) : sp_warp_max(v[i]);
