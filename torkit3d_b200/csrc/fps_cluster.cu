@@ -7,7 +7,7 @@
 // L2 in every step (4 clouds of 65536 points: 19 us per step).  Here a cluster of 4, 8 or 16 small
 // blocks shares a cloud: every block keeps a contiguous slice of the points and their running
 // minima in registers (8 to 32 points per thread), and the step has no block or cluster barrier at
-// all -- see fps_warpcast_kernel.  32 clouds of 8192 points, 1024 samples: 0.34 ms against 0.70 ms;
+// all -- see fps_warpcast_kernel.  32 clouds of 8192 points, 1024 samples: 0.33 ms against 0.70 ms;
 // 4 clouds of 65536 points, 2048 samples: 1.12 ms against 39.9 ms for the streaming kernel.
 //
 // Measured and dropped: the same clusters with 1024-thread blocks that reduce inside the block
@@ -44,10 +44,10 @@ constexpr int FC_MAX_CL = 16;  // 8 is the portable cluster size; 16 needs an op
 // closer to it than its running minimum.  Nothing else can be farther: a warp whose candidate has not
 // been taken has no point above it.  The first candidate always passes, so the sequence is the one
 // of single steps, bit for bit.  Counted on the CPU, an exchange yields 3.5 to 4.3 samples; taking one
-// costs about 0.15 us, an exchange 0.45 us and more.  32 clouds of 8192 points, 1024 samples: 0.34 ms,
+// costs about 0.15 us, an exchange 0.45 us and more.  32 clouds of 8192 points, 1024 samples: 0.33 ms,
 // one sample per exchange 0.56; 4 clouds of 65536 points, 2048 samples: 1.12 ms, 1.95.  Where most
-// distances tie (a lattice of 1000 positions) exchanges yield little more than one sample, at 1.05 to
-// 1.2 times the cost.
+// distances tie (all points the same, a lattice of fewer positions than points) exchanges yield little
+// more than one sample, at 1.06 to 1.35 times the cost.
 //
 // The candidate slots and mbarriers are double buffered by the parity of the exchange: a warp can send
 // for exchange i+2 only after it has seen every warp's candidate of exchange i+1, which those warps
@@ -195,23 +195,30 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
     const float2 dx = __fadd2_rn(qx_, nx), dy = __fadd2_rn(qy_, ny), dz = __fadd2_rn(qz_, nz);
     return __ffma2_rn(__ffma2_rn(__fmul2_rn(dx, dx), one2, __fmul2_rn(dy, dy)), one2, __fmul2_rn(dz, dz));
   };
+  // The thread's largest running minimum is taken along with few points (8192 points, 1024 samples: 338 -> 332 us, all
+  // points the same 655 -> 630), on its own with many (65536 points: 1157, taken along 1181).
+  constexpr bool FUSED = FW_P2 <= 4;
+  float bm = 0.f;
   auto apply = [&](float x, float y, float z) {
+    if constexpr (FUSED) bm = 0.f;
     const float2 nx = make_float2(-x, -x), ny = make_float2(-y, -y), nz = make_float2(-z, -z);
 #pragma unroll
     for (int i = 0; i < FW_P2; ++i) {
       const float2 d = dist2(i, nx, ny, nz);
       md[i].x = fminf(md[i].x, d.x);
       md[i].y = fminf(md[i].y, d.y);
+      if constexpr (FUSED) asm("max.f32 %0, %0, %1, %2;" : "+f"(bm) : "f"(md[i].x), "f"(md[i].y));
     }
   };
   auto thread_max = [&]() {
+    if constexpr (FUSED) return bm;
     float m = 0.f;
 #pragma unroll
     for (int i = 0; i < FW_P2; ++i) asm("max.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(md[i].x), "f"(md[i].y));
     return m;
   };
   apply(cx, cy, cz);  // sample 0
-  float bm = thread_max();
+  bm = thread_max();
 
   constexpr int CPL = FW_SLOTS / 32;  // candidates of a lane
   bool failed = false;
@@ -317,7 +324,9 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       }
       continue;
     }
-    // lane l holds candidates l, l + 32, ...
+    // lane l holds candidates l, l + 32, ...; without bounds four of them are not looked at beyond distance and index
+    // (131072 points all the same, 512 samples: 890 -> 824 us)
+    const bool whole = CPL <= 2 || ex >= again;
     unsigned cb[CPL];
     int ci[CPL];
     float kx[CPL], ky[CPL], kz[CPL];
@@ -327,12 +336,18 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       const int sl = lane + 32 * c;
       const bool has = sl < nw;
       // whole words: the slots are 32 bytes apart, and single words would meet in four banks
-      const uint4 v = *reinterpret_cast<const uint4 *>(&cand[par][has ? sl : 0]);
-      cb[c] = has ? v.x : 0u;
-      ci[c] = has ? (int)v.y : 0x7fffffff;
-      kx[c] = __uint_as_float(v.z);
-      ky[c] = __uint_as_float(v.w);
-      kz[c] = cand[par][has ? sl : 0].z;
+      if (whole) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(&cand[par][has ? sl : 0]);
+        cb[c] = has ? v.x : 0u;
+        ci[c] = has ? (int)v.y : 0x7fffffff;
+        kx[c] = __uint_as_float(v.z);
+        ky[c] = __uint_as_float(v.w);
+        kz[c] = cand[par][has ? sl : 0].z;
+      } else {
+        const uint2 v = *reinterpret_cast<const uint2 *>(&cand[par][has ? sl : 0]);
+        cb[c] = has ? v.x : 0u;
+        ci[c] = has ? (int)v.y : 0x7fffffff;
+      }
       reduced[c] = false;
     }
     unsigned bound = 0u;
@@ -377,15 +392,17 @@ fps_warpcast_kernel(const float *__restrict__ points, int N, int NL, int S, int6
       }
       ++n;
       ++taken;
+      if (whole) {
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        if (lane + 32 * c == src) {
-          cb[c] = 0u;
-          ci[c] = 0x7fffffff;
+        for (int c = 0; c < CPL; ++c) {
+          if (lane + 32 * c == src) {
+            cb[c] = 0u;
+            ci[c] = 0x7fffffff;
+          }
+          reduced[c] |= sqdist<float>(kx[c], ky[c], kz[c], cx, cy, cz) < __uint_as_float(cb[c]);
         }
-        reduced[c] |= sqdist<float>(kx[c], ky[c], kz[c], cx, cy, cz) < __uint_as_float(cb[c]);
+        if constexpr (CPL == 1) stale = __ballot_sync(0xffffffffu, reduced[0]);
       }
-      if constexpr (CPL == 1) stale = __ballot_sync(0xffffffffu, reduced[0]);
       // in the shadow of the next pick's reductions
       apply(cx, cy, cz);
       if (taken == FW_BATCH || n >= stop || ex < again) break;
@@ -654,10 +671,13 @@ static bool fps_warpcast_launch(const float *points, int64_t B, int64_t N, int64
 // 4097 to 16384 points and few clouds: up to 8192 points clusters of four blocks of 256 threads (8
 // points per thread), beyond that eight blocks of 128 threads (16 points per thread).  Measured on
 // two B200s, 512 samples, against one 1024-thread block per cloud (fps_resident_kernel), in ms:
-//   clouds                      4      32     64     96
-//   N =  8192  4 x 256 threads  0.26-0.27  0.28  0.33   0.40     one block  0.356
-//              8 x  64 threads  0.25-0.29  0.27-0.31  0.30-0.33  0.36   (faster on one GPU, slower on the other)
-//   N = 16384  8 x 128 threads  0.30   0.34-0.37  0.45   0.76     one block  0.699
+//   clouds                           4      32     64     96     148
+//   N =  8192  surface               0.182  0.196  0.262  0.333  0.532   one block  0.352
+//              lattice               0.244  0.245  0.327  0.419  0.663              0.366
+//              all the same          0.316  0.330  0.407  0.528  0.855              0.408
+//   N = 16384  surface               0.219  0.259  0.368  0.572  0.830   one block  0.694
+//              lattice               0.290  0.332  0.467  0.742  1.074              0.730
+//              all the same          0.321  0.384  0.495  0.812  1.194              0.812
 // Beyond about half a cloud per SM the blocks of several clusters share SMs and the one-block
 // kernel is as fast; up to 4096 points its step (0.43 us) is shorter than the exchange over
 // distributed shared memory (0.45 to 0.5 us).
@@ -673,7 +693,7 @@ static bool fps_warpcast_launch(const float *points, int64_t B, int64_t N, int64
 // `force`: the diagnostic entry, several always.
 static bool fps_cluster_dispatch(const float *points, int64_t B, int64_t N, int64_t S, int ps, int64_t cs,
                                  int64_t *index, float *sampled, cudaStream_t st, int *rc, FwWait wt, bool force) {
-  const bool batched = force || S >= (N <= 16384 ? 192 : 384);
+  const bool batched = force || S >= (N <= 16384 ? 160 : N <= 65536 ? 240 : 384);
   if (N > 4096 && N <= 16384) {
     if (N <= 8192) {
       if (!force && B * 15 > (int64_t)sm_count() * 7) return false;
