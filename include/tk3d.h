@@ -334,8 +334,9 @@ int tk3d_fps_gather(const void *points, int64_t B, int64_t N, int64_t num_sample
 /*
  * Set-abstraction grouping: ball query + group_points of the features + group_points of the
  * coordinates + centring + concatenation, i.e. everything SetAbstraction.forward does before its
- * MLP (torkit3d/layers/pointnet2.py:43-58 with query_neighbor = BallQuery), in two launches (one
- * transpose of the features into `scratch`, one fused kernel).
+ * MLP (torkit3d/layers/pointnet2.py:43-58 with query_neighbor = BallQuery), in two launches (neighbours and
+ * a gather by channel rows; a transpose of the features into `scratch` and one fused kernel for few entries and for clouds
+ * whose rows do not fit shared memory).
  *   points    [B,N,3]|[B,3,N]  in   coordinates of the N input points ("in_xyz")
  *   centroids [B,M,3]|[B,3,M]  in   coordinates of the M group centres ("out_xyz")
  *   feature   [B,C,N]          in   may be NULL when C == 0

@@ -6,6 +6,7 @@
 // a contiguous run of E elements indexed by the SAME E indices for every channel, so a thread
 // loads its indices once (the reference re-reads the int64 index tensor for every channel) and
 // then walks the channels.
+#include "chanrow.cuh"
 #include "rows.cuh"
 
 namespace tk3d {
@@ -128,148 +129,6 @@ group_bwd_kernel(const T *__restrict__ gout, const int64_t *__restrict__ index, 
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// Channel-row forward kernel (clouds whose N1 features fit shared memory twice): no transposed
-// copy of the features, no scratch.  (The mirror image for the backward -- gradient rows
-// accumulated with shared-memory reductions -- was measured slower than the vector reductions
-// into a transposed accumulator, 0.18 against 0.12 ms on 32 x 64 x 8192 <- 32768 entries: a
-// shared-memory float reduction per element is the bottleneck.)
-//
-// A block owns a chunk of the E = N2*K index entries of one cloud -- each thread keeps
-// its entries' indices in registers for the whole block -- and walks a group of channels.  The
-// N1 features of a channel are one contiguous row of the [B,C,N1] tensor: the row is brought into
-// shared memory with 16-byte cp.async copies, double buffered so that the next row lands while
-// the current one is gathered, and the gather itself is a shared-memory read per output element
-// followed by 16-byte streaming stores of four consecutive entries.  HBM sees every feature and
-// every index once (the row re-reads of neighbouring blocks hit L2) and the output once.
-// An index outside [0,N1) reads the zero kept behind the row.
-constexpr int CR_THREADS = 256;
-
-__device__ __forceinline__ void cr_cp_async16(void *smem, const void *gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
-               : "memory");
-}
-__device__ __forceinline__ void cr_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cr_cp_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-
-// R rounds of four consecutive entries per thread: a block covers CR_THREADS * 4 * R entries.
-template <typename T, typename IndexT, int R, bool VEC>
-__global__ void __launch_bounds__(CR_THREADS)
-group_fwd_chanrow_kernel(const T *__restrict__ in, const IndexT *__restrict__ index, int C, int N1, int64_t E,
-                         int cg, T *__restrict__ out, int32_t *__restrict__ status) {
-  extern __shared__ __align__(16) unsigned char cr_raw[];
-  T *cr_rows = reinterpret_cast<T *>(cr_raw);  // [2][N1 + 4]; slots N1..N1+3 of each hold 0
-  constexpr int PER16 = 16 / (int)sizeof(T);   // elements per 16-byte copy
-  const int tid = threadIdx.x;
-  const int64_t b = blockIdx.z;
-  const int c0 = blockIdx.y * cg, c1 = min(C, c0 + cg);
-  const int64_t e0 = (int64_t)blockIdx.x * (CR_THREADS * 4 * R);
-  const int stride = N1 + 4;
-
-  int id[R][4];
-  bool bad = false;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int64_t e = e0 + (int64_t)(r * CR_THREADS + tid) * 4 + v;
-      int64_t j = e < E ? (int64_t)index[b * E + e] : 0;
-      if (j < 0 || j >= N1) {
-        j = N1;  // the zero behind the row
-        bad = true;
-      }
-      id[r][v] = (int)j;
-    }
-  }
-  if (bad && status) atomicOr(status, 1);
-  if (tid < 8) cr_rows[(tid >> 2) * stride + N1 + (tid & 3)] = (T)0;
-
-  const T *src = in + (b * C + c0) * (int64_t)N1;
-  auto stage = [&](int c, int buf) {
-    const T *g = src + (int64_t)(c - c0) * N1;
-    T *d = cr_rows + buf * stride;
-    for (int q = tid; q < N1 / PER16; q += CR_THREADS) cr_cp_async16(d + PER16 * q, g + PER16 * q);
-    cr_cp_commit();
-  };
-  stage(c0, 0);
-  for (int c = c0; c < c1; ++c) {
-    const int buf = (c - c0) & 1;
-    if (c + 1 < c1) {
-      stage(c + 1, buf ^ 1);  // the other buffer was released by the barrier that ended the last round
-      cr_cp_wait<1>();
-    } else {
-      cr_cp_wait<0>();
-    }
-    __syncthreads();
-    const T *row = cr_rows + buf * stride;
-    T *o = out + (b * C + c) * E;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int64_t e = e0 + (int64_t)(r * CR_THREADS + tid) * 4;
-      if (e >= E) break;
-      const T v0 = row[id[r][0]], v1 = row[id[r][1]], v2 = row[id[r][2]], v3 = row[id[r][3]];
-      if (VEC) {
-        if constexpr (sizeof(T) == 4) {
-          __stcs(reinterpret_cast<float4 *>(o + e), make_float4(v0, v1, v2, v3));
-        } else {
-          __stcs(reinterpret_cast<double2 *>(o + e), make_double2(v0, v1));
-          __stcs(reinterpret_cast<double2 *>(o + e) + 1, make_double2(v2, v3));
-        }
-      } else {
-        o[e] = v0;
-        if (e + 1 < E) o[e + 1] = v1;
-        if (e + 2 < E) o[e + 2] = v2;
-        if (e + 3 < E) o[e + 3] = v3;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// Largest cloud the channel-row kernels take: two rows (forward) must fit the 227 KB of an SM
-// (24576 floats or 12288 doubles).
-constexpr int64_t CR_MAX_ROW_BYTES = 24576 * 4;
-
-inline bool chanrow_ok(const void *in, int64_t B, int64_t C, int64_t N1, int64_t E, int64_t elem = 4) {
-  return N1 >= 256 && N1 % 4 == 0 && N1 * elem <= CR_MAX_ROW_BYTES && E >= 1024 && B <= 65535 && C <= 65535 &&
-         (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-}
-
-template <typename T, typename IndexT>
-int group_fwd_chanrow(const T *in, const IndexT *index, int64_t B, int64_t C, int64_t N1, int64_t E, T *out,
-                      int32_t *status, cudaStream_t st) {
-  // entries per block: 8192 when that still leaves enough blocks, else 4096
-  const int64_t sms = sm_count();
-  const bool big = B * ((E + 8191) / 8192) * 4 >= 3 * sms;
-  const int64_t ech = big ? 8192 : 4096;
-  const int64_t chunks = (E + ech - 1) / ech;
-  // channel groups: enough blocks for about three per SM, as few groups as possible beyond that
-  int64_t groups = (3 * sms + B * chunks - 1) / (B * chunks);
-  groups = groups < 1 ? 1 : (groups > C ? C : groups);
-  const int cg = (int)((C + groups - 1) / groups);
-  groups = (C + cg - 1) / cg;
-  TK3D_REQUIRE(chunks < (1LL << 31), TK3D_ERR_SHAPE, "group_points: too many entries");
-  const size_t smem = (size_t)2 * (N1 + 4) * sizeof(T);
-  dim3 grid((unsigned)chunks, (unsigned)groups, (unsigned)B);
-  const bool vec = E % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-#define TK3D_CR_LAUNCH(RR, VV)                                                                                   \
-  {                                                                                                              \
-    TK3D_CUDA(raise_smem_limit((const void *)group_fwd_chanrow_kernel<T, IndexT, RR, VV>, (int)smem));             \
-    group_fwd_chanrow_kernel<T, IndexT, RR, VV><<<grid, CR_THREADS, smem, st>>>(in, index, (int)C, (int)N1, E, cg, \
-                                                                                out, status);                       \
-  }
-  if (big) {
-    if (vec) TK3D_CR_LAUNCH(8, true) else TK3D_CR_LAUNCH(8, false)
-  } else {
-    if (vec) TK3D_CR_LAUNCH(4, true) else TK3D_CR_LAUNCH(4, false)
-  }
-#undef TK3D_CR_LAUNCH
-  return check_launch("group_fwd_chanrow_kernel");
-}
-
 // How many channels one block walks: enough blocks to fill the GPU a few times over, but as few
 // channel groups as possible so the indices are read once per group.
 int64_t channels_per_block(int64_t tiles, int64_t B, int64_t C, int mult = 8) {
@@ -329,9 +188,8 @@ using namespace tk3d;
 
 extern "C" size_t tk3d_group_fwd_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K, int dtype) {
   if (dtype != TK3D_F32 || B <= 0 || C <= 0 || N1 <= 0 || N2 <= 0 || K <= 0 || B > 65535) return 0;
-  // shapes the channel-row kernels take need no scratch (given 16-byte aligned features; an
-  // unaligned tensor then runs the direct kernel)
-  if (chanrow_ok(nullptr, B, C, N1, N2 * K)) return 0;
+  // shapes the channel-row kernels take need no scratch
+  if (chanrow_ok(B, C, N1, N2 * K)) return 0;
   return rows_profitable(C, N1, N2 * K, 1) ? rows_scratch_bytes(B, C, N1) : 0;
 }
 
@@ -345,8 +203,8 @@ static int group_fwd_impl(const void *in, const IndexT *index, int64_t B, int64_
   TK3D_REQUIRE(index && out && (in || N1 == 0), TK3D_ERR_NULL, "group_fwd: a pointer is NULL");
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == TK3D_F32) {
-    if (chanrow_ok(in, B, C, N1, E))
-      return group_fwd_chanrow<float, IndexT>((const float *)in, index, B, C, N1, E, (float *)out, status, st);
+    if (chanrow_ok(B, C, N1, E))
+      return group_fwd_chanrow<float, IndexT>((const float *)in, index, B, C, N1, E, (float *)out, C * E, status, nullptr, st);
     const size_t want = tk3d_group_fwd_scratch_bytes(B, C, N1, N2, K, dtype);
     const size_t rows = rows_profitable(C, N1, E, 1) && B <= 65535 ? rows_scratch_bytes(B, C, N1) : 0;
     (void)want;
@@ -355,8 +213,9 @@ static int group_fwd_impl(const void *in, const IndexT *index, int64_t B, int64_
                                     (float *)scratch, st);
     return group_fwd_t<float, IndexT>((const float *)in, index, B, C, N1, E, (float *)out, status, st);
   }
-  if (chanrow_ok(in, B, C, N1, E, 8))
-    return group_fwd_chanrow<double, IndexT>((const double *)in, index, B, C, N1, E, (double *)out, status, st);
+  if (chanrow_ok(B, C, N1, E, 8))
+    return group_fwd_chanrow<double, IndexT>((const double *)in, index, B, C, N1, E, (double *)out, C * E, status, nullptr,
+                                             st);
   return group_fwd_t<double, IndexT>((const double *)in, index, B, C, N1, E, (double *)out, status, st);
 }
 

@@ -22,8 +22,10 @@
 // close to the sum of a ball query (0.13 ms) and a gather (0.11 ms); larger batches, whose blocks
 // come in several waves, let the sweep of one block overlap the traffic of another.
 //
-// Large problems whose scratch allows it find the neighbours over spatially ordered clouds first
-// (spatial_ball.cu); the kernel then starts from those lists.
+// This kernel serves clouds of more than 24576 or fewer than 256 points and small calls; elsewhere the neighbours are found
+// first and gathered by channel rows (sa_two_step).  Large problems whose scratch allows it find them over spatially
+// ordered clouds (spatial_ball.cu); the kernel then starts from those lists.
+#include "chanrow.cuh"
 #include "rows.cuh"
 #include "spatial.cuh"
 #include "sweep.cuh"
@@ -358,6 +360,14 @@ bool ball_order_pays(int64_t B, int64_t N1, int64_t N2);
 }
 static size_t sa_align(size_t n) { return (n + 255) & ~(size_t)255; }
 
+// Neighbours first, then a gather by channel rows, where rows fit shared memory and there are enough entries.  B200, us, the
+// fused kernel with its transposition / two kernels: 32 x 512 points, 128 centres, K = 64, C = 128 96 / 40 (few blocks for
+// the machine's size, each with both phases one behind the other); 1 x the same 91 / 14; 32 x 8192, 1024, 32, 64 202 / 166;
+// 2 x 24000, 2000, 64, 256 371 / 254; 8 x 24000, 4000, 16, 32 306 / 305.
+static bool sa_two_step(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K) {
+  return chanrow_ok(B, C, N, M * K);
+}
+
 extern "C" size_t tk3d_sa_group_scratch_bytes(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K, int dtype) {
   if (!tk3d_sa_group_supported(B, C, N, M, K, dtype) || C == 0) return 0;
   const size_t rows = rows_scratch_bytes(B, C, N);
@@ -379,22 +389,39 @@ extern "C" int tk3d_sa_group_fwd(const void *points, const void *centroids, cons
   TK3D_REQUIRE(centroids && out && (points || N == 0) && (feature || C == 0), TK3D_ERR_NULL,
                "sa_group_fwd: a pointer is NULL");
   cudaStream_t st = (cudaStream_t)stream;
+  const size_t rows = rows_scratch_bytes(B, C, N);
+  TK3D_REQUIRE(C == 0 || N == 0 || (scratch != nullptr && scratch_bytes >= rows), TK3D_ERR_SCRATCH,
+               "sa_group_fwd: scratch of %zu bytes required (got %zu)", rows, scratch_bytes);
+  const bool order = C > 0 && ball_order_pays(B, M, N) &&
+                     scratch_bytes >= tk3d_sa_group_scratch_bytes(B, C, N, M, K, dtype);
+  char *search = order ? (char *)scratch + sa_align(rows) : nullptr;
+  int32_t *lists = index32 ? index32 : order ? reinterpret_cast<int32_t *>(search + sp_search_bytes(B, M, N)) : nullptr;
+  const size_t list_bytes = sizeof(int32_t) * (size_t)(B * M * K);
+  if (!lists && scratch_bytes >= list_bytes) lists = (int32_t *)scratch;
+  if (N > 0 && lists && sa_two_step(B, C, N, M, K)) {
+    int rc = tk3d_ball_query_ws(centroids, points, B, M, N, radius, K, xyz_channel_first, lists, TK3D_I32, search,
+                                order ? sp_search_bytes(B, M, N) : 0, TK3D_F32, stream);
+    if (rc) return rc;
+    CrXyz xyz;
+    xyz.points = (const float *)points;
+    xyz.cent = (const float *)centroids;
+    xyz.pps = xyz_channel_first ? 1 : 3, xyz.pcs = xyz_channel_first ? (int)N : 1;
+    xyz.cps = xyz_channel_first ? 1 : 3, xyz.cpc = xyz_channel_first ? (int)M : 1;
+    xyz.K = (int)K, xyz.M = (int)M;
+    return group_fwd_chanrow<float, int32_t>((const float *)feature, lists, B, C, N, M * K, (float *)out, ctot * M * K,
+                                             status, use_xyz ? &xyz : nullptr, st);
+  }
   const float *featT = nullptr;
   if (C > 0 && N > 0) {
-    const size_t want = rows_scratch_bytes(B, C, N);
-    TK3D_REQUIRE(scratch != nullptr && scratch_bytes >= want, TK3D_ERR_SCRATCH,
-                 "sa_group_fwd: scratch of %zu bytes required (got %zu)", want, scratch_bytes);
     int rc = transpose_bcn((const float *)feature, (float *)scratch, B, C, N, st);
     if (rc) return rc;
     featT = (const float *)scratch;
   }
   const int32_t *given = nullptr;
-  if (C > 0 && ball_order_pays(B, M, N) &&
-      scratch_bytes >= tk3d_sa_group_scratch_bytes(B, C, N, M, K, dtype)) {
-    char *order = (char *)scratch + sa_align(rows_scratch_bytes(B, C, N));
-    int32_t *lists = index32 ? index32 : reinterpret_cast<int32_t *>(order + sp_search_bytes(B, M, N));
+  if (order) {
+    lists = index32 ? index32 : reinterpret_cast<int32_t *>(search + sp_search_bytes(B, M, N));
     int rc = sp_ball_query((const float *)centroids, (const float *)points, B, M, N, xyz_channel_first, radius * radius,
-                           (int)K, lists, 1, order, st);
+                           (int)K, lists, 1, search, st);
     if (rc) return rc;
     given = lists;
   }
