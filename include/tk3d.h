@@ -216,8 +216,8 @@ int tk3d_group_fwd(const void *in, const int64_t *index, int64_t B, int64_t C, i
  * Replaces group_points_backward_cuda (torkit3d/csrc/include/group_points.h:10-13,
  * torkit3d/csrc/cuda/group_points_kernel.cu:67-114).  Out-of-range indices are skipped and
  * reported through `status` as above.  `scratch` (optional, tk3d_group_bwd_scratch_bytes(...) bytes): the
- * gradients are accumulated with 16-byte vector atomics into a transposed [B,N1,C] buffer and transposed
- * back, instead of scattered single-float atomics.  Its contents on entry are ignored.
+ * gradients are accumulated with 16-byte vector atomics into rows [B,N1,C rounded up to 4] and written back channel by
+ * channel, instead of scattered single-float atomics.  Its contents on entry are ignored; 16-byte aligned, else unused.
  */
 size_t tk3d_group_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K, int dtype);
 int tk3d_group_bwd(const void *grad_out, const int64_t *index, int64_t B, int64_t C, int64_t N1, int64_t N2,
@@ -364,8 +364,10 @@ int tk3d_sa_group_fwd(const void *points, const void *centroids, const void *fea
  *   grad_feature   [B,C,N]            out, optional: scatter-add of the first C channels
  *   grad_points    like points        out, optional: scatter-add of the coordinate channels
  *   grad_centroids like centroids     out, optional: minus the sum over K of the coordinate channels
- * Each output is fully written (zeroed first where it accumulates).  `scratch` as in the forward.
+ * Each output is fully written (zeroed first where it accumulates).
+ *   scratch (optional, tk3d_sa_group_bwd_scratch_bytes(...) bytes): see tk3d_group_bwd
  */
+size_t tk3d_sa_group_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K, int dtype);
 int tk3d_sa_group_bwd(const void *grad_out, const int32_t *index32, int64_t B, int64_t C, int64_t N, int64_t M,
                       int64_t K, int xyz_channel_first, int use_xyz, void *grad_feature, void *grad_points,
                       void *grad_centroids, int32_t *status, void *scratch, size_t scratch_bytes, int dtype,
@@ -401,7 +403,7 @@ int tk3d_three_nn_interp_bwd(const void *grad_out, const int32_t *index32, const
  *       out[b,C+c,n,k] = query_feature[b,c,n]
  *   An index outside [0,N2) gathers 0 and ORs bit 0 into *status (optional).
  *   scratch (optional, tk3d_edge_feature_scratch_bytes(...) bytes; 0 = no fast path for the shape):
- *   same role as in tk3d_group_fwd / tk3d_group_bwd.
+ *   same role as in tk3d_group_fwd; the backward's is tk3d_edge_feature_bwd_scratch_bytes(...) bytes, see tk3d_group_bwd.
  * Backward: grad_key[b,c,index[b,n,k]] += grad_out[b,c,n,k];
  *           grad_query[b,c,n] = sum_k (grad_out[b,C+c,n,k] - grad_out[b,c,n,k]).
  * Either gradient pointer may be NULL; each one given is fully written.
@@ -410,6 +412,7 @@ size_t tk3d_edge_feature_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t
 int tk3d_edge_feature_fwd(const void *query_feature, const void *key_feature, const int64_t *index, int64_t B,
                           int64_t C, int64_t N1, int64_t N2, int64_t K, int include_query, void *out,
                           int32_t *status, void *scratch, size_t scratch_bytes, int dtype, void *stream);
+size_t tk3d_edge_feature_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K, int dtype);
 int tk3d_edge_feature_bwd(const void *grad_out, const int64_t *index, int64_t B, int64_t C, int64_t N1, int64_t N2,
                           int64_t K, int include_query, void *grad_query, void *grad_key, int32_t *status,
                           void *scratch, size_t scratch_bytes, int dtype, void *stream);

@@ -106,8 +106,7 @@ def sa_group_backward(grad_out, index32, C, N, use_xyz=True, channel_first=True,
             if (xyz and need_points) else None
         gcen = torch.empty((B, 3, M) if channel_first else (B, M, 3), dtype=torch.float32, device=dev) \
             if (xyz and need_centroids) else None
-        # the transposed gradient alone; the rest of that size is the forward's search
-        need = 4 * B * C * N if gfeat is not None and _lib.scratch_bytes("tk3d_sa_group", B, C, N, M, K, _lib.F32) else 0
+        need = _lib.scratch_bytes("tk3d_sa_group_bwd", B, C, N, M, K, _lib.F32) if gfeat is not None else 0
         scratch = _scratch(need, dev)
         check(lib.tk3d_sa_group_bwd(_ptr(grad_out), _ptr(index32), B, C, N, M, K, 1 if channel_first else 0,
                                     1 if use_xyz else 0, _ptr(gfeat) if gfeat is not None else None,
@@ -208,7 +207,7 @@ def edge_feature_backward(grad_out, index, C, N2, include_query=True, need_query
     with _on(dev):
         gq = torch.empty((B, C, N1), dtype=grad_out.dtype, device=dev) if need_query else None
         gk = torch.empty((B, C, N2), dtype=grad_out.dtype, device=dev) if need_key else None
-        need = _lib.scratch_bytes("tk3d_edge_feature", B, C, N1, N2, K, dt) if need_key else 0
+        need = _lib.scratch_bytes("tk3d_edge_feature_bwd", B, C, N1, N2, K, dt) if need_key else 0
         scratch = _scratch(need, dev)
         check(lib.tk3d_edge_feature_bwd(_ptr(grad_out), _ptr(index), B, C, N1, N2, K, 1 if include_query else 0,
                                         _ptr(gq) if need_query else None, _ptr(gk) if need_key else None, None,

@@ -54,6 +54,7 @@ SIGNATURES = {
     "tk3d_fps_gather": (_int, [_vp, _i64, _i64, _i64, _int, _vp, _vp, _vp, ctypes.c_size_t, _int, _vp]),
     "tk3d_sa_group_supported": (_int, [_i64, _i64, _i64, _i64, _i64, _int]),
     "tk3d_sa_group_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64, _i64, _int]),
+    "tk3d_sa_group_bwd_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64, _i64, _int]),
     "tk3d_sa_group_fwd": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, ctypes.c_float, _i64, _int, _int, _vp, _vp,
                                  _vp, _vp, ctypes.c_size_t, _int, _vp]),
     "tk3d_sa_group_bwd": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _i64, _int, _int, _vp, _vp, _vp, _vp, _vp,
@@ -64,6 +65,7 @@ SIGNATURES = {
     "tk3d_three_nn_interp_bwd": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp, _vp, ctypes.c_size_t, _int,
                                         _vp]),
     "tk3d_edge_feature_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64, _i64, _int]),
+    "tk3d_edge_feature_bwd_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64, _i64, _int]),
     "tk3d_edge_feature_fwd": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _int, _vp, _vp, _vp,
                                      ctypes.c_size_t, _int, _vp]),
     "tk3d_edge_feature_bwd": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _i64, _int, _vp, _vp, _vp, _vp,

@@ -10,6 +10,7 @@
 // the chunk-swizzled shared tile with 16-byte streaming stores.  Everything else takes a direct
 // kernel (one thread per output entry, walking the channels).
 #include "rows.cuh"
+#include "scatter.cuh"
 
 namespace tk3d {
 
@@ -205,6 +206,15 @@ extern "C" int tk3d_edge_feature_fwd(const void *query_feature, const void *key_
   return check_launch("edge_rows_vec4_kernel");
 }
 
+static bool edge_bwd_rows_ok(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K) {
+  return C >= 4 && C <= ROWS_MAX_C && scatter_ok(B, C, N2, N1, K) && scatter_pays(B, C, N1, K);
+}
+
+extern "C" size_t tk3d_edge_feature_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K,
+                                                      int dtype) {
+  return dtype == TK3D_F32 && edge_bwd_rows_ok(B, C, N1, N2, K) ? scatter_scratch_bytes(B, C, N2) : 0;
+}
+
 extern "C" int tk3d_edge_feature_bwd(const void *grad_out, const int64_t *index, int64_t B, int64_t C, int64_t N1,
                                      int64_t N2, int64_t K, int include_query, void *grad_query, void *grad_key,
                                      int32_t *status, void *scratch, size_t scratch_bytes, int dtype, void *stream) {
@@ -216,6 +226,27 @@ extern "C" int tk3d_edge_feature_bwd(const void *grad_out, const int64_t *index,
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t gstride = (include_query ? 2 * C : C) * E;
   const size_t elem = dtype == TK3D_F64 ? 8 : 4;
+  const bool rows = dtype == TK3D_F32 && grad_key && B * C * E > 0 && N2 > 0 && scratch != nullptr &&
+                    (reinterpret_cast<uintptr_t>(scratch) & 15) == 0 && edge_bwd_rows_ok(B, C, N1, N2, K) &&
+                    scratch_bytes >= scatter_scratch_bytes(B, C, N2);
+  if (rows) {
+    ScatterCall c;
+    c.gout = (const float *)grad_out;
+    c.index = index;
+    c.B = B, c.C = C, c.N = N2, c.M = N1, c.K = K;
+    c.gstride = gstride;
+    c.gin = (float *)grad_key;
+    if (grad_query && scatter_edge_ok(K)) {
+      c.gq = (float *)grad_query;
+      c.include_query = include_query;
+      grad_query = nullptr;
+    }
+    c.status = status;
+    c.scratch = scratch;
+    int rc = scatter_launch(c, st);
+    if (rc) return rc;
+    grad_key = nullptr;
+  }
   if (grad_query && B * C * N1 > 0) {
     const int64_t blocks = (B * C * N1 + 255) / 256, cap = (int64_t)sm_count() * 32;
     const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
@@ -229,20 +260,6 @@ extern "C" int tk3d_edge_feature_bwd(const void *grad_out, const int64_t *index,
     if (rc) return rc;
   }
   if (grad_key && B * C * N2 > 0) {
-    const size_t want = tk3d_edge_feature_scratch_bytes(B, C, N1, N2, K, dtype);
-    const bool rows = want != 0 && scratch != nullptr && scratch_bytes >= want && rows_vec_ok(C, E, grad_out, scratch);
-    if (rows) {
-      TK3D_CUDA(cudaMemsetAsync(scratch, 0, want, st));
-      const size_t smem = (size_t)C * ROWS_TE * sizeof(float);
-      if (smem > 48 * 1024)
-        TK3D_CUDA(raise_smem_limit((const void *)scatter_rows_vec4_kernel<1, int64_t>, (int)smem));
-      dim3 grid((unsigned)((E + ROWS_TE - 1) / ROWS_TE), (unsigned)B);
-      scatter_rows_vec4_kernel<1, int64_t><<<grid, ROWS_THREADS, smem, st>>>(
-          (const float *)grad_out, index, nullptr, (int)C, N2, E, gstride, (float *)scratch, status);
-      int rc = check_launch("scatter_rows_vec4_kernel");
-      if (rc) return rc;
-      return transpose_bcn((const float *)scratch, (float *)grad_key, B, N2, C, st);
-    }
     TK3D_CUDA(cudaMemsetAsync(grad_key, 0, elem * (size_t)(B * C * N2), st));
     if (E > 0) {
       const int64_t blocks = (B * C * E + 255) / 256, cap = (int64_t)sm_count() * 32;

@@ -8,6 +8,7 @@
 // then walks the channels.
 #include "chanrow.cuh"
 #include "rows.cuh"
+#include "scatter.cuh"
 
 namespace tk3d {
 
@@ -263,8 +264,9 @@ extern "C" int tk3d_group_fwd_rows(const void *rows, const void *index, int inde
 
 extern "C" size_t tk3d_group_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K, int dtype) {
   if (dtype != TK3D_F32 || B <= 0 || C <= 0 || N1 <= 0 || N2 <= 0 || K <= 0 || B > 65535) return 0;
-  if (C % 4 != 0 || (N2 * K) % 4 != 0 || (N1 + 31) / 32 > 65535) return 0;
-  return rows_profitable(C, N1, N2 * K, 1) ? rows_scratch_bytes(B, C, N1) : 0;
+  return scatter_ok(B, C, N1, N2, K) && scatter_pays(B, C, N2, K) && rows_profitable(C, N1, N2 * K, 1)
+             ? scatter_scratch_bytes(B, C, N1)
+             : 0;
 }
 
 extern "C" int tk3d_group_bwd(const void *gout, const int64_t *index, int64_t B, int64_t C, int64_t N1, int64_t N2,
@@ -279,9 +281,17 @@ extern "C" int tk3d_group_bwd(const void *gout, const int64_t *index, int64_t B,
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == TK3D_F32) {
     const size_t want = tk3d_group_bwd_scratch_bytes(B, C, N1, N2, K, dtype);
-    if (want != 0 && scratch != nullptr && scratch_bytes >= want && rows_vec_ok(C, E, gout, scratch))
-      return scatter_rows<1>((const float *)gout, index, nullptr, B, C, N1, E, (float *)gin, status, (float *)scratch,
-                             st);
+    if (want != 0 && scratch != nullptr && scratch_bytes >= want && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0) {
+      ScatterCall c;
+      c.gout = (const float *)gout;
+      c.index = index;
+      c.B = B, c.C = C, c.N = N1, c.M = N2, c.K = K;
+      c.gstride = C * E;
+      c.gin = (float *)gin;
+      c.status = status;
+      c.scratch = scratch;
+      return scatter_launch(c, st);
+    }
     return group_bwd_t<float>((const float *)gout, index, B, C, N1, E, (float *)gin, status, st);
   }
   return group_bwd_t<double>((const double *)gout, index, B, C, N1, E, (double *)gin, status, st);

@@ -27,6 +27,7 @@
 // ordered clouds (spatial_ball.cu); the kernel then starts from those lists.
 #include "chanrow.cuh"
 #include "rows.cuh"
+#include "scatter.cuh"
 #include "spatial.cuh"
 #include "sweep.cuh"
 
@@ -299,6 +300,8 @@ sa_group_fwd_kernel(const float *__restrict__ points, const float *__restrict__ 
 // Backward of the three coordinate channels: one warp per (cloud, centroid), lanes over K.
 //   grad_points[b, index, d]  += g[b, C+d, m, k]
 //   grad_centroids[b, m, d]   -= sum_k g[b, C+d, m, k]
+// Neighbours that follow one another with the same index (the padding of a ball) are summed by shuffles and added once:
+// what the kernel waits for are the atomics to one point (32 x 128 centroids, K = 64, two thirds padding: 15 us without).
 __global__ void __launch_bounds__(256)
 sa_group_bwd_xyz_kernel(const float *__restrict__ gout, const int32_t *__restrict__ index32, int64_t B, int C, int N,
                         int M, int K, int pps, int pcs, int cps, int cpc, float *__restrict__ gpoints,
@@ -313,17 +316,44 @@ sa_group_bwd_xyz_kernel(const float *__restrict__ gout, const int32_t *__restric
     const float *g = gout + (b * (C + 3) + C) * E + (int64_t)m * K;
     const int32_t *ip = index32 + b * E + (int64_t)m * K;
     float sx = 0.f, sy = 0.f, sz = 0.f;
-    for (int k = lane; k < K; k += 32) {
-      const float gx = g[k], gy = g[E + k], gz = g[2 * E + k];
+    for (int k0 = 0; k0 < K; k0 += 32) {
+      const int k = k0 + lane;
+      float gx = 0.f, gy = 0.f, gz = 0.f;
+      int id = -1;
+      if (k < K) {
+        gx = g[k];
+        gy = g[E + k];
+        gz = g[2 * E + k];
+        id = ip[k];
+      }
       sx += gx;
       sy += gy;
       sz += gz;
-      const int id = ip[k];
-      if (id >= 0 && id < N && gpoints) {
-        float *p = gpoints + b * 3 * (int64_t)N + (int64_t)id * pps;
-        atomicAdd(p, gx);
-        atomicAdd(p + pcs, gy);
-        atomicAdd(p + 2 * (int64_t)pcs, gz);
+      if (gpoints) {
+        const int prev = __shfl_up_sync(0xffffffffu, id, 1);
+        const bool head = lane == 0 || prev != id;
+        if (!__all_sync(0xffffffffu, head)) {  // sums over each run, complete in its first lane
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int other = __shfl_down_sync(0xffffffffu, id, o);
+            const float x = __shfl_down_sync(0xffffffffu, gx, o), y = __shfl_down_sync(0xffffffffu, gy, o);
+            const float z = __shfl_down_sync(0xffffffffu, gz, o);
+            const unsigned heads = __ballot_sync(0xffffffffu, head);
+            // the lane o further on belongs to this run when no run starts in between
+            const unsigned between = lane + o < 32 ? (heads >> (lane + 1)) & ((1u << o) - 1) : 1u;
+            if (!between && other == id) {
+              gx += x;
+              gy += y;
+              gz += z;
+            }
+          }
+        }
+        if (head && id >= 0 && id < N) {
+          float *p = gpoints + b * 3 * (int64_t)N + (int64_t)id * pps;
+          atomicAdd(p, gx);
+          atomicAdd(p + pcs, gy);
+          atomicAdd(p + 2 * (int64_t)pcs, gz);
+        }
       }
     }
 #pragma unroll
@@ -468,6 +498,13 @@ sa_group_bwd_feat_kernel(const float *__restrict__ gout, const int32_t *__restri
 }  // namespace
 }  // namespace tk3d
 
+extern "C" size_t tk3d_sa_group_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K, int dtype) {
+  if (!tk3d_sa_group_supported(B, C, N, M, K, dtype) || C < 4 || !scatter_ok(B, C, N, M, K) ||
+      !scatter_pays(B, C, M, K))
+    return 0;
+  return scatter_scratch_bytes(B, C, N);
+}
+
 extern "C" int tk3d_sa_group_bwd(const void *gout, const int32_t *index32, int64_t B, int64_t C, int64_t N, int64_t M,
                                  int64_t K, int xyz_channel_first, int use_xyz, void *gfeature, void *gpoints,
                                  void *gcentroids, int32_t *status, void *scratch, size_t scratch_bytes, int dtype,
@@ -481,22 +518,18 @@ extern "C" int tk3d_sa_group_bwd(const void *gout, const int32_t *index32, int64
   const int64_t gstride = ctot * E;
   TK3D_REQUIRE(B * E == 0 || (gout && index32), TK3D_ERR_NULL, "sa_group_bwd: a pointer is NULL");
   if (gfeature && B * C * N > 0) {
-    const bool vec = C % 4 == 0 && K % 4 == 0 && C >= 4 && (N + 31) / 32 <= 65535 && scratch != nullptr &&
-                     scratch_bytes >= rows_scratch_bytes(B, C, N) &&
-                     ((reinterpret_cast<uintptr_t>(gout) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
-    if (vec) {
-      TK3D_CUDA(cudaMemsetAsync(scratch, 0, rows_scratch_bytes(B, C, N), st));
-      if (E > 0) {
-        const size_t smem = (size_t)C * ROWS_TE * sizeof(float);
-        if (smem > 48 * 1024)
-          TK3D_CUDA(raise_smem_limit((const void *)scatter_rows_vec4_kernel<1, int32_t>, (int)smem));
-        dim3 grid((unsigned)((E + ROWS_TE - 1) / ROWS_TE), (unsigned)B);
-        scatter_rows_vec4_kernel<1, int32_t><<<grid, ROWS_THREADS, smem, st>>>(
-            (const float *)gout, index32, nullptr, (int)C, N, E, gstride, (float *)scratch, status);
-        int rc = check_launch("scatter_rows_vec4_kernel");
-        if (rc) return rc;
-      }
-      int rc = transpose_bcn((const float *)scratch, (float *)gfeature, B, N, C, st);
+    if (E > 0 && C >= 4 && scatter_pays(B, C, M, K) && scratch != nullptr &&
+        (reinterpret_cast<uintptr_t>(scratch) & 15) == 0 && scratch_bytes >= scatter_scratch_bytes(B, C, N)) {
+      ScatterCall c;
+      c.gout = (const float *)gout;
+      c.index = index32;
+      c.index_i32 = 1;
+      c.B = B, c.C = C, c.N = N, c.M = M, c.K = K;
+      c.gstride = gstride;
+      c.gin = (float *)gfeature;
+      c.status = status;
+      c.scratch = scratch;
+      int rc = scatter_launch(c, st);
       if (rc) return rc;
     } else {
       TK3D_CUDA(cudaMemsetAsync(gfeature, 0, sizeof(float) * (size_t)(B * C * N), st));
