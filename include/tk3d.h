@@ -429,6 +429,12 @@ int tk3d_edge_feature_bwd(const void *grad_out, const int64_t *index, int64_t B,
  */
 int tk3d_feature_knn(const void *query, const void *key, int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t k,
                      int channel_first, void *distance, int64_t *index, int dtype, void *stream);
+/* The same with `scratch` of tk3d_feature_knn_scratch_bytes(...) bytes (0: not served; 16-byte aligned, contents ignored on
+ * entry): a matrix product on the tensor cores decides which pairs get the exact distance.  Results are the same. */
+size_t tk3d_feature_knn_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t k, int dtype);
+int tk3d_feature_knn_ws(const void *query, const void *key, int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t k,
+                        int channel_first, void *dist, int64_t *index, void *scratch, size_t scratch_bytes, int dtype,
+                        void *stream);
 
 /*
  * Range-checked build.  libtk3d_b200_bounds.so is this library compiled with -DTK3D_BOUNDS: every

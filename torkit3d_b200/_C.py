@@ -433,8 +433,11 @@ def feature_knn_cuda(query, key, k, channel_first=True):
     with _on(query.device):
         distance = torch.empty((B, N1, k), dtype=query.dtype, device=query.device)
         index = torch.empty((B, N1, k), dtype=torch.int64, device=query.device)
-        check(lib.tk3d_feature_knn(_ptr(query), _ptr(key), B, C, N1, N2, k, 1 if channel_first else 0,
-                                   _ptr(distance), _ptr(index), _dtype(query), _stream(query)))
+        need = _lib.scratch_bytes("tk3d_feature_knn", B, C, N1, N2, k, _lib.F32)
+        scratch = _order_scratch(need, query.device) if need else None
+        check(lib.tk3d_feature_knn_ws(_ptr(query), _ptr(key), B, C, N1, N2, k, 1 if channel_first else 0,
+                                      _ptr(distance), _ptr(index), _ptr(scratch) if scratch is not None else None,
+                                      need if scratch is not None else 0, _dtype(query), _stream(query)))
     return [distance, index]
 
 

@@ -5,9 +5,10 @@
 // Squared distance of a (query, key) pair: acc = 0; for c = 0 .. C-1: acc = fma(d_c, d_c, acc) with
 // d_c = key_c - query_c -- one rounding per channel, summed in channel order, which a CPU loop with
 // fmaf() reproduces bit for bit.  (The reference's cdist goes through a matrix product and is
-// itself only accurate to about 1e-6 of |q|^2 + |r|^2; this form is cheaper than it looks -- two
-// FP32 instructions per pair and channel -- and needs no tensor cores at DGCNN's sizes: 32 clouds
-// of 1024 points with 64 channels are 4.3 GFLOP.)
+// itself only accurate to about 1e-6 of |q|^2 + |r|^2.)
+//
+// With scratch the tensor cores find the pairs that can matter (feature_filter.cu: k <= 48, C <= 128, 256 to 65536 keys);
+// this kernel evaluates all pairs, for the calls and the groups of queries that are left.
 //
 // Every warp owns four queries; the eight warps of a block share tiles of 256 keys, staged 16 channels at
 // a time with asynchronous copies into two buffers.  Lane l holds the 4 x 8 distances of its queries to
@@ -24,6 +25,7 @@
 // operations, the rest mostly selection.
 #include <limits.h>
 
+#include "feature_filter.cuh"
 #include "tk3d_common.cuh"
 
 namespace tk3d {
@@ -103,7 +105,8 @@ enum { FK_POINTS = 0, FK_CHANNELS = 1, FK_CHANNELS16 = 2 };
 template <int KS, int LAYOUT>
 __global__ void __launch_bounds__(FK_THREADS, KS <= 2 ? 3 : 2)
 feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ key, int C, int N1, int N2, int k,
-                   float *__restrict__ dist, int64_t *__restrict__ index, int64_t blocks_total) {
+                   float *__restrict__ dist, int64_t *__restrict__ index, int64_t blocks_total,
+                   const int *__restrict__ counts) {
   extern __shared__ __align__(16) unsigned char fk_smem[];
   constexpr int QW = FK_QW, V = LAYOUT == FK_CHANNELS16 ? 4 : 1;
   constexpr bool CF = LAYOUT != FK_POINTS;
@@ -118,6 +121,8 @@ feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ ke
   for (int64_t blk = blockIdx.x; blk < blocks_total; blk += gridDim.x) {
     const int64_t b = blk / chunks;
     const int q0 = (int)(blk % chunks) * QT;
+    // with counts only the groups that have a query without a result (ff_knn)
+    if (counts && !__syncthreads_or(tid < QT && q0 + tid < N1 && counts[b * N1 + q0 + tid] < 0)) continue;
     const float *qb = query + b * (int64_t)C * N1;
     const float *kb = key + b * (int64_t)C * N2;
     // slice `s` of the tile at key j0 goes to buffer `to`
@@ -236,10 +241,10 @@ feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ ke
 
 template <int KS>
 int launch(const float *query, const float *key, int64_t B, int C, int N1, int N2, int k, bool cf, float *dist,
-           int64_t *index, cudaStream_t st) {
+           int64_t *index, const int *counts, cudaStream_t st) {
   constexpr int QT = FK_QW * FK_WARPS;
   const int64_t total = B * ((N1 + QT - 1) / QT);
-  const int64_t cap = (int64_t)sm_count() * 32;
+  const int64_t cap = (int64_t)sm_count() * (counts ? 8 : 32);
   const unsigned grid = (unsigned)(total < cap ? total : cap);
   const size_t smem = cf ? sizeof(FkSmem<KS, false>) : sizeof(FkSmem<KS, true>);
   const bool wide = N1 % 4 == 0 && N2 % 4 == 0 &&
@@ -248,7 +253,7 @@ int launch(const float *query, const float *key, int64_t B, int C, int N1, int N
               : wide ? feature_knn_kernel<KS, FK_CHANNELS16>
                      : feature_knn_kernel<KS, FK_CHANNELS>;
   TK3D_CUDA(raise_smem_limit((const void *)kern, (int)smem));
-  kern<<<grid, FK_THREADS, smem, st>>>(query, key, C, N1, N2, k, dist, index, total);
+  kern<<<grid, FK_THREADS, smem, st>>>(query, key, C, N1, N2, k, dist, index, total, counts);
   return check_launch("feature_knn_kernel");
 }
 
@@ -257,8 +262,29 @@ int launch(const float *query, const float *key, int64_t B, int C, int N1, int N
 
 using namespace tk3d;
 
+namespace tk3d {
+namespace {
+// Five launches and a scratch buffer against one launch.  On the device, all pairs / filtered, us: 4 x 512 x 512, 16 channels
+// (5e7 by the measure below) 21 / 20, 8 x 300 x 300, 100 channels (9.5e7) 39 / 30, 1 x 1024 x 1024, 64 channels (1e8) 53 / 35;
+// but a caller that launches an EdgeConv layer's forward and backward waits for its own launches up to about 3e8: 5 x 737 x
+// 737, 37 channels (1.9e8) 168 / 186 for the whole pass, 2 x 1289 x 1289, 71 (3.4e8) 170 / 179, 1 x 1780 x 1780, 94 (4e8)
+// 242 / 207.
+bool ff_pays(int64_t B, int64_t C, int64_t N1, int64_t N2) { return (double)B * N1 * N2 * (C + 32) >= 3.5e8; }
+}  // namespace
+}  // namespace tk3d
+
+extern "C" size_t tk3d_feature_knn_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t k, int dtype) {
+  return dtype == TK3D_F32 && ff_pays(B, C, N1, N2) ? ff_scratch_bytes(B, C, N1, N2, k) : 0;
+}
+
 extern "C" int tk3d_feature_knn(const void *query, const void *key, int64_t B, int64_t C, int64_t N1, int64_t N2,
                                 int64_t k, int channel_first, void *dist, int64_t *index, int dtype, void *stream) {
+  return tk3d_feature_knn_ws(query, key, B, C, N1, N2, k, channel_first, dist, index, nullptr, 0, dtype, stream);
+}
+
+extern "C" int tk3d_feature_knn_ws(const void *query, const void *key, int64_t B, int64_t C, int64_t N1, int64_t N2,
+                                   int64_t k, int channel_first, void *dist, int64_t *index, void *scratch,
+                                   size_t scratch_bytes, int dtype, void *stream) {
   TK3D_RANGE("tk3d_feature_knn");
   TK3D_REQUIRE(dtype == TK3D_F32 || dtype == TK3D_F64, TK3D_ERR_DTYPE, "feature_knn: dtype %d", dtype);
   TK3D_REQUIRE(dtype == TK3D_F32, TK3D_ERR_UNSUPPORTED, "feature_knn: float32 only");
@@ -275,9 +301,15 @@ extern "C" int tk3d_feature_knn(const void *query, const void *key, int64_t B, i
   cudaStream_t st = (cudaStream_t)stream;
   const float *q = (const float *)query, *r = (const float *)key;
   const bool cf = channel_first != 0;
-  if (k <= 32) return launch<1>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, st);
-  if (k <= 64) return launch<2>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, st);
-  return launch<4>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, st);
+  const int *counts = nullptr;
+  const size_t need = scratch ? ff_scratch_bytes(B, C, N1, N2, k) : 0;
+  if (need != 0 && scratch_bytes >= need && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0) {
+    const int rc = ff_knn(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, scratch, &counts, st);
+    if (rc) return rc;
+  }
+  if (k <= 32) return launch<1>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, counts, st);
+  if (k <= 64) return launch<2>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, counts, st);
+  return launch<4>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, counts, st);
 }
 
 TK3D_BOUNDS_TU(feature_knn)
