@@ -12,7 +12,8 @@
 //     the issue slots) and the loads' latency between them, not the reductions (the interpolation's gradient reduces 2.4
 //     times as many bytes a second); walking over tiles with two buffers did not help (72 to 82 us).
 //   scatter_edge_kernel (edge features): a tile holds whole queries, and the sums over each query's K entries of both
-//     halves of gout come from the same pass.  64 x 1024 <- 1024 x 20: 45 and 76 for the sums apart -> 107 us.
+//     halves of gout come from the same pass.  64 x 1024 <- 1024 x 20: 45 and 76 for the sums apart -> 81 us (335 MB at
+//     4.1 TB/s; half of the issue slots, latency between them).
 // Clouds a few at a time, for rows that stay in L2 (32, 16, 8 MB of rows a pass), were no faster: 103, 104, 119, 150 us.
 #include "rows.cuh"
 #include "scatter.cuh"
@@ -143,25 +144,48 @@ __global__ void __launch_bounds__(SC_NT, 12) scatter_fold_kernel(const ScatterAr
 }
 
 // With query sums.  A block has the entries of a few whole queries in a slab of channels, and those of the second half of
-// gout beside them, so that all its loads are under way at once (the second half read as the sums go: 122 us, not 107).
+// gout beside them, so that all its loads are under way at once (the second half read as the sums go: 122 us).
 constexpr int SE_NT = 256;
 
-template <bool VEC, typename IndexT>
+// SLAB: tiles of 128 entries and slabs of 32 channels, with 16-byte loads; a thread's chunk is then the same in every row,
+// and its rows are 8 apart, which flips bits 1 and 2 of (c >> 2) & 7: addresses are constants apart (108 -> 81 us).
+template <bool VEC, bool SLAB, typename IndexT>
 __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a, const IndexT *__restrict__ index) {
   extern __shared__ __align__(16) float tile[];  // [halves][slab][TE], then int id[TE]
   constexpr int NW = SE_NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ql = lane & 7, el = lane >> 3;
-  const int TE = a.TE, halves = a.include_query ? 2 : 1;
-  int *sid = reinterpret_cast<int *>(tile + halves * a.slab * TE);
+  const int TE = SLAB ? 128 : a.TE, slab = SLAB ? 32 : a.slab, halves = a.include_query ? 2 : 1;
+  int *sid = reinterpret_cast<int *>(tile + halves * slab * TE);
   const int64_t b = blockIdx.y;
   const int64_t e0 = (int64_t)blockIdx.x * a.per;
   const int n = (int)min((int64_t)a.per, a.E - e0);
-  const int c0 = blockIdx.z * a.slab, nc = min(a.slab, a.C - c0);  // channels of this block
+  const int c0 = blockIdx.z * slab, nc = min(slab, a.C - c0);  // channels of this block
   const float *gb = a.gout + b * a.gstride + (int64_t)c0 * a.E + e0;
-  for (int h = 0; h < halves; ++h) {
+  const IndexT *ip = index + b * a.E + e0;
+  const int64_t id0 = tid < n ? (int64_t)ip[tid] : -1;  // requested ahead of gout
+  if (SLAB) {
+    const int e = lane << 2;
+    const float *src = gb + (int64_t)warp * a.E + e;
+    const int at = warp * 128 + (e ^ ((warp >> 2) << 2));
+    const int64_t step = 8 * a.E, other = (int64_t)a.C * a.E;
+    float4 v[2][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (h < halves && e < n && warp + 8 * i < nc)
+          v[h][i] = __ldcs(reinterpret_cast<const float4 *>(src + h * other + i * step));
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (h < halves && e < n && warp + 8 * i < nc)
+          *reinterpret_cast<float4 *>(tile + ((at + (h * 32 + 8 * i) * 128) ^ (8 * i))) = v[h][i];
+  }
+  for (int h = 0; !SLAB && h < halves; ++h) {
     const float *src = gb + (int64_t)h * a.C * a.E;
-    float *dst = tile + h * a.slab * TE;
+    float *dst = tile + h * slab * TE;
     if (VEC) {
       const int lc = a.lg - 2;
 #pragma unroll 4
@@ -182,7 +206,7 @@ __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a
   for (int i = nc * TE + tid; i < ((nc + 3) & ~3) * TE; i += SE_NT) tile[i] = 0.f;  // the row's padding channels
   bool bad = false;
   for (int e = tid; e < n; e += SE_NT) {
-    const int64_t v = index[b * a.E + e0 + e];
+    const int64_t v = e == tid ? id0 : (int64_t)ip[e];
     const bool out = v < 0 || v >= a.N;
     bad |= out;
     sid[e] = out ? -1 : (int)v;
@@ -200,7 +224,7 @@ __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a
   // gq[b,c,m] = sum_k (g[C+c] - g[c]), or minus the sum of the only half
   const int K = a.K, nq = n / K;
   const int64_t m0 = (int64_t)blockIdx.x * (a.per / K);
-  const float *second = tile + a.slab * TE;
+  const float *second = tile + slab * TE;
   for (int u = tid; u < nc * nq; u += SE_NT) {
     const int c = u / nq, m = u - c * nq;
     float sum = 0.f;
@@ -271,7 +295,9 @@ int scatter_go(ScatterArgs a, int64_t B, const IndexT *index, cudaStream_t st) {
     const int64_t tiles = (a.E + a.per - 1) / a.per;
     TK3D_REQUIRE(tiles < (1LL << 31), TK3D_ERR_SHAPE, "scatter: too many entries");
     const dim3 grid((unsigned)tiles, (unsigned)B, (unsigned)((a.C + a.slab - 1) / a.slab));
-    auto kern = aligned && a.per % 4 == 0 ? scatter_edge_kernel<true, IndexT> : scatter_edge_kernel<false, IndexT>;
+    auto kern = !(aligned && a.per % 4 == 0) ? scatter_edge_kernel<false, false, IndexT>
+                : a.lg == 7                  ? scatter_edge_kernel<true, true, IndexT>
+                                             : scatter_edge_kernel<true, false, IndexT>;
     if (smem > 48 * 1024) TK3D_CUDA(raise_smem_limit((const void *)kern, (int)smem));
     kern<<<grid, SE_NT, smem, st>>>(a, index);
     return check_launch("scatter_edge_kernel");
