@@ -608,15 +608,17 @@ spatial_nn_kernel(const __grid_constant__ SpSearch job, double *__restrict__ sum
 int sp_build(const SpCloud &a, const SpCloud *b, int64_t B, const SpUse &use, cudaStream_t st) {
   const int64_t clouds = b ? 2 * B : B;
   const int big = b && b->N > a.N ? b->N : a.N;
-  // Blocks per cloud: as many as leave every block an SM of its own.  With two blocks per SM the barriers of the cluster
-  // take longer than the halved passes save, and small clouds do not fill many blocks.  1 / 2 / 4 / 8 blocks, us:
-  // 40 clouds of 2048 10 / 12 / 14 / 26, 16 of 4096 14 / 13 / 11 / 14, 32 of 4096 13 / 13 / 12 / 18, 16 of 8192 21 / 17 /
-  // 13 / 15, 64 of 8192 25 / 21 / 23 / 40, 8 of 16384 36 / 24 / 16 / 13, 40 of 16384 36 / 24 / 26 / 36, 128 of 16384
-  // 39 / 43 / 52 / 79, 20 of 65536 124 / 68 / 39 / 40, 16 of 131072 293 / 140 / 76 / 46.
+  // Blocks per cloud: as many as leave every block an SM of its own (eight: two thirds of the SMs, for clouds of less than
+  // 16384 points).  With two blocks per SM the barriers of the cluster take longer than the halved passes save, and small
+  // clouds do not fill many blocks.  1 / 2 / 4 / 8 blocks, us: 40 clouds of 2048 10 / 12 / 14 / 26, 16 of 4096 14 / 13 / 11 /
+  // 14, 32 of 4096 13 / 13 / 12 / 18, 8 of 6000 - / - / 12 / 11, 16 of 8192 21 / 17 / 13 / 15, 64 of 8192 25 / 21 / 23 / 40,
+  // 8 of 16384 36 / 24 / 16 / 13, 40 of 16384 36 / 24 / 26 / 36, 128 of 16384 39 / 43 / 52 / 79, 20 of 65536 124 / 68 / 39 /
+  // 40, 16 of 131072 293 / 140 / 76 / 46.
   // Clouds of the smaller side count by their share of the larger one's points (63 of 1343 and 63 of 16251: 36 / 24 by 1 / 2).
-  const int64_t weight = b ? B * ((int64_t)a.N + b->N) / big : B;
+  const int64_t weight = b ? B * ((int64_t)a.N + b->N) / big : B, sms = sm_count();
   int CL = 1;
-  while (CL < 8 && weight * CL * 2 <= sm_count() && big >= (CL == 4 ? 12288 : 4096)) CL *= 2;
+  while (CL < 4 && weight * CL * 2 <= sms && big >= 3000) CL *= 2;
+  if (CL == 4 && weight * 8 <= (big >= 16384 ? sms : sms * 2 / 3) && big >= 4096) CL = 8;
   SpPair pair;
   pair.c[0] = a;
   pair.c[1] = b ? *b : a;
