@@ -15,7 +15,8 @@
 // each rounded or truncated at 2^-23 of the sum of magnitudes, in 3 C / 16 steps: C * 2^-21 of |a||b| with room; norms and
 // the exact distance are rounded C + 2 times at 2^-24 of at most X^2.  2 |a||b| <= X^2 / 2, so that
 // e = (C * 2^-21 + 2^-16) X^2 (+ 2^-110 for what underflows) covers all of them about twice.  A key with d <= the k-th d has
-// v <= (k-th smallest class minimum) + 2 e.
+// v <= (k-th smallest class minimum) + 2 e.  Against 64 bits the errors were at most 0.5 e for 3 channels (the halves), 0.07 e
+// for 64 and 0.05 e for 128 (normal, rectified, far from the origin, channels of different size, an outlier, huge).
 //
 // 32 x 1024 x 1024, 64 channels, k = 20: 229 us by all pairs, 89 now: preparing 7, filter 37, exact distances 41, looking
 // for what is left 4; 32 x 2000, 16 channels 388 / 138; 4 x 4096, 64 channels 458 / 117; 32 x 1024, 128 channels, k = 32
