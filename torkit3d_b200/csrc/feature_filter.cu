@@ -180,6 +180,7 @@ __device__ __forceinline__ void ff_mma(unsigned d, u64 a, u64 b, unsigned accumu
 __device__ __forceinline__ void ff_commit(unsigned bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// Instructions marked aligned want the whole warp; lanes that took a branch or polled a barrier meet at __syncwarp().
 // Requests 32 columns of the warp's lanes; ff_loaded() before they are used.
 __device__ __forceinline__ void ff_load32(unsigned taddr, unsigned (&r)[32]) {
   __syncwarp();
@@ -194,6 +195,7 @@ __device__ __forceinline__ void ff_load32(unsigned taddr, unsigned (&r)[32]) {
 }
 // The registers go through the wait, so that no use of them is moved ahead of it.
 __device__ __forceinline__ void ff_loaded(unsigned (&r)[32]) {
+  __syncwarp();
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));
@@ -239,6 +241,7 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ff_smem(&tmem_at)), "r"(2 * FF_T)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -409,8 +412,10 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
     }
     __syncthreads();
   }
-  if (warp == 0)
+  if (warp == 0) {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * FF_T) : "memory");
+  }
 }
 
 __device__ __forceinline__ u64 ff_exchange(u64 v, int o, bool low) {
