@@ -104,3 +104,19 @@ def test_edge(B, C, N, M, K, kind, include_query):
         _close(gk, ref, mag, count)
         if need_query:
             _close(gq, q, g.double().abs().sum(3).reshape(B, -1, C, M).sum(1), 2 * K)
+
+
+@pytest.mark.parametrize("N", [65535 * 32 + 1, 65535 * 64 + 4])
+def test_clouds_of_more_points_than_a_grid_has_rows(N):
+    """The rows are written back point by point: no size of a grid may limit the points."""
+    from torkit3d_b200 import _C, _fused
+
+    M, K = -(-N // 64), 16
+    index = _index("uniform", 1, M, K, N)
+    index[0, 0] = N - 1
+    g = torch.randn(1, 16, M, K, device=DEV)
+    _close(_C.group_points_backward_cuda(g, index, N), *_scatter(g, index, N))
+    index, g = index[:, :64].contiguous(), torch.randn(1, 8, 64, K, device=DEV)
+    ref = _scatter(g[:, :4], index, N)
+    _close(_fused.edge_feature_backward(g, index, 4, N)[1], *ref)
+    _close(_fused.sa_group_backward(g[:, :7].contiguous(), index.int(), 4, N)[0], *ref)

@@ -211,7 +211,7 @@ extern "C" int tk3d_edge_feature_fwd(const void *query_feature, const void *key_
 }
 
 static bool edge_bwd_rows_ok(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K) {
-  return C >= 4 && C <= ROWS_MAX_C && scatter_ok(B, C, N2, N1, K) && scatter_pays(B, C, N1, K);
+  return C >= 4 && C <= ROWS_MAX_C && scatter_ok(B, C, N2, N1, K) && scatter_pays(B, C, N2, N1, K);
 }
 
 extern "C" size_t tk3d_edge_feature_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K,

@@ -264,7 +264,7 @@ extern "C" int tk3d_group_fwd_rows(const void *rows, const void *index, int inde
 
 extern "C" size_t tk3d_group_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K, int dtype) {
   if (dtype != TK3D_F32 || B <= 0 || C <= 0 || N1 <= 0 || N2 <= 0 || K <= 0 || B > 65535) return 0;
-  return scatter_ok(B, C, N1, N2, K) && scatter_pays(B, C, N2, K) && rows_profitable(C, N1, N2 * K, 1)
+  return scatter_ok(B, C, N1, N2, K) && scatter_pays(B, C, N1, N2, K) && rows_profitable(C, N1, N2 * K, 1)
              ? scatter_scratch_bytes(B, C, N1)
              : 0;
 }

@@ -500,7 +500,7 @@ sa_group_bwd_feat_kernel(const float *__restrict__ gout, const int32_t *__restri
 
 extern "C" size_t tk3d_sa_group_bwd_scratch_bytes(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K, int dtype) {
   if (!tk3d_sa_group_supported(B, C, N, M, K, dtype) || C < 4 || !scatter_ok(B, C, N, M, K) ||
-      !scatter_pays(B, C, M, K))
+      !scatter_pays(B, C, N, M, K))
     return 0;
   return scatter_scratch_bytes(B, C, N);
 }
@@ -518,8 +518,8 @@ extern "C" int tk3d_sa_group_bwd(const void *gout, const int32_t *index32, int64
   const int64_t gstride = ctot * E;
   TK3D_REQUIRE(B * E == 0 || (gout && index32), TK3D_ERR_NULL, "sa_group_bwd: a pointer is NULL");
   if (gfeature && B * C * N > 0) {
-    if (E > 0 && C >= 4 && scatter_pays(B, C, M, K) && scratch != nullptr &&
-        (reinterpret_cast<uintptr_t>(scratch) & 15) == 0 && scratch_bytes >= scatter_scratch_bytes(B, C, N)) {
+    const size_t rows = tk3d_sa_group_bwd_scratch_bytes(B, C, N, M, K, dtype);
+    if (rows != 0 && scratch != nullptr && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0 && scratch_bytes >= rows) {
       ScatterCall c;
       c.gout = (const float *)gout;
       c.index = index32;

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a
   }
 }
 
-// rows [B][N][ld] -> gin [B][C][N] where C is no multiple of 4; a block moves 64 points x 64 channels.
+// rows [B][N][ld] -> gin [B][C][N] for any C and N; a block moves 64 points x 64 channels.
 __global__ void __launch_bounds__(256)
 unrow_kernel(const float *__restrict__ rows, int ld, int C, int N, float *__restrict__ gin) {
   __shared__ __align__(16) float t[64 * 64];  // [channel][point], chunks of four points swizzled
@@ -345,7 +345,7 @@ int scatter_launch(const ScatterCall &c, cudaStream_t st) {
   const int rc = c.index_i32 ? scatter_go<int32_t>(a, c.B, (const int32_t *)c.index, st)
                              : scatter_go<int64_t>(a, c.B, (const int64_t *)c.index, st);
   if (rc) return rc;
-  if (c.C % 4 == 0) return transpose_bcn(a.rows, c.gin, c.B, c.N, c.C, st);
+  if (c.C % 4 == 0 && c.N <= SCATTER_TRANSPOSED) return transpose_bcn(a.rows, c.gin, c.B, c.N, c.C, st);
   const dim3 grid((unsigned)((c.N + 63) / 64), (unsigned)((c.C + 63) / 64), (unsigned)c.B);
   unrow_kernel<<<grid, 256, 0, st>>>(a.rows, a.ld, a.C, a.N, c.gin);
   return check_launch("unrow_kernel");

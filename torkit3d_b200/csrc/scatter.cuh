@@ -22,7 +22,12 @@ inline size_t scatter_scratch_bytes(int64_t B, int64_t C, int64_t N) {
 }
 // Sizes that 16-byte accesses do not fit take the direct kernels while they are small: three launches and a scratch buffer
 // cost the caller 7 us more than two (10 x 111 channels, 231 x 36 entries 128 -> 135; 7 x 24, 3557 x 22 192 -> 163).
-inline bool scatter_pays(int64_t B, int64_t C, int64_t M, int64_t K) {
+// Clouds of more points than the transposition takes have their rows written back by unrow_kernel, for few channels a
+// small part of a tile: 4 x 2097121 <- 64 x 16 entries 22 us direct and 60 by rows, 4 x 2097121 <- 524288 37 / 77, 64 x
+// 4200000 <- 32768 263 / 492, but 16 x 2097121 <- 524288 191 / 117, 32 x 3000001 <- 1600000 1853 / 325.
+constexpr int64_t SCATTER_TRANSPOSED = 65535 * 32;  // points: they are a grid's y there
+inline bool scatter_pays(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K) {
+  if (N > SCATTER_TRANSPOSED && (C < 16 || 4 * M * K < N)) return false;
   return (C % 4 == 0 && (M * K) % 4 == 0) || B * C * M * K >= 12000000;
 }
 // Whether the sizes are served; whether gq can be summed in the same pass.
