@@ -120,3 +120,29 @@ def test_clouds_of_more_points_than_a_grid_has_rows(N):
     ref = _scatter(g[:, :4], index, N)
     _close(_fused.edge_feature_backward(g, index, 4, N)[1], *ref)
     _close(_fused.sa_group_backward(g[:, :7].contiguous(), index.int(), 4, N)[0], *ref)
+
+
+@pytest.mark.parametrize("B,C,N,M,K", [(2, 37, 900, 4100, 41), (2, 64, 1024, 256, 16)])
+def test_no_memory_for_the_rows(B, C, N, M, K, monkeypatch):
+    """The rows are an option: where they cannot be allocated the direct kernels run."""
+    from torkit3d_b200 import _C, _fused
+
+    index = _index("padded", B, M, K, N)
+    g = torch.randn(B, 2 * C, M, K, device=DEV)
+    half, sa = g[:, :C].contiguous(), g[:, :C + 3].contiguous()
+    ref = _scatter(half, index, N)
+    empty, refused = torch.empty, []
+
+    def none_for_scratch(*args, **kwargs):
+        if kwargs.get("dtype") is torch.uint8:
+            refused.append(args)
+            raise torch.cuda.OutOfMemoryError("no memory")
+        return empty(*args, **kwargs)
+
+    monkeypatch.setattr(torch, "empty", none_for_scratch)
+    got = (_C.group_points_backward_cuda(half, index, N), _fused.edge_feature_backward(g, index, C, N)[1],
+           _fused.sa_group_backward(sa, index.int(), C, N)[0])
+    monkeypatch.undo()
+    assert len(refused) == 3
+    for x in got:
+        _close(x, *ref)

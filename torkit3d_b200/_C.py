@@ -125,9 +125,10 @@ def _ptr(t):
 
 
 def _order_scratch(need, device, least=0):
-    """Scratch of ``need`` bytes for a search over spatially ordered clouds (about 21 bytes a point and 16 KB a cloud,
-    512 MB at most: larger batches are cut).  Where that much is not free, ``least`` bytes (0: None), with which the
-    library sweeps all pairs."""
+    """Scratch of ``need`` bytes for a faster path that the call can do without: a search over spatially ordered clouds
+    (about 21 bytes a point and 16 KB a cloud, 512 MB at most: larger batches are cut), the tensor cores' filter of
+    feature-space neighbours (512 MB at most), the rows of a gradient (as much as the gradient).  Where that much is not
+    free, ``least`` bytes (0: None), with which the library takes its path without."""
     try:
         return torch.empty((need,), dtype=torch.uint8, device=device)
     except torch.cuda.OutOfMemoryError:
@@ -247,9 +248,10 @@ def group_points_backward_cuda(grad_output, index, n1):
     with _on(grad_output.device):
         gin = torch.empty((B, C, n1), dtype=grad_output.dtype, device=grad_output.device)
         need = _lib.scratch_bytes("tk3d_group_bwd", B, C, n1, N2, K, _dtype(grad_output))
-        scratch = torch.empty((need,), dtype=torch.uint8, device=grad_output.device) if need else None
+        scratch = _order_scratch(need, grad_output.device) if need else None
         check(lib.tk3d_group_bwd(_ptr(grad_output), _ptr(index), B, C, n1, N2, K, _ptr(gin), None,
-                                 _ptr(scratch) if need else None, need, _dtype(grad_output), _stream(grad_output)))
+                                 _ptr(scratch) if scratch is not None else None, need if scratch is not None else 0,
+                                 _dtype(grad_output), _stream(grad_output)))
     return gin
 
 

@@ -107,7 +107,8 @@ def sa_group_backward(grad_out, index32, C, N, use_xyz=True, channel_first=True,
         gcen = torch.empty((B, 3, M) if channel_first else (B, M, 3), dtype=torch.float32, device=dev) \
             if (xyz and need_centroids) else None
         need = _lib.scratch_bytes("tk3d_sa_group_bwd", B, C, N, M, K, _lib.F32) if gfeat is not None else 0
-        scratch = _scratch(need, dev)
+        scratch = _order_scratch(need, dev) if need else None
+        need = need if scratch is not None else 0
         check(lib.tk3d_sa_group_bwd(_ptr(grad_out), _ptr(index32), B, C, N, M, K, 1 if channel_first else 0,
                                     1 if use_xyz else 0, _ptr(gfeat) if gfeat is not None else None,
                                     _ptr(gpts) if gpts is not None else None,
@@ -208,7 +209,8 @@ def edge_feature_backward(grad_out, index, C, N2, include_query=True, need_query
         gq = torch.empty((B, C, N1), dtype=grad_out.dtype, device=dev) if need_query else None
         gk = torch.empty((B, C, N2), dtype=grad_out.dtype, device=dev) if need_key else None
         need = _lib.scratch_bytes("tk3d_edge_feature_bwd", B, C, N1, N2, K, dt) if need_key else 0
-        scratch = _scratch(need, dev)
+        scratch = _order_scratch(need, dev) if need else None
+        need = need if scratch is not None else 0
         check(lib.tk3d_edge_feature_bwd(_ptr(grad_out), _ptr(index), B, C, N1, N2, K, 1 if include_query else 0,
                                         _ptr(gq) if need_query else None, _ptr(gk) if need_key else None, None,
                                         _ptr(scratch) if need else None, need, dt, _stream(grad_out)))
