@@ -102,7 +102,9 @@ __device__ __noinline__ u64 fk_flush(u64 *buf, u64 *list, int n, int k, int lane
 // copied by four bytes, or by sixteen (N1 and N2 multiples of four, 16-byte aligned tensors).
 enum { FK_POINTS = 0, FK_CHANNELS = 1, FK_CHANNELS16 = 2 };
 
-template <int KS, int LAYOUT>
+// LEFT: only the groups that have a query without a result (a negative count, see ff_knn), a block for each.  A template
+// argument: as a test of `counts` in every call's loop the kernel took 119 us instead of 114 (2 x 1289 x 1289, 71 channels).
+template <int KS, int LAYOUT, bool LEFT>
 __global__ void __launch_bounds__(FK_THREADS, KS <= 2 ? 3 : 2)
 feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ key, int C, int N1, int N2, int k,
                    float *__restrict__ dist, int64_t *__restrict__ index, int64_t blocks_total,
@@ -121,8 +123,7 @@ feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ ke
   for (int64_t blk = blockIdx.x; blk < blocks_total; blk += gridDim.x) {
     const int64_t b = blk / chunks;
     const int q0 = (int)(blk % chunks) * QT;
-    // with counts only the groups that have a query without a result (ff_knn)
-    if (counts && !__syncthreads_or(tid < QT && q0 + tid < N1 && counts[b * N1 + q0 + tid] < 0)) continue;
+    if (LEFT && !__syncthreads_or(tid < QT && q0 + tid < N1 && counts[b * N1 + q0 + tid] < 0)) return;
     const float *qb = query + b * (int64_t)C * N1;
     const float *kb = key + b * (int64_t)C * N2;
     // slice `s` of the tile at key j0 goes to buffer `to`
@@ -235,23 +236,24 @@ feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ ke
         }
       }
     }
+    if (LEFT) return;
     __syncthreads();  // the next task's first slice may land in a buffer that a slower warp still reads
   }
 }
 
-template <int KS>
+template <int KS, bool LEFT>
 int launch(const float *query, const float *key, int64_t B, int C, int N1, int N2, int k, bool cf, float *dist,
            int64_t *index, const int *counts, cudaStream_t st) {
   constexpr int QT = FK_QW * FK_WARPS;
   const int64_t total = B * ((N1 + QT - 1) / QT);
-  const int64_t cap = (int64_t)sm_count() * (counts ? 8 : 32);
-  const unsigned grid = (unsigned)(total < cap ? total : cap);
+  const int64_t cap = (int64_t)sm_count() * 32;
+  const unsigned grid = (unsigned)(LEFT || total < cap ? total : cap);
   const size_t smem = cf ? sizeof(FkSmem<KS, false>) : sizeof(FkSmem<KS, true>);
   const bool wide = N1 % 4 == 0 && N2 % 4 == 0 &&
                     ((reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(key)) & 15) == 0;
-  auto kern = !cf    ? feature_knn_kernel<KS, FK_POINTS>
-              : wide ? feature_knn_kernel<KS, FK_CHANNELS16>
-                     : feature_knn_kernel<KS, FK_CHANNELS>;
+  auto kern = !cf    ? feature_knn_kernel<KS, FK_POINTS, LEFT>
+              : wide ? feature_knn_kernel<KS, FK_CHANNELS16, LEFT>
+                     : feature_knn_kernel<KS, FK_CHANNELS, LEFT>;
   TK3D_CUDA(raise_smem_limit((const void *)kern, (int)smem));
   kern<<<grid, FK_THREADS, smem, st>>>(query, key, C, N1, N2, k, dist, index, total, counts);
   return check_launch("feature_knn_kernel");
@@ -307,9 +309,14 @@ extern "C" int tk3d_feature_knn_ws(const void *query, const void *key, int64_t B
     const int rc = ff_knn(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, scratch, &counts, st);
     if (rc) return rc;
   }
-  if (k <= 32) return launch<1>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, counts, st);
-  if (k <= 64) return launch<2>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, counts, st);
-  return launch<4>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, (float *)dist, index, counts, st);
+  float *d = (float *)dist;
+  if (counts) {  // k <= 48
+    if (k <= 32) return launch<1, true>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, d, index, counts, st);
+    return launch<2, true>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, d, index, counts, st);
+  }
+  if (k <= 32) return launch<1, false>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, d, index, nullptr, st);
+  if (k <= 64) return launch<2, false>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, d, index, nullptr, st);
+  return launch<4, false>(q, r, B, (int)C, (int)N1, (int)N2, (int)k, cf, d, index, nullptr, st);
 }
 
 TK3D_BOUNDS_TU(feature_knn)
