@@ -1,28 +1,40 @@
 // k nearest neighbours in a C-dimensional feature space by tensor cores: which keys can be among a query's k nearest is
 // decided from a matrix product, and only those pairs (25 for k = 20) get the exact distance of feature_knn.cu.
 //
-// 1. ff_prep_kernel: every feature, less the mean of four keys (what is common to all would only cost digits), as a sum of two bf16 (its upper and lower half, 2^-18 of it is lost), in the order that
-//    tcgen05.mma reads (tiles of 128 points: half, eight channels, point), squared norms, and rows of float32.
+// 1. ff_prep_kernel: every feature, less a common centre (what all have in common would only cost digits: the middle two of
+//    four keys, channel by channel), as a sum of two bf16 (its upper and lower half, 2^-18 of it is lost), in the order that
+//    tcgen05.mma reads (tiles of 128 points: half, eight channels, point), two bounds of the squared norm, and rows of float32.
 // 2. ff_filter_kernel: a block holds 128 queries, the lanes of tensor memory.  Tiles of 128 keys arrive by bulk
 //    copies; a . b = ah . bh + ah . bl + al . bh is accumulated in tensor memory, two tiles in flight, while the threads
 //    read the tile before: v = |key|^2 - 2 query . key, the distance less the query's own norm.
-//    First over all keys: the minima over 64 classes of keys; their k-th smallest (a sorting network in registers) plus
-//    twice the error bounds the k-th neighbour's v.  Then over all keys again: those below go to the query's list.
+//    First over all keys: the minima of v's upper bound over 64 classes of keys; their k-th smallest (a sorting network in
+//    registers) plus the query's part of the error bounds the k-th neighbour's v.  Then over all keys again: those whose lower
+//    bound is below go to the query's list.
 // 3. ff_exact_kernel: a warp per query, lane = candidate; exact distances, the nearest kept sorted by (distance, index).
-// 4. feature_knn_kernel redoes the groups of queries that have one whose list overflowed or whose numbers are not finite.
+// 4. feature_knn_kernel redoes the groups of 32 queries that have one without a list.
 //
-// Error of v: let X = |query| + max |key|, both less the mean; the differences are rounded once (2^-24).  The halves leave out 3 * 2^-18 of |a||b|; a step of the product adds 17 numbers,
-// each rounded or truncated at 2^-23 of the sum of magnitudes, in 3 C / 16 steps: C * 2^-21 of |a||b| with room; norms and
-// the exact distance are rounded C + 2 times at 2^-24 of at most X^2.  2 |a||b| <= X^2 / 2, so that
-// e = (C * 2^-21 + 2^-16) X^2 (+ 2^-110 for what underflows) covers all of them about twice.  A key with d <= the k-th d has
-// v <= (k-th smallest class minimum) + 2 e.  Against 64 bits the errors were at most 0.5 e for 3 channels (the halves), 0.07 e
-// for 64 and 0.05 e for 128 (normal, rectified, far from the origin, channels of different size, an outlier, huge).
+// Error of v: let X = |query| + |key|, both less the centre; the differences are rounded once (2^-24).  The halves leave out
+// 3 * 2^-18 of |a||b|; a step of the product adds 17 numbers, taken to be rounded or truncated at 2^-23 of the sum of
+// magnitudes each, in 3 C / 16 steps: C * 2^-21 of |a||b| with room; norms and the exact distance are rounded C + 2 times at
+// 2^-24 of at most X^2.  2 |a||b| <= X^2 / 2, so that e = c X^2, c = C * 2^-21 + 2^-16 (+ 2^-110 for what underflows) covers
+// all of them about twice.  How the tensor cores round inside a step is written nowhere: what stands behind that part are the
+// errors measured against 64 bits, at most 0.5 e for 3 channels (the halves), 0.07 e for 64 and 0.05 e for 128 (normal,
+// rectified, far from the origin, channels of different size, an outlier, huge).
+// X^2 <= 2 |query|^2 + 2 |key|^2, so that a key's part, 2 c |key|^2, is put into its norm's two bounds: a key far from the
+// others widens the bounds of no other (with the largest norm in its place, one key at 100 times the others' distance left
+// nothing to filter).  A key with d <= the k-th d has its lower v <= (k-th smallest class minimum) + 4 c |query|^2.
+//
+// What the filter cannot tell apart it leaves to the kernel for all pairs, and is quick to find out: keys whose norms are not
+// finite or vanish (no product is made), queries with a key in reach in 57 or more classes (some 140 keys, more than the
+// lists take; with 53 a lattice of ties took 139 instead of 87 us), groups with such a query.  All pairs / the filter in vain,
+// us, 32 x 1024 x 1024, 64 channels, k = 20: equal points 185 / 202, not a number 230 / 246, eight tight clusters 230 / 262;
+// 16 x 2000 x 2000, 16 channels, k = 16, clusters about as large as the lists 257 / 319.
 //
 // 32 x 1024 x 1024, 64 channels, k = 20: 229 us by all pairs, 89 now: preparing 7, filter 37, exact distances 41, looking
-// for what is left 4; 32 x 2000, 16 channels 388 / 138; 4 x 4096, 64 channels 458 / 117; 32 x 1024, 128 channels, k = 32
+// for what is left 3; 32 x 2000, 16 channels 388 / 138; 4 x 4096, 64 channels 458 / 117; 32 x 1024, 128 channels, k = 32
 // 384 / 220.  The filter's product is 16 % of it; the rest is reading tensor memory (two loads of 32 columns a thread and
 // tile), the minima and the comparisons.  With one thread per query it took 61 to 77 us.  The exact distances wait for
-// shared memory.  Where all distances are equal nothing can be left out: 184 -> 232.
+// shared memory.
 #include "feature_filter.cuh"
 
 namespace tk3d {
@@ -33,20 +45,25 @@ constexpr int FF_CLASSES = 64;
 constexpr int FF_CAP = 64;       // candidates per query
 constexpr int FF_MAX_C = 128;
 constexpr int FF_MAX_K = 48;     // the 48th of 64 class minima lies near the 89th key
+constexpr int FF_CROWD = 57;     // classes with a key in reach of a query that is given up
+constexpr float FF_HUGE = 1e37f; // squared norms: no distance below overflows
 constexpr int FF_PREP = 32;      // points of a preparing block
 constexpr unsigned FULL = 0xffffffffu;
 using u64 = unsigned long long;
 
 // One side (queries or keys) in scratch.
 struct FfSide {
-  unsigned char *tiles;  // [B][tiles][tile_bytes]: halves [2][Cp / 8][128][8] bf16, squared norms [128]
+  unsigned char *tiles;  // [B][tiles][tile_bytes]: halves [2][Cp / 8][128][8] bf16, norms' upper and lower bounds [2][128]
   float *rows;           // [B][N][Cr]
   float *block_max;      // [B][ceil(N / 32)] largest squared norm
 };
 
 __host__ __device__ inline int ff_cp(int C) { return (C + 15) / 16 * 16; }
 __host__ __device__ inline int ff_cr(int C) { return (C + 3) / 4 * 4; }
-__host__ __device__ inline int ff_tile_bytes(int C) { return 2 * ff_cp(C) * FF_T * 2 + FF_T * 4; }
+__host__ __device__ inline int ff_tile_bytes(int C) { return 2 * ff_cp(C) * FF_T * 2 + 2 * FF_T * 4; }
+__host__ __device__ inline int ff_upper(int C) { return ff_tile_bytes(C) - 2 * FF_T * 4; }  // where the bounds lie
+__host__ __device__ inline int ff_lower(int C) { return ff_tile_bytes(C) - FF_T * 4; }
+__device__ __forceinline__ float ff_error(int C) { return (float)C * 4.76837158e-7f + 1.52587891e-5f; }  // c
 __host__ __device__ inline int ff_tiles(int N) { return (N + FF_T - 1) / FF_T; }
 
 // Where a point lies in its tile: tiles are turned against each other, so that points whose indices differ by a multiple of
@@ -62,7 +79,8 @@ __device__ __forceinline__ unsigned ff_bf16(float x) {  // nearest bf16, as the 
 
 // Warp w of a block takes the channel groups w, w + 8, ...; lane = point.
 template <bool CF>
-__global__ void __launch_bounds__(256) ff_prep_kernel(const float *__restrict__ in, const float *__restrict__ key, int C, int N, int N2, FfSide s) {
+__global__ void __launch_bounds__(256)
+ff_prep_kernel(const float *__restrict__ in, const float *__restrict__ key, int C, int N, int N2, FfSide s) {
   __shared__ float part[8][FF_PREP];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t b = blockIdx.y;
@@ -78,9 +96,8 @@ __global__ void __launch_bounds__(256) ff_prep_kernel(const float *__restrict__ 
       const int64_t j = (int64_t)(2 * (lane >> 3) + 1) * N2 / 8;
       mid = 0.f;
       if (c < C) mid = CF ? key[(b * C + c) * (int64_t)N2 + j] : key[(b * N2 + j) * (int64_t)C + c];
-      mid += __shfl_xor_sync(FULL, mid, 8);
-      mid += __shfl_xor_sync(FULL, mid, 16);
-      mid *= 0.25f;
+      const float other = __shfl_xor_sync(FULL, mid, 8), lo = fminf(mid, other), hi = fmaxf(mid, other);
+      mid = 0.5f * (fmaxf(lo, __shfl_xor_sync(FULL, lo, 16)) + fminf(hi, __shfl_xor_sync(FULL, hi, 16)));
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -118,8 +135,9 @@ __global__ void __launch_bounds__(256) ff_prep_kernel(const float *__restrict__ 
     sum = 0.f;
 #pragma unroll
     for (int w = 0; w < 8; ++w) sum += part[w][lane];
-    // no padding point is ever near
-    reinterpret_cast<float *>(tile + bytes - FF_T * 4)[ff_place(n)] = there ? sum : __int_as_float(0x7f800000);
+    const float inf = __int_as_float(0x7f800000), e = 2.f * ff_error(C);  // no padding point is ever near
+    reinterpret_cast<float *>(tile + ff_upper(C))[ff_place(n)] = there ? fmaf(sum, e, sum) : inf;
+    reinterpret_cast<float *>(tile + ff_lower(C))[ff_place(n)] = there ? fmaf(sum, -e, sum) : inf;
     unsigned top = there ? __float_as_uint(sum) & 0x7fffffffu : 0u;  // NaN above infinity above every number
     top = __reduce_max_sync(FULL, top);
     if (lane == 0 && blockIdx.x * FF_PREP < N)
@@ -230,6 +248,7 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
   extern __shared__ __align__(1024) unsigned char ff_raw[];  // queries, two tiles of keys, [16][128] minima
   __shared__ __align__(8) unsigned long long bars[5];  // keys arrived [2], product done [2], queries arrived
   __shared__ unsigned tmem_at;
+  __shared__ int lost[FF_T / FF_GROUP];  // groups of queries that are redone anyway
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = tid >> 7, row = tid & (FF_T - 1);
   const int64_t b = blockIdx.y;
   const int bytes = ff_tile_bytes(C), lower = ff_cp(C) * FF_T * 2, tiles = ff_tiles(N2), steps = 2 * tiles;
@@ -240,6 +259,7 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
     for (int i = 0; i < 5; ++i) ff_bar_init(ff_smem(bars + i));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (tid < FF_T / FF_GROUP) lost[tid] = 0;
   if (warp == 0) {
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ff_smem(&tmem_at)), "r"(2 * FF_T)
@@ -285,10 +305,26 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
     for (int i = lane; i < nb; i += 32) top = max(top, __float_as_uint(ks.block_max[b * nb + i]));
     r2 = __uint_as_float(__reduce_max_sync(FULL, top));
   }
+  auto leave = [&]() {
+    if (warp == 0) {
+      __syncwarp();
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * FF_T) : "memory");
+    }
+  };
   ok = ff_wait(bar_q, 0);
-  if (tid == 0) ok = ok && product(0);
   const int q = ff_point(blockIdx.x, row);
-  const float qn = *reinterpret_cast<const float *>(ff_raw + bytes - FF_T * 4 + 4 * row);
+  if (!(r2 < FF_HUGE) || r2 < 1e-30f) {  // numbers that overflow or are none, or nothing to tell apart
+    if (q < N1) found[(b * N1 + q) * 2 + half] = FF_BAD;
+    if (tid == 0) {
+      ff_wait(bar_k, 0);
+      ff_wait(bar_k + 8, 0);
+    }
+    __syncthreads();
+    leave();
+    return;
+  }
+  if (tid == 0) ok = ok && product(0);
+  const float qn = *reinterpret_cast<const float *>(ff_raw + ff_upper(C) + 4 * row);
   float m[FF_CLASSES];  // this thread's 32, and later the other's
 #pragma unroll
   for (int i = 0; i < FF_CLASSES; ++i) m[i] = __int_as_float(0x7f800000);
@@ -305,7 +341,7 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
     ok = ok && ff_wait(bar_k + 8 * (s & 1), (s >> 1) & 1) && ff_wait(bar_d + 8 * (s & 1), (s >> 1) & 1);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned ta = tmem + (s & 1) * FF_T + half * 64 + ((unsigned)((warp & 3) * 32) << 16);
-    norm = reinterpret_cast<const float4 *>(ff_raw + bytes + (s & 1) * bytes + bytes - FF_T * 4) + half * 16;
+    norm = reinterpret_cast<const float4 *>(ff_raw + bytes + (s & 1) * bytes + (s < tiles ? ff_upper(C) : ff_lower(C))) + half * 16;
     ff_load32(ta, r0);
     ff_load32(ta + 32, r1);
     if (tid == 0 && s + 1 < steps) ok = ok && product(s + 1);
@@ -355,20 +391,19 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
     }
     if (half == 0) {
       ff_sort<1>(m);
-      const float size = sqrtf(qn) + sqrtf(r2);
-      const float e = ((float)C * 4.76837158e-7f + 1.52587891e-5f) * size * size + 7.7e-34f;
+      const float e = fmaf(4.f * ff_error(C), qn, 1.6e-33f);
 #pragma unroll
       for (int i = 0; i < FF_CLASSES; ++i)
-        if (i == k - 1) limit = m[i] + 2.f * e;
-      // every class has a key below it: more than the exact kernel takes (many equal distances, say)
-      if (m[FF_CLASSES - 1] <= limit) limit = __int_as_float(0x7f800000);
+        if (i == k - 1) limit = m[i] + e;
+      if (m[FF_CROWD - 1] <= limit || !(qn < FF_HUGE)) limit = __int_as_float(0x7f800000);
       *x = limit;
+      if (!(fabsf(limit) < 3e38f) && q < N1) lost[(q % FF_T) / FF_GROUP] = 1;
     }
     __syncthreads();
     limit = *x;
   }
   // Neither infinite nor not a number, and a query at all; else nothing is below the limit.
-  const bool live = fabsf(limit) < 3e38f && q < N1;
+  const bool live = fabsf(limit) < 3e38f && q < N1 && !lost[(q % FF_T) / FF_GROUP];
   const float2 over = live ? make_float2(-limit, -limit) : make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
   if (going && !__syncthreads_or(live)) {  // nothing to look for: the tiles and the product under way, and that is all
     ok = ff_wait(bar_k + 8 * (s & 1), (s >> 1) & 1) && ff_wait(bar_d + 8 * (s & 1), (s >> 1) & 1) &&
@@ -412,10 +447,7 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
     }
     __syncthreads();
   }
-  if (warp == 0) {
-    __syncwarp();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * FF_T) : "memory");
-  }
+  leave();
 }
 
 __device__ __forceinline__ u64 ff_exchange(u64 v, int o, bool low) {
@@ -453,9 +485,14 @@ ff_exact_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, const uint16
   const int q = blockIdx.x * (FF_EXACT / 32) + warp, b = blockIdx.y;
   if (q >= N1) return;
   const int64_t query = (int64_t)b * N1 + q;
-  const int2 parts = *reinterpret_cast<const int2 *>(found + 2 * query);
-  const int n = parts.x + parts.y;
-  const bool bad = n > 2 * FF_CAP || n < k;
+  // the lists of the whole group: one without sends all of it to the other kernel
+  int2 parts = make_int2(k, 0);
+  if ((q & ~(FF_GROUP - 1)) + lane < N1)
+    parts = *reinterpret_cast<const int2 *>(found + 2 * ((int64_t)b * N1 + (q & ~(FF_GROUP - 1)) + lane));
+  int n = parts.x + parts.y;
+  const bool bad = __any_sync(FULL, n > 2 * FF_CAP || n < k);
+  parts.x = __shfl_sync(FULL, parts.x, q & (FF_GROUP - 1));
+  n = __shfl_sync(FULL, n, q & (FF_GROUP - 1));
   if (lane == 0) counts[query] = bad ? -1 : n;
   if (bad) return;
   const int Cr = ff_cr(C), L = Cr / 4, stride = 16 * (L | 1);

@@ -115,6 +115,7 @@ feature_knn_kernel(const float *__restrict__ query, const float *__restrict__ ke
   using Smem = FkSmem<KS, LAYOUT == FK_POINTS>;
   Smem &sm = *reinterpret_cast<Smem *>(fk_smem);
   constexpr int QT = QW * FK_WARPS;
+  static_assert(!LEFT || QT == FF_GROUP, "the filter gives up groups of this size");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chunks = (N1 + QT - 1) / QT;
   const int slices = (C + FK_CS - 1) / FK_CS;
