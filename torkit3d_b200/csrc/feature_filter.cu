@@ -2,7 +2,7 @@
 // decided from a matrix product, and only those pairs (25 for k = 20) get the exact distance of feature_knn.cu.
 //
 // 1. ff_prep_kernel: every feature, less a common centre (what all have in common would only cost digits: the middle two of
-//    four keys, channel by channel), as a sum of two bf16 (its upper and lower half, 2^-18 of it is lost), in the order that
+//    four keys, channel by channel), as a sum of two bf16 (its upper and lower half, 2^-17 of it is lost), in the order that
 //    tcgen05.mma reads (tiles of 128 points: half, eight channels, point), two bounds of the squared norm, and rows of float32.
 // 2. ff_filter_kernel: a block holds 128 queries, the lanes of tensor memory.  Tiles of 128 keys arrive by bulk
 //    copies; a . b = ah . bh + ah . bl + al . bh is accumulated in tensor memory, two tiles in flight, while the threads
@@ -13,13 +13,15 @@
 // 3. ff_exact_kernel: a warp per query, lane = candidate; exact distances, the nearest kept sorted by (distance, index).
 // 4. feature_knn_kernel redoes the groups of 32 queries that have one without a list.
 //
-// Error of v: let X = |query| + |key|, both less the centre; the differences are rounded once (2^-24).  The halves leave out
-// 3 * 2^-18 of |a||b|; a step of the product adds 17 numbers, taken to be rounded or truncated at 2^-23 of the sum of
-// magnitudes each, in 3 C / 16 steps: C * 2^-21 of |a||b| with room; norms and the exact distance are rounded C + 2 times at
-// 2^-24 of at most X^2.  2 |a||b| <= X^2 / 2, so that e = c X^2, c = C * 2^-21 + 2^-16 (+ 2^-110 for what underflows) covers
-// all of them about twice.  How the tensor cores round inside a step is written nowhere: what stands behind that part are the
-// errors measured against 64 bits, at most 0.5 e for 3 channels (the halves), 0.07 e for 64 and 0.05 e for 128 (normal,
-// rectified, far from the origin, channels of different size, an outlier, huge).
+// Error of v: let X = |query| + |key|, both less the centre, and count in u = 2^-24 X^2; 2 |a||b| <= X^2 / 2.
+//   halves: bf16 has eight digits, so that the upper half is off by 2^-8 of a number at most and both halves by 2^-17; left out
+//     are al . bl and what both halves miss, (2^-16 + 2 * 2^-17) of |a||b|, in v twice that: 256 u;
+//   product: 3 (C + C / 16) numbers are added, taken to be rounded or truncated at 2^-23 of the sum of magnitudes each;
+//   rounding of the norm and of the exact distance, C + 2 u each, of the centred features 2 u, of v, its bounds and the limit 4.
+// Together 256 + 5 C + 3 C / 16 + 13 u at most; e = c X^2, c = C * 2^-21 + 1.25 * 2^-16, is 320 + 8 C u (and 2^-110 for what
+// underflows).  How the tensor cores round inside a step is written nowhere: what stands behind the product's part are the
+// errors measured against 64 bits, at most 0.70, 0.62, 0.41, 0.20 and 0.07 e for 1, 3, 16, 64 and 128 channels (normal,
+// rectified, far from the origin, of one sign, channels and points of different size, far points).
 // X^2 <= 2 |query|^2 + 2 |key|^2, so that a key's part, 2 c |key|^2, is put into its norm's two bounds: a key far from the
 // others widens the bounds of no other (with the largest norm in its place, one key at 100 times the others' distance left
 // nothing to filter).  A key with d <= the k-th d has its lower v <= (k-th smallest class minimum) + 4 c |query|^2.
@@ -63,7 +65,7 @@ __host__ __device__ inline int ff_cr(int C) { return (C + 3) / 4 * 4; }
 __host__ __device__ inline int ff_tile_bytes(int C) { return 2 * ff_cp(C) * FF_T * 2 + 2 * FF_T * 4; }
 __host__ __device__ inline int ff_upper(int C) { return ff_tile_bytes(C) - 2 * FF_T * 4; }  // where the bounds lie
 __host__ __device__ inline int ff_lower(int C) { return ff_tile_bytes(C) - FF_T * 4; }
-__device__ __forceinline__ float ff_error(int C) { return (float)C * 4.76837158e-7f + 1.52587891e-5f; }  // c
+__device__ __forceinline__ float ff_error(int C) { return (float)C * 4.76837158e-7f + 1.90734863e-5f; }  // c
 __host__ __device__ inline int ff_tiles(int N) { return (N + FF_T - 1) / FF_T; }
 
 // Where a point lies in its tile: tiles are turned against each other, so that points whose indices differ by a multiple of
@@ -341,7 +343,8 @@ ff_filter_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, unsigned ch
     ok = ok && ff_wait(bar_k + 8 * (s & 1), (s >> 1) & 1) && ff_wait(bar_d + 8 * (s & 1), (s >> 1) & 1);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned ta = tmem + (s & 1) * FF_T + half * 64 + ((unsigned)((warp & 3) * 32) << 16);
-    norm = reinterpret_cast<const float4 *>(ff_raw + bytes + (s & 1) * bytes + (s < tiles ? ff_upper(C) : ff_lower(C))) + half * 16;
+    norm = reinterpret_cast<const float4 *>(ff_raw + bytes + (s & 1) * bytes + (s < tiles ? ff_upper(C) : ff_lower(C)));
+    norm += half * 16;
     ff_load32(ta, r0);
     ff_load32(ta + 32, r1);
     if (tid == 0 && s + 1 < steps) ok = ok && product(s + 1);
