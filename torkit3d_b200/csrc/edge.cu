@@ -133,6 +133,33 @@ edge_bwd_query_kernel(const T *__restrict__ gout, int64_t B, int64_t C, int64_t 
   }
 }
 
+// The same with a warp per query, for long lists: a thread's list is a line or more of its own.  8 x 64 channels x 1024 queries,
+// thread / warp, us: K = 33 45 / 87, 65 93 / 100, 70 106 / 104, 85 129 / 105, 130 201 / 127, 160 590 / 138, 256 941 / 177
+// (float64 K = 33 80 / 103, 65 157 / 124, 160 594 / 199).
+constexpr int64_t EDGE_WARP_K = 68;
+template <typename T>
+__global__ void __launch_bounds__(256)
+edge_bwd_query_warp_kernel(const T *__restrict__ gout, int64_t B, int64_t C, int64_t N1, int64_t K, int include_query,
+                           T *__restrict__ gq) {
+  const int64_t E = N1 * K;
+  const int64_t ctot = include_query ? 2 * C : C;
+  const int lane = threadIdx.x & 31;
+  for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < B * C * N1;
+       t += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int64_t n = t % N1;
+    const int64_t bc = t / N1;
+    const int64_t b = bc / C, c = bc - b * C;
+    const T *g0 = gout + (b * ctot + c) * E + n * K;
+    const T *g1 = g0 + C * E;
+    T acc = 0;
+#pragma unroll 4
+    for (int64_t k = lane; k < K; k += 32) acc += include_query ? g1[k] - g0[k] : -g0[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) gq[t] = acc;
+  }
+}
+
 // grad_key without the row path: scalar atomics.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -240,7 +267,7 @@ extern "C" int tk3d_edge_feature_bwd(const void *grad_out, const int64_t *index,
     c.B = B, c.C = C, c.N = N2, c.M = N1, c.K = K;
     c.gstride = gstride;
     c.gin = (float *)grad_key;
-    if (grad_query && scatter_edge_ok(K)) {
+    if (grad_query && scatter_edge_entries(grad_out, E, gstride, K) > 0) {
       c.gq = (float *)grad_query;
       c.include_query = include_query;
       grad_query = nullptr;
@@ -252,14 +279,16 @@ extern "C" int tk3d_edge_feature_bwd(const void *grad_out, const int64_t *index,
     grad_key = nullptr;
   }
   if (grad_query && B * C * N1 > 0) {
-    const int64_t blocks = (B * C * N1 + 255) / 256, cap = (int64_t)sm_count() * 32;
+    const bool warps = K >= EDGE_WARP_K;
+    const int64_t blocks = (B * C * N1 * (warps ? 32 : 1) + 255) / 256, cap = (int64_t)sm_count() * 32;
     const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
-    if (dtype == TK3D_F32)
-      edge_bwd_query_kernel<float><<<grid, 256, 0, st>>>((const float *)grad_out, B, C, N1, K, include_query,
-                                                         (float *)grad_query);
-    else
-      edge_bwd_query_kernel<double><<<grid, 256, 0, st>>>((const double *)grad_out, B, C, N1, K, include_query,
-                                                          (double *)grad_query);
+    if (dtype == TK3D_F32) {
+      auto kern = warps ? edge_bwd_query_warp_kernel<float> : edge_bwd_query_kernel<float>;
+      kern<<<grid, 256, 0, st>>>((const float *)grad_out, B, C, N1, K, include_query, (float *)grad_query);
+    } else {
+      auto kern = warps ? edge_bwd_query_warp_kernel<double> : edge_bwd_query_kernel<double>;
+      kern<<<grid, 256, 0, st>>>((const double *)grad_out, B, C, N1, K, include_query, (double *)grad_query);
+    }
     int rc = check_launch("edge_bwd_query_kernel");
     if (rc) return rc;
   }

@@ -11,9 +11,11 @@
 //     (a third padding) 71 -> 65 us, 128 x 512 <- 128 x 64 (two thirds) 49 -> 36.  What bounds it: instructions (0.56 of
 //     the issue slots) and the loads' latency between them, not the reductions (the interpolation's gradient reduces 2.4
 //     times as many bytes a second); walking over tiles with two buffers did not help (72 to 82 us).
-//   scatter_edge_kernel (edge features): a tile holds whole queries, and the sums over each query's K entries of both
-//     halves of gout come from the same pass.  64 x 1024 <- 1024 x 20: 45 and 76 for the sums apart -> 81 us (335 MB at
-//     4.1 TB/s; half of the issue slots, latency between them).
+//   scatter_edge_kernel (edge features, lists of up to 128): a tile holds whole queries, and the sums over each query's K
+//     entries of both halves of gout come from the same pass.  64 x 1024 <- 1024 x 20: 45 and 76 for the sums apart -> 81 us
+//     (335 MB at 4.1 TB/s).  Tiles hold as many queries as make a multiple of four entries, for 16-byte accesses: as many as
+//     fit, element by element where that is no multiple, took twice the time (B = 8, K = 14 40 us / 21, 22 78 / 34, 34 133 / 57),
+//     and for lists of odd length above 32 or of more than 128 longer than the sums apart (K = 65 348 / 128, 130 1264 / 193).
 // Clouds a few at a time, for rows that stay in L2 (32, 16, 8 MB of rows a pass), were no faster: 103, 104, 119, 150 us.
 #include "rows.cuh"
 #include "scatter.cuh"
@@ -30,8 +32,7 @@ struct ScatterArgs {
   float *rows;
   int32_t *status;
   // query sums
-  int TE, lg, per;   // entries of a tile's memory (a power of two, lg its exponent) and entries it holds
-  int slab;          // channels of a block
+  int per;           // entries of a tile
   int M, K, include_query;
   float *gq;
 };
@@ -143,31 +144,30 @@ __global__ void __launch_bounds__(SC_NT, 12) scatter_fold_kernel(const ScatterAr
   }
 }
 
-// With query sums.  A block has the entries of a few whole queries in a slab of channels, and those of the second half of
-// gout beside them, so that all its loads are under way at once (the second half read as the sums go: 122 us).
-constexpr int SE_NT = 256;
+// With query sums.  A block has the entries of a few whole queries, at most 128, in a slab of 32 channels, and those of the
+// second half of gout beside them, so that all its loads are under way at once (the second half read as the sums go: 122 us).
+// A thread's chunk of four entries is the same in every row, and its rows are 8 apart, which flips bits 1 and 2 of
+// (c >> 2) & 7: addresses are constants apart (108 -> 81 us).
+constexpr int SE_NT = 256, SE_TE = 128, SE_C = 32;
 
-// SLAB: tiles of 128 entries and slabs of 32 channels, with 16-byte loads; a thread's chunk is then the same in every row,
-// and its rows are 8 apart, which flips bits 1 and 2 of (c >> 2) & 7: addresses are constants apart (108 -> 81 us).
-template <bool VEC, bool SLAB, typename IndexT>
+template <typename IndexT>
 __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a, const IndexT *__restrict__ index) {
-  extern __shared__ __align__(16) float tile[];  // [halves][slab][TE], then int id[TE]
+  extern __shared__ __align__(16) float tile[];  // [halves][SE_C][SE_TE], then int id[SE_TE]
   constexpr int NW = SE_NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ql = lane & 7, el = lane >> 3;
-  const int TE = SLAB ? 128 : a.TE, slab = SLAB ? 32 : a.slab, halves = a.include_query ? 2 : 1;
-  int *sid = reinterpret_cast<int *>(tile + halves * slab * TE);
+  const int halves = a.include_query ? 2 : 1;
+  int *sid = reinterpret_cast<int *>(tile + halves * SE_C * SE_TE);
   const int64_t b = blockIdx.y;
   const int64_t e0 = (int64_t)blockIdx.x * a.per;
-  const int n = (int)min((int64_t)a.per, a.E - e0);
-  const int c0 = blockIdx.z * slab, nc = min(slab, a.C - c0);  // channels of this block
+  const int n = (int)min((int64_t)a.per, a.E - e0);  // a multiple of 4
+  const int c0 = blockIdx.z * SE_C, nc = min(SE_C, a.C - c0);  // channels of this block
   const float *gb = a.gout + b * a.gstride + (int64_t)c0 * a.E + e0;
-  const IndexT *ip = index + b * a.E + e0;
-  const int64_t id0 = tid < n ? (int64_t)ip[tid] : -1;  // requested ahead of gout
-  if (SLAB) {
+  const int64_t id0 = tid < n ? (int64_t)index[b * a.E + e0 + tid] : -1;  // requested ahead of gout
+  {
     const int e = lane << 2;
     const float *src = gb + (int64_t)warp * a.E + e;
-    const int at = warp * 128 + (e ^ ((warp >> 2) << 2));
+    const int at = warp * SE_TE + (e ^ ((warp >> 2) << 2));
     const int64_t step = 8 * a.E, other = (int64_t)a.C * a.E;
     float4 v[2][4];
 #pragma unroll
@@ -181,58 +181,35 @@ __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         if (h < halves && e < n && warp + 8 * i < nc)
-          *reinterpret_cast<float4 *>(tile + ((at + (h * 32 + 8 * i) * 128) ^ (8 * i))) = v[h][i];
+          *reinterpret_cast<float4 *>(tile + ((at + (h * SE_C + 8 * i) * SE_TE) ^ (8 * i))) = v[h][i];
   }
-  for (int h = 0; !SLAB && h < halves; ++h) {
-    const float *src = gb + (int64_t)h * a.C * a.E;
-    float *dst = tile + h * slab * TE;
-    if (VEC) {
-      const int lc = a.lg - 2;
-#pragma unroll 4
-      for (int u = tid; u < nc << lc; u += SE_NT) {
-        const int c = u >> lc, e = (u & ((1 << lc) - 1)) << 2;
-        if (e < n)
-          *reinterpret_cast<float4 *>(dst + sc_at(c, e, TE)) =
-              __ldcs(reinterpret_cast<const float4 *>(src + (int64_t)c * a.E + e));
-      }
-    } else {
-#pragma unroll 4
-      for (int u = tid; u < nc << a.lg; u += SE_NT) {
-        const int c = u >> a.lg, e = u & (TE - 1);
-        if (e < n) dst[sc_at(c, e, TE)] = __ldcs(src + (int64_t)c * a.E + e);
-      }
-    }
+  for (int i = nc * SE_TE + tid; i < ((nc + 3) & ~3) * SE_TE; i += SE_NT) tile[i] = 0.f;  // the row's padding channels
+  if (tid < n) {
+    const bool out = id0 < 0 || id0 >= a.N;
+    sid[tid] = out ? -1 : (int)id0;
+    if (out && a.status) atomicOr(a.status, 1);
   }
-  for (int i = nc * TE + tid; i < ((nc + 3) & ~3) * TE; i += SE_NT) tile[i] = 0.f;  // the row's padding channels
-  bool bad = false;
-  for (int e = tid; e < n; e += SE_NT) {
-    const int64_t v = e == tid ? id0 : (int64_t)ip[e];
-    const bool out = v < 0 || v >= a.N;
-    bad |= out;
-    sid[e] = out ? -1 : (int)v;
-  }
-  if (bad && a.status) atomicOr(a.status, 1);
   __syncthreads();
   const int L = (nc + 3) >> 2;
   float *rb = a.rows + b * (int64_t)a.N * a.ld + c0 + 4 * ql;
   for (int s = warp * 4 + el; s < n; s += NW * 4) {
     const int id = sid[s];
     if (id < 0) continue;
-    const float *src = tile + 4 * ql * TE + (s ^ (ql << 2));
-    if (ql < L) red_add4(rb + (int64_t)id * a.ld, src[0], src[TE], src[2 * TE], src[3 * TE]);
+    const float *src = tile + 4 * ql * SE_TE + (s ^ (ql << 2));
+    if (ql < L) red_add4(rb + (int64_t)id * a.ld, src[0], src[SE_TE], src[2 * SE_TE], src[3 * SE_TE]);
   }
   // gq[b,c,m] = sum_k (g[C+c] - g[c]), or minus the sum of the only half
   const int K = a.K, nq = n / K;
   const int64_t m0 = (int64_t)blockIdx.x * (a.per / K);
-  const float *second = tile + slab * TE;
+  const float *second = tile + SE_C * SE_TE;
   for (int u = tid; u < nc * nq; u += SE_NT) {
     const int c = u / nq, m = u - c * nq;
     float sum = 0.f;
-    if (VEC && (K & 3) == 0) {
+    if ((K & 3) == 0) {
       for (int e = m * K; e < m * K + K; e += 4) {
-        const float4 g0 = *reinterpret_cast<const float4 *>(tile + sc_at(c, e, TE));
+        const float4 g0 = *reinterpret_cast<const float4 *>(tile + sc_at(c, e, SE_TE));
         float4 g1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a.include_query) g1 = *reinterpret_cast<const float4 *>(second + sc_at(c, e, TE));
+        if (a.include_query) g1 = *reinterpret_cast<const float4 *>(second + sc_at(c, e, SE_TE));
         sum += g1.x - g0.x;
         sum += g1.y - g0.y;
         sum += g1.z - g0.z;
@@ -240,7 +217,7 @@ __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a
       }
     } else {
       for (int e = m * K; e < m * K + K; ++e) {
-        const int at = sc_at(c, e, TE);
+        const int at = sc_at(c, e, SE_TE);
         sum += a.include_query ? second[at] - tile[at] : -tile[at];
       }
     }
@@ -285,21 +262,12 @@ template <typename IndexT>
 int scatter_go(ScatterArgs a, int64_t B, const IndexT *index, cudaStream_t st) {
   const bool aligned = a.E % 4 == 0 && a.gstride % 4 == 0 && (reinterpret_cast<uintptr_t>(a.gout) & 15) == 0;
   if (a.gq) {
-    // tiles of 128 entries (one query where it is longer) and slabs of 32 channels (8 beside long queries)
-    a.lg = 7;
-    while ((1 << a.lg) < a.K) ++a.lg;
-    a.TE = 1 << a.lg;
-    a.per = a.TE / a.K * a.K;
-    a.slab = a.lg <= 8 ? 32 : 8;
-    const size_t smem = sizeof(float) * (size_t)(a.include_query ? 2 : 1) * a.slab * a.TE + sizeof(int) * (size_t)a.TE;
+    a.per = scatter_edge_entries(a.gout, a.E, a.gstride, a.K);
+    const size_t smem = sizeof(float) * (size_t)(a.include_query ? 2 : 1) * SE_C * SE_TE + sizeof(int) * SE_TE;
     const int64_t tiles = (a.E + a.per - 1) / a.per;
     TK3D_REQUIRE(tiles < (1LL << 31), TK3D_ERR_SHAPE, "scatter: too many entries");
-    const dim3 grid((unsigned)tiles, (unsigned)B, (unsigned)((a.C + a.slab - 1) / a.slab));
-    auto kern = !(aligned && a.per % 4 == 0) ? scatter_edge_kernel<false, false, IndexT>
-                : a.lg == 7                  ? scatter_edge_kernel<true, true, IndexT>
-                                             : scatter_edge_kernel<true, false, IndexT>;
-    if (smem > 48 * 1024) TK3D_CUDA(raise_smem_limit((const void *)kern, (int)smem));
-    kern<<<grid, SE_NT, smem, st>>>(a, index);
+    const dim3 grid((unsigned)tiles, (unsigned)B, (unsigned)((a.C + SE_C - 1) / SE_C));
+    scatter_edge_kernel<IndexT><<<grid, SE_NT, smem, st>>>(a, index);
     return check_launch("scatter_edge_kernel");
   }
   const size_t smem = sizeof(float) * (size_t)a.ld * ROWS_TE;
@@ -325,7 +293,11 @@ bool scatter_ok(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K) {
          M * K < (1LL << 36);
 }
 
-bool scatter_edge_ok(int64_t K) { return K <= 1024; }
+int scatter_edge_entries(const void *gout, int64_t E, int64_t gstride, int64_t K) {
+  if (K > SE_TE || E % 4 != 0 || gstride % 4 != 0 || (reinterpret_cast<uintptr_t>(gout) & 15) != 0) return 0;
+  const int whole = K % 4 == 0 ? 1 : K % 2 == 0 ? 2 : 4;  // queries whose entries are a multiple of 4
+  return (int)(SE_TE / (K * whole) * (K * whole));
+}
 
 int scatter_launch(const ScatterCall &c, cudaStream_t st) {
   ScatterArgs a;

@@ -11,7 +11,7 @@ struct ScatterCall {
   int index_i32 = 0;
   int64_t B = 0, C = 0, N = 0, M = 0, K = 0, gstride = 0;
   float *gin = nullptr;         // [B][C][N]
-  float *gq = nullptr;          // [B][C][M]: sums over each query's K entries, see scatter_edge_ok
+  float *gq = nullptr;          // [B][C][M]: sums over each query's K entries, see scatter_edge_entries
   int include_query = 0;
   int32_t *status = nullptr;
   void *scratch = nullptr;      // scatter_scratch_bytes(B, C, N), 16-byte aligned
@@ -30,9 +30,10 @@ inline bool scatter_pays(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K) 
   if (N > SCATTER_TRANSPOSED && (C < 16 || 4 * M * K < N)) return false;
   return (C % 4 == 0 && (M * K) % 4 == 0) || B * C * M * K >= 12000000;
 }
-// Whether the sizes are served; whether gq can be summed in the same pass.
+// Whether the sizes are served.
 bool scatter_ok(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K);
-bool scatter_edge_ok(int64_t K);
+// Entries of a tile where gq can be summed in the same pass, else 0.
+int scatter_edge_entries(const void *gout, int64_t E, int64_t gstride, int64_t K);
 int scatter_launch(const ScatterCall &c, cudaStream_t st);
 
 }  // namespace tk3d
