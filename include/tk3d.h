@@ -348,7 +348,7 @@ int tk3d_fps_gather(const void *points, int64_t B, int64_t N, int64_t num_sample
  *   status    int32            in/out optional: bit 0 is OR-ed in when a centre has no neighbour
  *                                   (its K entries are -1; its feature channels are 0 and its
  *                                   coordinate channels are -centroid)
- *   scratch   tk3d_sa_group_scratch_bytes(...) bytes, required when C > 0
+ *   scratch   tk3d_sa_group_scratch_bytes(...) bytes; at least B*C*N*4 required when C > 0 (the faster paths want all of it)
  * tk3d_sa_group_supported() tells whether the shape is served (fp32, C <= 512, 1 <= K <= 128);
  * otherwise compose tk3d_ball_query and tk3d_group_fwd.
  */

@@ -81,7 +81,7 @@ def sa_group_forward(points, centroids, feature, radius, max_neighbors, use_xyz=
         index32 = torch.empty((B, M, K), dtype=torch.int32, device=dev) if want_index else None
         need = _lib.scratch_bytes("tk3d_sa_group", B, C, N, M, K, _lib.F32)
         scratch = _order_scratch(need, dev, 4 * B * C * N) if need else None
-        need = scratch.numel() if need else 0
+        need = scratch.numel() if scratch is not None else 0
         check(lib.tk3d_sa_group_fwd(_ptr(points), _ptr(centroids), _ptr(feature) if C else None, B, C, N, M,
                                     float(radius), K, 1 if channel_first else 0, 1 if use_xyz else 0, _ptr(out),
                                     _ptr(index32) if want_index else None, None, _ptr(scratch) if need else None,

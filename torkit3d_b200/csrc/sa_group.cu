@@ -399,10 +399,10 @@ static bool sa_two_step(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K) {
 }
 
 extern "C" size_t tk3d_sa_group_scratch_bytes(int64_t B, int64_t C, int64_t N, int64_t M, int64_t K, int dtype) {
-  if (!tk3d_sa_group_supported(B, C, N, M, K, dtype) || C == 0) return 0;
-  const size_t rows = rows_scratch_bytes(B, C, N);
-  return ball_order_pays(B, M, N) ? sa_align(rows) + sp_search_bytes(B, M, N) + sizeof(int32_t) * (size_t)(B * M * K)
-                                  : rows;
+  if (!tk3d_sa_group_supported(B, C, N, M, K, dtype)) return 0;
+  const size_t rows = rows_scratch_bytes(B, C, N), lists = sizeof(int32_t) * (size_t)(B * M * K);
+  if (C > 0 && ball_order_pays(B, M, N)) return sa_align(rows) + sp_search_bytes(B, M, N) + lists;
+  return sa_two_step(B, C, N, M, K) && lists > rows ? lists : rows;  // the rows' place, for a call without index32
 }
 
 extern "C" int tk3d_sa_group_fwd(const void *points, const void *centroids, const void *feature, int64_t B, int64_t C,
