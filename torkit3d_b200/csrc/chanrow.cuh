@@ -176,11 +176,11 @@ inline bool chanrow_ok(int64_t B, int64_t C, int64_t N1, int64_t E, int64_t elem
   return N1 >= 256 && N1 * elem <= CR_MAX_ROW_BYTES && E >= 1024 && B <= 65535 && C <= 65532;
 }
 
-// out [B] slabs of ostride elements; xyz (float32): three more channels behind the C of `in`.
-template <typename T, typename IndexT>
+// out [B] slabs of ostride elements; XYZ (float32): three more channels behind the C of `in`.
+template <bool XYZ, typename T, typename IndexT>
 int group_fwd_chanrow(const T *in, const IndexT *index, int64_t B, int64_t C, int64_t N1, int64_t E, T *out,
-                      int64_t ostride, int32_t *status, const CrXyz *xyz, cudaStream_t st) {
-  const int64_t sms = sm_count(), ctot = C + (xyz ? 3 : 0);
+                      int64_t ostride, int32_t *status, const CrXyz &xyz, cudaStream_t st) {
+  const int64_t sms = sm_count(), ctot = C + (XYZ ? 3 : 0);
   // Entries per block: every block of a cloud copies the rows of its channels, so that long rows want many entries
   // (8 x 64 x 16000 -> 4000 x 32: 150 us with 4096 entries, 100 with 8192, 75 with 16384), short ones many blocks
   // (4 x 64 x 2000 -> 500 x 32: 7, 7 and 12).
@@ -201,30 +201,20 @@ int group_fwd_chanrow(const T *in, const IndexT *index, int64_t B, int64_t C, in
   const size_t smem = (size_t)(2 * rb * rowb);
   dim3 grid((unsigned)chunks, (unsigned)groups, (unsigned)B);
   const bool vec = E % 4 == 0 && (ostride * sizeof(T)) % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-  CrXyz none = {};
-#define TK3D_CR_LAUNCH(NT, RR, VV, XX)                                                                                \
+#define TK3D_CR_LAUNCH(NT, RR, VV)                                                                                    \
   {                                                                                                                   \
     if (smem > 48 * 1024)                                                                                             \
-      TK3D_CUDA(raise_smem_limit((const void *)group_fwd_chanrow_kernel<T, IndexT, NT, RR, VV, XX>, (int)smem));      \
-    group_fwd_chanrow_kernel<T, IndexT, NT, RR, VV, XX><<<grid, NT, smem, st>>>(                                      \
-        in, index, (int)C, (int)N1, E, cg, (int)rb, out, ostride, status, xyz ? *xyz : none);                         \
+      TK3D_CUDA(raise_smem_limit((const void *)group_fwd_chanrow_kernel<T, IndexT, NT, RR, VV, XYZ>, (int)smem));     \
+    group_fwd_chanrow_kernel<T, IndexT, NT, RR, VV, XYZ><<<grid, NT, smem, st>>>(                                     \
+        in, index, (int)C, (int)N1, E, cg, (int)rb, out, ostride, status, xyz);                                       \
   }
-#define TK3D_CR_PICK(XX)                                                                    \
-  if (pick == 3) {                                                                          \
-    if (vec) TK3D_CR_LAUNCH(512, 8, true, XX) else TK3D_CR_LAUNCH(512, 8, false, XX)        \
-  } else if (pick == 2) {                                                                   \
-    if (vec) TK3D_CR_LAUNCH(256, 8, true, XX) else TK3D_CR_LAUNCH(256, 8, false, XX)        \
-  } else {                                                                                  \
-    if (vec) TK3D_CR_LAUNCH(256, 4, true, XX) else TK3D_CR_LAUNCH(256, 4, false, XX)        \
+  if (pick == 3) {
+    if (vec) TK3D_CR_LAUNCH(512, 8, true) else TK3D_CR_LAUNCH(512, 8, false)
+  } else if (pick == 2) {
+    if (vec) TK3D_CR_LAUNCH(256, 8, true) else TK3D_CR_LAUNCH(256, 8, false)
+  } else {
+    if (vec) TK3D_CR_LAUNCH(256, 4, true) else TK3D_CR_LAUNCH(256, 4, false)
   }
-  if constexpr (sizeof(T) == 4) {
-    if (xyz) {
-      TK3D_CR_PICK(true)
-      return check_launch("group_fwd_chanrow_kernel");
-    }
-  }
-  TK3D_CR_PICK(false)
-#undef TK3D_CR_PICK
 #undef TK3D_CR_LAUNCH
   return check_launch("group_fwd_chanrow_kernel");
 }

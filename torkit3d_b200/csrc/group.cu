@@ -205,7 +205,7 @@ static int group_fwd_impl(const void *in, const IndexT *index, int64_t B, int64_
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == TK3D_F32) {
     if (chanrow_ok(B, C, N1, E))
-      return group_fwd_chanrow<float, IndexT>((const float *)in, index, B, C, N1, E, (float *)out, C * E, status, nullptr, st);
+      return group_fwd_chanrow<false>((const float *)in, index, B, C, N1, E, (float *)out, C * E, status, CrXyz{}, st);
     const size_t want = tk3d_group_fwd_scratch_bytes(B, C, N1, N2, K, dtype);
     const size_t rows = rows_profitable(C, N1, E, 1) && B <= 65535 ? rows_scratch_bytes(B, C, N1) : 0;
     (void)want;
@@ -215,8 +215,7 @@ static int group_fwd_impl(const void *in, const IndexT *index, int64_t B, int64_
     return group_fwd_t<float, IndexT>((const float *)in, index, B, C, N1, E, (float *)out, status, st);
   }
   if (chanrow_ok(B, C, N1, E, 8))
-    return group_fwd_chanrow<double, IndexT>((const double *)in, index, B, C, N1, E, (double *)out, C * E, status, nullptr,
-                                             st);
+    return group_fwd_chanrow<false>((const double *)in, index, B, C, N1, E, (double *)out, C * E, status, CrXyz{}, st);
   return group_fwd_t<double, IndexT>((const double *)in, index, B, C, N1, E, (double *)out, status, st);
 }
 

@@ -438,8 +438,8 @@ extern "C" int tk3d_sa_group_fwd(const void *points, const void *centroids, cons
     xyz.pps = xyz_channel_first ? 1 : 3, xyz.pcs = xyz_channel_first ? (int)N : 1;
     xyz.cps = xyz_channel_first ? 1 : 3, xyz.cpc = xyz_channel_first ? (int)M : 1;
     xyz.K = (int)K, xyz.M = (int)M;
-    return group_fwd_chanrow<float, int32_t>((const float *)feature, lists, B, C, N, M * K, (float *)out, ctot * M * K,
-                                             status, use_xyz ? &xyz : nullptr, st);
+    auto gather = use_xyz ? group_fwd_chanrow<true, float, int32_t> : group_fwd_chanrow<false, float, int32_t>;
+    return gather((const float *)feature, lists, B, C, N, M * K, (float *)out, ctot * M * K, status, xyz, st);
   }
   const float *featT = nullptr;
   if (C > 0 && N > 0) {
