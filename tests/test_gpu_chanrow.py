@@ -36,6 +36,7 @@ def test_group(B, C, N, M, K, dt):
             assert lib.tk3d_group_fwd_layout(f.data_ptr(), ix.data_ptr(), t, B, C, N, M, K, out.data_ptr(), status.data_ptr(),
                                              None, 0, code, torch.cuda.current_stream().cuda_stream) == 0
             assert torch.equal(out, _gather(f, index)) and int(status) == 1
+            assert bool(out_raw[:shift].isnan().all()) and bool(out_raw[shift + B * C * M * K:].isnan().all())
 
 
 @pytest.mark.parametrize("cf", [True, False])
@@ -62,3 +63,28 @@ def test_set_abstraction(B, C, N, M, K, cf, use_xyz, want_index):
     assert torch.equal(out, torch.cat(parts, 1))
     if want_index:
         assert torch.equal(index.long(), ref)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float64])
+@pytest.mark.parametrize("B,C,N,M,K", [(2, 40, 1023, 1300, 33), (1, 131, 4099, 1101, 16), (1, 12, 12287, 11201, 17),
+                                       (3, 1, 301, 44667, 15), (64, 3, 257, 345, 31), (1, 64, 255, 1024, 31)])
+def test_rows_in_pieces(B, C, N, M, K, dt):
+    """Outputs large enough for rows that are no whole 16-byte lines; nothing beside the output is written."""
+    from torkit3d_b200 import _lib
+
+    lib = _lib.load()
+    index = torch.randint(-1, N + 1, (B, M, K), device=DEV)
+    index[0, 0, 0] = N
+    n = B * C * M * K
+    raw = torch.randn(B * C * N + 3, dtype=dt, device=DEV)
+    out_raw = torch.empty(n + 64, dtype=dt, device=DEV)
+    for shift in (0, 1, 3):
+        f = raw[shift:shift + B * C * N].view(B, C, N)
+        out_raw.fill_(7.5)
+        out = out_raw[32 + shift:32 + shift + n].view(B, C, M, K)
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        assert lib.tk3d_group_fwd(f.data_ptr(), index.data_ptr(), B, C, N, M, K, out.data_ptr(), status.data_ptr(), None, 0,
+                                  _lib.F32 if dt == torch.float32 else _lib.F64,
+                                  torch.cuda.current_stream().cuda_stream) == 0
+        assert torch.equal(out, _gather(f, index)) and int(status) == 1
+        assert bool((out_raw[:32 + shift] == 7.5).all()) and bool((out_raw[32 + shift + n:] == 7.5).all())

@@ -176,15 +176,28 @@ inline bool chanrow_ok(int64_t B, int64_t C, int64_t N1, int64_t E, int64_t elem
   return N1 >= 256 && N1 * elem <= CR_MAX_ROW_BYTES && E >= 1024 && B <= 65535 && C <= 65532;
 }
 
+// Rows that are not whole 16-byte lines, copied in pieces: worth it from 2e6 elements of output and a quarter as many entries as
+// points on; below, the direct gather (us, direct / channel rows: 1 x 64 x 1185 -> 18960 4.5 / 5.2, 14 x 12 x 1185 -> 4740 4.1 /
+// 5.3, 64 x 12 x 20411 -> 3060 11 / 15; 1 x 64 x 8191 -> 32764 9.1 / 6.6, 64 x 12 x 8191 -> 3276 12.8 / 8.3).
+inline bool chanrow_pieces_pay(int64_t B, int64_t C, int64_t N1, int64_t E) {
+  return B * C * E >= 2000000 && 4 * E >= N1;
+}
+
 // out [B] slabs of ostride elements; XYZ (float32): three more channels behind the C of `in`.
 template <bool XYZ, typename T, typename IndexT>
 int group_fwd_chanrow(const T *in, const IndexT *index, int64_t B, int64_t C, int64_t N1, int64_t E, T *out,
                       int64_t ostride, int32_t *status, const CrXyz &xyz, cudaStream_t st) {
   const int64_t sms = sm_count(), ctot = C + (XYZ ? 3 : 0);
-  // Entries per block: every block of a cloud copies the rows of its channels, so that long rows want many entries
-  // (8 x 64 x 16000 -> 4000 x 32: 150 us with 4096 entries, 100 with 8192, 75 with 16384), short ones many blocks
-  // (4 x 64 x 2000 -> 500 x 32: 7, 7 and 12).
-  const int pick = N1 >= 9000 ? 3 : N1 >= 4096 || B * ((E + 8191) / 8192) * 4 >= 3 * sms ? 2 : 1;
+  // Entries per block: every block of a cloud copies the rows of its channels, so that large calls want many entries, small
+  // ones many blocks; rows of 14000 points leave room for one block per SM, which wants more threads.  4096 / 8192 / 16384
+  // entries, us: 1 x 131 x 24000 -> 24000 13.6 / 12.0 / 12.4, 4 x 64 x 24000 -> 96000 75 / 46 / 40, 32 x 64 x 12000 -> 12000 46 / 47 / 42,
+  // 43 x 12 x 12000 -> 48000 42 / 34 / 39, 8 x 64 x 12000
+  // -> 48000 43 / 35 / 36, 11 x 64 x 8192 -> 32768 35 / 29 / 34, 1 x 131 x 4096 -> 65536 10.6 / 13.7 / 16.5, 1 x 12 x 12000 ->
+  // 48000 3.7 / 4.8 / 7.2, 64 x 64 x 300 -> 4800 25 / 20 / 27.
+  const int64_t work = B * C * E;
+  const bool long_rows = N1 >= 14000 ? work >= 3500000 : N1 >= 9000 && C >= 48 && work >= 10000000;
+  const bool many = B * ((E + 8191) / 8192) * 4 >= 3 * sms || (N1 >= 4096 && work >= 10000000);
+  const int pick = E > 8192 && long_rows ? 3 : E > 4096 && many ? 2 : 1;
   const int64_t ech = pick == 3 ? 16384 : pick == 2 ? 8192 : 4096;
   const int64_t chunks = (E + ech - 1) / ech;
   // channel groups: enough blocks for about three per SM, as few groups as possible beyond that

@@ -187,10 +187,23 @@ int check_group_args(const char *what, const void *a, const int64_t *index, cons
 
 using namespace tk3d;
 
+// Features of N1 points as whole 16-byte lines, wherever they start?  N1 % 4 for float64 too.
+static bool group_lines(const void *in, int64_t N1) { return N1 % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0; }
+
+static bool group_by_channels(const void *in, int64_t B, int64_t C, int64_t N1, int64_t E, int64_t elem) {
+  return chanrow_ok(B, C, N1, E, elem) && (group_lines(in, N1) || chanrow_pieces_pay(B, C, N1, E));
+}
+
+// Many entries per point gather from transposed rows with 16-byte accesses rather than from channel rows in pieces (us, rows /
+// channel rows: 1 x 64 x 20411 -> 326576 23 / 35, 5 x 64 x 4879 -> 78064 27 / 34; 20 x 64 x 4879 -> 19516 38 / 34).
+static bool group_by_points(int64_t C, int64_t N1, int64_t E) {
+  return N1 % 4 != 0 && C % 4 == 0 && E % 4 == 0 && rows_profitable(C, N1, E, 1) && E >= (N1 >= 14000 ? 3 : 8) * N1;
+}
+
 extern "C" size_t tk3d_group_fwd_scratch_bytes(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t K, int dtype) {
   if (dtype != TK3D_F32 || B <= 0 || C <= 0 || N1 <= 0 || N2 <= 0 || K <= 0 || B > 65535) return 0;
   // shapes the channel-row kernels take need no scratch
-  if (chanrow_ok(B, C, N1, N2 * K)) return 0;
+  if (group_by_channels(nullptr, B, C, N1, N2 * K, 4) && !group_by_points(C, N1, N2 * K)) return 0;
   return rows_profitable(C, N1, N2 * K, 1) ? rows_scratch_bytes(B, C, N1) : 0;
 }
 
@@ -204,17 +217,16 @@ static int group_fwd_impl(const void *in, const IndexT *index, int64_t B, int64_
   TK3D_REQUIRE(index && out && (in || N1 == 0), TK3D_ERR_NULL, "group_fwd: a pointer is NULL");
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == TK3D_F32) {
-    if (chanrow_ok(B, C, N1, E))
-      return group_fwd_chanrow<false>((const float *)in, index, B, C, N1, E, (float *)out, C * E, status, CrXyz{}, st);
-    const size_t want = tk3d_group_fwd_scratch_bytes(B, C, N1, N2, K, dtype);
     const size_t rows = rows_profitable(C, N1, E, 1) && B <= 65535 ? rows_scratch_bytes(B, C, N1) : 0;
-    (void)want;
-    if (rows != 0 && scratch != nullptr && scratch_bytes >= rows)
+    const bool fits = rows != 0 && scratch != nullptr && scratch_bytes >= rows;
+    if (group_by_channels(in, B, C, N1, E, 4) && !(fits && group_by_points(C, N1, E)))
+      return group_fwd_chanrow<false>((const float *)in, index, B, C, N1, E, (float *)out, C * E, status, CrXyz{}, st);
+    if (fits)
       return gather_rows<1, IndexT>((const float *)in, index, nullptr, B, C, N1, E, (float *)out, status,
                                     (float *)scratch, st);
     return group_fwd_t<float, IndexT>((const float *)in, index, B, C, N1, E, (float *)out, status, st);
   }
-  if (chanrow_ok(B, C, N1, E, 8))
+  if (group_by_channels(in, B, C, N1, E, 8))
     return group_fwd_chanrow<false>((const double *)in, index, B, C, N1, E, (double *)out, C * E, status, CrXyz{}, st);
   return group_fwd_t<double, IndexT>((const double *)in, index, B, C, N1, E, (double *)out, status, st);
 }
