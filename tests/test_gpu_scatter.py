@@ -146,3 +146,13 @@ def test_no_memory_for_the_rows(B, C, N, M, K, monkeypatch):
     assert len(refused) == 3
     for x in got:
         _close(x, *ref)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "padded", "bad"])
+@pytest.mark.parametrize("B,C,N,M,K", [(4, 512, 300, 331, 16), (2, 64, 1000, 1303, 64), (2, 64, 1000, 1303, 60)])
+def test_group_on_both_sides_of_the_folding_limit(B, C, N, M, K, kind):
+    from torkit3d_b200 import _C
+
+    index = _index(kind, B, M, K, N)
+    g = torch.randn(B, C, M, K, device=DEV)
+    _close(_C.group_points_backward_cuda(g, index, N), *_scatter(g, index, N))

@@ -190,10 +190,9 @@ int group_fwd_chanrow(const T *in, const IndexT *index, int64_t B, int64_t C, in
   const int64_t sms = sm_count(), ctot = C + (XYZ ? 3 : 0);
   // Entries per block: every block of a cloud copies the rows of its channels, so that large calls want many entries, small
   // ones many blocks; rows of 14000 points leave room for one block per SM, which wants more threads.  4096 / 8192 / 16384
-  // entries, us: 1 x 131 x 24000 -> 24000 13.6 / 12.0 / 12.4, 4 x 64 x 24000 -> 96000 75 / 46 / 40, 32 x 64 x 12000 -> 12000 46 / 47 / 42,
-  // 43 x 12 x 12000 -> 48000 42 / 34 / 39, 8 x 64 x 12000
-  // -> 48000 43 / 35 / 36, 11 x 64 x 8192 -> 32768 35 / 29 / 34, 1 x 131 x 4096 -> 65536 10.6 / 13.7 / 16.5, 1 x 12 x 12000 ->
-  // 48000 3.7 / 4.8 / 7.2, 64 x 64 x 300 -> 4800 25 / 20 / 27.
+  // entries, us: 1 x 131 x 24000 -> 24000 13.6 / 12.0 / 12.4, 4 x 64 x 24000 -> 96000 75 / 46 / 40, 32 x 64 x 12000 -> 12000
+  // 46 / 47 / 42, 43 x 12 x 12000 -> 48000 42 / 34 / 39, 8 x 64 x 12000 -> 48000 43 / 35 / 36, 11 x 64 x 8192 -> 32768 35 / 29 /
+  // 34, 1 x 131 x 4096 -> 65536 10.6 / 13.7 / 16.5, 1 x 12 x 12000 -> 48000 3.7 / 4.8 / 7.2, 64 x 64 x 300 -> 4800 25 / 20 / 27.
   const int64_t work = B * C * E;
   const bool long_rows = N1 >= 14000 ? work >= 3500000 : N1 >= 9000 && C >= 48 && work >= 10000000;
   const bool many = B * ((E + 8191) / 8192) * 4 >= 3 * sms || (N1 >= 4096 && work >= 10000000);

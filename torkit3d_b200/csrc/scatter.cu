@@ -274,8 +274,12 @@ int scatter_go(ScatterArgs a, int64_t B, const IndexT *index, cudaStream_t st) {
   const int64_t tiles = (a.E + ROWS_TE - 1) / ROWS_TE;
   TK3D_REQUIRE(tiles < (1LL << 31), TK3D_ERR_SHAPE, "scatter: too many entries");
   const dim3 grid((unsigned)tiles, (unsigned)B);
-  // Folding pays from 64 channels on: 8 x 24000 <- 4000 x 16 with 32 channels, a third padding, 23 us without and 29 with it
-  if (aligned && a.C % 4 == 0 && a.C < 64) {
+  // Folding pays from 64 channels on (8 x 24000 <- 4000 x 16 with 32 channels, a third padding, 23 us without and 29 with it) and
+  // from 1e7 elements on, whatever the padding: without / with it, none, a third and two thirds padded, us: 1 x 256 x 128 <-
+  // 512 7.4 / 8.3, 8.8, 8.4, 16 x 256 x 512 <- 2048 18 / 18.4, 19.9, 17.5, 64 x 64 x 2048 <- 8192 50 / 46, 48, 44, 16 x 512 x
+  // 2048 <- 8192 171 / 139, 169, 155.
+  if (aligned && a.C % 4 == 0 && (a.C < 64 || B * a.C * a.E < 10000000)) {
+    if (smem > 48 * 1024) TK3D_CUDA(raise_smem_limit((const void *)scatter_rows_vec4_kernel<1, IndexT>, (int)smem));
     scatter_rows_vec4_kernel<1, IndexT><<<grid, ROWS_THREADS, smem, st>>>(a.gout, index, nullptr, a.C, a.N, a.E, a.gstride,
                                                                           a.rows, a.status);
     return check_launch("scatter_rows_vec4_kernel");
