@@ -437,9 +437,10 @@ int tk3d_feature_knn_ws(const void *query, const void *key, int64_t B, int64_t C
                         void *stream);
 
 /*
- * Range-checked build.  libtk3d_b200_bounds.so is this library compiled with -DTK3D_BOUNDS: every
- * coordinate load and every index-tensor access of the operators is checked against the extent of
- * its tensor, a violation is counted and redirected to element 0.  tk3d_bounds_violations()
+ * Range-checked build.  libtk3d_b200_bounds.so is this library compiled with -DTK3D_BOUNDS: the
+ * coordinate loads and index writes of the searches, the index reads of the gathers and the rows and outputs that
+ * the channel-row gathers and the gradients by rows address are checked against the extent of their
+ * tensor, a violation is counted and redirected to element 0 (stores are left out).  tk3d_bounds_violations()
  * synchronises the device and returns the number of violations since the library was loaded; in the
  * regular build, which carries no checks, it returns -1.  (The reference's only run-time checks on
  * this path are the device-side asserts of torkit3d/csrc/cuda/group_points_kernel.cu:62 and

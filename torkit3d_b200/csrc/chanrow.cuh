@@ -72,7 +72,7 @@ group_fwd_chanrow_kernel(const T *__restrict__ in, const IndexT *__restrict__ in
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       const int e = entry(r, v);
-      int64_t j = e < left ? (int64_t)index[b * E + e0 + e] : 0;
+      int64_t j = e < left ? (int64_t)index[TK3D_AT(b * E + e0 + e, gridDim.z * E)] : 0;
       if (j < 0 || j >= N1) {
         j = N1;  // the zero behind the row
         bad = true;
@@ -137,7 +137,8 @@ group_fwd_chanrow_kernel(const T *__restrict__ in, const IndexT *__restrict__ in
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if (entry(r, 0) >= left) break;
-        T v[4] = {row[id[r][0]], row[id[r][1]], row[id[r][2]], row[id[r][3]]};
+        T v[4] = {row[TK3D_AT(id[r][0], N1 + 1)], row[TK3D_AT(id[r][1], N1 + 1)], row[TK3D_AT(id[r][2], N1 + 1)],
+                  row[TK3D_AT(id[r][3], N1 + 1)]};
         if constexpr (XYZ) {
           if (coord) {
             const float *q = xyz.cent + b * 3 * (int64_t)xyz.M + (int64_t)(c - C) * xyz.cpc;
@@ -150,6 +151,7 @@ group_fwd_chanrow_kernel(const T *__restrict__ in, const IndexT *__restrict__ in
         }
         if constexpr (VEC) {
           const int e = entry(r, 0);
+          if (!TK3D_IN(o + e + 3 - out, (int64_t)gridDim.z * ostride)) continue;
           if constexpr (sizeof(T) == 4) {
             __stcs(reinterpret_cast<float4 *>(o + e), make_float4(v[0], v[1], v[2], v[3]));
           } else {
@@ -160,7 +162,7 @@ group_fwd_chanrow_kernel(const T *__restrict__ in, const IndexT *__restrict__ in
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const int e = entry(r, k);
-            if (e < left) __stcs(o + e, v[k]);
+            if (e < left && TK3D_IN(o + e - out, (int64_t)gridDim.z * ostride)) __stcs(o + e, v[k]);
           }
         }
       }

@@ -35,7 +35,7 @@ edge_rows_vec4_kernel(const float *__restrict__ keyT, const float *__restrict__ 
   for (int g = warp; g < (n >> 2); g += ROWS_THREADS / 32) {
     int id[1];
     float w[1];
-    rows_load_index<1, int64_t>(index, nullptr, b * E + e0 + 4 * g + el, N2, true, id, w, bad);
+    rows_load_index<1, int64_t>(index, nullptr, b * E + e0 + 4 * g + el, gridDim.y * E, N2, true, id, w, bad);
     const float4 *row = fb + (int64_t)(id[0] < 0 ? 0 : id[0]) * L;
     float *dst = tile + 4 * ql * ROWS_TE + (((g ^ ql) & (ROWS_TE / 4 - 1)) << 2) + el;
     row += ql;
@@ -96,7 +96,7 @@ edge_direct_kernel(const T *__restrict__ key, const T *__restrict__ qfeat, const
   const int64_t ctot = include_query ? 2 * C : C;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < B * E; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = t / E, e = t - b * E, n = e / K;
-    int64_t id = index[t];
+    int64_t id = index[TK3D_AT(t, B * E)];
     if (id < 0 || id >= N2) {
       id = -1;
       if (status) atomicOr(status, 1);
@@ -170,7 +170,7 @@ edge_bwd_key_kernel(const T *__restrict__ gout, const int64_t *__restrict__ inde
     const int64_t e = t % E;
     const int64_t bc = t / E;
     const int64_t b = bc / C, c = bc - b * C;
-    const int64_t id = index[b * E + e];
+    const int64_t id = index[TK3D_AT(b * E + e, B * E)];
     if (id < 0 || id >= N2) {
       if (status) atomicOr(status, 1);
       continue;

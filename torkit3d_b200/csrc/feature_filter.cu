@@ -34,9 +34,9 @@
 //
 // 32 x 1024 x 1024, 64 channels, k = 20: 229 us by all pairs, 89 now: preparing 7, filter 37, exact distances 41, looking
 // for what is left 3; 32 x 2000, 16 channels 388 / 138; 4 x 4096, 64 channels 458 / 117; 32 x 1024, 128 channels, k = 32
-// 384 / 220.  The filter's product is 16 % of it; the rest is reading tensor memory (two loads of 32 columns a thread and
-// tile), the minima and the comparisons.  With one thread per query it took 61 to 77 us.  The exact distances wait for
-// shared memory.
+// 384 / 220.  The tensor pipe is active for 37 % of the filter; the rest is reading tensor memory (two loads of 32 columns a
+// thread and tile), the minima and the comparisons.  With one thread per query it took 61 to 77 us.  The exact distances
+// wait for shared memory.
 #include "feature_filter.cuh"
 
 namespace tk3d {
@@ -146,12 +146,6 @@ ff_prep_kernel(const float *__restrict__ in, const float *__restrict__ key, int 
       s.block_max[b * ((N + FF_PREP - 1) / FF_PREP) + blockIdx.x] = __uint_as_float(top);
   }
 }
-
-#ifdef TK3D_BOUNDS
-#define FF_AT(i, n) ((int)tk3d_checked((i), (n)))
-#else
-#define FF_AT(i, n) (i)
-#endif
 
 __device__ __forceinline__ unsigned ff_smem(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ff_bar_init(unsigned bar) {
@@ -512,7 +506,7 @@ ff_exact_kernel(FfSide qs, FfSide ks, int C, int N1, int N2, int k, const uint16
     const int c = c0 + lane, here = min(32, n - c0);
     int j = 0;
     if (c < n) j = list[c < parts.x ? c : FF_CAP + c - parts.x];
-    const unsigned off = FF_AT(j, N2) * (unsigned)(Cr * 4);
+    const unsigned off = (unsigned)TK3D_AT(j, N2) * (unsigned)(Cr * 4);
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < 8; ++i) {  // four rows a step, eight lanes each

@@ -34,7 +34,7 @@ group_fwd_direct_kernel(const T *__restrict__ in, const IndexT *__restrict__ ind
   bool bad = false;
 #pragma unroll
   for (int v = 0; v < GP_VEC; ++v) {
-    id[v] = v < n ? (int64_t)ip[v] : 0;
+    id[v] = v < n ? (int64_t)ip[TK3D_AT(e0 + v, E) - e0] : 0;
     if (id[v] < 0 || id[v] >= N1) {
       id[v] = -1;
       bad |= v < n;
@@ -85,7 +85,7 @@ group_bwd_kernel(const T *__restrict__ gout, const int64_t *__restrict__ index, 
   bool bad = false;
 #pragma unroll
   for (int v = 0; v < GP_VEC; ++v) {
-    id[v] = v < n ? ip[v] : -1;
+    id[v] = v < n ? ip[TK3D_AT(e0 + v, E) - e0] : -1;
     if (v < n && (id[v] < 0 || id[v] >= N1)) {
       id[v] = -1;
       bad = true;

@@ -29,7 +29,7 @@ interp_fwd_direct_kernel(const T *__restrict__ in, const int64_t *__restrict__ i
   bool bad = false;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    id[i] = index[(b * N2 + m) * 3 + i];
+    id[i] = index[TK3D_AT((b * N2 + m) * 3 + i, gridDim.z * N2 * 3)];
     w[i] = weight[(b * N2 + m) * 3 + i];
     if (id[i] < 0 || id[i] >= N1) {
       id[i] = 0;
@@ -68,7 +68,7 @@ interp_bwd_kernel(const T *__restrict__ gout, const int64_t *__restrict__ index,
   bool bad = false;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    id[i] = index[(b * N2 + m) * 3 + i];
+    id[i] = index[TK3D_AT((b * N2 + m) * 3 + i, gridDim.z * N2 * 3)];
     w[i] = weight[(b * N2 + m) * 3 + i];
     if (id[i] < 0 || id[i] >= N1) {
       id[i] = -1;

@@ -123,7 +123,7 @@ gather_rows_kernel(const float *__restrict__ featT, const IndexT *__restrict__ i
 
   bool bad = false;
   for (int t = tid; t < n * NSRC; t += ROWS_THREADS) {
-    int64_t id = index[(b * E + e0) * NSRC + t];
+    int64_t id = index[TK3D_AT((b * E + e0) * NSRC + t, gridDim.y * E * NSRC)];
     if (id < 0 || id >= N1) {
       id = -1;
       bad = true;
@@ -179,11 +179,11 @@ gather_rows_kernel(const float *__restrict__ featT, const IndexT *__restrict__ i
 // loads, 16-byte streaming stores.
 template <int NSRC, typename IndexT>
 __device__ __forceinline__ void rows_load_index(const IndexT *__restrict__ index, const float *__restrict__ weight,
-                                                int64_t at, int64_t N1, bool live, int (&id)[NSRC], float (&w)[NSRC],
-                                                bool &bad) {
+                                                int64_t at, int64_t count, int64_t N1, bool live, int (&id)[NSRC],
+                                                float (&w)[NSRC], bool &bad) {
 #pragma unroll
   for (int i = 0; i < NSRC; ++i) {
-    int64_t v = live ? (int64_t)index[at * NSRC + i] : 0;  // a group beyond the tile reads nothing
+    int64_t v = live ? (int64_t)index[TK3D_AT(at * NSRC + i, count * NSRC)] : 0;  // a group beyond the tile reads nothing
     w[i] = 1.f;
     if (NSRC > 1) w[i] = live ? weight[at * NSRC + i] : 0.f;
     if (v < 0 || v >= N1) {
@@ -216,7 +216,8 @@ gather_rows_vec4_kernel(const float *__restrict__ featT, const IndexT *__restric
 #pragma unroll
   for (int j = 0; j < ROWS_GPW; ++j) {
     const int g = warp + j * (ROWS_THREADS / 32);
-    rows_load_index<NSRC, IndexT>(index, weight, b * E + e0 + 4 * g + el, N1, g < (n >> 2), ids[j], ws[j], bad);
+    rows_load_index<NSRC, IndexT>(index, weight, b * E + e0 + 4 * g + el, gridDim.y * E, N1, g < (n >> 2), ids[j], ws[j],
+                                  bad);
   }
 #pragma unroll
   for (int j = 0; j < ROWS_GPW; ++j) {
@@ -316,7 +317,8 @@ scatter_rows_vec4_kernel(const float *__restrict__ gout, const IndexT *__restric
 #pragma unroll
   for (int j = 0; j < ROWS_GPW; ++j) {
     const int g = warp + j * (ROWS_THREADS / 32);
-    rows_load_index<NSRC, IndexT>(index, weight, b * E + e0 + 4 * g + el, N1, g < nchunks, ids[j], ws[j], bad);
+    rows_load_index<NSRC, IndexT>(index, weight, b * E + e0 + 4 * g + el, gridDim.y * E, N1, g < nchunks, ids[j], ws[j],
+                                  bad);
   }
   __syncthreads();
 

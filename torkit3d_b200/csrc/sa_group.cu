@@ -187,7 +187,7 @@ sa_group_fwd_kernel(const float *__restrict__ points, const float *__restrict__ 
     __syncthreads();  // the lists' first entries are visible to every warp
     if constexpr (GIVEN) {  // complete lists
       const int32_t *gp = given + b * E + (int64_t)m0 * K;
-      for (int e = tid; e < nv * K; e += THREADS) sidx[(e / K) * S1 + (e % K)] = gp[e];
+      for (int e = tid; e < nv * K; e += THREADS) sidx[(e / K) * S1 + (e % K)] = given[TK3D_AT(gp + e - given, B * E)];
       if (part == 0 && valid && status && gp[(int64_t)lane * K] < 0) atomicOr(status, 1);
     } else if (done < K) {   // short lists repeat their first hit; empty ones (and padding lanes) hold -1
       const int first = valid && done > 0 ? row[0] : -1;
@@ -324,7 +324,7 @@ sa_group_bwd_xyz_kernel(const float *__restrict__ gout, const int32_t *__restric
         gx = g[k];
         gy = g[E + k];
         gz = g[2 * E + k];
-        id = ip[k];
+        id = ip[TK3D_AT(k, K)];
       }
       sx += gx;
       sy += gy;
@@ -486,7 +486,7 @@ sa_group_bwd_feat_kernel(const float *__restrict__ gout, const int32_t *__restri
     const int64_t bc = t / E;
     const int64_t b = bc / C;
     const int c = (int)(bc - b * C);
-    const int id = index32[b * E + e];
+    const int id = index32[TK3D_AT(b * E + e, B * E)];
     if (id < 0 || id >= N) {
       if (status) atomicOr(status, 1);
       continue;

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(SC_NT, 12) scatter_fold_kernel(const ScatterAr
   const int n = (int)min((int64_t)TE, a.E - e0);
   const float *gb = a.gout + b * a.gstride + e0;
   // the index is requested ahead of gout and looked at behind it
-  int64_t id = tid < n ? (int64_t)index[b * a.E + e0 + tid] : -1;
+  int64_t id = tid < n ? (int64_t)index[TK3D_AT(b * a.E + e0 + tid, gridDim.y * a.E)] : -1;
   if (VEC) {
     // a thread's chunk is the same in every row; rows are 16 apart: (c >> 2) & 7 flips its highest bit
     const int c0 = tid >> 3, e = (tid & 7) << 2;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(SC_NT, 12) scatter_fold_kernel(const ScatterAr
   const float *mine = tile + 4 * ql * TE;
   for (int i = warp * 4 + el; i < nruns[0]; i += NW * 4) {
     const int s = runs[0][i] & 255;
-    float *dst = rb + (int64_t)sid[s] * a.ld + 4 * ql;
+    float *dst = rb + TK3D_AT(sid[s], a.N) * (int64_t)a.ld + 4 * ql;
     const float *src = mine + (s ^ (ql << 2));
 #pragma unroll 2
     for (int q = ql; q < L; q += 8, src += 32 * TE, dst += 32) red_add4(dst, src[0], src[TE], src[2 * TE], src[3 * TE]);
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(SC_NT, 12) scatter_fold_kernel(const ScatterAr
   // longer runs, one per warp: every fourth entry per el
   for (int i = warp; i < nruns[1]; i += NW) {
     const int s = runs[1][i] & 255, len = runs[1][i] >> 8;
-    float *dst = rb + (int64_t)sid[s] * a.ld + 4 * ql;
+    float *dst = rb + TK3D_AT(sid[s], a.N) * (int64_t)a.ld + 4 * ql;
     const float *src = mine;
     for (int q0 = 0; q0 < L; q0 += 8, src += 32 * TE, dst += 32) {
       float x = 0.f, y = 0.f, z = 0.f, w = 0.f;
@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a
   const int n = (int)min((int64_t)a.per, a.E - e0);  // a multiple of 4
   const int c0 = blockIdx.z * SE_C, nc = min(SE_C, a.C - c0);  // channels of this block
   const float *gb = a.gout + b * a.gstride + (int64_t)c0 * a.E + e0;
-  const int64_t id0 = tid < n ? (int64_t)index[b * a.E + e0 + tid] : -1;  // requested ahead of gout
+  // requested ahead of gout
+  const int64_t id0 = tid < n ? (int64_t)index[TK3D_AT(b * a.E + e0 + tid, gridDim.y * a.E)] : -1;
   {
     const int e = lane << 2;
     const float *src = gb + (int64_t)warp * a.E + e;
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a
     const int id = sid[s];
     if (id < 0) continue;
     const float *src = tile + 4 * ql * SE_TE + (s ^ (ql << 2));
-    if (ql < L) red_add4(rb + (int64_t)id * a.ld, src[0], src[SE_TE], src[2 * SE_TE], src[3 * SE_TE]);
+    if (ql < L) red_add4(rb + TK3D_AT(id, a.N) * (int64_t)a.ld, src[0], src[SE_TE], src[2 * SE_TE], src[3 * SE_TE]);
   }
   // gq[b,c,m] = sum_k (g[C+c] - g[c]), or minus the sum of the only half
   const int K = a.K, nq = n / K;
@@ -221,7 +222,8 @@ __global__ void __launch_bounds__(SE_NT) scatter_edge_kernel(const ScatterArgs a
         sum += a.include_query ? second[at] - tile[at] : -tile[at];
       }
     }
-    a.gq[(b * a.C + c0 + c) * (int64_t)a.M + m0 + m] = sum;
+    const int64_t at = (b * a.C + c0 + c) * (int64_t)a.M + m0 + m;
+    if (TK3D_IN(at, (int64_t)gridDim.y * a.C * a.M)) a.gq[at] = sum;
   }
 }
 
@@ -255,7 +257,8 @@ unrow_kernel(const float *__restrict__ rows, int ld, int C, int N, float *__rest
   const int nc = min(64, C - c0), nl = tid & 63;
   if (n0 + nl < N)
     for (int cl = tid >> 6; cl < nc; cl += 4)
-      dst[(int64_t)cl * N + nl] = t[cl * 64 + ((((nl >> 2) ^ (cl >> 2)) & 15) << 2) + (nl & 3)];
+      if (TK3D_IN(dst + (int64_t)cl * N + nl - gin, (int64_t)gridDim.z * C * N))
+        dst[(int64_t)cl * N + nl] = t[cl * 64 + ((((nl >> 2) ^ (cl >> 2)) & 15) << 2) + (nl & 3)];
 }
 
 template <typename IndexT>

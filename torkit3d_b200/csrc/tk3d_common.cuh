@@ -98,6 +98,10 @@ __device__ __forceinline__ int64_t tk3d_checked(int64_t i, int64_t n) {
   }
   return i;
 }
+// TK3D_AT: an index, element 0 where it is out of range; TK3D_IN: whether it is in range, for stores that are left out.
+#define TK3D_AT(i, n) tk3d_checked((i), (n))
+__device__ __forceinline__ bool tk3d_in(int64_t i, int64_t n) { return tk3d_checked(i, n) == i && n > 0; }
+#define TK3D_IN(i, n) tk3d_in((i), (n))
 #define TK3D_BOUNDS_TU(tag)                                                   \
   extern "C" unsigned long long tk3d_bounds_count_##tag(void) {               \
     unsigned long long v = 0;                                                 \
@@ -105,6 +109,8 @@ __device__ __forceinline__ int64_t tk3d_checked(int64_t i, int64_t n) {
     return v;                                                                 \
   }
 #else
+#define TK3D_AT(i, n) (i)
+#define TK3D_IN(i, n) true
 #define TK3D_BOUNDS_TU(tag)
 #endif
 
