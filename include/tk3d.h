@@ -479,6 +479,12 @@ int tk3d_diag_fps_wait_limit(const void *points, int64_t B, int64_t N, int64_t n
  * roofline of the distance kernels.  `sink` is a device float that is never actually written.
  */
 int tk3d_diag_ffma(int64_t iters, float *sink, double *flop, void *stream);
+/*
+ * tk3d_diag_feature_filter() says where in its scratch tk3d_feature_knn_ws leaves what the filter found, for tests: byte
+ * offsets of the candidates [B][N1][2][64] uint16, of their numbers [B][N1][2] int32 (above 64: none) and of the queries'
+ * counts [B][N1] int32 (negative: left to the kernel for all pairs).  same: query and key are one tensor.
+ */
+int tk3d_diag_feature_filter(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t k, int same, size_t offset[3]);
 
 /*
  * Diagnostic with no counterpart in the reference: the name of the kernel that tk3d_chamfer_fwd, the sweep

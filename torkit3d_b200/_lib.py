@@ -74,6 +74,7 @@ SIGNATURES = {
     "tk3d_fps_expired_waits": (ctypes.c_longlong, []),
     "tk3d_diag_fps_wait_limit": (_int, [_vp, _i64, _i64, _i64, _vp, _i64, _i64, _vp]),
     "tk3d_diag_ffma": (_int, [_i64, _vp, ctypes.POINTER(ctypes.c_double), _vp]),
+    "tk3d_diag_feature_filter": (_int, [_i64, _i64, _i64, _i64, _i64, _int, ctypes.POINTER(ctypes.c_size_t)]),
     "tk3d_feature_knn": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _i64, _int, _vp, _vp, _int, _vp]),
     "tk3d_feature_knn_scratch_bytes": (ctypes.c_size_t, [_i64, _i64, _i64, _i64, _i64, _int]),
     "tk3d_feature_knn_ws": (_int, [_vp, _vp, _i64, _i64, _i64, _i64, _i64, _int, _vp, _vp, _vp, ctypes.c_size_t, _int,

@@ -643,4 +643,18 @@ int ff_knn(const float *query, const float *key, int64_t B, int C, int N1, int N
 
 }  // namespace tk3d
 
+using namespace tk3d;
+
+extern "C" int tk3d_diag_feature_filter(int64_t B, int64_t C, int64_t N1, int64_t N2, int64_t k, int same,
+                                        size_t offset[3]) {
+  TK3D_REQUIRE(offset != nullptr, TK3D_ERR_NULL, "diag_feature_filter: offset is NULL");
+  TK3D_REQUIRE(ff_scratch_bytes(B, C, N1, N2, k) != 0, TK3D_ERR_SHAPE, "diag_feature_filter: sizes that are not served");
+  char *const base = reinterpret_cast<char *>(256);
+  const FfLayout l = ff_layout(B, (int)C, (int)N1, (int)N2, same != 0 && N1 == N2, base);
+  offset[0] = (size_t)(reinterpret_cast<char *>(l.lists) - base);
+  offset[1] = (size_t)(reinterpret_cast<char *>(l.found) - base);
+  offset[2] = (size_t)(reinterpret_cast<char *>(l.counts) - base);
+  return TK3D_OK;
+}
+
 TK3D_BOUNDS_TU(feature_filter)
