@@ -6,7 +6,8 @@ Cases: c1_chamfer, c2_knn, c3_fps, c3_ball, c3_group_fwd, c3_group_bwd, c4_chamf
 c4_chamfer_bwd, c5_three_nn, c5_three_nn_slab8, c5_interp_fwd, c5_interp_fwd_rows, c5_feature_rows, c5_interp_bwd, and the layer front ends on the same
 inputs in channel-first layout, fused and spelled operator by operator: c3_fps_gather,
 c3_fps_chain, c3_sa_fused, c3_sa_chain, c3_sa_fused_bwd, c5_fp_fused, c5_fp_chain; and the EdgeConv edge
-features of a DGCNN layer (B=32, 1024 points, C=64, K=20): edge_fused, edge_chain; and its feature-space
+features of a DGCNN layer (B=32, 1024 points, C=64, K=20): edge_fused, edge_chain, edge_fused_bwd;
+and its feature-space
 KNN: feature_knn, feature_knn_chain (cdist + topk in PyTorch); knn_f64 (float64 KNN, 8 x 2048 x 2048, k=16); knn_k200 (float32, 4 x 4096 x 4096, k=200); fps_large (4 clouds of 65536 points -> 2048 samples).  ``--scale-batch`` overrides the batch
 size of the configuration (smaller captures for ``ncu``).  Prints the mean CUDA-event time.
 """
@@ -70,6 +71,11 @@ def build_case(name, batch, dev):
         _, ind = knn_points(pts, pts, 20)
         if name == "edge_fused":
             return lambda: get_edge_feature(x, x, ind)
+        if name == "edge_fused_bwd":
+            from torkit3d_b200 import _fused
+
+            go = torch.randn(B, 128, 1024, 20, generator=g).to(dev)
+            return lambda: _fused.edge_feature_backward(go, ind, 64, 1024)
 
         def edge_chain():
             grouped = group_points(x, ind)

@@ -2,9 +2,9 @@
 
     python -m torkit3d_b200.build [--force] [--verbose] [--bounds]
 
-``--bounds`` builds libtk3d_b200_bounds.so instead: the same sources with -DTK3D_BOUNDS, in which every
-coordinate load and index-tensor access is range checked and violations are counted
-(tk3d_bounds_violations()).  The tests run a set of shapes through it; it is not what the operators load.
+``--bounds`` builds libtk3d_b200_bounds.so instead: the same sources with -DTK3D_BOUNDS, in which the
+searches' coordinate loads, index-tensor accesses and the rows that gathers and gradients address are range
+checked and violations are counted (tk3d_bounds_violations()).  The tests run a set of shapes through it; it is not what the operators load.
 
 The library has no dependency on torch or Python headers (plain CUDA runtime), so a full rebuild
 takes seconds.  Objects are cached under ``torkit3d_b200/csrc/build/`` by source mtime.
